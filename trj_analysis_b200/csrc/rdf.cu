@@ -13,17 +13,12 @@
 // the counts equal the all-pairs sweep exactly.  Axes with fewer than 3 cells are not split
 // (one cell along that axis); a frame with no split axis is the all-pairs case.
 //
-// Within a cell, atoms are ordered along a Morton curve over S^3 sub-cells, so the 64 home atoms of
-// a warp (two per lane, consecutive in that order) fill a small box.  Each warp tests 32 staged
-// neighbour atoms at a time against that box grown by the cutoff (one ballot) and runs the exact
-// pair test only for the neighbours that can be in range: a conservative cull, the counts are
-// those of the full stencil.
-//
-// Neighbour-cell atoms are staged into shared memory with 1-D TMA bulk copies
-// (cp.async.bulk, no multicast) into two slots, each on its own mbarrier.  Warps walk the task
-// sequence independently: the last warp to release a slot refills it with the next task, so there
-// is no CTA barrier per task.  Warps count into uint32 shared histogram replicas (warp w uses
-// replica w mod nrep); replicas are merged with 64-bit global atomics at exit.
+// Each cell is divided into boxes of about 28 atoms ("groups"), and the atoms are sorted by
+// (cell, group).  A warp takes the up to 32 atoms of one group as homes, one per lane, and walks the
+// groups of the neighbour cells: groups, then single atoms, farther from the homes' bounding box than
+// the cutoff are skipped (conservatively: the counts are those of the full stencil), and the survivors
+// are compacted into a buffer of the warp in shared memory, from which the exact pair test runs with
+// every lane busy, two neighbours per packed FP32 instruction.
 #include <curand_kernel.h>
 #include <math.h>
 
@@ -35,48 +30,83 @@
 
 namespace {
 
-constexpr int kThreads = 256;       // threads per CTA
-constexpr int kHomeChunk = 2 * kThreads;  // two home atoms per thread: a warp holds 64 consecutive atoms
-constexpr int kJChunk = 512;        // neighbour atoms per staged buffer (8 KB)
-constexpr int kSlots = 2;           // staged buffers (tasks in flight per CTA)
+constexpr int kGroup = 32;            // home atoms of a round, one per lane
+constexpr double kGroupFill = 28.0;   // average atoms per group aimed at: few groups then exceed 32
+constexpr int kRing = 128;            // surviving neighbours buffered per warp (arrays x, y, z, w)
+constexpr int kRingRun = 64;          // survivors tested per run
+constexpr int kMaxWarps = 32;         // per SM: 64 registers a thread (24 warps of 80 registers: 4 % slower at 1e6 atoms)
 constexpr int kMaxOffsets = 14;
 
-struct RdfParams {
+typedef unsigned long long u64;
+
+// Frame flags raised by cell_assign_kernel: how far coordinates reach outside [0, L).  They decide
+// whether |d| < 3L/2 holds for every pair of the frame (see frame_within).
+enum : unsigned { kFrameLow = 1u, kFrameVeryLow = 2u, kFrameHigh = 4u };
+
+// What one pair's test and bin need.
+struct PairGeom {
     float L[3];
+    float inv_L[3];
     float h1[3], h2[3];         // |dx| < h1: nint(dx/L) = 0; h1 <= |dx| < h2: +-1; else the division
     float side2, side2_lo, side2_hi;
+    float side2_win;            // side2_hi - side2, the larger half of that window
     float deltar, inv_deltar;
-    int lsmax, nsp, nit;
+    float edge_thr;             // distance of q from the nearest integer above which a bin edge may be near
+    int lsmax, nsp;
     int floor_bins;             // 0: bin nint(r/deltar) (reference); 1: bin floor(r/deltar)+1
-    int nc[3];
-    int ncell;
-    int noff;
-    int hsplit, jsplit;
-    int nrep;
-    int fast_ok;                // every axis split into >= 5 cells
-    float cull2;                // (cutoff * (1 + 2^-10))^2: neighbours farther from a warp's box are skipped
-    float cull_pad;             // added to the box half-widths: covers the FP32 rounding of the cull test
-    int sbits;                  // sub-cells per cell axis: 2^sbits (Morton order inside a cell)
-    long long wait_clocks;      // limit of a warp's wait for a staged neighbour chunk
-    int stall_test;             // 1: each warp's first wait is on a barrier nothing arrives on (timeout test)
-    int off[kMaxOffsets][3];
-    int64_t nitems;
+    int row_words;              // words of a shared histogram row: lsmax + 2 (first and last: not counted)
+    int want_edge;              // edge statistics are collected
+    float one;                  // 1.0f, from the host: not a constant the assembler could fold
 };
 
-struct TaskInfo {
-    int sa, na;        // home cell start/count in the sorted array
-    int sb;            // first staged neighbour atom (global index into sorted)
-    int jcount;        // staged atoms
-    int jlocal0;       // index within the neighbour cell of the first staged atom
-    int hc;            // home chunk
-    int self;          // home cell == neighbour cell
-    int fast;          // no minimum image needed for any pair of the task
-    int cull;          // both cells hold only coordinates in [-L, L): the box cull applies (wrapped values)
-    float img[3];      // periodic image of the neighbour cell: 0 or -+L per axis
-    int valid;         // 0 = no more tasks
-    int oct;           // 1: warp w's homes are octant w of the home cell (ostart[w] .. ostart[w + 1])
-    short ostart[9];   // octant starts within the home cell (oct = 1)
+struct RdfParams {
+    PairGeom g;
+    int nit;
+    int nc[3];                  // cells per axis (1: the axis is not split)
+    int sub[3], nsub;           // groups per cell: sub[0] x sub[1] x sub[2] boxes, z fastest
+    float inv_sub[3];           // 1 / sub
+    float edge[3];              // cell edge
+    float half[3];              // half edge of a group's box, with the cull pad
+    int noff;
+    int nseg, per_seg;          // segments of a home group's neighbour list (one work item each); their length
+    int split_all;              // every axis of the geometry is split (in two dimensions: x and y)
+    float cull2;                // (cutoff * (1 + 2^-10))^2: neighbours farther from the homes' box are skipped
+    float cull_pad;             // added to half-widths: covers the FP32 rounding of the cull test
+    long long wait_clocks;      // limit of the stall test's wait
+    int stall_test;             // 1: every warp waits on a barrier nothing arrives on (timeout test)
+    int off[kMaxOffsets][3];
+    unsigned nitems;
 };
+
+// ---- packed FP32 (two independent IEEE operations per instruction, each rounded to nearest once) ----
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ u64 pack2(float lo, float hi) {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ float fast_sqrt(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 
 __device__ __forceinline__ float min_image_exact(float d, float L) {
     float n = roundf(__fdiv_rn(d, L));
@@ -103,115 +133,20 @@ __device__ __forceinline__ int outcome(float rr2, float side2, float deltar, int
     return (ind <= lsmax && ind > 0) ? ind : 0;
 }
 
-// Task iterator, run by one thread at a time (the thread that refills a slot): items are taken from
-// a global counter (dynamic balance); item = (cell, offset, home round, neighbour segment);
-// tasks = (home round of up to 512 atoms, neighbour chunk of up to 512 atoms).
-struct TaskGen {
-    int64_t w;
-    int hc, jc;
-    int started;
-};
-
 __device__ __forceinline__ int wrapc(int c, int n) { return c < 0 ? c + n : (c >= n ? c - n : c); }
 
-// Octant starts of cell c (atoms sa .. sa + na of the sorted array) from the sub-cell starts; returns 1
-// when no octant holds more than 64 atoms.  Not inlined: it runs on the refill path only, and its
-// loads would otherwise add to the register pressure of the pair loop.
-__device__ __noinline__ int octant_starts(const int32_t* __restrict__ fstart, int c, int sa, int na, int sbits,
-                                          short* ostart) {
-    const int64_t kb = (int64_t)c << (3 * sbits);
-    const int step = 1 << (3 * (sbits - 1));
-    int mx = 0, prev = 0;
-    ostart[0] = 0;
-    for (int o = 1; o <= 8; ++o) {
-        const int v = o < 8 ? fstart[kb + o * step] - sa : na;
-        ostart[o] = (short)v;
-        mx = max(mx, v - prev);
-        prev = v;
-    }
-    return mx <= 64;
-}
-
-__device__ bool next_task(TaskGen& g, const RdfParams& p, const int32_t* __restrict__ cstart,
-                          const int32_t* __restrict__ ccount, const int32_t* __restrict__ cflag,
-                          const int32_t* __restrict__ fstart, unsigned long long* work, TaskInfo& t) {
-    for (;;) {
-        if (!g.started) {
-            g.started = 1;
-            g.w = (int64_t)atomicAdd(work, 1ull);
-            g.hc = -1;
-            g.jc = 0;
-        }
-        if (g.w >= p.nitems) {
-            t.valid = 0;
-            return false;
-        }
-        int64_t w = g.w;
-        const int seg = (int)(w % p.jsplit);
-        w /= p.jsplit;
-        const int h = (int)(w % p.hsplit);
-        w /= p.hsplit;
-        const int o = (int)(w % p.noff);
-        const int c = (int)(w / p.noff);
-        const int cz = c % p.nc[2];
-        const int cy = (c / p.nc[2]) % p.nc[1];
-        const int cx = c / (p.nc[2] * p.nc[1]);
-        const int ex = cx + p.off[o][0], ey = cy + p.off[o][1], ez = cz + p.off[o][2];
-        const int c2 = (wrapc(ex, p.nc[0]) * p.nc[1] + wrapc(ey, p.nc[1])) * p.nc[2] + wrapc(ez, p.nc[2]);
-        const int na = ccount[c], nb = ccount[c2];
-        const int self = (o == 0);
-        if (g.hc < 0) {
-            g.hc = h;
-            g.jc = 0;
-        }
-        while (true) {
-            if (g.hc * kHomeChunk >= na) break;  // item done
-            const int jfirst = self ? g.hc * kHomeChunk : 0;
-            const int jtot = nb - jfirst;
-            const int s0 = jfirst + (int)((int64_t)jtot * seg / p.jsplit);
-            const int s1 = jfirst + (int)((int64_t)jtot * (seg + 1) / p.jsplit);
-            const int jstart = s0 + g.jc * kJChunk;
-            if (jtot <= 0 || jstart >= s1) {
-                g.hc += p.hsplit;
-                g.jc = 0;
-                continue;
-            }
-            const bool wraps = ex < 0 || ex >= p.nc[0] || ey < 0 || ey >= p.nc[1] || ez < 0 || ez >= p.nc[2];
-            t.sa = cstart[c];
-            t.na = na;
-            t.sb = cstart[c2] + jstart;
-            t.jcount = min(kJChunk, s1 - jstart);
-            t.jlocal0 = jstart;
-            t.hc = g.hc;
-            t.self = self;
-            t.fast = p.fast_ok && !wraps && !cflag[c] && !cflag[c2];
-            t.cull = !((cflag[c] | cflag[c2]) & 2);
-            t.img[0] = ex < 0 ? -p.L[0] : (ex >= p.nc[0] ? p.L[0] : 0.f);
-            t.img[1] = ey < 0 ? -p.L[1] : (ey >= p.nc[1] ? p.L[1] : 0.f);
-            t.img[2] = ez < 0 ? -p.L[2] : (ez >= p.nc[2] ? p.L[2] : 0.f);
-            t.valid = 1;
-            // Octant homes: a cell of one home round whose eight Morton octants (sub-cell keys
-            // o * 8^(sbits-1) ..) each hold at most 64 atoms gives warp w octant w, a box of half the
-            // cell edge, instead of 64 consecutive atoms that may span two octants.
-            t.oct = (p.sbits >= 1 && na <= kHomeChunk) ? octant_starts(fstart, c, t.sa, na, p.sbits, t.ostart) : 0;
-            g.jc += 1;
-            return true;
-        }
-        g.w = (int64_t)atomicAdd(work, 1ull);
-        g.hc = -1;
-    }
-}
-
 struct PairCounters {
-    unsigned long long ulp = 0, fma = 0, counted = 0;
+    unsigned ulp = 0, fma = 0;
+    u64 counted = 0;
 };
 
-// Exact reference outcome of a pair near a bin edge or the cutoff, with its edge statistics:
+// Exact reference outcome of a pair near a bin edge or the cutoff, with its edge statistics when wanted:
 // returns the bin | 2^29 if a one-ulp change of rr2 changes it | 2^30 if the FMA-contracted rr2
 // does.  Scalars by value: nothing of the caller's needs an address (no local-memory copies).
 __device__ __noinline__ int exact_bin(float rr2, float x2, float dy, float dz, float side2, float deltar, int lsmax,
-                                      int floor_bins) {
+                                      int floor_bins, int want_edge = 1) {
     const int ind = outcome(rr2, side2, deltar, lsmax, floor_bins);
+    if (!want_edge) return ind;
     const int olo = outcome(nextafterf(rr2, -INFINITY), side2, deltar, lsmax, floor_bins);
     const int ohi = outcome(nextafterf(rr2, INFINITY), side2, deltar, lsmax, floor_bins);
     const float rr2f = fmaf(dz, dz, fmaf(dy, dy, x2));
@@ -219,77 +154,209 @@ __device__ __noinline__ int exact_bin(float rr2, float x2, float dy, float dz, f
     return ind | ((olo != ind || ohi != ind) ? (1 << 29) : 0) | (fma ? (1 << 30) : 0);
 }
 
-// QMODE: also adds the charge product q_a*q_b of every counted pair to the bin (FP64; the product
-// of two FP32 charges is exact in FP64).  rdf.cuf:469-472.
-// FLOOR: bins floor(r/deltar)+1 (rdfxy) instead of nint(r/deltar).
-template <bool FLOOR, bool QMODE>
-__device__ __forceinline__ void bin_pair(float rr2, float x2, float dy, float dz, int row, const RdfParams& p,
-                                         unsigned* myhist, PairCounters& pc, double* myq, float qa,
-                                         const float* qbp) {
-    const float q = rr2 * rsqrtf(rr2) * p.inv_deltar;
-    // Nearest integer of q by adding and removing 1.5*2^23 (q < 2^22): qb holds it in its low
-    // mantissa bits; d = q - r in [-1/2, 1/2] exactly.
-    const float qb = __fadd_rn(q, 12582912.0f);
-    const float d = __fsub_rn(q, __fsub_rn(qb, 12582912.0f));
-    const float win = fmaf(q, 1.9073486e-6f, 9.5367432e-7f);  // q*2^-19 + 2^-20
-    // distance of q from the nearest bin edge: integers (floor bins) or half-integers (nint bins)
-    const float edge = FLOOR ? fabsf(d) : 0.5f - fabsf(d);
-    int ind;
-    if (rr2 >= p.side2_lo || !(edge > win)) {  // NaN (rr2 == 0) takes this path too
-        const int e = exact_bin(rr2, x2, dy, dz, p.side2, p.deltar, p.lsmax, p.floor_bins);
-        pc.ulp += (e >> 29) & 1;
-        pc.fma += (e >> 30) & 1;
-        ind = e & ((1 << 29) - 1);
-    } else {
-        // Away from an edge, round-to-nearest-even and NINT agree, and floor(q) = r - (d < 0).
-        const int r = __float_as_int(qb) - 0x4B400000;
-        ind = FLOOR ? r + (d > 0.f ? 1 : 0) : r;
-        if (ind > p.lsmax) ind = 0;
+// How the minimum image of a pair is formed.  All forms give the reference's d - L*nint(fl(d/L)) for
+// every pair that can be in range, up to its sign, which drops out in the squares.
+//   kImgNone   d: both cells hold only coordinates in [0, L), every axis is split (>= 3 cells of edge >=
+//              cutoff) and the task does not wrap: a pair with another image is beyond the cutoff in
+//              either one (its |d| here is >= L/2 >= 1.5 cutoffs, its true image >= one cell edge).
+//   kImgShift  the same on tasks that wrap: nint = -+1 on the wrapped axes, d + img with img = +-L or 0
+//              (adding 0 leaves d as it is).
+//   kImgRound  d - L*n with n = d/L rounded by the 1.5*2^23 trick: every axis split, coordinates in [-L, L)
+//              (|n| <= 2, so L*n is exact).  A pair in range has |d - L*n| <= L/3, far from where the
+//              approximate quotient could round to another integer; a pair near there is >= L/2 away.
+//   kImgFold   min(|d|, ||d| - L|) per axis, for frames in which |d| < 3L/2 (frame_within): below L/2 it
+//              is |d| (the rounded L - |d| is >= L/2), from L/2 on |d| - L is exact (Sterbenz) and the
+//              smaller one; h1 is L/2 itself, so this is the reference's choice, ties included.
+//   kImgAny    the thresholds h1, h2 and the division beyond them.
+enum { kImgNone = 0, kImgShift = 1, kImgRound = 2, kImgFold = 3, kImgAny = 4 };
+
+// Constants of one axis: img (kImgShift), or 1/L (kImgRound).
+template <int MODE>
+__device__ __forceinline__ float image_1(float b, float na, float cst, float L, float h1, float h2) {
+    const float d = __fadd_rn(b, na);
+    if (MODE == kImgShift) return __fadd_rn(d, cst);
+    if (MODE == kImgRound) return __fmaf_rn(__fsub_rn(__fmaf_rn(d, cst, 12582912.0f), 12582912.0f), -L, d);
+    if (MODE == kImgFold) {
+        const float a = fabsf(d);
+        return fminf(a, fabsf(__fsub_rn(a, L)));
     }
-    if (ind > 0) {
-        atomicAdd(&myhist[row * p.lsmax + ind - 1], 1u);
-        if (QMODE) atomicAdd(&myq[ind - 1], (double)qa * (double)__ldg(qbp));
-    }
+    if (MODE == kImgAny) return min_image(d, L, h1, h2);
+    return d;
 }
 
-template <bool FAST, bool FLOOR, bool QMODE>
-__device__ __forceinline__ void pair(const float4& a, const float4& b, bool valid, int si, const RdfParams& p,
-                                     const int* rowtab, unsigned* myhist, PairCounters& pc, double* myq,
-                                     float qa, const float* qbp) {
-    float dx = __fsub_rn(b.x, a.x);
-    float dy = __fsub_rn(b.y, a.y);
-    float dz = __fsub_rn(b.z, a.z);
-    if (!FAST) {
-        dx = min_image(dx, p.L[0], p.h1[0], p.h2[0]);
-        dy = min_image(dy, p.L[1], p.h1[1], p.h2[1]);
-        dz = min_image(dz, p.L[2], p.h1[2], p.h2[2]);
+template <int MODE>
+__device__ __forceinline__ u64 image_2(u64 b, u64 na, u64 cst, float L, float h1, float h2) {
+    u64 d = add2(b, na);
+    if (MODE == kImgShift) return add2(d, cst);
+    if (MODE == kImgRound) {
+        const u64 magic = pack2(12582912.0f, 12582912.0f), nmagic = pack2(-12582912.0f, -12582912.0f);
+        return fma2(add2(fma2(d, cst, magic), nmagic), pack2(-L, -L), d);
     }
-    const float x2 = __fmul_rn(dx, dx);
-    const float rr2 = __fadd_rn(__fadd_rn(x2, __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-    if (valid && rr2 < p.side2_hi) {
-        const int sj = __float_as_int(b.w);
-        if ((unsigned)sj < (unsigned)p.nsp)
-            bin_pair<FLOOR, QMODE>(rr2, x2, dy, dz, rowtab[si * p.nsp + sj], p, myhist, pc, myq, qa, qbp);
+    if (MODE == kImgFold || MODE == kImgAny) {
+        float lo, hi;
+        unpack2(d, lo, hi);
+        if (MODE == kImgFold) {
+            lo = fabsf(lo);
+            hi = fabsf(hi);
+            lo = fminf(lo, fabsf(__fsub_rn(lo, L)));
+            hi = fminf(hi, fabsf(__fsub_rn(hi, L)));
+        } else {
+            lo = min_image(lo, L, h1, h2);
+            hi = min_image(hi, L, h1, h2);
+        }
+        d = pack2(lo, hi);
     }
+    return d;
 }
 
-// Box of the warp's home atoms, centred on the neighbour cell's periodic image: a neighbour b can be
-// within the cutoff of some home atom only if |b - c| - h, clipped at 0 per axis, has squared length
-// <= cull2.  Unsplit axes (one cell) get an infinite half-width: no cull along them.
-struct WarpBox {
-    float4 c, h;  // centre (x, y, z) and half-widths (x, y, z); .w unused
+__device__ __forceinline__ float max3_abs(float a, float b, float c) { return fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c)); }
+
+// Low bits of 1.5*2^23: an FP32 sum of it and q < 2^22 holds kBinBias + nint(q) as an integer.
+constexpr unsigned kBinBias = 0x4B400000u;
+
+// A lane's home atom against the survivors in its warp's buffer.
+struct Home {
+    float nx, ny, nz;   // negated coordinates
+    unsigned hist;      // square layout: shared-memory address of its species' first row of bins, minus 4 *
+                        // kBinBias; triangular layout: address of its species' entry in the row table
+    float q;            // charge
 };
 
-__device__ __forceinline__ void axis_box(float v0, bool has0, float v1, bool has1, bool split, float img, float pad,
-                                         float& c, float& h) {
-    // Wrapped coordinates of cull tasks lie in [0, L]: their bit patterns order like the values (+0 for -0).
-    const unsigned b0 = __float_as_uint(v0 + 0.0f), b1 = __float_as_uint(v1 + 0.0f);
-    const unsigned lo = min(has0 ? b0 : 0x7f800000u, has1 ? b1 : 0x7f800000u);
-    const unsigned hi = max(has0 ? b0 : 0u, has1 ? b1 : 0u);
-    const float mn = __uint_as_float(__reduce_min_sync(0xffffffffu, lo));
-    const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, hi));
-    c = 0.5f * (mn + mx) - img;
-    h = split ? 0.5f * (mx - mn) + pad : INFINITY;
+// Tests `n4` blocks of four survivors from ring position `head` (SELF: the round's own atoms in lane order
+// from position 0, pairs j > i).  w of a survivor: bytes to add to Home::hist (square layout: species * row
+// bytes; triangular layout: species * 64, a row of the 16 x 16 table).
+//
+// Per survivor and home: the reference's rr2 with every operation rounded once (two survivors per packed
+// instruction), then the bin from an approximate root.  q = r/deltar is off by less than 0.32 q 2^-20
+// (sqrt.approx 2^-23, 1/deltar 2^-24, the reference's own root and quotient 2^-24 each), and less than
+// 0.47 q 2^-20 after a change of rr2 by one ulp (2^-24) or to its FMA-contracted value (1.25*2^-23); so a
+// pair whose q is farther than edge_thr allows from any bin edge has the reference's bin, and no edge
+// statistic.  rr2 < side2 is exact.  FLOOR: floor(q) + 1 = the integer nearest to q + 1/2.
+// Every pair in range is counted at once in its approximate bin; a block in which some test lies in the
+// window of an edge (or, with EDGE, within 2^-20 of the cutoff, where one-ulp changes decide) is looked at
+// again and the few wrong counts are moved.  QMODE instead leaves those out of the first count, since a
+// charge product cannot be taken back exactly.
+template <int MODE, bool SELF, bool FLOOR, bool QMODE, bool SQUARE, bool EDGE>
+__device__ __forceinline__ void test_run(const float* __restrict__ ring, const double* __restrict__ ring_q, int head,
+                                         int n4, const Home& h, bool has, float ix, float iy, float iz,
+                                         const PairGeom& g, PairCounters& pc, double* myq) {
+    const float cx = MODE == kImgRound ? g.inv_L[0] : ix, cy = MODE == kImgRound ? g.inv_L[1] : iy,
+                cz = MODE == kImgRound ? g.inv_L[2] : iz;
+    const u64 nx = pack2(h.nx, h.nx), ny = pack2(h.ny, h.ny), nz = pack2(h.nz, h.nz);
+    const u64 jx = pack2(cx, cx), jy = pack2(cy, cy), jz = pack2(cz, cz);
+    const u64 inv = pack2(g.inv_deltar, g.inv_deltar);
+    const u64 magic = pack2(12582912.0f, 12582912.0f);  // 1.5*2^23: its sum with q holds nint(q) in the low bits
+    const u64 one = pack2(g.one, g.one);
+    const u64 neg1 = pack2(-1.0f, -1.0f), half = pack2(0.5f, 0.5f);
+    const float thr = g.edge_thr;
+    const float lo = has ? (QMODE ? g.side2_lo : g.side2) : 0.0f, hi = has ? g.side2_hi : 0.0f;
+    const int lane = (int)(threadIdx.x & 31u);
+#pragma unroll 1
+    for (int k = 0; k < n4; ++k) {
+        const int e = (head + 4 * k) & (kRing - 1);
+        const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(ring + e);
+        const ulonglong2 Y = *reinterpret_cast<const ulonglong2*>(ring + kRing + e);
+        const ulonglong2 Z = *reinterpret_cast<const ulonglong2*>(ring + 2 * kRing + e);
+        const uint4 W = *reinterpret_cast<const uint4*>(ring + 3 * kRing + e);
+        float r[4];
+        unsigned bits[4];
+        float d[4];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const u64 dx = image_2<MODE>(p ? X.y : X.x, nx, jx, g.L[0], g.h1[0], g.h2[0]);
+            const u64 dy = image_2<MODE>(p ? Y.y : Y.x, ny, jy, g.L[1], g.h1[1], g.h2[1]);
+            const u64 dz = image_2<MODE>(p ? Z.y : Z.x, nz, jz, g.L[2], g.h1[2], g.h2[2]);
+            // the two sums as a*1 + b: the assembler contracts a packed product and sum into an fma
+            const u64 rr = fma2(fma2(mul2(dx, dx), one, mul2(dy, dy)), one, mul2(dz, dz));
+            unpack2(rr, r[2 * p], r[2 * p + 1]);
+            const u64 s = pack2(fast_sqrt(r[2 * p]), fast_sqrt(r[2 * p + 1]));
+            u64 t, dd;
+            if (FLOOR) {
+                const u64 q = fma2(s, inv, half);
+                t = add2(q, magic);
+                dd = add2(q, fma2(t, neg1, magic));
+            } else {
+                t = fma2(s, inv, magic);
+                dd = fma2(s, inv, fma2(t, neg1, magic));
+            }
+            unpack2(dd, d[2 * p], d[2 * p + 1]);
+            bits[2 * p] = (unsigned)t;
+            bits[2 * p + 1] = (unsigned)(t >> 32);
+        }
+        const unsigned w[4] = {W.x, W.y, W.z, W.w};
+        auto row_of = [&](unsigned wt) {
+            unsigned row = h.hist + wt;
+            if (!SQUARE) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(row) : "r"(row));
+            return row;
+        };
+        bool again;
+        if constexpr (QMODE) {
+            again = false;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const bool in = (!SELF || 4 * k + t > lane) && r[t] < hi;
+                const bool fast = in && r[t] < lo && fabsf(d[t]) <= thr;
+                if (fast) {
+                    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(row_of(w[t]) + (bits[t] << 2)) : "memory");
+                    atomicAdd(&myq[bits[t] - kBinBias], (double)h.q * ring_q[e + t]);
+                }
+                again = again || (in && !fast);
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                // predicated, not branched over: a branch per test costs more than the idle lanes
+                const float top = (SELF && 4 * k + t <= lane) ? 0.0f : lo;
+                asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %0, %1;\n\t@p red.shared.add.u32 [%2], 1;\n\t}" ::"f"(r[t]),
+                             "f"(top), "r"(row_of(w[t]) + (bits[t] << 2))
+                             : "memory");
+            }
+            again = fmaxf(max3_abs(d[0], d[1], d[2]), fabsf(d[3])) > thr;
+            if (EDGE) {
+                const u64 m = pack2(-g.side2, -g.side2);
+                float z[4];
+                unpack2(add2(pack2(r[0], r[1]), m), z[0], z[1]);
+                unpack2(add2(pack2(r[2], r[3]), m), z[2], z[3]);
+                const float zm = fminf(fminf(fabsf(z[0]), fabsf(z[1])), fminf(fabsf(z[2]), fabsf(z[3])));
+                again = again || zm <= g.side2_win;
+            }
+        }
+        if (again) {
+            const float lo2 = (EDGE || QMODE) ? g.side2_lo : INFINITY;
+            unsigned which = 0;
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if ((!SELF || 4 * k + t > lane) && r[t] < (EDGE || QMODE ? hi : lo) && (fabsf(d[t]) > thr || r[t] >= lo2))
+                    which |= 1u << t;
+#pragma unroll 1
+            while (which) {
+                const int t = __ffs(which) - 1;
+                which &= which - 1u;
+                const float rr2 = t < 2 ? (t == 0 ? r[0] : r[1]) : (t == 2 ? r[2] : r[3]);
+                const unsigned was = (t < 2 ? (t == 0 ? bits[0] : bits[1]) : (t == 2 ? bits[2] : bits[3]));
+                float x2 = 0.f, dy = 0.f, dz = 0.f;
+                if (EDGE || QMODE) {  // the statistics look at the FMA-contracted rr2 as well
+                    const float dx = image_1<MODE>(ring[e + t], h.nx, cx, g.L[0], g.h1[0], g.h2[0]);
+                    dy = image_1<MODE>(ring[kRing + e + t], h.ny, cy, g.L[1], g.h1[1], g.h2[1]);
+                    dz = image_1<MODE>(ring[2 * kRing + e + t], h.nz, cz, g.L[2], g.h1[2], g.h2[2]);
+                    x2 = __fmul_rn(dx, dx);
+                }
+                const int x = exact_bin(rr2, x2, dy, dz, g.side2, g.deltar, g.lsmax, g.floor_bins,
+                                        (EDGE || QMODE) && g.want_edge);
+                pc.ulp += (x >> 29) & 1;
+                pc.fma += (x >> 30) & 1;
+                const unsigned ind = (x & ((1 << 29) - 1)) + kBinBias;
+                const unsigned row = row_of(__float_as_uint(ring[3 * kRing + e + t]));
+                if (QMODE) {
+                    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(row + (ind << 2)) : "memory");
+                    atomicAdd(&myq[ind - kBinBias], (double)h.q * ring_q[e + t]);
+                } else if (rr2 < g.side2 && ind != was) {
+                    asm volatile("red.shared.add.u32 [%0], 0xffffffff;" ::"r"(row + (was << 2)) : "memory");
+                    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(row + (ind << 2)) : "memory");
+                }
+            }
+        }
+    }
 }
 
 // Wrapped coordinate of a folded one in [-L, L): x, or x + L for x < 0 (the same FP32 value the cell
@@ -297,235 +364,283 @@ __device__ __forceinline__ void axis_box(float v0, bool has0, float v1, bool has
 // negative coordinates negative; the cull works on the wrapped values.
 __device__ __forceinline__ float wrap_cull(float x, float L) { return x < 0.f ? __fadd_rn(x, L) : x; }
 
-__device__ __forceinline__ bool maybe_near(const float4& b, const float4& c, const float4& h, float cull2,
-                                           const float (&L)[3]) {
-    const float gx = fmaxf(fabsf(wrap_cull(b.x, L[0]) - c.x) - h.x, 0.f);
-    const float gy = fmaxf(fabsf(wrap_cull(b.y, L[1]) - c.y) - h.y, 0.f);
-    const float gz = fmaxf(fabsf(wrap_cull(b.z, L[2]) - c.z) - h.z, 0.f);
-    return fmaf(gz, gz, fmaf(gy, gy, gx * gx)) <= cull2;
+// Distance along one axis from a point (or box centre) to the homes' box, clipped at 0.  PERIODIC: of the
+// nearest image.
+template <bool PERIODIC>
+__device__ __forceinline__ float axis_gap(float b, float c, float h, float L) {
+    float t = fabsf(b - c);
+    if (PERIODIC) t = fminf(t, L - t);
+    return fmaxf(t - h, 0.f);
 }
 
-// One task for one warp: its 64 home atoms (a0 = atom il0, a1 = atom il0 + 32 per lane) against the
-// staged neighbour chunk.  Blocks of 32 neighbours are culled against the warp's box (kept in shared
-// memory, `wb`) with one ballot; the survivors are tested exactly.  Returns the candidate pairs tested.
-// Lanes whose bit index k has jj0 + k > lim: the neighbours of a block that pair with a home.
-__device__ __forceinline__ unsigned after_mask(int lim, int jj0) {
-    const int s = lim - jj0;
-    return s < 0 ? 0xffffffffu : (s >= 31 ? 0u : (0xffffffffu << (s + 1)));
+// The warp's home atoms' bounding box along one axis (wrapped coordinates, in [0, L]: their bit patterns
+// order like the values; + 0 turns -0 into +0).
+__device__ __forceinline__ void axis_box(float v, bool has, float pad, float& c, float& h) {
+    const unsigned b = __float_as_uint(v + 0.0f);
+    const float mn = __uint_as_float(__reduce_min_sync(0xffffffffu, has ? b : 0x7f800000u));
+    const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, has ? b : 0u));
+    c = 0.5f * (mn + mx);
+    h = 0.5f * (mx - mn) + pad;
 }
 
-// SELF: home and neighbour cell are the same cell (pairs need j > i within it).
-template <bool FAST, bool SELF, bool FLOOR, bool QMODE>
-__device__ __forceinline__ unsigned run_task(const TaskInfo& ti, const float4* __restrict__ bj, const float4& a0,
-                                             const float4& a1, bool h0, bool h1, int il0, int il0w, int s0, int s1,
-                                             unsigned lane, const RdfParams& p, const int* rowtab, unsigned* myhist,
-                                             PairCounters& pc, double* myq, float qa0, float qa1, const float* qj,
-                                             WarpBox* wb) {
-    if (ti.cull) {
-        float cx, cy, cz, hx, hy, hz;
-        axis_box(wrap_cull(a0.x, p.L[0]), h0, wrap_cull(a1.x, p.L[0]), h1, p.nc[0] > 1, ti.img[0], p.cull_pad, cx, hx);
-        axis_box(wrap_cull(a0.y, p.L[1]), h0, wrap_cull(a1.y, p.L[1]), h1, p.nc[1] > 1, ti.img[1], p.cull_pad, cy, hy);
-        axis_box(wrap_cull(a0.z, p.L[2]), h0, wrap_cull(a1.z, p.L[2]), h1, p.nc[2] > 1, ti.img[2], p.cull_pad, cz, hz);
-        if (lane == 0) {
-            wb->c = make_float4(cx, cy, cz, 0.f);
-            wb->h = make_float4(hx, hy, hz, 0.f);
-        }
-        __syncwarp();
-    }
-    const int jbeg = SELF ? max(0, il0w + 1 - ti.jlocal0) : 0;
-    const int lim0 = SELF ? il0 - ti.jlocal0 : -1;  // a0 pairs need jj > lim0
-    const int lim1 = SELF ? lim0 + 32 : -1;         // a1 pairs need jj > lim1
-    unsigned tested = 0;
-    for (int jj0 = jbeg; jj0 < ti.jcount; jj0 += 32) {
-        const int jl = jj0 + (int)lane;
-        bool keep = jl < ti.jcount;
-        if (ti.cull && keep) keep = maybe_near(bj[jl], wb->c, wb->h, p.cull2, p.L);
-        unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (SELF)
-            tested += (h0 ? __popc(m & after_mask(lim0, jj0)) : 0) + (h1 ? __popc(m & after_mask(lim1, jj0)) : 0);
-        else
-            tested += __popc(m) * ((unsigned)h0 + (unsigned)h1);
-        while (m) {
-            const int k0 = __ffs(m) - 1;
-            m &= m - 1u;
-            const int j0 = jj0 + k0;
-            const float4 b0 = bj[j0];
-            pair<FAST, FLOOR, QMODE>(a0, b0, SELF ? (h0 && j0 > lim0) : h0, s0, p, rowtab, myhist, pc, myq, qa0,
-                                     qj + j0);
-            pair<FAST, FLOOR, QMODE>(a1, b0, SELF ? (h1 && j0 > lim1) : h1, s1, p, rowtab, myhist, pc, myq, qa1,
-                                     qj + j0);
-        }
-    }
-    return tested;
+// |d| < 3L/2 for every pair of the frame: no coordinate below -0.499 L, or none below -0.749 L while none
+// reaches 0.749 L (frames centred on the origin).  (Coordinates outside [-L, L) are flagged per cell.)
+__device__ __forceinline__ bool frame_within(unsigned f) {
+    return !(f & kFrameLow) || !(f & (kFrameVeryLow | kFrameHigh));
 }
 
-// Arms the next phase of a staging slot: the next task's neighbour chunk by bulk copy, or a plain
-// arrival with valid = 0 when the work is exhausted (readers of that phase leave the task loop).
-__device__ __forceinline__ void refill_slot(int slot, TaskGen& gen, const RdfParams& p,
-                                            const int32_t* __restrict__ cstart, const int32_t* __restrict__ ccount,
-                                            const int32_t* __restrict__ cflag, const int32_t* __restrict__ fstart,
-                                            unsigned long long* work,
-                                            const float4* __restrict__ sorted, TaskInfo* tinfo, uint64_t* bars,
-                                            unsigned* phases, float4* buf) {
-    TaskInfo nx;
-    const bool ok = next_task(gen, p, cstart, ccount, cflag, fstart, work, nx);
-    tinfo[slot] = nx;
-    phases[slot] += 1u;
-    if (ok) {
-        // The slot's previous contents were read through the generic proxy; order those reads before
-        // the bulk copy (async proxy) overwrites them.
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        trj_mbar_arrive_expect_tx(&bars[slot], nx.jcount * 16u);
-        trj_bulk_g2s(buf + slot * kJChunk, sorted + nx.sb, nx.jcount * 16u, &bars[slot]);
-    } else {
-        trj_mbar_arrive(&bars[slot]);
-    }
-}
-
-// QMODE: sorted_q holds the charges in cell order and gqq_frame (lsmax doubles) receives this
-// frame's sum of q_a*q_b per bin; the charge replicas (lsmax doubles each, warp w uses w mod nrep)
-// follow the count replicas in shared memory.
-template <bool FLOOR, bool QMODE>
-__global__ void __launch_bounds__(kThreads, 4) rdf_pairs_kernel(RdfParams p, const float4* __restrict__ sorted,
-                                                             const int32_t* __restrict__ cstart,
-                                                             const int32_t* __restrict__ ccount,
-                                                             const int32_t* __restrict__ cflag,
-                                                             const int32_t* __restrict__ fstart,
-                                                             unsigned long long* __restrict__ work,
-                                                             unsigned long long* __restrict__ hist_g,
-                                                             unsigned long long* __restrict__ edge_g,
-                                                             unsigned* __restrict__ status,
-                                                             const float* __restrict__ sorted_q,
-                                                             double* __restrict__ gqq_frame) {
+// Work item = (home group, segment of its neighbour list), taken from a global counter by one warp at a
+// time; no warp waits for another.  Shared memory: bin rows (count), charge rows (QMODE, FP64 [row_words]),
+// the warps' buffers.  SQUARE: a bin row per ordered species pair, so that a pair's row address is a sum of
+// two registers; otherwise the rows of ind_ij through a 16 x 16 table of addresses.
+//
+// What bounds it: instruction issue (76 % of the slots at 62,500 atoms), not the 22 MB it moves.  At 1e6
+// atoms (3 species, 0.86e9 pairs in range) 1.75e9 pairs are tested, in 17.6e6 blocks of four survivors x 32
+// homes of about 100 instructions each, and 4.6e6 neighbour groups read and culled, together a quarter of
+// the time.  Measured: 7.25 -> 2.9 ms at 1e6 atoms, 1.62 -> 0.41 ms at 62,500 (cutoff 10, four cells per
+// axis), 19.3 -> 6.0 ms for the 4e6-atom slab, against 64-atom homes (two per lane) that a CTA walks over
+// staged neighbour cells with a branch per pair.
+template <bool FLOOR, bool QMODE, bool SQUARE, bool EDGE>
+__global__ void __launch_bounds__(kMaxWarps * 32, 1)
+    rdf_pairs_kernel(const __grid_constant__ RdfParams p, const float4* __restrict__ sorted,
+                     const int32_t* __restrict__ fstart, const int32_t* __restrict__ fcount,
+                     const int32_t* __restrict__ cflag, const unsigned* __restrict__ fflag, unsigned* __restrict__ work,
+                     u64* __restrict__ hist_g, u64* __restrict__ edge_g, unsigned* __restrict__ status,
+                     const float* __restrict__ sorted_q, double* __restrict__ gqq_frame) {
     extern __shared__ __align__(128) unsigned char smem[];
-    float4* buf = reinterpret_cast<float4*>(smem);                       // [kSlots][kJChunk]
-    unsigned* hist = reinterpret_cast<unsigned*>(smem + kSlots * kJChunk * sizeof(float4));
-    __shared__ __align__(8) uint64_t bars[kSlots];
     __shared__ __align__(8) uint64_t never;  // no thread arrives on it: the target of the stall test
-    __shared__ TaskInfo tinfo[kSlots];
-    __shared__ unsigned released[kSlots];  // warps done with the slot's task
-    __shared__ unsigned phases[kSlots];    // phases armed per slot
-    __shared__ TaskGen gen;                // task iterator, used by one refilling thread at a time
-    __shared__ int rowtab[16 * 16];
-    __shared__ int abort_flag;
-    __shared__ WarpBox wboxes[kThreads / 32];
-
-    const int tid = threadIdx.x, warp = tid / 32;
-    const unsigned lane = (unsigned)tid & 31u;
-    const int hsz = p.nit * p.lsmax;
-    unsigned* myhist = hist + (size_t)(warp % p.nrep) * hsz;
-    for (int k = tid; k < p.nrep * hsz; k += blockDim.x) hist[k] = 0u;
-    double* qhist = nullptr;
-    double* myq = nullptr;
-    if (QMODE) {
-        qhist = reinterpret_cast<double*>(hist + (((size_t)p.nrep * hsz + 1) & ~(size_t)1));
-        myq = qhist + (size_t)(warp % p.nrep) * p.lsmax;
-        for (int k = tid; k < p.nrep * p.lsmax; k += blockDim.x) qhist[k] = 0.0;
-    }
-    for (int k = tid; k < p.nsp * p.nsp; k += blockDim.x) rowtab[k] = trj_pair_row(k / p.nsp, k % p.nsp, p.nsp);
+    __shared__ unsigned rowtab[SQUARE ? 1 : 256];
+    __shared__ int stalled;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarp = blockDim.x >> 5;
+    const PairGeom& g = p.g;
+    const int nsp = g.nsp, rw = g.row_words;
+    const int nrow = SQUARE ? nsp * nsp : p.nit;
+    // [warps' buffers][QMODE: warps' charge buffers, FP64 rows][count rows]
+    float* ring = reinterpret_cast<float*>(smem) + (size_t)warp * 4 * kRing;
+    double* ring_q = reinterpret_cast<double*>(smem + (size_t)nwarp * 16 * kRing) + (QMODE ? warp * kRing : 0);
+    double* qhist = reinterpret_cast<double*>(smem + (size_t)nwarp * 16 * kRing) + (QMODE ? nwarp * kRing : 0);
+    unsigned* hist = reinterpret_cast<unsigned*>(qhist + (QMODE ? rw : 0));
+    for (int k = tid; k < nrow * rw; k += blockDim.x) hist[k] = 0u;
+    if (QMODE)
+        for (int k = tid; k < rw; k += blockDim.x) qhist[k] = 0.0;
+    const unsigned hist_base = trj_smem_addr(hist);
+    if (!SQUARE)
+        for (int k = tid; k < nsp * nsp; k += blockDim.x)
+            rowtab[(k / nsp) * 16 + k % nsp] =
+                hist_base + (unsigned)(trj_pair_row(k / nsp, k % nsp, nsp) * rw * 4) - 4u * kBinBias;
     if (tid == 0) {
-        gen.started = 0;
-        abort_flag = 0;
-        for (int sl = 0; sl < kSlots; ++sl) {
-            trj_mbar_init(&bars[sl], 1);
-            released[sl] = 0u;
-            phases[sl] = 0u;
-        }
         trj_mbar_init(&never, 1);
         trj_fence_mbar_init();
-        for (int sl = 0; sl < kSlots; ++sl) refill_slot(sl, gen, p, cstart, ccount, cflag, fstart, work, sorted, tinfo, bars, phases, buf);
+        stalled = 0;
     }
     __syncthreads();
+    if (p.stall_test && !trj_mbar_wait_limit(&never, 0u, p.wait_clocks)) {
+        if (lane == 0) trj_raise(status, TRJ_DEV_TIMEOUT);
+        stalled = 1;
+    }
+    __syncthreads();
+    if (stalled) return;
+
+    const unsigned lt = (1u << lane) - 1u;
+    const bool frame_ok = frame_within(*fflag);
     PairCounters pc;
-    unsigned long long n_tested = 0;
-    // Warps walk the task sequence independently: task t sits in slot t % kSlots; the last warp to
-    // release a slot refills it with the next task, so a warp may run up to kSlots - 1 tasks ahead of
-    // the slowest one instead of meeting it at a CTA barrier after every task.
-    for (int t = 0;; ++t) {
-        const int slot = t % kSlots;
-        if (__shfl_sync(0xffffffffu, *(volatile int*)&abort_flag, 0)) break;  // warp-uniform
-        // Warp-uniform outcome: the task loop below uses full-warp ballots.
-        const bool stall = p.stall_test && t == 0;
-        if (!__all_sync(0xffffffffu, trj_mbar_wait_limit(stall ? &never : &bars[slot],
-                                                         stall ? 0u : (unsigned)(t / kSlots) & 1u,
-                                                         p.wait_clocks))) {
-            if (lane == 0) {
-                trj_raise(status, TRJ_DEV_TIMEOUT);
-                *(volatile int*)&abort_flag = 1;
-            }
-            break;
-        }
-        const TaskInfo ti = tinfo[slot];
-        if (!ti.valid) break;
-        // The warp's home atoms [hbeg, hend) within the cell: its octant, or 64 consecutive atoms of the round.
-        const int hbeg = ti.oct ? (int)tinfo[slot].ostart[warp] : ti.hc * kHomeChunk + 64 * warp;
-        const int hend = ti.oct ? (int)tinfo[slot].ostart[warp + 1] : min(ti.na, hbeg + 64);
-        const int il0 = hbeg + (int)lane, il1 = il0 + 32;
-        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 a0 = il0 < hend ? sorted[ti.sa + il0] : z4;
-        const float4 a1 = il1 < hend ? sorted[ti.sa + il1] : z4;
-        const int s0 = __float_as_int(a0.w), s1 = __float_as_int(a1.w);
-        // A species outside 0..nsp-1 can only come from a frame already flagged as bad data.
-        const bool h0 = il0 < hend && (unsigned)s0 < (unsigned)p.nsp;
-        const bool h1 = il1 < hend && (unsigned)s1 < (unsigned)p.nsp;
-        const float qa0 = (QMODE && il0 < hend) ? sorted_q[ti.sa + il0] : 0.f;
-        const float qa1 = (QMODE && il1 < hend) ? sorted_q[ti.sa + il1] : 0.f;
-        const float* qj = QMODE ? sorted_q + ti.sb : nullptr;
-        const float4* bj = buf + slot * kJChunk;
-        WarpBox* wb = &wboxes[warp];
-#define TRJ_RUN(F, S)                                                                                       \
-    run_task<F, S, FLOOR, QMODE>(ti, bj, a0, a1, h0, h1, il0, hbeg, s0, s1, lane, p, rowtab, myhist, pc, myq, qa0, \
-                                 qa1, qj, wb)
-        if (hbeg < hend) {  // warp-uniform: the warp has home atoms in this task
-            if (ti.fast)
-                n_tested += ti.self ? TRJ_RUN(true, true) : TRJ_RUN(true, false);
-            else
-                n_tested += ti.self ? TRJ_RUN(false, true) : TRJ_RUN(false, false);
-        }
+    u64 n_tested = 0;
+    for (;;) {
+        unsigned item = 0;
+        if (lane == 0) item = atomicAdd(work, 1u);
+        item = __shfl_sync(0xffffffffu, item, 0);
+        if (item >= p.nitems) break;
+        const int key = (int)(item / (unsigned)p.nseg), seg = (int)(item - (unsigned)key * (unsigned)p.nseg);
+        const int hbeg = fstart[key], hend = hbeg + fcount[key];
+        if (hbeg >= hend) continue;
+        const int c = key / p.nsub, own = key - c * p.nsub;
+        const int cz = c % p.nc[2], cxy = c / p.nc[2], cy = cxy % p.nc[1], cx = cxy / p.nc[1];
+        const int fl = cflag[c];
+        const int list = p.noff * p.nsub;  // the (offset, neighbour group) list, cut into segments
+        const int t0 = seg * p.per_seg, t1 = min(list, t0 + p.per_seg);
+        for (int h0 = hbeg; h0 < hend; h0 += kGroup) {
+            const int nh = min(kGroup, hend - h0);
+            const bool has = lane < nh;
+            const float4 a = has ? sorted[h0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+            Home h;
+            h.nx = -a.x;
+            h.ny = -a.y;
+            h.nz = -a.z;
+            h.q = (QMODE && has) ? sorted_q[h0 + lane] : 0.f;
+            const unsigned wa = __float_as_uint(a.w);  // species * row bytes (64 with the row table)
+            h.hist = SQUARE ? hist_base + wa * (unsigned)nsp - 4u * kBinBias : trj_smem_addr(rowtab) + (wa >> 4);
+            float bx, by, bz, wx, wy, wz;  // the homes' box: centre and half-widths
+            axis_box(wrap_cull(a.x, g.L[0]), has, p.cull_pad, bx, wx);
+            axis_box(wrap_cull(a.y, g.L[1]), has, p.cull_pad, by, wy);
+            axis_box(wrap_cull(a.z, g.L[2]), has, p.cull_pad, bz, wz);
+            for (int t = t0; t < t1;) {
+                const int o = t / p.nsub, s_lo = t - o * p.nsub, s_hi = min(p.nsub, t1 - o * p.nsub);
+                t = o * p.nsub + s_hi;
+                const int ex = cx + p.off[o][0], ey = cy + p.off[o][1], ez = cz + p.off[o][2];
+                const int c2 = (wrapc(ex, p.nc[0]) * p.nc[1] + wrapc(ey, p.nc[1])) * p.nc[2] + wrapc(ez, p.nc[2]);
+                const int f2 = fl | cflag[c2];
+                const bool far = f2 & 2;
+                const float ix = ex < 0 ? -g.L[0] : (ex >= p.nc[0] ? g.L[0] : 0.f);
+                const float iy = ey < 0 ? -g.L[1] : (ey >= p.nc[1] ? g.L[1] : 0.f);
+                const float iz = ez < 0 ? -g.L[2] : (ez >= p.nc[2] ? g.L[2] : 0.f);
+                const bool plain = p.split_all && !(f2 & 1);  // image known from the cells
+                const int mode = plain ? ((ix != 0.f || iy != 0.f || iz != 0.f) ? kImgShift : kImgNone)
+                                       : far ? kImgAny : p.split_all ? kImgRound : frame_ok ? kImgFold : kImgAny;
+                const int kb = c2 * p.nsub;
+                int head = 0, tail = 0;
+                auto append = [&](const float4& b, float qb, bool keep) {
+                    const unsigned m = __ballot_sync(0xffffffffu, keep);
+                    if (keep) {
+                        const int e = (tail + __popc(m & lt)) & (kRing - 1);
+                        ring[e] = b.x;
+                        ring[kRing + e] = b.y;
+                        ring[2 * kRing + e] = b.z;
+                        ring[3 * kRing + e] = b.w;
+                        if (QMODE) ring_q[e] = (double)qb;
+                    }
+                    tail += __popc(m);
+                };
+                // Fills the buffer up to a multiple of four with NaN entries (in no range, near no edge).
+                auto pad = [&]() {
+                    const int n = tail - head, up = (n + 3) & ~3;
+                    if (lane < up - n) {
+                        const int e = (tail + lane) & (kRing - 1);
+                        ring[e] = ring[kRing + e] = ring[2 * kRing + e] = NAN;
+                        ring[3 * kRing + e] = 0.f;
+                        if (QMODE) ring_q[e] = 0.0;
+                    }
+                    return up >> 2;
+                };
+#define TRJ_RUN(M, S, N4) test_run<M, S, FLOOR, QMODE, SQUARE, EDGE>(ring, ring_q, head, N4, h, has, ix, iy, iz, g, pc, qhist)
+                if (o == 0 && s_lo <= own && own < s_hi) {
+                    // pairs j > i of the round's own atoms, through the buffer in lane order
+                    append(a, h.q, has);
+                    const int n4 = pad();
+                    __syncwarp();
+                    if (plain) TRJ_RUN(kImgNone, true, n4);
+                    else TRJ_RUN(kImgAny, true, n4);
+                    __syncwarp();
+                    if (EDGE && has) n_tested += (unsigned)(nh - 1 - lane);
+                    tail = 0;
+                }
+                int s0 = s_lo - 32, j = 0, je = 0, gs = 0, gn = 0;  // gs, gn: start and atoms of lane's group
+                unsigned m = 0;
+                bool more = true;
+                do {
+                    // survivors into the buffer until a run is full or the segment's groups are used up
+                    while (tail - head < kRingRun) {
+                        if (j >= je) {
+                            if (!m) {
+                                s0 += 32;
+                                if (s0 >= s_hi) {
+                                    more = false;
+                                    break;
+                                }
+                                // lanes over the neighbour groups: which can hold an atom in range of the homes' box
+                                const int s = s0 + lane;
+                                bool near = s < s_hi && (o > 0 || s >= own);
+                                if (near && !far) {
+                                    const int q = (int)(((float)s + 0.5f) * p.inv_sub[2]), sz = s - q * p.sub[2];
+                                    const int sx = (int)(((float)q + 0.5f) * p.inv_sub[1]), sy = q - sx * p.sub[1];
+                                    const float gx = ((float)ex + ((float)sx + 0.5f) * p.inv_sub[0]) * p.edge[0];
+                                    const float gy = ((float)ey + ((float)sy + 0.5f) * p.inv_sub[1]) * p.edge[1];
+                                    const float gz = ((float)ez + ((float)sz + 0.5f) * p.inv_sub[2]) * p.edge[2];
+                                    float dx, dy, dz;
+                                    if (p.split_all) {
+                                        dx = axis_gap<false>(gx, bx, wx + p.half[0], 0.f);
+                                        dy = axis_gap<false>(gy, by, wy + p.half[1], 0.f);
+                                        dz = axis_gap<false>(gz, bz, wz + p.half[2], 0.f);
+                                    } else {
+                                        dx = axis_gap<true>(gx - ix, bx, wx + p.half[0], g.L[0]);
+                                        dy = axis_gap<true>(gy - iy, by, wy + p.half[1], g.L[1]);
+                                        dz = axis_gap<true>(gz - iz, bz, wz + p.half[2], g.L[2]);
+                                    }
+                                    near = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
+                                }
+                                if (near) {
+                                    gs = fstart[kb + s];
+                                    gn = fcount[kb + s];
+                                }
+                                m = __ballot_sync(0xffffffffu, near);
+                                continue;
+                            }
+                            const int k = __ffs(m) - 1;
+                            m &= m - 1u;
+                            j = __shfl_sync(0xffffffffu, gs, k);
+                            je = j + __shfl_sync(0xffffffffu, gn, k);
+                            if (o == 0 && s0 + k == own) j = h0 + nh;  // the round's own atoms are done
+                            continue;
+                        }
+                        bool keep = j + lane < je;
+                        const float4 b = keep ? sorted[j + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+                        const float qb = (QMODE && keep) ? sorted_q[j + lane] : 0.f;
+                        j += 32;
+                        if (keep && !far) {
+                            float dx, dy, dz;
+                            if (plain) {
+                                dx = axis_gap<false>(b.x, bx - ix, wx, 0.f);
+                                dy = axis_gap<false>(b.y, by - iy, wy, 0.f);
+                                dz = axis_gap<false>(b.z, bz - iz, wz, 0.f);
+                            } else {
+                                dx = axis_gap<true>(wrap_cull(b.x, g.L[0]), bx, wx, g.L[0]);
+                                dy = axis_gap<true>(wrap_cull(b.y, g.L[1]), by, wy, g.L[1]);
+                                dz = axis_gap<true>(wrap_cull(b.z, g.L[2]), bz, wz, g.L[2]);
+                            }
+                            keep = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
+                        }
+                        const int before = tail;
+                        append(b, qb, keep);
+                        if (EDGE && has) n_tested += (unsigned)(tail - before);
+                    }
+                    const int n4 = tail - head >= kRingRun ? kRingRun / 4 : pad();
+                    __syncwarp();  // the other lanes' entries
+                    if (mode == kImgNone) TRJ_RUN(kImgNone, false, n4);
+                    else if (mode == kImgShift) TRJ_RUN(kImgShift, false, n4);
+                    else if (mode == kImgRound) TRJ_RUN(kImgRound, false, n4);
+                    else if (mode == kImgFold) TRJ_RUN(kImgFold, false, n4);
+                    else TRJ_RUN(kImgAny, false, n4);
+                    __syncwarp();
+                    head += 4 * n4;
+                } while (more);
 #undef TRJ_RUN
-        // Release the slot; the last warp refills it.
-        __syncwarp();
-        if (lane == 0) {
-            __threadfence_block();
-            if (atomicAdd(&released[slot], 1u) == kThreads / 32 - 1) {
-                released[slot] = 0u;
-                __threadfence_block();
-                refill_slot(slot, gen, p, cstart, ccount, cflag, fstart, work, sorted, tinfo, bars, phases, buf);
             }
         }
-        __syncwarp();
     }
     __syncthreads();
-    if (tid == 0 && abort_flag) {
-        // Let copies still in flight land before the CTA exits (bounded by the default limit, not by
-        // the plan's wait limit: a copy always lands).
-        for (int sl = 0; sl < kSlots; ++sl)
-            if (phases[sl]) trj_mbar_wait(&bars[sl], (phases[sl] - 1) & 1);
-    }
-    __syncthreads();
-    // Merge replicas into the global uint64 histogram (their total is the counted pairs).
+    // Merge into the global uint64 histogram (the total is the counted pairs).
+    const int hsz = p.nit * g.lsmax;
+    int row = 0, sa = 0, sb = 0;  // species of the row of element k
     for (int k = tid; k < hsz; k += blockDim.x) {
-        unsigned long long s = 0;
-        for (int r = 0; r < p.nrep; ++r) s += hist[(size_t)r * hsz + k];
+        while (row < k / g.lsmax) {
+            ++row;
+            if (++sb == nsp) sb = ++sa;
+        }
+        const int bin = k - row * g.lsmax + 1;
+        u64 s;
+        if (SQUARE) {
+            s = hist[(sa * nsp + sb) * rw + bin];
+            if (sa != sb) s += hist[(sb * nsp + sa) * rw + bin];
+        } else {
+            s = hist[row * rw + bin];
+        }
         if (s) atomicAdd(&hist_g[k], s);
         pc.counted += s;
     }
     if (QMODE) {
-        for (int k = tid; k < p.lsmax; k += blockDim.x) {
-            double s = 0.0;
-            for (int r = 0; r < p.nrep; ++r) s += qhist[(size_t)r * p.lsmax + k];
+        for (int k = tid; k < g.lsmax; k += blockDim.x) {
+            const double s = qhist[k + 1];
             if (s != 0.0) atomicAdd(&gqq_frame[k], s);
         }
     }
     if (edge_g) {
-        unsigned long long n_ulp = pc.ulp, n_fma = pc.fma, n_counted = pc.counted;
+        u64 n_ulp = pc.ulp, n_fma = pc.fma, n_counted = pc.counted;
         for (int off = 16; off > 0; off >>= 1) {
             n_ulp += __shfl_down_sync(0xffffffffu, n_ulp, off);
             n_fma += __shfl_down_sync(0xffffffffu, n_fma, off);
             n_counted += __shfl_down_sync(0xffffffffu, n_counted, off);
             n_tested += __shfl_down_sync(0xffffffffu, n_tested, off);
         }
-        if ((tid & 31) == 0) {
+        if (lane == 0) {
             if (n_ulp) atomicAdd(&edge_g[TRJ_EDGE_ULP], n_ulp);
             if (n_fma) atomicAdd(&edge_g[TRJ_EDGE_FMA], n_fma);
             if (n_counted) atomicAdd(&edge_g[TRJ_EDGE_COUNTED], n_counted);
@@ -534,81 +649,90 @@ __global__ void __launch_bounds__(kThreads, 4) rdf_pairs_kernel(RdfParams p, con
     }
 }
 
-// Cell of each atom from its wrapped coordinate, and its sub-cell: the cell is split into
-// 2^sbits parts per axis and the parts are numbered along a Morton curve (bits interleaved x, y, z
-// from the lowest), so atoms sorted by key = cell * 8^sbits + sub-cell are cell-contiguous and
-// spatially ordered inside each cell.  Per-key and per-cell counts, per-key slots.
-__global__ void cell_assign_kernel(const float4* __restrict__ packed, int64_t n, float Lx, float Ly,
-                                   float Lz, int ncx, int ncy, int ncz, int sbits, int32_t* __restrict__ fcount,
-                                   int32_t* __restrict__ ccount, int32_t* __restrict__ cflag,
-                                   int32_t* __restrict__ akey, int32_t* __restrict__ aslot) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 v = packed[i];
-    float L[3] = {Lx, Ly, Lz};
-    int nc[3] = {ncx, ncy, ncz};
-    float r[3] = {v.x, v.y, v.z};
-    int k[3], sub[3];
-    const int S = 1 << sbits;
-    bool outside = false, far = false;
+// Cell of each atom from its wrapped coordinate, and its group: the cell is divided into sub[0] x sub[1] x
+// sub[2] boxes numbered z fastest, so atoms sorted by key = cell * nsub + box are cell-contiguous and
+// grouped by box.  Per-key counts and slots, cell and frame flags.
+__global__ void cell_assign_kernel(const float4* __restrict__ packed, int64_t n, const __grid_constant__ RdfParams p,
+                                   int32_t* __restrict__ fcount, int32_t* __restrict__ cflag,
+                                   unsigned* __restrict__ fflag, int32_t* __restrict__ akey,
+                                   int32_t* __restrict__ aslot) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned ff = 0;
+    if (i < n) {
+        const float4 v = packed[i];
+        const float r[3] = {v.x, v.y, v.z};
+        int k[3], sub[3];
+        bool outside = false, far = false;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        outside |= !(r[d] >= 0.0f && r[d] < L[d]);
-        far |= !(r[d] >= -L[d] && r[d] < L[d]);
-        float w = r[d] - L[d] * floorf(r[d] / L[d]);
-        float t = w * ((float)nc[d] / L[d]);
-        int c = (int)t;
-        c = c < 0 ? 0 : (c >= nc[d] ? nc[d] - 1 : c);
-        k[d] = c;
-        int sc = (int)((t - (float)c) * (float)S);
-        sub[d] = sc < 0 ? 0 : (sc >= S ? S - 1 : sc);  // also catches NaN coordinates (sc = 0)
+        for (int d = 0; d < 3; ++d) {
+            const float L = p.g.L[d];
+            outside |= !(r[d] >= 0.0f && r[d] < L);
+            far |= !(r[d] >= -L && r[d] < L);
+            ff |= (r[d] < -0.499f * L ? kFrameLow : 0u) | (r[d] < -0.749f * L ? kFrameVeryLow : 0u) |
+                  (r[d] >= 0.749f * L ? kFrameHigh : 0u);
+            const float w = r[d] - L * floorf(r[d] / L);
+            const float t = w * ((float)p.nc[d] / L);
+            int c = (int)t;
+            c = c < 0 ? 0 : (c >= p.nc[d] ? p.nc[d] - 1 : c);
+            k[d] = c;
+            const int sc = (int)((t - (float)c) * (float)p.sub[d]);
+            sub[d] = sc < 0 ? 0 : (sc >= p.sub[d] ? p.sub[d] - 1 : sc);  // also catches NaN coordinates (sc = 0)
+        }
+        const int c = (k[0] * p.nc[1] + k[1]) * p.nc[2] + k[2];
+        const int key = c * p.nsub + (sub[0] * p.sub[1] + sub[1]) * p.sub[2] + sub[2];
+        // A species outside 0..nsp-1 can only come from a frame already flagged as bad data: not placed.
+        const bool ok = __float_as_uint(v.w) < (unsigned)p.g.nsp;
+        akey[i] = ok ? key : -1;
+        if (ok) aslot[i] = atomicAdd(&fcount[key], 1);
+        // bit 0: a coordinate outside [0, L) (pairs of the cell need the minimum image);
+        // bit 1: a coordinate outside [-L, L) or NaN (its wrapped value is not x or x + L: no cull)
+        if (outside) atomicOr(&cflag[c], far ? 3 : 1);
     }
-    int m = 0;
-    for (int b = 0; b < sbits; ++b)
-        m |= (((sub[0] >> b) & 1) << (3 * b)) | (((sub[1] >> b) & 1) << (3 * b + 1)) |
-             (((sub[2] >> b) & 1) << (3 * b + 2));
-    int c = (k[0] * ncy + k[1]) * ncz + k[2];
-    const int key = (c << (3 * sbits)) | m;
-    akey[i] = key;
-    aslot[i] = atomicAdd(&fcount[key], 1);
-    atomicAdd(&ccount[c], 1);
-    // bit 0: a coordinate outside [0, L) (pairs of the cell need the minimum image);
-    // bit 1: a coordinate outside [-L, L) or NaN (its wrapped value is not x or x + L: no box cull)
-    if (outside) atomicOr(&cflag[c], far ? 3 : 1);
+    ff = __reduce_or_sync(0xffffffffu, ff);
+    if ((threadIdx.x & 31) == 0 && (ff & ~*(volatile unsigned*)fflag)) atomicOr(fflag, ff);
 }
 
-// Start of every (cell, sub-cell) key: the cell's start plus the exclusive prefix of its sub-cell
-// counts.  One warp per cell.
-__global__ void sub_offsets_kernel(const int32_t* __restrict__ fcount, const int32_t* __restrict__ cstart, int ncell,
-                                   int sbits, int32_t* __restrict__ fstart) {
-    const int c = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-    const unsigned lane = threadIdx.x & 31u;
-    if (c >= ncell) return;
-    const int nsub = 1 << (3 * sbits);
-    const int64_t base = (int64_t)c << (3 * sbits);
-    int carry = cstart[c];
-    for (int s0 = 0; s0 < nsub; s0 += 32) {
-        const int s = s0 + (int)lane;
-        const int v = s < nsub ? fcount[base + s] : 0;
-        int x = v;
+// Start of every group in the sorted array.  Groups need only be contiguous, not in key order, so a block
+// takes the room of its 256 groups from a counter instead of waiting for the sums before it: one short
+// kernel in place of a scan over all keys.
+__global__ void __launch_bounds__(256) group_offsets_kernel(const int32_t* __restrict__ fcount, int nkey,
+                                                            int32_t* __restrict__ total, int32_t* __restrict__ fstart) {
+    __shared__ int wsum[8], base;
+    const int k = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int v = k < nkey ? fcount[k] : 0;
+    int x = v;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if ((int)lane >= o) x += y;
-        }
-        if (s < nsub) fstart[base + s] = carry + x - v;
-        carry += __shfl_sync(0xffffffffu, x, 31);
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
     }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int sum = 0;
+        for (int w = 0; w < 8; ++w) {
+            const int y = wsum[w];
+            wsum[w] = sum;
+            sum += y;
+        }
+        base = atomicAdd(total, sum);
+    }
+    __syncthreads();
+    if (k < nkey) fstart[k] = base + wsum[warp] + x - v;
 }
 
 __global__ void cell_scatter_kernel(const float4* __restrict__ packed, int64_t n,
                                     const int32_t* __restrict__ akey, const int32_t* __restrict__ aslot,
-                                    const int32_t* __restrict__ fstart, float4* __restrict__ sorted,
+                                    const int32_t* __restrict__ fstart, unsigned wscale, float4* __restrict__ sorted,
                                     const float* __restrict__ q, float* __restrict__ sorted_q) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int64_t d = fstart[akey[i]] + aslot[i];
-    sorted[d] = packed[i];
+    const int key = akey[i];
+    if (key < 0) return;
+    const int64_t d = fstart[key] + aslot[i];
+    float4 v = packed[i];
+    v.w = __uint_as_float(__float_as_uint(v.w) * wscale);  // species as the pair kernel adds it to addresses
+    sorted[d] = v;
     if (q) sorted_q[d] = q[i];
 }
 
@@ -633,36 +757,13 @@ __global__ void gqq_finish_kernel(const float* __restrict__ q, int64_t n, const 
     for (int k = threadIdx.x; k < lsmax; k += blockDim.x) gqq[k] += gqq_frame[k] / (double)avq2;
 }
 
-// Single-block exclusive scan of int32 counts (length up to a few million).
-__global__ void scan_exclusive_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, int n) {
-    __shared__ int32_t part[1024];
-    int per = (n + blockDim.x - 1) / blockDim.x;
-    int b0 = threadIdx.x * per, b1 = min(n, b0 + per);
-    int32_t s = 0;
-    for (int k = b0; k < b1; ++k) s += in[k];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int off = 1; off < (int)blockDim.x; off <<= 1) {
-        int32_t v = threadIdx.x >= (unsigned)off ? part[threadIdx.x - off] : 0;
-        __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
-    }
-    int32_t run = part[threadIdx.x] - s;
-    for (int k = b0; k < b1; ++k) {
-        out[k] = run;
-        run += in[k];
-    }
-    if (threadIdx.x == blockDim.x - 1) out[n] = part[threadIdx.x];
-}
-
 // Number fluctuations (s2D3_sh, rdf.cuf:489-553): block b draws one point uniformly in the box with
 // the reference's generator and seed (XORWOW, curand_init(b + 12345, 0, 0), b 1-based), counts the
 // atoms within each radius r_k = k*deltar (cumulative over nint(r/deltar) bins, the reference's
 // gi_s(ind:lsmax) += 1) from the cells around it, and adds N_k and N_k^2 to the int64 sums.
-__global__ void s2n_kernel(const float4* __restrict__ sorted, const int32_t* __restrict__ cstart,
-                           const int32_t* __restrict__ ccount, float Lx, float Ly, float Lz, int ncx, int ncy,
-                           int ncz, float side2, float deltar, int lsmax, unsigned long long* __restrict__ gi,
+__global__ void s2n_kernel(const float4* __restrict__ sorted, const int32_t* __restrict__ fstart,
+                           const int32_t* __restrict__ fcount, int nsub, float Lx, float Ly, float Lz, int ncx,
+                           int ncy, int ncz, float side2, float deltar, int lsmax, unsigned long long* __restrict__ gi,
                            unsigned long long* __restrict__ g2i, float* __restrict__ points, int dim) {
     extern __shared__ unsigned long long cnt[];  // lsmax + 1
     __shared__ float pt[3];
@@ -695,9 +796,10 @@ __global__ void s2n_kernel(const float4* __restrict__ sorted, const int32_t* __r
             for (int dz = -rz; dz <= rz; ++dz) {
                 const int cx = (pc[0] + dx + ncx) % ncx, cy = (pc[1] + dy + ncy) % ncy, cz = (pc[2] + dz + ncz) % ncz;
                 const int c = (cx * ncy + cy) * ncz + cz;
-                const int a0 = cstart[c], na = ccount[c];
-                for (int j = threadIdx.x; j < na; j += blockDim.x) {
-                    const float4 a = sorted[a0 + j];
+                for (int sg = threadIdx.x >> 5; sg < nsub; sg += blockDim.x >> 5) {  // a warp per group of the cell
+                  const int j0 = fstart[c * nsub + sg], je = j0 + fcount[c * nsub + sg];
+                  for (int j = j0 + (int)(threadIdx.x & 31u); j < je; j += 32) {
+                    const float4 a = sorted[j];
                     // rdf.cuf:533-541: difference point - atom, minimum image, (x^2 + y^2) + z^2, FP32
                     float xd = __fsub_rn(pt[0], a.x), yd = __fsub_rn(pt[1], a.y), zd = __fsub_rn(pt[2], a.z);
                     xd = __fsub_rn(xd, __fmul_rn(Lx, roundf(__fdiv_rn(xd, Lx))));
@@ -708,6 +810,7 @@ __global__ void s2n_kernel(const float4* __restrict__ sorted, const int32_t* __r
                         const int ind = (int)roundf(__fdiv_rn(__fsqrt_rn(rr2), deltar));
                         if (ind >= 0 && ind <= lsmax) atomicAdd(&cnt[ind], 1ull);
                     }
+                  }
                 }
             }
     __syncthreads();
@@ -738,14 +841,58 @@ __global__ void s2n_kernel(const float4* __restrict__ sorted, const int32_t* __r
 // a CTA keeps the counts of one item in two shared replicas (even and odd warps) and merges them into
 // that item's uint64 histogram when its next unit belongs to another item, and at exit.
 template <bool FLOOR>
+__device__ __forceinline__ void bin_pair(float rr2, float x2, float dy, float dz, int row, const PairGeom& p,
+                                         unsigned* myhist, PairCounters& pc) {
+    const float q = rr2 * rsqrtf(rr2) * p.inv_deltar;
+    // Nearest integer of q by adding and removing 1.5*2^23 (q < 2^22): qb holds it in its low
+    // mantissa bits; d = q - r in [-1/2, 1/2] exactly.
+    const float qb = __fadd_rn(q, 12582912.0f);
+    const float d = __fsub_rn(q, __fsub_rn(qb, 12582912.0f));
+    const float win = fmaf(q, 1.9073486e-6f, 9.5367432e-7f);  // q*2^-19 + 2^-20
+    // distance of q from the nearest bin edge: integers (floor bins) or half-integers (nint bins)
+    const float edge = FLOOR ? fabsf(d) : 0.5f - fabsf(d);
+    int ind;
+    if (rr2 >= p.side2_lo || !(edge > win)) {  // NaN (rr2 == 0) takes this path too
+        const int e = exact_bin(rr2, x2, dy, dz, p.side2, p.deltar, p.lsmax, p.floor_bins);
+        pc.ulp += (e >> 29) & 1;
+        pc.fma += (e >> 30) & 1;
+        ind = e & ((1 << 29) - 1);
+    } else {
+        // Away from an edge, round-to-nearest-even and NINT agree, and floor(q) = r - (d < 0).
+        const int r = __float_as_int(qb) - 0x4B400000;
+        ind = FLOOR ? r + (d > 0.f ? 1 : 0) : r;
+        if (ind > p.lsmax) ind = 0;
+    }
+    if (ind > 0) atomicAdd(&myhist[row * p.lsmax + ind - 1], 1u);
+}
+
+template <bool FLOOR>
+__device__ __forceinline__ void pair(const float4& a, const float4& b, bool valid, int si, const PairGeom& p,
+                                     const int* rowtab, unsigned* myhist, PairCounters& pc) {
+    float dx = __fsub_rn(b.x, a.x);
+    float dy = __fsub_rn(b.y, a.y);
+    float dz = __fsub_rn(b.z, a.z);
+    dx = min_image(dx, p.L[0], p.h1[0], p.h2[0]);
+    dy = min_image(dy, p.L[1], p.h1[1], p.h2[1]);
+    dz = min_image(dz, p.L[2], p.h1[2], p.h2[2]);
+    const float x2 = __fmul_rn(dx, dx);
+    const float rr2 = __fadd_rn(__fadd_rn(x2, __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+    if (valid && rr2 < p.side2_hi) {
+        const int sj = __float_as_int(b.w);
+        if ((unsigned)sj < (unsigned)p.nsp)
+            bin_pair<FLOOR>(rr2, x2, dy, dz, rowtab[si * p.nsp + sj], p, myhist, pc);
+    }
+}
+
+template <bool FLOOR>
 __device__ __forceinline__ unsigned batch_tile_pairs(const float4* __restrict__ tile, int jcount, const float4& a,
-                                                     bool has_a, int il, bool diag, int si, const RdfParams& P,
+                                                     bool has_a, int il, bool diag, int si, const PairGeom& P,
                                                      const int* rowtab, unsigned* myhist, PairCounters& pc) {
     unsigned tested = 0;
     for (int jj = 0; jj < jcount; ++jj) {
         const bool valid = has_a && (!diag || jj > il);
         tested += valid ? 1u : 0u;
-        pair<false, FLOOR, false>(a, tile[jj], valid, si, P, rowtab, myhist, pc, nullptr, 0.f, nullptr);
+        pair<FLOOR>(a, tile[jj], valid, si, P, rowtab, myhist, pc);
     }
     return tested;
 }
@@ -794,7 +941,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(BatchHead
     const int nitems = hdr->nitems;
     const int64_t total = hdr->total_pair;
     int cur = -1;
-    RdfParams P;
+    PairGeom P;
     int n = 0, ntile = 0;
     int64_t off = 0;
     PairCounters pc;
@@ -821,7 +968,6 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(BatchHead
                 P.inv_deltar = it.inv_deltar;
                 P.lsmax = it.lsmax;
                 P.nsp = it.nsp;
-                P.nit = it.nit;
                 P.floor_bins = it.floor_bins;
                 n = it.n;
                 ntile = it.ntile;
@@ -867,19 +1013,19 @@ struct trj_rdf_plan {
     float deltar = 0.f, rcrdf_eff = 0.f, side2 = 0.f;
     int64_t n_max = 0;
     int ncell_cap = 0;
-    int nc[3] = {1, 1, 1};
-    int32_t* ccount = nullptr;  // ncell_cap
-    int32_t* cflag = nullptr;   // ncell_cap: bit 0 a coordinate outside [0, L), bit 1 outside [-L, L)
-    unsigned long long* work = nullptr;  // item counter of the pair kernel
-    int32_t* cstart = nullptr;  // ncell_cap + 1
-    int64_t fine_cap = 0;       // capacity of the per-(cell, sub-cell) arrays
-    int32_t* fcount = nullptr;  // fine_cap
-    int32_t* fstart = nullptr;  // fine_cap + 1
-    int32_t* akey = nullptr;    // n_max: (cell, sub-cell) key per atom
+    int nc[3] = {1, 1, 1};      // cells per axis of the cutoff
+    int64_t key_cap = 0;        // capacity of the per-group arrays
+    int32_t* fstart = nullptr;  // key_cap: first atom of every (cell, group) in `sorted`
+    // Zeroed per frame by one memset: work counter (8 bytes), atoms placed, frame flags, cell flags
+    // (ncell: bit 0 a coordinate outside [0, L), bit 1 outside [-L, L)), atoms per group (nkey).
+    int32_t* zeroed = nullptr;  // 4 + ncell_cap + key_cap
+    int32_t* akey = nullptr;    // n_max: (cell, group) key per atom
     int32_t* aslot = nullptr;   // n_max
+    int grid_nc[3] = {1, 1, 1}, nsub = 1;  // cells and groups per cell of the last accumulated frame
     float4* sorted = nullptr;   // n_max
     float* sorted_q = nullptr;  // n_max charges in cell order (first charged call)
-    int cells_valid = 0;        // sorted/cstart/ccount hold the last accumulated frame
+    int32_t* fcount_last = nullptr;  // atoms per group of the last accumulated frame (in `zeroed`)
+    int cells_valid = 0;        // sorted, fstart and the counts hold the last accumulated frame
     float box_last[3] = {0.f, 0.f, 0.f};
     double* gqq_frame = nullptr;  // lsmax: this frame's charge-product sums
     int64_t scratch_bytes = 0;
@@ -918,6 +1064,127 @@ static void cells_for(const float L[3], float side2, int nc[3], int dim = 3) {
     if (dim == 2) nc[2] = 1;
 }
 
+// Shared memory kept back from the largest histogram a plan may have.
+constexpr size_t kHistReserve = 20480;
+
+// What a pair's test needs, from the frame's box and the plan's cutoff and bins.
+static void fill_geom(PairGeom& g, const float box[3], float side2, float deltar, int lsmax, int nsp, int floor_bins,
+                      bool want_edge) {
+    for (int d = 0; d < 3; ++d) {
+        g.L[d] = box[d];
+        g.inv_L[d] = 1.0f / box[d];
+        g.h1[d] = nint_threshold(box[d], 0.5f);
+        g.h2[d] = nint_threshold(box[d], 1.5f);
+    }
+    g.side2 = side2;
+    g.side2_lo = (float)((double)side2 * (1.0 - 1.0 / 1048576.0));
+    g.side2_hi = (float)((double)side2 * (1.0 + 1.0 / 1048576.0));
+    g.side2_win = fmaxf(g.side2_hi - side2, side2 - g.side2_lo);
+    g.deltar = deltar;
+    g.inv_deltar = 1.0f / deltar;
+    // Window around a bin edge outside which the approximate q has the reference's bin (test_run): 0.34 (with
+    // edge statistics 0.5) x 2^-20 of the largest q of a pair in range, plus 2^-22.  Cutoffs whose squares leave the normal range (and bins
+    // beyond the integer trick) take the exact path throughout.
+    const double qmax = sqrt((double)g.side2_hi) / (double)deltar + 1.0;
+    const double thr = 0.5 - (qmax * (want_edge ? 0.5 : 0.34) / 1048576.0 + 1.0 / 4194304.0);
+    g.edge_thr = (side2 > 1e-30f && thr > 0.0) ? (float)thr : -1.0f;
+    g.lsmax = lsmax;
+    g.nsp = nsp;
+    g.floor_bins = floor_bins;
+    g.row_words = lsmax + 2;
+    g.want_edge = want_edge;
+    g.one = 1.0f;
+}
+
+// Volume (2D: area) of the region within r of a box of edges e: what the homes of one group are tested against.
+static double reach(const double e[3], double r, int dim) {
+    if (dim == 2) return e[0] * e[1] + 2.0 * r * (e[0] + e[1]) + M_PI * r * r;
+    return e[0] * e[1] * e[2] + 2.0 * r * (e[0] * e[1] + e[1] * e[2] + e[2] * e[0]) +
+           M_PI * r * r * (e[0] + e[1] + e[2]) + 4.0 / 3.0 * M_PI * r * r * r;
+}
+
+// Cells (nc, in: the most the cutoff allows) and groups per cell (sub) of an n-atom frame.  A group wants
+// about 28 atoms, one per lane with room for fluctuations: sparse cells are merged (never below 3 per axis)
+// and dense ones divided, into the split of lowest cost = groups x volume tested per group.
+static void choose_groups(int64_t n, const float box[3], double rc, int dim, int64_t key_cap, int nc[3], int sub[3]) {
+    const int nd = dim == 2 ? 2 : 3;
+    double m = (double)n / ((double)nc[0] * nc[1] * nc[2]);
+    if (m < 0.75 * kGroupFill) {
+        const double f = pow(kGroupFill / std::max(m, 1e-3), 1.0 / nd);
+        for (int d = 0; d < nd; ++d)
+            if (nc[d] >= 3) nc[d] = std::max(3, (int)(nc[d] / f));
+        m = (double)n / ((double)nc[0] * nc[1] * nc[2]);
+    }
+    sub[0] = sub[1] = sub[2] = 1;
+    if (m <= kGroupFill) return;
+    double e[3], vol = 1.0;
+    for (int d = 0; d < 3; ++d) e[d] = (double)box[d] / nc[d];
+    for (int d = 0; d < nd; ++d) vol *= e[d];
+    const double ideal = pow(vol * kGroupFill / m, 1.0 / nd);
+    const int64_t most = std::max<int64_t>(1, key_cap / ((int64_t)nc[0] * nc[1] * nc[2]));
+    double best = -1.0;
+    int lo[3], hi[3];
+    for (int d = 0; d < 3; ++d) {
+        lo[d] = d < nd ? std::max(1, (int)(e[d] / ideal) - 1) : 1;
+        hi[d] = d < nd ? std::max(1, (int)(e[d] / ideal) + 2) : 1;
+    }
+    for (int a = lo[0]; a <= hi[0]; ++a)
+        for (int b = lo[1]; b <= hi[1]; ++b)
+            for (int c = lo[2]; c <= hi[2]; ++c) {
+                const double groups = (double)a * b * c;
+                if (m / groups > kGroupFill || groups > (double)most) continue;
+                const double edge[3] = {e[0] / a, e[1] / b, e[2] / c};
+                const double cost = groups * reach(edge, rc, dim);
+                if (best < 0.0 || cost < best) {
+                    best = cost;
+                    sub[0] = a;
+                    sub[1] = b;
+                    sub[2] = c;
+                }
+            }
+}
+
+struct PairShape {
+    int ctas, warps;  // per SM, per CTA
+    bool square;      // a bin row per ordered species pair
+    size_t smem;      // dynamic shared memory of a CTA
+};
+
+// Launch shape of the pair kernel: 32 warps per SM (64 registers a thread) in CTAs of 8 while their
+// histograms fit, then fewer, larger CTAs that share one, then fewer warps.  The square row layout is
+// taken where it does not cost warps.
+static bool pair_shape(const trj_ctx* ctx, int nsp, int nit, int row_words, bool charged, PairShape* out) {
+    static const int kCtas[] = {4, 2, 1, 1, 1, 1, 1};
+    static const int kWarps[] = {8, 16, 32, 24, 16, 8, 4};
+    const size_t optin = ctx->smem_optin, per_sm = optin + 1024;
+    for (int i = 0; i < 7; ++i)
+        for (int square = 1; square >= 0; --square) {
+            const size_t rows = square ? (size_t)nsp * nsp : (size_t)nit;
+            const size_t smem = (size_t)kWarps[i] * kRing * (16 + (charged ? 8 : 0)) +
+                                (size_t)row_words * (4 * rows + (charged ? 8 : 0)) + 16;
+            // the driver's reserve and the static shared memory of a CTA
+            if (smem + 1200 > optin || (smem + 1024 + 1200) * kCtas[i] > per_sm) continue;
+            out->ctas = kCtas[i];
+            out->warps = kWarps[i];
+            out->square = square;
+            out->smem = smem;
+            return true;
+        }
+    return false;
+}
+
+typedef void (*PairKernel)(RdfParams, const float4*, const int32_t*, const int32_t*, const int32_t*, const unsigned*, unsigned*,
+                           u64*, u64*, unsigned*, const float*, double*);
+template <bool FLOOR, bool SQUARE>
+static PairKernel pair_kernel_of(bool charged, bool edge) {
+    return charged ? rdf_pairs_kernel<FLOOR, true, SQUARE, true>
+                   : (edge ? rdf_pairs_kernel<FLOOR, false, SQUARE, true> : rdf_pairs_kernel<FLOOR, false, SQUARE, false>);
+}
+static PairKernel pair_kernel(int floor_bins, bool charged, bool square, bool edge) {
+    if (floor_bins) return square ? pair_kernel_of<true, true>(charged, edge) : pair_kernel_of<true, false>(charged, edge);
+    return square ? pair_kernel_of<false, true>(charged, edge) : pair_kernel_of<false, false>(charged, edge);
+}
+
 static int rdf_plan_create_impl(trj_ctx* ctx, int nsp, float deltar, float rcrdf, const float box[3],
                                 int64_t n_max, int dim, trj_rdf_plan** out) {
     if (!ctx || !out || !box) return TRJ_ERR_INVALID;
@@ -945,7 +1212,7 @@ static int rdf_plan_create_impl(trj_ctx* ctx, int nsp, float deltar, float rcrdf
     p->lsmax = nint_host(rc / deltar) + 1;
     p->n_max = n_max;
     size_t hist_bytes = (size_t)p->nit * p->lsmax * 4;
-    size_t budget = ctx->smem_optin - kSlots * kJChunk * sizeof(float4) - 4096;
+    size_t budget = ctx->smem_optin - kHistReserve;
     if (hist_bytes > budget) {
         delete p;
         return trj_fail(ctx, TRJ_ERR_UNSUPPORTED,
@@ -957,26 +1224,21 @@ static int rdf_plan_create_impl(trj_ctx* ctx, int nsp, float deltar, float rcrdf
     // Room for a box up to 25% smaller per axis (more cells) without re-planning.
     p->ncell_cap = std::max(ncell * 2 + 64, 64);
     trj_device_guard g(ctx->device);
-    // Sub-cell keys: up to 64 per cell, never more entries than atoms (or cells).
-    p->fine_cap = std::max<int64_t>(p->ncell_cap, std::min<int64_t>((int64_t)p->ncell_cap * 64, n_max));
-    size_t bytes = 64 + sizeof(int32_t) * (size_t)(3 * p->ncell_cap + 1) +
-                   sizeof(int32_t) * (size_t)(2 * p->fine_cap + 1) +
-                   (sizeof(int32_t) * 2 + sizeof(float4)) * (size_t)std::max<int64_t>(n_max, 1);
+    // Groups: one per cell, or at least 16 atoms per group on average (choose_groups).
+    p->key_cap = (int64_t)p->ncell_cap + n_max / 16 + 64;
+    const size_t na = (size_t)std::max<int64_t>(n_max, 1);
+    size_t bytes = 64 + sizeof(int32_t) * (size_t)(4 + p->ncell_cap + 2 * p->key_cap) +
+                   (sizeof(int32_t) * 2 + sizeof(float4)) * na;
     char* base = nullptr;
     if (trj_dev_alloc(ctx, (void**)&base, bytes + 256) != cudaSuccess) {
         delete p;
         return trj_fail(ctx, TRJ_ERR_NOMEM, "rdf plan: %zu bytes of scratch", bytes);
     }
     p->sorted = reinterpret_cast<float4*>(base);
-    p->akey = reinterpret_cast<int32_t*>(p->sorted + std::max<int64_t>(n_max, 1));
-    p->aslot = p->akey + std::max<int64_t>(n_max, 1);
-    p->ccount = p->aslot + std::max<int64_t>(n_max, 1);
-    p->cstart = p->ccount + p->ncell_cap;
-    p->cflag = p->cstart + p->ncell_cap + 1;
-    p->fcount = p->cflag + p->ncell_cap;
-    p->fstart = p->fcount + p->fine_cap;
-    p->work = reinterpret_cast<unsigned long long*>(
-        (reinterpret_cast<uintptr_t>(p->fstart + p->fine_cap + 1) + 15) & ~(uintptr_t)15);
+    p->akey = reinterpret_cast<int32_t*>(p->sorted + na);
+    p->aslot = p->akey + na;
+    p->zeroed = reinterpret_cast<int32_t*>((reinterpret_cast<uintptr_t>(p->aslot + na) + 15) & ~(uintptr_t)15);
+    p->fstart = p->zeroed + 4 + p->ncell_cap + p->key_cap;
     p->scratch_bytes = (int64_t)bytes;
     *out = p;
     return TRJ_OK;
@@ -1089,31 +1351,33 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
 
     RdfParams P;
     memset(&P, 0, sizeof(P));
-    for (int d = 0; d < 3; ++d) {
-        P.L[d] = box[d];
-        P.h1[d] = nint_threshold(box[d], 0.5f);
-        P.h2[d] = nint_threshold(box[d], 1.5f);
-    }
-    P.side2 = plan->side2;
-    P.side2_lo = (float)((double)plan->side2 * (1.0 - 1.0 / 1048576.0));
-    P.side2_hi = (float)((double)plan->side2 * (1.0 + 1.0 / 1048576.0));
-    P.deltar = plan->deltar;
-    P.inv_deltar = 1.0f / plan->deltar;
-    P.lsmax = plan->lsmax;
-    P.floor_bins = plan->floor_bins;
+    fill_geom(P.g, box, plan->side2, plan->deltar, plan->lsmax, plan->nsp, plan->floor_bins, edge_dev != nullptr);
     P.wait_clocks = plan->wait_clocks;
     P.stall_test = plan->stall_test;
-    P.nsp = plan->nsp;
     P.nit = plan->nit;
     cells_for(box, plan->side2, P.nc, plan->dim);
-    P.ncell = P.nc[0] * P.nc[1] * P.nc[2];
-    if (P.ncell > plan->ncell_cap)
-        return trj_fail(ctx, TRJ_ERR_CAPACITY, "rdf accumulate: %d cells exceed plan capacity %d", P.ncell,
-                        plan->ncell_cap);
     for (int d = 0; d < 3; ++d) {
         plan->nc[d] = P.nc[d];
         plan->box_last[d] = box[d];
     }
+    if (P.nc[0] * P.nc[1] * P.nc[2] > plan->ncell_cap)
+        return trj_fail(ctx, TRJ_ERR_CAPACITY, "rdf accumulate: %d cells exceed plan capacity %d",
+                        P.nc[0] * P.nc[1] * P.nc[2], plan->ncell_cap);
+    choose_groups(n, box, plan->rcrdf_eff, plan->dim, plan->key_cap, P.nc, P.sub);
+    const int ncell = P.nc[0] * P.nc[1] * P.nc[2];
+    P.nsub = P.sub[0] * P.sub[1] * P.sub[2];
+    const int nkey = ncell * P.nsub;
+    // Cull radius 2^-10 above the cutoff (the exact test needs rr2 < side2*(1 + 2^-20)); the pad,
+    // 2^-16 of the largest edge, exceeds the rounding of the box and gap arithmetic (a few ulps of
+    // coordinates below 2L).
+    P.cull2 = (float)((double)plan->side2 * (1.0 + 1.0 / 1024.0) * (1.0 + 1.0 / 1024.0));
+    P.cull_pad = (float)((double)std::max(box[0], std::max(box[1], box[2])) / 65536.0);
+    for (int d = 0; d < 3; ++d) {
+        P.inv_sub[d] = 1.0f / (float)P.sub[d];
+        P.edge[d] = box[d] / (float)P.nc[d];
+        P.half[d] = 0.5f * P.edge[d] / (float)P.sub[d] + P.cull_pad;
+    }
+    P.split_all = P.nc[0] >= 3 && P.nc[1] >= 3 && (P.nc[2] >= 3 || plan->dim == 2);
     // Half-shell stencil over the split axes: (0,0,0) first, then offsets > 0 lexicographically.
     int no = 0;
     P.off[no][0] = P.off[no][1] = P.off[no][2] = 0;
@@ -1130,81 +1394,49 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
                 ++no;
             }
     P.noff = no;
-    double avg = (double)n / P.ncell;
-    P.hsplit = std::max(1, (int)ceil(avg / kHomeChunk));
-    // No minimum image needed away from the wrap (2D: z differences are 0, z is never wrapped).
-    P.fast_ok = P.nc[0] >= 5 && P.nc[1] >= 5 && (P.nc[2] >= 5 || plan->dim == 2);
-    // Cull radius 2^-10 above the cutoff (the exact test needs rr2 < side2*(1 + 2^-20)); the pad,
-    // 2^-16 of the largest edge, exceeds the rounding of the box and gap arithmetic (a few ulps of
-    // coordinates below 2L).
-    P.cull2 = (float)((double)plan->side2 * (1.0 + 1.0 / 1024.0) * (1.0 + 1.0 / 1024.0));
-    P.cull_pad = (float)((double)std::max(box[0], std::max(box[1], box[2])) / 65536.0);
-    // Split neighbour ranges when there are too few (cell, offset, home chunk) items to fill the GPU.
-    int64_t base_items = (int64_t)P.ncell * P.noff * P.hsplit;
-    int64_t want = (int64_t)ctx->sm_count * 4;
-    P.jsplit = (int)std::max<int64_t>(1, std::min<int64_t>(64, (want + base_items - 1) / base_items));
-    P.nitems = base_items * P.jsplit;
+    // Launch shape: as many warps per SM as the histogram leaves room for, with a row per ordered species
+    // pair where that costs no warps.
+    PairShape shape;
+    if (!pair_shape(ctx, plan->nsp, plan->nit, P.g.row_words, charged, &shape))
+        return trj_fail(ctx, TRJ_ERR_UNSUPPORTED, "rdf accumulate: histogram too large");
+    // Segments: about twelve items per resident warp, so that the last ones end together (six: 62,500 atoms
+    // 485 us instead of 455; twenty-four: 459), but at least six neighbour groups per item.
+    const int64_t warps = (int64_t)ctx->sm_count * shape.ctas * shape.warps;
+    const int64_t list = (int64_t)P.noff * P.nsub;
+    P.nseg = (int)std::max<int64_t>(1, std::min<int64_t>((12 * warps + nkey - 1) / nkey, list / 6));
+    P.per_seg = (int)((list + P.nseg - 1) / P.nseg);
+    P.nitems = (unsigned)nkey * (unsigned)P.nseg;  // below 2^32: nseg > 1 only for few keys
 
-    // Shared memory: two staging buffers + histogram replicas (+ FP64 charge replicas).
-    size_t hist_bytes = (size_t)P.nit * P.lsmax * 4 + (charged ? (size_t)P.lsmax * 8 + 8 : 0);
-    size_t stage = kSlots * kJChunk * sizeof(float4);
-    size_t optin = ctx->smem_optin;
-    // Most CTAs per SM (up to 4, i.e. 32 warps) that still hold >= 2 histogram replicas each;
-    // a single CTA per SM otherwise.
-    const size_t sm_smem = optin + 1024;  // per-SM shared memory (the opt-in limit plus the driver's block reserve)
-    int ctas_per_sm = 1, nrep = 0;
-    for (int k = 4; k >= 2; --k) {
-        size_t per_cta = sm_smem / k - 1024 - 2048;  // driver reserve + static shared memory
-        int r = per_cta > stage ? (int)std::min<size_t>(8, (per_cta - stage) / hist_bytes) : 0;
-        if (r >= 2) {
-            ctas_per_sm = k;
-            nrep = r;
-            break;
-        }
-    }
-    if (nrep < 2) nrep = (int)std::min<size_t>(8, (optin - 2048 - stage) / hist_bytes);
-    if (nrep < 1) return trj_fail(ctx, TRJ_ERR_UNSUPPORTED, "rdf accumulate: histogram too large");
-    P.nrep = nrep;
-    size_t smem = stage + (size_t)nrep * hist_bytes;
-    void (*kern)(RdfParams, const float4*, const int32_t*, const int32_t*, const int32_t*, const int32_t*,
-                 unsigned long long*, unsigned long long*, unsigned long long*, unsigned*, const float*, double*) =
-        plan->floor_bins ? (charged ? rdf_pairs_kernel<true, true> : rdf_pairs_kernel<true, false>)
-                         : (charged ? rdf_pairs_kernel<false, true> : rdf_pairs_kernel<false, false>);
-    TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const PairKernel kern = pair_kernel(plan->floor_bins, charged, shape.square, edge_dev != nullptr);
+    TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem));
 
-    // Sub-cells per cell axis: 4 (64 per cell) from 128 atoms per cell on, 2 from 16 on, within the
-    // key capacity.
-    const double per_cell = (double)n / P.ncell;
-    int sbits = per_cell >= 128.0 ? 2 : (per_cell >= 16.0 ? 1 : 0);
-    while (sbits > 0 && ((int64_t)P.ncell << (3 * sbits)) > plan->fine_cap) --sbits;
-    const int nkey = P.ncell << (3 * sbits);
-    P.sbits = sbits;
-
-    // Cell binning: count, scan over cells, sub-cell offsets, scatter.
-    TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->fcount, 0, sizeof(int32_t) * nkey, s));
-    TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->ccount, 0, sizeof(int32_t) * P.ncell, s));
-    TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->cflag, 0, sizeof(int32_t) * P.ncell, s));
-    TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->work, 0, sizeof(unsigned long long), s));
+    // Cell binning: count, group offsets, scatter.
+    unsigned* work = reinterpret_cast<unsigned*>(plan->zeroed);
+    int32_t* total = plan->zeroed + 2;
+    unsigned* fflag = reinterpret_cast<unsigned*>(plan->zeroed + 3);
+    int32_t* cflag = plan->zeroed + 4;
+    int32_t* fcount = cflag + ncell;
+    plan->fcount_last = fcount;
+    plan->nsub = P.nsub;
+    for (int d = 0; d < 3; ++d) plan->grid_nc[d] = P.nc[d];
+    TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->zeroed, 0, sizeof(int32_t) * (size_t)(4 + ncell + nkey), s));
     unsigned nb = (unsigned)((n + 255) / 256);
-    cell_assign_kernel<<<nb, 256, 0, s>>>((const float4*)packed_dev, n, box[0], box[1], box[2], P.nc[0],
-                                          P.nc[1], P.nc[2], sbits, plan->fcount, plan->ccount, plan->cflag,
-                                          plan->akey, plan->aslot);
-    scan_exclusive_kernel<<<1, 1024, 0, s>>>(plan->ccount, plan->cstart, P.ncell);
-    sub_offsets_kernel<<<(unsigned)((P.ncell + 7) / 8), 256, 0, s>>>(plan->fcount, plan->cstart, P.ncell, sbits,
-                                                                    plan->fstart);
+    cell_assign_kernel<<<nb, 256, 0, s>>>((const float4*)packed_dev, n, P, fcount, cflag, fflag, plan->akey,
+                                          plan->aslot);
+    group_offsets_kernel<<<(unsigned)((nkey + 255) / 256), 256, 0, s>>>(fcount, nkey, total, plan->fstart);
     cell_scatter_kernel<<<nb, 256, 0, s>>>((const float4*)packed_dev, n, plan->akey, plan->aslot, plan->fstart,
-                                           plan->sorted, charged ? charge_dev : nullptr, plan->sorted_q);
+                                           shape.square ? 4u * (unsigned)P.g.row_words : 64u, plan->sorted, charged ? charge_dev : nullptr, plan->sorted_q);
     if (charged) TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->gqq_frame, 0, sizeof(double) * plan->lsmax, s));
-    int64_t grid = std::min<int64_t>((int64_t)ctx->sm_count * ctas_per_sm, P.nitems);
+    const int64_t grid = std::min<int64_t>((int64_t)ctx->sm_count * shape.ctas,
+                                           ((int64_t)P.nitems + shape.warps - 1) / shape.warps);
     plan->timer.begin(ctx, s);
-    kern<<<(unsigned)grid, kThreads, smem, s>>>(P, plan->sorted, plan->cstart, plan->ccount, plan->cflag, plan->fstart,
-                                                plan->work,
-                                                (unsigned long long*)hist_dev, (unsigned long long*)edge_dev,
-                                                ctx->status_dev, charged ? plan->sorted_q : nullptr,
-                                                charged ? plan->gqq_frame : nullptr);
+    kern<<<(unsigned)grid, shape.warps * 32, shape.smem, s>>>(P, plan->sorted, plan->fstart, fcount, cflag, fflag, work,
+                                                              (u64*)hist_dev, (u64*)edge_dev, ctx->status_dev,
+                                                              charged ? plan->sorted_q : nullptr,
+                                                              charged ? plan->gqq_frame : nullptr);
     plan->timer.end(ctx, s);
     plan->cells_valid = 1;
-    ctx->launches += 5;
+    ctx->launches += 4;
     if (charged) {
         gqq_finish_kernel<<<1, 1024, 0, s>>>(charge_dev, n, plan->gqq_frame, plan->lsmax, gqq_dev);
         ctx->launches += 1;
@@ -1243,8 +1475,8 @@ extern "C" int trj_rdf_s2n(trj_rdf_plan* plan, int nrandom, uint64_t* gi_dev, ui
     if (smem > 48 * 1024)
         TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(s2n_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     s2n_kernel<<<(unsigned)nrandom, 256, smem, (cudaStream_t)stream>>>(
-        plan->sorted, plan->cstart, plan->ccount, plan->box_last[0], plan->box_last[1], plan->box_last[2],
-        plan->nc[0], plan->nc[1], plan->nc[2], plan->side2, plan->deltar, plan->lsmax,
+        plan->sorted, plan->fstart, plan->fcount_last, plan->nsub, plan->box_last[0], plan->box_last[1],
+        plan->box_last[2], plan->grid_nc[0], plan->grid_nc[1], plan->grid_nc[2], plan->side2, plan->deltar, plan->lsmax,
         (unsigned long long*)gi_dev, (unsigned long long*)g2i_dev, points_dev, plan->dim);
     ctx->launches += 1;
     TRJ_CUDA_TRY(ctx, cudaGetLastError());

@@ -151,8 +151,8 @@ class RdfPlan:
               "trj_rdf_plan_set_binning")
 
     def set_wait(self, clocks: int = 0, stall_test: bool = False) -> None:
-        """Limit (SM clocks, 0 = default) of the pair kernel's waits for staged chunks; stall_test makes
-        every launch run out of it once (see trj_rdf_plan_set_wait)."""
+        """stall_test makes every launch of the pair kernel run out of a bounded wait of ``clocks`` SM clocks
+        (0 = default; see trj_rdf_plan_set_wait)."""
         check(self.ctx.lib.trj_rdf_plan_set_wait(self.h, int(clocks), 1 if stall_test else 0), self.ctx.h,
               "trj_rdf_plan_set_wait")
 
