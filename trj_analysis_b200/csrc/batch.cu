@@ -202,7 +202,7 @@ extern "C" int trj_batch_add(trj_batch* b, int buf, trj_rdf_plan* rdf, trj_sq_pl
     h->total_chunk += it.nchunk;
     h->total_pair += (int64_t)it.ntile * (it.ntile + 1) / 2;
     if (sq && it.nvec > 0) {
-        h->total_sq += (int64_t)it.nvblk * it.nsplit;
+        h->total_sq += (int64_t)it.nvblk * it.nsplit * it.parts;
         h->total_red += it.nbins;
     }
     h->total_atoms += n;
@@ -228,7 +228,7 @@ extern "C" int trj_batch_launch(trj_batch* b, int buf, void* stream) {
     trj_batch_launch_layout(hdr, items, B.xyz_map, B.sp_map, B.raw, B.chunk_counts, B.packed, B.phase,
                             ctx->status_dev, b->grid_layout, s);
     trj_batch_launch_pairs(hdr, items, B.packed, b->hist_words, b->grid_pairs, s);
-    trj_batch_launch_sq(hdr, items, B.phase, b->grid_sq, b->grid_red, s);
+    trj_batch_launch_sq(hdr, items, B.phase, ctx->turn_dev, b->grid_sq, b->grid_red, s);
     b->timer.end(ctx, s);
     ctx->launches += 5;
     TRJ_CUDA_TRY(ctx, cudaGetLastError());

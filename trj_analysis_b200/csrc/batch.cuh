@@ -37,12 +37,12 @@ struct __align__(16) BatchItem {
     const double* w;
     const int32_t* bin_start;
     const int64_t* sp_off_dev;
-    double2* part;                       // [nsplit][nsp][nvec]
+    double2* part;                       // [nsplit * parts][nsp][nvec]
     double2* rho;                        // [nsp][nvec]
     double* out;                         // [nbins][nit] accumulator
     int32_t nvec, nsplit, vpt, nbins;
-    int32_t nvblk;                       // vector blocks: ceil(nvec / (kBatchThreads * vpt))
-    int32_t pad0;
+    int32_t nvblk;                       // vector blocks of the direct sum
+    int32_t parts, tv, tg;               // rest of its shape (sq.cu PlainShape)
     // first work unit of the item in each kernel's list
     int64_t chunk_begin, pair_begin, sq_begin, red_begin;
 };
@@ -78,8 +78,8 @@ void trj_batch_launch_pairs(BatchHeader* hdr, const BatchItem* items, const floa
 size_t trj_batch_pairs_smem(int hist_words);                                                  // rdf.cu
 int trj_batch_pairs_prepare(int hist_words);                                                  // rdf.cu
 int trj_batch_pairs_occupancy(int hist_words, int* per_sm);                                   // rdf.cu
-void trj_batch_launch_sq(BatchHeader* hdr, const BatchItem* items, const uint4* phase, int grid_sq, int grid_red,
-                         cudaStream_t s);                                                     // sq.cu
+void trj_batch_launch_sq(BatchHeader* hdr, const BatchItem* items, const uint4* phase, const float2* turn, int grid_sq,
+                         int grid_red, cudaStream_t s);                                       // sq.cu
 int trj_batch_sq_occupancy(int* per_sm_sq, int* per_sm_red);                                   // sq.cu
 struct trj_rdf_plan;
 struct trj_sq_plan;

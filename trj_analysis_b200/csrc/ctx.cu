@@ -22,6 +22,14 @@ int trj_fail(trj_ctx* ctx, int code, const char* fmt, ...) {
     return code;
 }
 
+namespace {
+__global__ void turn_table_kernel(float2* turn) {
+    double s, c;
+    sincospi((double)threadIdx.x / 128.0, &s, &c);
+    turn[threadIdx.x] = make_float2((float)c, (float)s);
+}
+}  // namespace
+
 extern "C" int trj_abi_version(void) { return TRJ_ABI_VERSION; }
 
 extern "C" int trj_ctx_create(int device, trj_ctx** out) {
@@ -48,13 +56,16 @@ extern "C" int trj_ctx_create(int device, trj_ctx** out) {
     }
     ctx->sm_count = prop.multiProcessorCount;
     ctx->smem_optin = prop.sharedMemPerBlockOptin;
-    if (cudaMalloc(&ctx->status_dev, 8 * sizeof(unsigned)) != cudaSuccess ||
+    // status words, then the 256-entry turn table of the direct sums
+    if (cudaMalloc(&ctx->status_dev, 8 * sizeof(unsigned) + 256 * sizeof(float2)) != cudaSuccess ||
         cudaMallocHost(&ctx->status_host, 8 * sizeof(unsigned)) != cudaSuccess) {
         if (ctx->status_dev) cudaFree(ctx->status_dev);
         delete ctx;
         return TRJ_ERR_NOMEM;
     }
     cudaMemset(ctx->status_dev, 0, 8 * sizeof(unsigned));
+    ctx->turn_dev = reinterpret_cast<float2*>(ctx->status_dev + 8);
+    turn_table_kernel<<<1, 256>>>(ctx->turn_dev);
     cudaDeviceSynchronize();
     *out = ctx;
     return TRJ_OK;

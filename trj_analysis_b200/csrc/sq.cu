@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "batch.cuh"
@@ -23,10 +24,39 @@
 
 namespace {
 
-constexpr int kPlainThreads = 256;
-constexpr int kPlainVPT = 4;           // k-vectors per thread
-constexpr int kPlainChunk = 1024;      // atoms staged per pass
-constexpr int kPlainSub = 64;          // FP32 partial-sum length before the FP64 add
+constexpr int kPlainThreads = 256;     // most threads of a direct-sum block
+constexpr int kPlainSub = 64;          // atoms of an FP32 partial sum before the FP64 add ("run")
+constexpr int kPlainSlice = 2048;      // least atoms of a slice (see plain_shape)
+constexpr int kPlainStage = 512;       // atoms staged per pass, at most
+constexpr int kPlainCtas = 4;          // direct-sum blocks of 256 threads per SM
+constexpr int kTurnCopies = 16;        // copies of the turn table in shared memory, one per lane of a half-warp
+
+typedef unsigned long long u64;
+
+// Packed FP32: two independent IEEE operations per instruction, each rounded to nearest once.
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ u64 pack2(float lo, float hi) {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
 
 // Fixed-point phase coordinates of every atom.  With charges (q non-null) every atom is written a
 // second time at n + i as a member of the charge species qsp, its charge (FP32 bits) in place of the
@@ -45,128 +75,213 @@ __global__ void phase_coords_kernel(const float4* __restrict__ packed, int64_t n
     if (q) out[n + i] = make_uint4(u[0], u[1], u[2], __float_as_uint(q[i]));
 }
 
-// cos and sin of the angle 2 pi ph / 2^32 (ph a 32-bit fixed-point fraction of a turn): the nearest of
-// 256 table angles (the table holds cos, sin of 2 pi k / 256, each rounded once from FP64), rotated by the
-// remainder |theta| <= pi/256 through its Taylor polynomials (theta - theta^3/6; 1 - theta^2/2 +
-// theta^4/24, truncation below 3e-12).  Every step rounds to nearest once, so the error has no
-// systematic part, which matters because it is added once per atom.
-__device__ __forceinline__ void sincos_turn(unsigned ph, const float2* __restrict__ tab, float& sn, float& cs) {
-    const unsigned hi = (ph + 0x800000u) >> 24;         // nearest table angle (mod 256)
-    const int lo = (int)(ph - (hi << 24));               // remainder in [-2^23, 2^23): exact as a float
-    const float th = (float)lo * 1.4629180792671596e-09f;  // 2 pi / 2^32
-    const float t2 = th * th;
-    const float sl = th * fmaf(t2, -0.16666667f, 1.0f);
-    const float cl = fmaf(t2, fmaf(t2, 0.041666668f, -0.5f), 1.0f);
-    const float2 t = tab[hi & 255u];
-    cs = fmaf(t.x, cl, -(t.y * sl));
-    sn = fmaf(t.y, cl, t.x * sl);
+// Terms of two vectors for one atom: cos and sin of the angles 2 pi ph / 2^32 (ph a 32-bit fixed-point
+// fraction of a turn): the nearest of 256 table angles (cos, sin of 2 pi k / 256, each rounded once from
+// FP64), rotated by the remainder |theta| <= pi/256 through its Taylor polynomials (theta - theta^3/6;
+// 1 - theta^2/2 + theta^4/24, truncation below 3e-12).  Every step rounds to nearest once, so the error has
+// no systematic part, which matters because it is added once per atom.  `tab` is this lane's column of the
+// replicated table (lanes of a half-warp read different banks).
+__device__ __forceinline__ void terms2(unsigned pa, unsigned pb, const char* tab, u64& ta, u64& tb) {
+    // remainder in [-2^23, 2^23): the low 24 bits, sign-extended (exact as a float)
+    const float fa = (float)((int)(pa << 8) >> 8), fb = (float)((int)(pb << 8) >> 8);
+    const u64 th = mul2(pack2(fa, fb), pack2(1.4629180792671596e-09f, 1.4629180792671596e-09f));  // 2 pi / 2^32
+    const u64 t2 = mul2(th, th), one = pack2(1.0f, 1.0f);
+    const u64 sl = mul2(th, fma2(t2, pack2(-0.16666667f, -0.16666667f), one));
+    const u64 cl = fma2(t2, fma2(t2, pack2(0.041666668f, 0.041666668f), pack2(-0.5f, -0.5f)), one);
+    float sa, sb, ca, cb;
+    unpack2(sl, sa, sb);
+    unpack2(cl, ca, cb);
+    // nearest table angle, times the 128 bytes of an entry's copies
+    const float2 A = *reinterpret_cast<const float2*>(tab + (((pa + 0x800000u) >> 17) & 0x7f80u));
+    const float2 B = *reinterpret_cast<const float2*>(tab + (((pb + 0x800000u) >> 17) & 0x7f80u));
+    ta = pack2(__fmaf_rn(A.x, ca, -__fmul_rn(A.y, sa)), __fmaf_rn(A.y, ca, __fmul_rn(A.x, sa)));
+    tb = pack2(__fmaf_rn(B.x, cb, -__fmul_rn(B.y, sb)), __fmaf_rn(B.y, cb, __fmul_rn(B.x, sb)));
 }
 
-// cos, sin(2 pi k / 256), k = 0..255, each rounded once from FP64 (the table of sincos_turn).
-__device__ __forceinline__ void fill_turn_table(float2* turn_tab) {
-    for (int k = threadIdx.x; k < 256; k += blockDim.x) {
-        double sd, cd;
-        sincospi((double)k / 128.0, &sd, &cd);
-        turn_tab[k] = make_float2((float)cd, (float)sd);
+// Shape of a direct sum.  A slice (of nsplit) is the unit of the FP32 partial sums: runs of 64 atoms are
+// counted from its start within each species; parts cut a slice's runs further, between blocks.  A block
+// takes tv threads x VPT vectors and walks tg runs at a time (tv * tg <= 256 threads).
+struct PlainShape {
+    int vpt, tv, tg, nvblk, nsplit, parts;
+};
+
+// Shared memory of a direct-sum block: replicated turn table, staged atoms, FP64 sums of the tg > 1 threads.
+struct PlainSmem {
+    float2 turn[256 * kTurnCopies];
+    union {
+        uint4 atoms[kPlainStage];
+        double2 red[kPlainThreads];
+    };
+};
+
+__device__ __forceinline__ void fill_turn_table(PlainSmem& sm, const float2* __restrict__ turn) {
+    for (int k = threadIdx.x; k < 256 * kTurnCopies / 2; k += blockDim.x) {  // two copies per 16-byte store
+        const float2 t = turn[k / (kTurnCopies / 2)];
+        reinterpret_cast<float4*>(sm.turn)[k] = make_float4(t.x, t.y, t.x, t.y);
     }
 }
 
-// Direct sum of one block of vectors (bx) over one slice (by of nsplit) of every species: thread owns
-// VPT vectors.  Species qsp (if any) is the charge species: each term is weighted by the charge in the
-// entry's w.  Partials by position in the subset: part[by][species][nsub].  turn_tab must be filled
-// (fill_turn_table) before the call; the barrier at the top of the chunk loop orders it.
+// Sums of one block of vectors (bx) over one part (by = slice * parts + part) of every species.  Species qsp
+// (if any) is the charge species: each term is weighted by the charge in the entry's w.  Partials by position
+// in the subset: part[by][species][nsub].  The turn table must be filled; the first barrier orders it.
+//
+// What bounds it: the FP32 pipes and the issue slots they take (22 instructions, 25 clocks per term and
+// scheduler in a loop of nothing else: 1.46e12 terms/s; all-scalar FP32 27 clocks, without the integer
+// multiply-adds of the phase 22.7).  One copy of the table had a lane's load conflict with three to six
+// others'.  62,500 atoms x 14,116 vectors: 846 -> 700 us; 1e6 atoms x 363 vectors: 538 -> 360 us;
+// 16,379 atoms with the reference's vectors, where eight slices left most SMs idle: 144 -> 43 us; 4,000 atoms,
+// one slice: 235 -> 12 us.
 template <int VPT>
 __device__ __forceinline__ void plain_block(const uint4* __restrict__ phase, const int64_t* __restrict__ sp_off,
                                             int nsp, int qsp, const int4* __restrict__ vecs,
-                                            const int32_t* __restrict__ subset, int nsub, int nsplit,
-                                            double2* __restrict__ part, int64_t bx, int64_t by, uint4* atoms,
-                                            const float2* turn_tab) {
-    const int tid = threadIdx.x;
-    const int64_t vbase = bx * kPlainThreads * VPT;
+                                            const int32_t* __restrict__ subset, int nsub, const PlainShape& shape,
+                                            double2* __restrict__ part, int64_t bx, int64_t by, PlainSmem& sm) {
+    const int tid = threadIdx.x, tv = shape.tv, tg = shape.tg;
+    const int g = tid / tv, v = tid - g * tv;  // run lane and vector lane; g >= tg: a thread that only stages
+    const int stage_runs = kPlainStage / kPlainSub / tg * tg;  // runs staged at a time: a multiple of tg
+    const bool busy = g < tg;
+    const char* tab = reinterpret_cast<const char*>(sm.turn + (tid & (kTurnCopies - 1)));
+    const int64_t vbase = bx * tv * VPT + v;
     unsigned nx[VPT], ny[VPT], nz[VPT];
-    int vidx[VPT];
 #pragma unroll
     for (int q = 0; q < VPT; ++q) {
-        int64_t s = vbase + q * kPlainThreads + tid;
-        vidx[q] = s < nsub ? subset[s] : -1;
-        int4 v = vidx[q] >= 0 ? vecs[vidx[q]] : make_int4(0, 0, 0, 0);
-        nx[q] = (unsigned)v.x;
-        ny[q] = (unsigned)v.y;
-        nz[q] = (unsigned)v.z;
+        const int64_t s = vbase + (int64_t)q * tv;
+        const int4 n = busy && s < nsub ? vecs[subset[s]] : make_int4(0, 0, 0, 0);
+        nx[q] = (unsigned)n.x;
+        ny[q] = (unsigned)n.y;
+        nz[q] = (unsigned)n.z;
     }
+    const int64_t slice = by / shape.parts, cut = by - slice * shape.parts;
     for (int a = 0; a < nsp; ++a) {
-        int64_t a0 = sp_off[a], a1 = sp_off[a + 1];
-        int64_t len = a1 - a0;
-        int64_t s0 = a0 + len * by / nsplit, s1 = a0 + len * (by + 1) / nsplit;
+        const int64_t a0 = sp_off[a], len = sp_off[a + 1] - a0;
+        const int64_t s0 = a0 + len * slice / shape.nsplit, s1 = a0 + len * (slice + 1) / shape.nsplit;
+        const int64_t runs = (s1 - s0 + kPlainSub - 1) / kPlainSub;
+        const int64_t r0 = runs * cut / shape.parts, r1 = runs * (cut + 1) / shape.parts;
         double accr[VPT], acci[VPT];
 #pragma unroll
         for (int q = 0; q < VPT; ++q) accr[q] = acci[q] = 0.0;
         const bool weighted = a == qsp;
-        for (int64_t c0 = s0; c0 < s1; c0 += kPlainChunk) {
-            int cnt = (int)((s1 - c0) < (int64_t)kPlainChunk ? (s1 - c0) : (int64_t)kPlainChunk);
+        for (int64_t r = r0; r < r1; r += stage_runs) {
+            const int64_t c0 = s0 + r * kPlainSub, c1 = min(s1, s0 + min(r + stage_runs, r1) * kPlainSub);
+            const int cnt = (int)(c1 - c0);
             __syncthreads();
-            for (int k = tid; k < cnt; k += kPlainThreads) atoms[k] = phase[c0 + k];
+            for (int k = tid; k < cnt; k += blockDim.x) sm.atoms[k] = phase[c0 + k];
             __syncthreads();
-            for (int j0 = 0; j0 < cnt; j0 += kPlainSub) {
-                int j1 = min(cnt, j0 + kPlainSub);
-                float fr[VPT], fi[VPT];
+            for (int j0 = busy ? g * kPlainSub : cnt; j0 < cnt; j0 += tg * kPlainSub) {
+                const int j1 = min(cnt, j0 + kPlainSub);
+                u64 f[VPT];
 #pragma unroll
-                for (int q = 0; q < VPT; ++q) fr[q] = fi[q] = 0.f;
-                for (int j = j0; j < j1; ++j) {
-                    uint4 u = atoms[j];
-                    const float w = weighted ? __uint_as_float(u.w) : 1.0f;  // fma with 1: the plain sum
+                for (int q = 0; q < VPT; ++q) f[q] = 0ull;
+                auto walk = [&](auto has_weight) {
+#pragma unroll 2
+                    for (int j = j0; j < j1; ++j) {
+                        const uint4 u = sm.atoms[j];
+                        const u64 w = pack2(__uint_as_float(u.w), __uint_as_float(u.w));
 #pragma unroll
-                    for (int q = 0; q < VPT; ++q) {
-                        unsigned ph = nx[q] * u.x + ny[q] * u.y + nz[q] * u.z;
-                        // an unbiased sine/cosine: a biased fast one adds its mean error once per
-                        // atom, which at 10^6 atoms is a few 1e-5 of |rho|^2 on a shell of three vectors
-                        float sn, cs;
-                        sincos_turn(ph, turn_tab, sn, cs);
-                        fr[q] = fmaf(w, cs, fr[q]);
-                        fi[q] = fmaf(w, sn, fi[q]);
+                        for (int q = 0; q < VPT; q += 2) {
+                            u64 ta, tb;
+                            terms2(nx[q] * u.x + ny[q] * u.y + nz[q] * u.z,
+                                   nx[q + 1] * u.x + ny[q + 1] * u.y + nz[q + 1] * u.z, tab, ta, tb);
+                            f[q] = has_weight ? fma2(w, ta, f[q]) : add2(f[q], ta);
+                            f[q + 1] = has_weight ? fma2(w, tb, f[q + 1]) : add2(f[q + 1], tb);
+                        }
                     }
-                }
+                };
+                if (weighted) walk(std::true_type());
+                else walk(std::false_type());
 #pragma unroll
                 for (int q = 0; q < VPT; ++q) {
-                    accr[q] += (double)fr[q];
-                    acci[q] += (double)fi[q];
+                    float re, im;
+                    unpack2(f[q], re, im);
+                    accr[q] += (double)re;
+                    acci[q] += (double)im;
                 }
             }
         }
 #pragma unroll
-        for (int q = 0; q < VPT; ++q)
-            if (vidx[q] >= 0)  // partials by position in the subset: [split][species][nsub]
-                part[(by * nsp + a) * nsub + vbase + q * kPlainThreads + tid] = make_double2(accr[q], acci[q]);
+        for (int q = 0; q < VPT; ++q) {
+            double2 sum = make_double2(accr[q], acci[q]);
+            if (tg > 1) {  // the run lanes of a vector, in order
+                __syncthreads();
+                sm.red[tid] = sum;
+                __syncthreads();
+                if (g == 0)
+                    for (int k = 1; k < tg; ++k) {
+                        sum.x += sm.red[k * tv + v].x;
+                        sum.y += sm.red[k * tv + v].y;
+                    }
+            }
+            const int64_t s = vbase + (int64_t)q * tv;
+            if (g == 0 && s < nsub) part[(by * nsp + a) * nsub + s] = sum;
+        }
     }
 }
 
 template <int VPT>
-__global__ void __launch_bounds__(kPlainThreads) sq_plain_kernel(
+__global__ void __launch_bounds__(kPlainThreads, kPlainCtas) sq_plain_kernel(
     const uint4* __restrict__ phase, const int64_t* __restrict__ sp_off, int nsp, int qsp,
-    const int4* __restrict__ vecs, const int32_t* __restrict__ subset, int nsub, int64_t nvec,
-    int nsplit, double2* __restrict__ part) {
-    __shared__ uint4 atoms[kPlainChunk];
-    __shared__ float2 turn_tab[256];
-    fill_turn_table(turn_tab);
-    plain_block<VPT>(phase, sp_off, nsp, qsp, vecs, subset, nsub, nsplit, part, blockIdx.x, blockIdx.y, atoms,
-                     turn_tab);
+    const int4* __restrict__ vecs, const int32_t* __restrict__ subset, int nsub, PlainShape shape,
+    const float2* __restrict__ turn, double2* __restrict__ part) {
+    __shared__ __align__(16) PlainSmem sm;
+    fill_turn_table(sm, turn);
+    plain_block<VPT>(phase, sp_off, nsp, qsp, vecs, subset, nsub, shape, part, blockIdx.x, blockIdx.y, sm);
 }
 
-// rho[a][v] = sum over splits (fixed order) for the subset's vectors.
-__global__ void gather_plain_kernel(const double2* __restrict__ part, const int32_t* __restrict__ subset,
-                                    int nsub, int64_t nvec, int nsp, int nsplit, double2* __restrict__ rho) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)nsub * nsp) return;
-    int a = (int)(t / nsub);
-    const int64_t pos = t % nsub;
-    int v = subset[pos];
-    double re = 0.0, im = 0.0;
-    for (int s = 0; s < nsplit; ++s) {
-        double2 p = part[((int64_t)s * nsp + a) * nsub + pos];
-        re += p.x;
-        im += p.y;
-    }
-    rho[(int64_t)a * nvec + v] = make_double2(re, im);
+// Sums over `n` partials `stride` apart for 32 vectors at a time (consecutive vectors in a warp's lanes:
+// coalesced): chain l of 32 takes partials l, l + 32, ..., and warp 0 adds the chains in order and returns the
+// sum.  A CTA of NW warps gives each warp 32 / NW chains; the order does not depend on NW.
+constexpr int kSumChains = 32;
+template <int NW>
+__device__ __forceinline__ double2 sum_partials(const double2* __restrict__ p, int64_t stride, int n, bool valid,
+                                                double2 (*red)[32]) {
+    constexpr int kOwn = kSumChains / NW;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double2 t[kOwn];
+#pragma unroll
+    for (int c = 0; c < kOwn; ++c) t[c] = make_double2(0.0, 0.0);
+    if (valid)
+        for (int s = 0; s < n; s += kSumChains) {
+#pragma unroll
+            for (int c = 0; c < kOwn; ++c) {
+                const int k = s + warp + NW * c;
+                const double2 x = k < n ? p[(int64_t)k * stride] : make_double2(0.0, 0.0);
+                t[c].x += x.x;
+                t[c].y += x.y;
+            }
+        }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < kOwn; ++c) red[warp + NW * c][lane] = t[c];
+    __syncthreads();
+    double2 sum = red[0][lane];
+    if (warp == 0)
+        for (int k = 1; k < min(kSumChains, n); ++k) {
+            sum.x += red[k][lane].x;
+            sum.y += red[k][lane].y;
+        }
+    return sum;
+}
+
+// rho[a][v] = sum over the parts (fixed order) for the subset's vectors; grid (vector blocks of 32, species).
+template <int NW>
+__global__ void __launch_bounds__(32 * NW) gather_plain_kernel(const double2* __restrict__ part,
+                                                               const int32_t* __restrict__ subset, int nsub,
+                                                               int64_t nvec, int nsp, int nparts,
+                                                               double2* __restrict__ rho) {
+    __shared__ double2 red[kSumChains][32];
+    const int a = blockIdx.y, pos = blockIdx.x * 32 + (int)(threadIdx.x & 31u);
+    const bool valid = pos < nsub;
+    const double2 r = sum_partials<NW>(part + (int64_t)a * nsub + pos, (int64_t)nsp * nsub, nparts, valid, red);
+    if (valid && threadIdx.x < 32) rho[(int64_t)a * nvec + subset[pos]] = r;
+}
+
+void launch_gather(const double2* part, const int32_t* subset, int64_t nsub, int64_t nvec, int nsp, int nparts,
+                   double2* rho, cudaStream_t s) {
+    const dim3 grid((unsigned)((nsub + 31) / 32), (unsigned)nsp);
+    if (nparts > 128)  // a chain per warp: the loads of many parts in flight
+        gather_plain_kernel<32><<<grid, 1024, 0, s>>>(part, subset, (int)nsub, nvec, nsp, nparts, rho);
+    else
+        gather_plain_kernel<8><<<grid, 256, 0, s>>>(part, subset, (int)nsub, nvec, nsp, nparts, rho);
 }
 
 // rho[a][v] for tensor-tile vectors from the FP64 tile blocks.
@@ -186,36 +301,53 @@ __global__ void gather_dense_kernel(const double* __restrict__ tc_out, const int
     }
 }
 
-// out[bin][pair] += sum_v w_v Re(rho_a conj(rho_b)) over the bin's vectors [v0, v1), by one CTA of
-// 256 threads in a fixed order (thread-strided FP64 sums, warp shuffles, warps in order).
+// out[bin][pair] += sum_v w_v Re(rho_a conj(rho_b)) over the bin's vectors [v0, v1), in a fixed order: 256
+// threads take every 256th vector, four pairs (a, b .. b + 3) in one pass over them, then warp shuffles and
+// warps in order.  Each 256 threads of the CTA work on a pass of their own (the order does not depend on how
+// many there are).  red: 4 doubles per warp.  1e6-atom frame (3 species, 171 shells of up to 4,700 vectors):
+// 109 us with one pair per pass and 256 threads, 36 us so.
+constexpr int kBinPairs = 4;
 __device__ __forceinline__ void bin_reduce_block(const double2* __restrict__ rho, const double* __restrict__ w,
                                                  int v0, int v1, int64_t nvec, int nsp, int bin,
                                                  double* __restrict__ out, double* red) {
-    const int nit = nsp * (nsp + 1) / 2;
-    for (int a = 0; a < nsp; ++a)
-        for (int b = a; b < nsp; ++b) {
-            double s = 0.0;
-            for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
-                double2 ra = rho[(int64_t)a * nvec + v], rb = rho[(int64_t)b * nvec + v];
-                s += w[v] * (ra.x * rb.x + ra.y * rb.y);
+    const int nit = nsp * (nsp + 1) / 2, t = threadIdx.x & 255, team = threadIdx.x >> 8, nteam = blockDim.x >> 8;
+    int a = 0, b = 0;
+    for (int pass = 0; a < nsp; ++pass) {
+        if (pass % nteam == team) {
+            double s[kBinPairs] = {};
+            for (int v = v0 + t; v < v1; v += 256) {
+                const double2 ra = rho[(int64_t)a * nvec + v];
+                const double wv = w[v];
+#pragma unroll
+                for (int k = 0; k < kBinPairs; ++k)
+                    if (b + k < nsp) {
+                        const double2 rb = rho[(int64_t)(b + k) * nvec + v];
+                        s[k] += wv * (ra.x * rb.x + ra.y * rb.y);
+                    }
             }
-            for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double t = 0.0;
-                for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += red[k];
-                out[(int64_t)bin * nit + trj_pair_row(a, b, nsp)] += t;
+#pragma unroll
+            for (int k = 0; k < kBinPairs; ++k) {
+                for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], off);
+                if ((t & 31) == 0) red[(threadIdx.x >> 5) * kBinPairs + k] = s[k];
             }
-            __syncthreads();
+            asm volatile("bar.sync %0, 256;" ::"r"(1 + team) : "memory");  // the team's warps
+            if (t < kBinPairs && b + t < nsp) {
+                double sum = 0.0;
+                for (int k = 0; k < 8; ++k) sum += red[(team * 8 + k) * kBinPairs + t];
+                out[(int64_t)bin * nit + trj_pair_row(a, b + t, nsp)] += sum;
+            }
+            asm volatile("bar.sync %0, 256;" ::"r"(1 + team) : "memory");
         }
+        b += kBinPairs;
+        if (b >= nsp) b = ++a;
+    }
 }
 
 // One CTA per bin.
-__global__ void bin_reduce_kernel(const double2* __restrict__ rho, const double* __restrict__ w,
-                                  const int32_t* __restrict__ bin_start, int64_t nvec, int nsp,
-                                  double* __restrict__ out) {
-    __shared__ double red[32];
+__global__ void __launch_bounds__(1024) bin_reduce_kernel(const double2* __restrict__ rho, const double* __restrict__ w,
+                                                          const int32_t* __restrict__ bin_start, int64_t nvec, int nsp,
+                                                          double* __restrict__ out) {
+    __shared__ double red[32 * kBinPairs];
     const int bin = blockIdx.x;
     const int v0 = bin_start[bin], v1 = bin_start[bin + 1];
     if (v0 >= v1) return;
@@ -230,11 +362,11 @@ __global__ void bin_reduce_kernel(const double2* __restrict__ rho, const double*
 // bin) for the reduction.
 __global__ void __launch_bounds__(kPlainThreads, 2) batch_sq_kernel(BatchHeader* __restrict__ hdr,
                                                                     const BatchItem* __restrict__ items,
-                                                                    const uint4* __restrict__ phase) {
-    __shared__ uint4 atoms[kPlainChunk];
-    __shared__ float2 turn_tab[256];
+                                                                    const uint4* __restrict__ phase,
+                                                                    const float2* __restrict__ turn) {
+    __shared__ __align__(16) PlainSmem sm;
     __shared__ long long unit_s;
-    fill_turn_table(turn_tab);
+    fill_turn_table(sm, turn);
     const int nitems = hdr->nitems;
     const int64_t total = hdr->total_sq;
     while (true) {
@@ -244,19 +376,21 @@ __global__ void __launch_bounds__(kPlainThreads, 2) batch_sq_kernel(BatchHeader*
         __syncthreads();
         if (u >= total) break;
         const BatchItem& it = items[batch_item_of<&BatchItem::sq_begin>(items, nitems, u)];
+        const PlainShape shape = {it.vpt, it.tv, it.tg, it.nvblk, it.nsplit, it.parts};
         const int64_t t = u - it.sq_begin, bx = t % it.nvblk, by = t / it.nvblk;
-        if (it.vpt == 1)
-            plain_block<1>(phase + it.atom_off, it.sp_off_dev, it.nsp, -1, it.vecs, it.subset, it.nvec, it.nsplit,
-                           it.part, bx, by, atoms, turn_tab);
+        if (it.vpt == 2)
+            plain_block<2>(phase + it.atom_off, it.sp_off_dev, it.nsp, -1, it.vecs, it.subset, it.nvec, shape,
+                           it.part, bx, by, sm);
         else
-            plain_block<kPlainVPT>(phase + it.atom_off, it.sp_off_dev, it.nsp, -1, it.vecs, it.subset, it.nvec,
-                                   it.nsplit, it.part, bx, by, atoms, turn_tab);
+            plain_block<4>(phase + it.atom_off, it.sp_off_dev, it.nsp, -1, it.vecs, it.subset, it.nvec, shape,
+                           it.part, bx, by, sm);
     }
 }
 
-__global__ void __launch_bounds__(256, 2) batch_reduce_kernel(BatchHeader* __restrict__ hdr,
+__global__ void __launch_bounds__(256, 4) batch_reduce_kernel(BatchHeader* __restrict__ hdr,
                                                            const BatchItem* __restrict__ items) {
-    __shared__ double red[32];
+    __shared__ double red[8 * kBinPairs];
+    __shared__ double2 psum[kSumChains][32];
     __shared__ long long unit_s;
     const int nitems = hdr->nitems;
     const int64_t total = hdr->total_red;
@@ -270,19 +404,16 @@ __global__ void __launch_bounds__(256, 2) batch_reduce_kernel(BatchHeader* __res
         const int bin = (int)(u - it.red_begin);
         const int v0 = it.bin_start[bin], v1 = it.bin_start[bin + 1];
         if (v0 >= v1) continue;  // block-uniform
-        // rho of the bin's vectors: the splits' partials in order (gather_plain_kernel; the subset is
-        // every vector, so position = vector)
+        // rho of the bin's vectors: the parts' sums in order (gather_plain_kernel; the subset is every
+        // vector, so position = vector)
         const int nb = v1 - v0, nsp = it.nsp, nvec = it.nvec;
-        for (int q = threadIdx.x; q < nb * nsp; q += blockDim.x) {
-            const int a = q / nb, v = v0 + q % nb;
-            double re = 0.0, im = 0.0;
-            for (int s = 0; s < it.nsplit; ++s) {
-                const double2 p = it.part[((int64_t)s * nsp + a) * nvec + v];
-                re += p.x;
-                im += p.y;
+        for (int a = 0; a < nsp; ++a)
+            for (int b0 = 0; b0 < nb; b0 += 32) {
+                const int v = v0 + b0 + (int)(threadIdx.x & 31u);
+                const double2 r = sum_partials<8>(it.part + (int64_t)a * nvec + v, (int64_t)nsp * nvec,
+                                                  it.nsplit * it.parts, v < v1, psum);
+                if (v < v1 && threadIdx.x < 32) it.rho[(int64_t)a * nvec + v] = r;
             }
-            it.rho[(int64_t)a * nvec + v] = make_double2(re, im);
-        }
         __syncthreads();
         bin_reduce_block(it.rho, it.w, v0, v1, nvec, nsp, bin, it.out, red);
     }
@@ -304,22 +435,57 @@ __global__ void check_counts_kernel(const uint4* __restrict__ phase, const int64
     if (s < 0 || s >= nsp || i < sp_off[s] || i >= sp_off[s + 1]) trj_raise(status, TRJ_DEV_COUNT_MISMATCH);
 }
 
-// Vectors per thread: 4 for large vector sets; 1 when 4 per thread would leave most lanes idle
-// (the few hundred axis vectors next to the tensor tiles).
-int plain_vpt(int64_t nsub) { return nsub < (int64_t)kPlainThreads * kPlainVPT * 32 ? 1 : kPlainVPT; }
-
+// Slices of a direct sum of nsub vectors over n_total atoms: they fix which atoms share an FP32 partial sum,
+// whatever the launch shape.
 int plain_nsplit(const trj_ctx* ctx, int64_t nsub, int64_t n_total) {
-    const int vpt = plain_vpt(nsub);
-    int64_t blocks_v = (nsub + kPlainThreads * vpt - 1) / (kPlainThreads * vpt);
+    const int per_block = kPlainThreads * (nsub < (int64_t)kPlainThreads * 4 * 32 ? 1 : 4);
+    int64_t blocks_v = (nsub + per_block - 1) / per_block;
     if (blocks_v <= 0) return 1;
     int64_t target = (int64_t)ctx->sm_count * 8;
     int64_t ns = (target + blocks_v - 1) / blocks_v;
-    int64_t by_atoms = std::max<int64_t>(1, n_total / (2 * kPlainChunk));
+    int64_t by_atoms = std::max<int64_t>(1, n_total / kPlainSlice);
     ns = std::min<int64_t>(ns, by_atoms);
     // partials are nsplit x species x vectors x 16 bytes: allow more splits for small vector sets
     const int64_t cap = nsub <= 32768 ? 1024 : 128;
     ns = std::max<int64_t>(1, std::min<int64_t>(ns, cap));
     return (int)ns;
+}
+
+// Launch shape: four vectors per thread where that still makes enough warps, two otherwise (one packed
+// instruction serves two); tv threads cover a block's vectors with the fewest idle lanes, the other threads
+// take further runs.  Slices are cut into parts, at least a run per run lane, while the partials stay below
+// 256 MB.
+PlainShape plain_shape(const trj_ctx* ctx, int64_t nsub, int64_t n_total, int nsp) {
+    PlainShape s;
+    s.nsplit = plain_nsplit(ctx, nsub, n_total);
+    const int64_t n = std::max<int64_t>(1, nsub);
+    // warps of four vectors per thread over single runs: enough to fill the SMs' schedulers?
+    const int64_t warps4 = (n + 127) / 128 * ((n_total + kPlainSub - 1) / kPlainSub);
+    s.vpt = n >= 2 * kPlainThreads && warps4 >= (int64_t)ctx->sm_count * 24 ? 4 : 2;
+    s.nvblk = (int)((n + (int64_t)kPlainThreads * s.vpt - 1) / ((int64_t)kPlainThreads * s.vpt));
+    const int64_t per = (n + s.nvblk - 1) / s.nvblk;  // vectors of a block
+    s.tv = (int)std::min<int64_t>(kPlainThreads, ((per + s.vpt - 1) / s.vpt + 31) / 32 * 32);
+    s.nvblk = (int)((n + (int64_t)s.tv * s.vpt - 1) / ((int64_t)s.tv * s.vpt));
+    s.tg = std::min(kPlainThreads / s.tv, kPlainStage / kPlainSub);
+    const int64_t blocks = (int64_t)s.nvblk * s.nsplit;
+    const int64_t runs = std::max<int64_t>(1, n_total / ((int64_t)s.nsplit * nsp * kPlainSub * s.tg));
+    const int64_t room = std::max<int64_t>(1, ((int64_t)256 << 20) / (16 * (int64_t)s.nsplit * nsp * n));
+    // blocks resident at a time (64 registers a thread, 41 KB of shared memory), and the number of parts that
+    // wastes least of the last wave: three waves at least where the runs allow, six at most
+    const double slots = (double)ctx->sm_count * std::min(5, kPlainThreads * kPlainCtas / (s.tv * s.tg));
+    const int64_t most = std::min(runs, room);
+    const int64_t lo = std::max<int64_t>(1, std::min(most, (int64_t)ceil(3.0 * slots / blocks)));
+    const int64_t hi = std::max(lo, std::min(most, (int64_t)(6.0 * slots / blocks)));
+    double best = 0.0;
+    s.parts = (int)lo;
+    for (int64_t k = lo; k <= hi; ++k) {
+        const double waves = (double)(blocks * k) / slots, use = waves / ceil(waves);
+        if (use > best + 0.01) {
+            best = use;
+            s.parts = (int)k;
+        }
+    }
+    return s;
 }
 
 }  // namespace
@@ -501,12 +667,13 @@ extern "C" int trj_sq_plan_create(trj_ctx* ctx, int nsp, int64_t nvec, const int
         }
         acct += (int64_t)tb;
     }
-    p->nsplit_all = plain_nsplit(ctx, nvec, p->n_total);
-    p->nsplit_sparse = plain_nsplit(ctx, p->n_sparse, p->n_total);
+    const PlainShape all_shape = plain_shape(ctx, nvec, p->n_total, nsp);
+    const PlainShape sparse_shape = plain_shape(ctx, p->n_sparse, p->n_total, nsp);
+    auto part_rows = [](const PlainShape& s) { return (size_t)s.nsplit * s.parts; };
     size_t phase_b = sizeof(uint4) * (size_t)std::max<int64_t>(1, p->n_total);
     size_t part_b = sizeof(double2) * (size_t)nsp *
-                    std::max<size_t>((size_t)p->nsplit_all * std::max<int64_t>(1, nvec),
-                                     (size_t)p->nsplit_sparse * std::max<int64_t>(1, p->n_sparse));
+                    std::max<size_t>(part_rows(all_shape) * std::max<int64_t>(1, nvec),
+                                     part_rows(sparse_shape) * std::max<int64_t>(1, p->n_sparse));
     size_t rho_b = sizeof(double2) * (size_t)nsp * (size_t)std::max<int64_t>(1, nvec);
     if (trj_dev_alloc(ctx, (void**)&p->phase_dev, phase_b) != cudaSuccess ||
         trj_dev_alloc(ctx, (void**)&p->part_dev, part_b) != cudaSuccess ||
@@ -560,23 +727,20 @@ extern "C" int trj_sq_plan_info(const trj_sq_plan* p, int64_t* n_dense, int64_t*
     return TRJ_OK;
 }
 
-static int run_plain(trj_sq_plan* p, const int32_t* subset, int64_t nsub, int nsplit, cudaStream_t s,
-                     bool timed) {
+static void launch_plain(const trj_ctx* ctx, const PlainShape& sh, const uint4* phase, const int64_t* sp_off, int nsp,
+                         int qsp, const int4* vecs, const int32_t* subset, int64_t nsub, double2* part, cudaStream_t s) {
+    const dim3 grid((unsigned)sh.nvblk, (unsigned)(sh.nsplit * sh.parts));
+    auto kern = sh.vpt == 2 ? sq_plain_kernel<2> : sq_plain_kernel<4>;
+    kern<<<grid, sh.tv * sh.tg, 0, s>>>(phase, sp_off, nsp, qsp, vecs, subset, (int)nsub, sh, ctx->turn_dev, part);
+}
+
+static int run_plain(trj_sq_plan* p, const int32_t* subset, int64_t nsub, cudaStream_t s, bool timed) {
     if (nsub <= 0) return TRJ_OK;
-    const int vpt = plain_vpt(nsub);
-    dim3 grid((unsigned)((nsub + kPlainThreads * vpt - 1) / (kPlainThreads * vpt)), (unsigned)nsplit);
+    const PlainShape sh = plain_shape(p->ctx, nsub, p->n_total, p->nsp);
     if (timed) p->timer.begin(p->ctx, s);
-    if (vpt == 1)
-        sq_plain_kernel<1><<<grid, kPlainThreads, 0, s>>>(p->phase_dev, p->species_off_dev, p->nsp, p->qsp, p->vec_dev,
-                                                          subset, (int)nsub, p->nvec, nsplit, p->part_dev);
-    else
-        sq_plain_kernel<kPlainVPT><<<grid, kPlainThreads, 0, s>>>(p->phase_dev, p->species_off_dev, p->nsp, p->qsp,
-                                                                  p->vec_dev, subset, (int)nsub, p->nvec, nsplit,
-                                                                  p->part_dev);
+    launch_plain(p->ctx, sh, p->phase_dev, p->species_off_dev, p->nsp, p->qsp, p->vec_dev, subset, nsub, p->part_dev, s);
     if (timed) p->timer.end(p->ctx, s);
-    int64_t tot = nsub * p->nsp;
-    gather_plain_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(p->part_dev, subset, (int)nsub, p->nvec,
-                                                                      p->nsp, nsplit, p->rho_dev);
+    launch_gather(p->part_dev, subset, nsub, p->nvec, p->nsp, sh.nsplit * sh.parts, p->rho_dev, s);
     p->ctx->launches += 2;
     return TRJ_OK;
 }
@@ -608,16 +772,17 @@ static int sq_accumulate_impl(trj_sq_plan* p, const float* packed_dev, const flo
         ctx->launches += 2;
     }
     if (method == TRJ_SQ_PLAIN_FP32 || p->tiles.empty()) {
-        run_plain(p, p->plain_all_dev, p->nvec, p->nsplit_all, s, true);
+        run_plain(p, p->plain_all_dev, p->nvec, s, true);
     } else {
         int rc = trj_sq_tc_run(p, box, s);
         if (rc != TRJ_OK) return rc;
         gather_dense_kernel<<<(unsigned)((p->nvec + 255) / 256), 256, 0, s>>>(
             p->tc_out_dev, p->dense_src_dev, p->nvec, p->nsp, p->dense_src_dev + p->nvec, p->rho_dev);
         ctx->launches += 1;
-        run_plain(p, p->plain_sparse_dev, p->n_sparse, p->nsplit_sparse, s, false);
+        run_plain(p, p->plain_sparse_dev, p->n_sparse, s, false);
     }
-    bin_reduce_kernel<<<p->nbins, 256, 0, s>>>(p->rho_dev, p->weight_dev, p->bin_start_dev, p->nvec, p->nsp,
+    const int teams = std::min(4, p->nsp + p->nsp * (p->nsp - 1) / 8);  // as many as there are passes
+    bin_reduce_kernel<<<p->nbins, 256 * teams, 0, s>>>(p->rho_dev, p->weight_dev, p->bin_start_dev, p->nvec, p->nsp,
                                               out_dev);
     ctx->launches += 1;
     p->last_method = method;
@@ -663,7 +828,8 @@ extern "C" int trj_sq_rho_groups(trj_sq_plan* p, const float* packed_dev, int64_
     if (p->nvec == 0) return TRJ_OK;
     trj_device_guard g(ctx->device);
     cudaStream_t s = (cudaStream_t)stream;
-    const int nsplit = plain_nsplit(ctx, p->nvec, std::max<int64_t>(n, 1));
+    const PlainShape sh = plain_shape(ctx, p->nvec, std::max<int64_t>(n, 1), ngroups);
+    const int nsplit = sh.nsplit * sh.parts;
     const size_t phase_need = sizeof(uint4) * (size_t)std::max<int64_t>(n, 1);
     const size_t part_need = sizeof(double2) * (size_t)nsplit * ngroups * p->nvec;
     const size_t rho_need = sizeof(double2) * (size_t)ngroups * p->nvec;
@@ -692,17 +858,9 @@ extern "C" int trj_sq_rho_groups(trj_sq_plan* p, const float* packed_dev, int64_
         phase_coords_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((const float4*)packed_dev, n, (double)box[0],
                                                                        (double)box[1], (double)box[2], phase, nullptr,
                                                                        p->z_from_y);
-    const int vpt = plain_vpt(p->nvec);
-    dim3 grid((unsigned)((p->nvec + kPlainThreads * vpt - 1) / (kPlainThreads * vpt)), (unsigned)nsplit);
-    if (vpt == 1)
-        sq_plain_kernel<1><<<grid, kPlainThreads, 0, s>>>(phase, off, ngroups, -1, p->vec_dev, p->plain_all_dev,
-                                                          (int)p->nvec, p->nvec, nsplit, part);
-    else
-        sq_plain_kernel<kPlainVPT><<<grid, kPlainThreads, 0, s>>>(phase, off, ngroups, -1, p->vec_dev,
-                                                                  p->plain_all_dev, (int)p->nvec, p->nvec, nsplit, part);
+    launch_plain(ctx, sh, phase, off, ngroups, -1, p->vec_dev, p->plain_all_dev, p->nvec, part, s);
     const int64_t tot = p->nvec * ngroups;
-    gather_plain_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(part, p->plain_all_dev, (int)p->nvec, p->nvec,
-                                                                      ngroups, nsplit, rho);
+    launch_gather(part, p->plain_all_dev, p->nvec, p->nvec, ngroups, nsplit, rho, s);
     unpermute_rho_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(rho, p->vec_dev, p->nvec, ngroups,
                                                                        (double2*)rho_out);
     ctx->launches += 4;
@@ -737,9 +895,9 @@ extern "C" int trj_sq_plan_set_z_from_y(trj_sq_plan* p, int mul) {
 
 // ---- fused multi-request launch: host side of the direct sum -----------------------------------
 
-void trj_batch_launch_sq(BatchHeader* hdr, const BatchItem* items, const uint4* phase, int grid_sq, int grid_red,
-                         cudaStream_t s) {
-    batch_sq_kernel<<<grid_sq, kPlainThreads, 0, s>>>(hdr, items, phase);
+void trj_batch_launch_sq(BatchHeader* hdr, const BatchItem* items, const uint4* phase, const float2* turn, int grid_sq,
+                         int grid_red, cudaStream_t s) {
+    batch_sq_kernel<<<grid_sq, kPlainThreads, 0, s>>>(hdr, items, phase, turn);
     batch_reduce_kernel<<<grid_red, 256, 0, s>>>(hdr, items);
 }
 
@@ -768,10 +926,14 @@ int trj_batch_fill_sq(trj_sq_plan* p, int64_t n, BatchItem* it) {
     it->part = p->part_dev;
     it->rho = p->rho_dev;
     it->nvec = (int32_t)p->nvec;
-    it->nsplit = p->nsplit_all;
-    it->vpt = plain_vpt(p->nvec);
+    const PlainShape sh = plain_shape(ctx, p->nvec, p->n_total, p->nsp);
+    it->nsplit = sh.nsplit;
+    it->parts = sh.parts;
+    it->vpt = sh.vpt;
+    it->tv = sh.tv;
+    it->tg = sh.tg;
     it->nbins = p->nbins;
-    it->nvblk = (int32_t)((p->nvec + (int64_t)kPlainThreads * it->vpt - 1) / ((int64_t)kPlainThreads * it->vpt));
+    it->nvblk = sh.nvblk;
     p->last_method = TRJ_SQ_PLAIN_FP32;
     return TRJ_OK;
 }

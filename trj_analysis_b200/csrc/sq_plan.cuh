@@ -45,8 +45,7 @@ struct trj_sq_plan {
     int64_t* dense_src_dev = nullptr;      // per plan vector: offset into TC output (re at +0, im at +128) or -1
     // scratch
     uint4* phase_dev = nullptr;            // n_total x (ux, uy, uz, species)
-    double2* part_dev = nullptr;           // direct-sum partials [nsplit][nsp][nvec]
-    int nsplit_all = 1, nsplit_sparse = 1;
+    double2* part_dev = nullptr;           // direct-sum partials [slice, part][nsp][nvec]
     double* tc_out_dev = nullptr;          // tensor-core rho blocks (FP64)
     double2* rho_dev = nullptr;            // [nsp][nvec] final rho in plan order
     int last_method = -1;

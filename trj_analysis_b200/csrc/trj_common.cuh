@@ -24,6 +24,7 @@ struct trj_ctx {
     size_t smem_optin = 0;
     unsigned* status_dev = nullptr;     // [0] status bits, [1..7] diagnostics
     unsigned* status_host = nullptr;    // pinned mirror
+    float2* turn_dev = nullptr;         // cos, sin(2 pi k / 256), k = 0..255, each rounded once from FP64
     struct PackScratch {
         void* ptr = nullptr;
         size_t bytes = 0;
