@@ -210,7 +210,7 @@ TRJ_API int trj_rdf_accumulate(trj_rdf_plan* plan, const float* packed_dev, int6
  * charge_packed_dev: the charges written by trj_frame_pack_charges.  Products
  * and sums are FP64 (the reference adds FP32 products with FP32 atomics).  An
  * all-zero charge set gives avq2 = 0 and non-finite gqq, as in the reference.
- * The first charged call on a plan allocates 4*n_max + 8*lsmax bytes. */
+ * The first charged call on a plan allocates 4*n_max + 8*(lsmax + n_max/256) bytes. */
 TRJ_API int trj_rdf_accumulate_charged(trj_rdf_plan* plan, const float* packed_dev, const float* charge_packed_dev,
                                        int64_t n, const float box[3], uint64_t* hist_dev, uint64_t* edge_dev,
                                        double* gqq_dev, void* stream);

@@ -196,61 +196,122 @@ __global__ void pack_count_kernel(const float* __restrict__ xyz, const int32_t* 
     if (threadIdx.x < nsp) block_counts[(int64_t)blockIdx.x * nsp + threadIdx.x] = cnt[threadIdx.x];
 }
 
-// One block: exclusive scan of per-block counts, species after species.
-__global__ void pack_scan_kernel(int32_t* __restrict__ block_counts, int64_t nblocks, int nsp,
-                                 int64_t* __restrict__ counts_out, int64_t* __restrict__ block_base) {
-    __shared__ int64_t partial[1024];
-    __shared__ int64_t species_base;
-    if (threadIdx.x == 0) species_base = 0;
-    __syncthreads();
-    int64_t per = (nblocks + blockDim.x - 1) / blockDim.x;
+// One block: exclusive scan of per-block counts, species after species, 1,024 blocks at a time.
+__global__ void __launch_bounds__(1024) pack_scan_kernel(const int32_t* __restrict__ block_counts, int64_t nblocks,
+                                                         int nsp, int64_t* __restrict__ counts_out,
+                                                         int64_t* __restrict__ block_base) {
+    __shared__ int warp_sum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t run = 0;  // atoms placed before this tile (all threads keep it)
     for (int s = 0; s < nsp; ++s) {
-        int64_t b0 = threadIdx.x * per, b1 = b0 + per < nblocks ? b0 + per : nblocks;
-        int64_t sum = 0;
-        for (int64_t b = b0; b < b1; ++b) sum += block_counts[b * nsp + s];
-        partial[threadIdx.x] = sum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int64_t run = 0;
-            for (unsigned t = 0; t < blockDim.x; ++t) {
-                int64_t v = partial[t];
-                partial[t] = run;
-                run += v;
+        const int64_t first = run;
+        for (int64_t b0 = 0; b0 < nblocks; b0 += 1024) {
+            const int64_t b = b0 + threadIdx.x;
+            const int v = b < nblocks ? block_counts[b * nsp + s] : 0;
+            int x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
             }
-            counts_out[s] = run;
+            if (lane == 31) warp_sum[warp] = x;
+            __syncthreads();
+            int w = warp_sum[lane];  // every warp scans the warps' sums
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += y;
+            }
+            const int before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+            if (b < nblocks) block_base[b * nsp + s] = run + (warp > 0 ? before : 0) + x - v;
+            run += __shfl_sync(0xffffffffu, w, 31);
+            __syncthreads();
         }
-        __syncthreads();
-        int64_t run = species_base + partial[threadIdx.x];
-        for (int64_t b = b0; b < b1; ++b) {
-            block_base[b * nsp + s] = run;
-            run += block_counts[b * nsp + s];
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) species_base += counts_out[s];
-        __syncthreads();
+        if (threadIdx.x == 0) counts_out[s] = run - first;
     }
 }
 
-__global__ void pack_scatter_kernel(const float* __restrict__ xyz, const int32_t* __restrict__ sp,
-                                    int64_t n, int nsp, float Lx, float Ly, float Lz,
-                                    const int64_t* __restrict__ block_base,
-                                    float4* __restrict__ packed, const float* __restrict__ q,
-                                    float* __restrict__ qpacked, const int32_t* __restrict__ lut, int nlut) {
+// Where a block's atoms of each species go.  kBaseScan: block_base of pack_scan_kernel.  kBaseCounts: from the
+// per-block counts, each block adding up those before it (frames of few blocks: one launch less).  kBaseAtoms:
+// from the species column itself, which small frames re-read in every block (the counting launch goes as well;
+// this kernel then checks its own atoms).
+enum { kBaseScan = 0, kBaseCounts = 1, kBaseAtoms = 2 };
+constexpr int64_t kPackCountBlocks = 128;  // most blocks of a kBaseCounts frame (131,072 atoms)
+constexpr int64_t kPackAtomsMax = 8192;    // most atoms of a kBaseAtoms frame
+
+template <int BASE>
+__global__ void __launch_bounds__(kPackThreads) pack_scatter_kernel(
+    const float* __restrict__ xyz, const int32_t* __restrict__ sp, int64_t n, int nsp, float Lx, float Ly, float Lz,
+    const int64_t* __restrict__ block_base, const int32_t* __restrict__ block_counts, int64_t* __restrict__ counts_out,
+    unsigned* status, float4* __restrict__ packed, const float* __restrict__ q, float* __restrict__ qpacked,
+    const int32_t* __restrict__ lut, int nlut) {
+    constexpr int kWarps = kPackThreads / 32;
     __shared__ int64_t base[kMaxSpecies];
-    __shared__ int warp_cnt[kPackThreads / 32][kMaxSpecies];
+    __shared__ int warp_cnt[kWarps][kMaxSpecies];
+    __shared__ int all_s[kMaxSpecies], before_s[kMaxSpecies];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    if (threadIdx.x < nsp) base[threadIdx.x] = block_base[(int64_t)blockIdx.x * nsp + threadIdx.x];
-    for (int k = threadIdx.x; k < (kPackThreads / 32) * kMaxSpecies; k += blockDim.x)
-        (&warp_cnt[0][0])[k] = 0;
+    if (BASE == kBaseScan) {
+        if (threadIdx.x < nsp) base[threadIdx.x] = block_base[(int64_t)blockIdx.x * nsp + threadIdx.x];
+    } else {
+        if (threadIdx.x < kMaxSpecies) all_s[threadIdx.x] = before_s[threadIdx.x] = 0;
+        __syncthreads();
+        if (BASE == kBaseCounts) {
+            for (int a = warp; a < nsp; a += kWarps) {
+                int all = 0, before = 0;
+                for (int b = lane; b < (int)gridDim.x; b += 32) {
+                    const int v = block_counts[(int64_t)b * nsp + a];
+                    all += v;
+                    before += b < (int)blockIdx.x ? v : 0;
+                }
+                all = __reduce_add_sync(0xffffffffu, all);
+                before = __reduce_add_sync(0xffffffffu, before);
+                if (lane == 0) {
+                    all_s[a] = all;
+                    before_s[a] = before;
+                }
+            }
+        } else {
+            // whole warps of 32 atoms: a warp's atoms lie in one block's chunk
+            const int first = (int)blockIdx.x * kPackChunk;
+            for (int a = 0; a < nsp; ++a) {
+                int all = 0, before = 0;
+#pragma unroll 4
+                for (int i = warp * 32; i < (int)n; i += kPackThreads) {
+                    const int s = i + lane < (int)n ? species_of(sp, i + lane, lut, nlut) : -1;
+                    const int c = __popc(__ballot_sync(0xffffffffu, s == a));
+                    all += c;
+                    before += i < first ? c : 0;
+                }
+                if (lane == 0) {
+                    atomicAdd(&all_s[a], all);
+                    atomicAdd(&before_s[a], before);
+                }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < nsp) {
+            int64_t b = before_s[threadIdx.x];
+            for (int a = 0; a < (int)threadIdx.x; ++a) b += all_s[a];
+            base[threadIdx.x] = b;
+            if (blockIdx.x == 0) counts_out[threadIdx.x] = all_s[threadIdx.x];
+        }
+    }
+    for (int k = threadIdx.x; k < kWarps * kMaxSpecies; k += blockDim.x) (&warp_cnt[0][0])[k] = 0;
     __syncthreads();
     const unsigned lt_mask = (1u << lane) - 1u;
     int64_t start = (int64_t)blockIdx.x * kPackChunk;
     for (int r = 0; r < kPackRounds; ++r) {
         int64_t i = start + r * kPackThreads + threadIdx.x;
         int s = -1;
+        float x = 0.f, y = 0.f, z = 0.f;
         if (i < n) {
             s = species_of(sp, i, lut, nlut);
-            if (s < 0 || s >= nsp) s = -1;  // flagged by pack_count_kernel; dropped here
+            x = xyz[3 * i];
+            y = xyz[3 * i + 1];
+            z = xyz[3 * i + 2];
+            if (s < 0 || s >= nsp) s = -1;  // flagged as bad data; dropped here
+            if (BASE == kBaseAtoms && (s < 0 || !isfinite(x) || !isfinite(y) || !isfinite(z)))
+                trj_raise(status, TRJ_DEV_BAD_DATA);
         }
         unsigned peers = __match_any_sync(0xffffffffu, s);
         int rank = __popc(peers & lt_mask);
@@ -261,9 +322,9 @@ __global__ void pack_scatter_kernel(const float* __restrict__ xyz, const int32_t
             for (int w = 0; w < warp; ++w) off += warp_cnt[w][s];
             off += rank;
             float4 v;
-            v.x = trj_fold_ref(xyz[3 * i], Lx);
-            v.y = trj_fold_ref(xyz[3 * i + 1], Ly);
-            v.z = trj_fold_ref(xyz[3 * i + 2], Lz);
+            v.x = trj_fold_ref(x, Lx);
+            v.y = trj_fold_ref(y, Ly);
+            v.z = trj_fold_ref(z, Lz);
             v.w = __int_as_float(s);
             packed[off] = v;
             if (q) qpacked[off] = q[i];  // charges follow their atoms (netcdf.f90:656-658)
@@ -281,6 +342,33 @@ __global__ void pack_scatter_kernel(const float* __restrict__ xyz, const int32_t
     }
 }
 
+
+// The layout launches of a frame; scratch holds nblocks * nsp block bases, then as many counts.
+int launch_pack(trj_ctx* ctx, const float* xyz, const int32_t* sp, int64_t n, int nsp, const float box[3], void* scratch,
+                int64_t* counts, float4* packed, const float* q, float* qpacked, const int32_t* lut, int nlut,
+                cudaStream_t s) {
+    const int64_t nblocks = (n + kPackChunk - 1) / kPackChunk;
+    int64_t* base = (int64_t*)scratch;
+    int32_t* block_counts = (int32_t*)(base + nblocks * nsp);
+    if (n > kPackAtomsMax) {
+        pack_count_kernel<<<(unsigned)nblocks, kPackThreads, 0, s>>>(xyz, sp, n, nsp, block_counts, ctx->status_dev, lut,
+                                                                     nlut);
+        ctx->launches += 1;
+    }
+    auto scatter = pack_scatter_kernel<kBaseAtoms>;
+    if (nblocks > kPackCountBlocks) {
+        pack_scan_kernel<<<1, 1024, 0, s>>>(block_counts, nblocks, nsp, counts, base);
+        ctx->launches += 1;
+        scatter = pack_scatter_kernel<kBaseScan>;
+    } else if (n > kPackAtomsMax) {
+        scatter = pack_scatter_kernel<kBaseCounts>;
+    }
+    scatter<<<(unsigned)nblocks, kPackThreads, 0, s>>>(xyz, sp, n, nsp, box[0], box[1], box[2], base, block_counts, counts,
+                                                       ctx->status_dev, packed, q, qpacked, lut, nlut);
+    ctx->launches += 1;
+    TRJ_CUDA_TRY(ctx, cudaGetLastError());
+    return TRJ_OK;
+}
 
 // ---- fused multi-request launch: frame layout -------------------------------------------------
 //
@@ -458,17 +546,8 @@ static int frame_pack_impl(trj_ctx* ctx, const char* name, const float* xyz_dev,
             return trj_fail(ctx, TRJ_ERR_NOMEM, "%s: scratch of %zu bytes", name, need);
         ps.bytes = need;
     }
-    int64_t* block_base = (int64_t*)ps.ptr;
-    int32_t* block_counts = (int32_t*)(block_base + nblocks * nsp);
-    pack_count_kernel<<<(unsigned)nblocks, kPackThreads, 0, s>>>(xyz_dev, species_dev, n, nsp,
-                                                                 block_counts, ctx->status_dev, lut_dev, nlut);
-    pack_scan_kernel<<<1, 1024, 0, s>>>(block_counts, nblocks, nsp, counts_dev, block_base);
-    pack_scatter_kernel<<<(unsigned)nblocks, kPackThreads, 0, s>>>(xyz_dev, species_dev, n, nsp, box[0], box[1],
-                                                                   box[2], block_base, (float4*)packed_dev,
-                                                                   charge_dev, charge_packed_dev, lut_dev, nlut);
-    ctx->launches += 3;
-    TRJ_CUDA_TRY(ctx, cudaGetLastError());
-    return TRJ_OK;
+    return launch_pack(ctx, xyz_dev, species_dev, n, nsp, box, ps.ptr, counts_dev, (float4*)packed_dev, charge_dev,
+                       charge_packed_dev, lut_dev, nlut, s);
 }
 
 extern "C" int trj_frame_pack(trj_ctx* ctx, const float* xyz_dev, const int32_t* species_dev,
@@ -500,7 +579,7 @@ extern "C" int trj_frame_pack_charges(trj_ctx* ctx, const float* xyz_dev, const 
 // ---------------------------------------------------------------------------
 // Frame layout without allocation.
 //
-// trj_frame_pack_static runs the same three layout kernels as trj_frame_pack, but its
+// trj_frame_pack_static runs the same layout kernels as trj_frame_pack, but its
 // per-block species counts and block offsets live in the fixed device array below instead of
 // context scratch grown with cudaMalloc.  It serves callers that may not allocate device memory
 // from inside the library: applications whose device memory is owned by another allocator (a
@@ -573,17 +652,8 @@ extern "C" int trj_frame_pack_static(trj_ctx* ctx, const float* xyz_dev, const i
     void* scratch = nullptr;
     int rc = pack_static_address(ctx, &scratch);
     if (rc != TRJ_OK) return rc;
-    int64_t* block_base = (int64_t*)scratch;
-    int32_t* block_counts = (int32_t*)(block_base + nblocks * nsp);
-    pack_count_kernel<<<(unsigned)nblocks, kPackThreads, 0, s>>>(xyz_dev, species_dev, n, nsp, block_counts,
-                                                                 ctx->status_dev, nullptr, 0);
-    pack_scan_kernel<<<1, 1024, 0, s>>>(block_counts, nblocks, nsp, counts_dev, block_base);
-    pack_scatter_kernel<<<(unsigned)nblocks, kPackThreads, 0, s>>>(xyz_dev, species_dev, n, nsp, box[0], box[1],
-                                                                   box[2], block_base, (float4*)packed_dev, nullptr,
-                                                                   nullptr, nullptr, 0);
-    ctx->launches += 3;
-    TRJ_CUDA_TRY(ctx, cudaGetLastError());
-    return TRJ_OK;
+    return launch_pack(ctx, xyz_dev, species_dev, n, nsp, box, scratch, counts_dev, (float4*)packed_dev, nullptr, nullptr,
+                       nullptr, 0, s);
 }
 
 void trj_batch_launch_layout(const BatchHeader* hdr, const BatchItem* items, const float* xyz_staged,

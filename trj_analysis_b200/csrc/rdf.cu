@@ -59,6 +59,15 @@ struct PairGeom {
     float one;                  // 1.0f, from the host: not a constant the assembler could fold
 };
 
+// Division of n < 2^31 by a launch constant: n * ceil(2^(31+l) / d) >> (31+l), l = ceil(log2 d).
+struct FastDiv {
+    unsigned d, mul;
+    int shift;
+};
+__device__ __forceinline__ int fast_div(int n, const FastDiv& f) {
+    return f.d == 1u ? n : (int)(__umulhi((unsigned)n, f.mul) >> f.shift);
+}
+
 struct RdfParams {
     PairGeom g;
     int nit;
@@ -67,8 +76,11 @@ struct RdfParams {
     float inv_sub[3];           // 1 / sub
     float edge[3];              // cell edge
     float half[3];              // half edge of a group's box, with the cull pad
-    int noff;
-    int nseg, per_seg;          // segments of a home group's neighbour list (one work item each); their length
+    FastDiv div_nsub, div_nc1, div_nc2, div_nseg;
+    // A home group's neighbour list: its own cell's groups at distance 0 .. nsub / 2 after it (cyclically, so
+    // that every group has the same share), then all groups of each further stencil cell.
+    int nself, list;            // entries of the own cell, of the list
+    int nseg, per_seg;          // segments of the list (one work item each); their length
     int split_all;              // every axis of the geometry is split (in two dimensions: x and y)
     float cull2;                // (cutoff * (1 + 2^-10))^2: neighbours farther from the homes' box are skipped
     float cull_pad;             // added to half-widths: covers the FP32 rounding of the cull test
@@ -450,14 +462,14 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
         if (lane == 0) item = atomicAdd(work, 1u);
         item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= p.nitems) break;
-        const int key = (int)(item / (unsigned)p.nseg), seg = (int)(item - (unsigned)key * (unsigned)p.nseg);
+        const int key = fast_div((int)item, p.div_nseg), seg = (int)item - key * p.nseg;
         const int hbeg = fstart[key], hend = hbeg + fcount[key];
         if (hbeg >= hend) continue;
-        const int c = key / p.nsub, own = key - c * p.nsub;
-        const int cz = c % p.nc[2], cxy = c / p.nc[2], cy = cxy % p.nc[1], cx = cxy / p.nc[1];
+        const int c = fast_div(key, p.div_nsub), own = key - c * p.nsub;
+        const int cxy = fast_div(c, p.div_nc2), cz = c - cxy * p.nc[2];
+        const int cx = fast_div(cxy, p.div_nc1), cy = cxy - cx * p.nc[1];
         const int fl = cflag[c];
-        const int list = p.noff * p.nsub;  // the (offset, neighbour group) list, cut into segments
-        const int t0 = seg * p.per_seg, t1 = min(list, t0 + p.per_seg);
+        const int t0 = seg * p.per_seg, t1 = min(p.list, t0 + p.per_seg);
         for (int h0 = hbeg; h0 < hend; h0 += kGroup) {
             const int nh = min(kGroup, hend - h0);
             const bool has = lane < nh;
@@ -474,8 +486,11 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
             axis_box(wrap_cull(a.y, g.L[1]), has, p.cull_pad, by, wy);
             axis_box(wrap_cull(a.z, g.L[2]), has, p.cull_pad, bz, wz);
             for (int t = t0; t < t1;) {
-                const int o = t / p.nsub, s_lo = t - o * p.nsub, s_hi = min(p.nsub, t1 - o * p.nsub);
-                t = o * p.nsub + s_hi;
+                // entries [e_lo, e_hi) of offset o: group e, or (own cell) the e-th after the homes' own
+                const int o = t < p.nself ? 0 : 1 + fast_div(t - p.nself, p.div_nsub);
+                const int first = o == 0 ? 0 : p.nself + (o - 1) * p.nsub;
+                const int e_lo = t - first, e_hi = min(o == 0 ? p.nself : p.nsub, t1 - first);
+                t = first + e_hi;
                 const int ex = cx + p.off[o][0], ey = cy + p.off[o][1], ez = cz + p.off[o][2];
                 const int c2 = (wrapc(ex, p.nc[0]) * p.nc[1] + wrapc(ey, p.nc[1])) * p.nc[2] + wrapc(ez, p.nc[2]);
                 const int f2 = fl | cflag[c2];
@@ -512,18 +527,20 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
                     return up >> 2;
                 };
 #define TRJ_RUN(M, S, N4) test_run<M, S, FLOOR, QMODE, SQUARE, EDGE>(ring, ring_q, head, N4, h, has, ix, iy, iz, g, pc, qhist)
-                if (o == 0 && s_lo <= own && own < s_hi) {
+                if (o == 0 && e_lo == 0) {
                     // pairs j > i of the round's own atoms, through the buffer in lane order
                     append(a, h.q, has);
                     const int n4 = pad();
                     __syncwarp();
                     if (plain) TRJ_RUN(kImgNone, true, n4);
+                    else if (mode == kImgRound) TRJ_RUN(kImgRound, true, n4);
+                    else if (mode == kImgFold) TRJ_RUN(kImgFold, true, n4);
                     else TRJ_RUN(kImgAny, true, n4);
                     __syncwarp();
                     if (EDGE && has) n_tested += (unsigned)(nh - 1 - lane);
                     tail = 0;
                 }
-                int s0 = s_lo - 32, j = 0, je = 0, gs = 0, gn = 0;  // gs, gn: start and atoms of lane's group
+                int e0 = e_lo - 32, j = 0, je = 0, gs = 0, gn = 0;  // gs, gn: start and atoms of lane's group
                 unsigned m = 0;
                 bool more = true;
                 do {
@@ -531,14 +548,17 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
                     while (tail - head < kRingRun) {
                         if (j >= je) {
                             if (!m) {
-                                s0 += 32;
-                                if (s0 >= s_hi) {
+                                e0 += 32;
+                                if (e0 >= e_hi) {
                                     more = false;
                                     break;
                                 }
                                 // lanes over the neighbour groups: which can hold an atom in range of the homes' box
-                                const int s = s0 + lane;
-                                bool near = s < s_hi && (o > 0 || s >= own);
+                                const int e = e0 + lane;
+                                int s = o == 0 ? own + e : e;
+                                if (s >= p.nsub) s -= p.nsub;
+                                // half-way round an even number of groups each pair is met twice: the lower has it
+                                bool near = e < e_hi && (o > 0 || 2 * e != p.nsub || 2 * own < p.nsub);
                                 if (near && !far) {
                                     const int q = (int)(((float)s + 0.5f) * p.inv_sub[2]), sz = s - q * p.sub[2];
                                     const int sx = (int)(((float)q + 0.5f) * p.inv_sub[1]), sy = q - sx * p.sub[1];
@@ -568,7 +588,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
                             m &= m - 1u;
                             j = __shfl_sync(0xffffffffu, gs, k);
                             je = j + __shfl_sync(0xffffffffu, gn, k);
-                            if (o == 0 && s0 + k == own) j = h0 + nh;  // the round's own atoms are done
+                            if (o == 0 && e0 + k == 0) j = h0 + nh;  // the round's own atoms are done
                             continue;
                         }
                         bool keep = j + lane < je;
@@ -649,6 +669,45 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     }
 }
 
+// Group of a folded coordinate along one axis: cell, then box within the cell (NaN: the first ones).
+__device__ __forceinline__ int cell_of(float r, float L, int nc, int nsub, int& box) {
+    const float w = r - L * floorf(r / L);
+    const float t = w * ((float)nc / L);
+    int c = (int)t;
+    c = c < 0 ? 0 : (c >= nc ? nc - 1 : c);
+    const int sc = (int)((t - (float)c) * (float)nsub);
+    box = sc < 0 ? 0 : (sc >= nsub ? nsub - 1 : sc);
+    return c;
+}
+
+// Key, cell, cell flags (bit 0: a coordinate outside [0, L); bit 1: outside [-L, L) or NaN) and frame flags of
+// an atom.
+struct AtomCell {
+    int key, cell;
+    int flag;
+    unsigned frame;
+};
+__device__ __forceinline__ AtomCell place(const float4& v, const RdfParams& p) {
+    const float r[3] = {v.x, v.y, v.z};
+    int k[3], sub[3];
+    bool outside = false, far = false;
+    AtomCell a;
+    a.frame = 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float L = p.g.L[d];
+        outside |= !(r[d] >= 0.0f && r[d] < L);
+        far |= !(r[d] >= -L && r[d] < L);
+        a.frame |= (r[d] < -0.499f * L ? kFrameLow : 0u) | (r[d] < -0.749f * L ? kFrameVeryLow : 0u) |
+                   (r[d] >= 0.749f * L ? kFrameHigh : 0u);
+        k[d] = cell_of(r[d], L, p.nc[d], p.sub[d], sub[d]);
+    }
+    a.cell = (k[0] * p.nc[1] + k[1]) * p.nc[2] + k[2];
+    a.key = a.cell * p.nsub + (sub[0] * p.sub[1] + sub[1]) * p.sub[2] + sub[2];
+    a.flag = outside ? (far ? 3 : 1) : 0;
+    return a;
+}
+
 // Cell of each atom from its wrapped coordinate, and its group: the cell is divided into sub[0] x sub[1] x
 // sub[2] boxes numbered z fastest, so atoms sorted by key = cell * nsub + box are cell-contiguous and
 // grouped by box.  Per-key counts and slots, cell and frame flags.
@@ -660,33 +719,13 @@ __global__ void cell_assign_kernel(const float4* __restrict__ packed, int64_t n,
     unsigned ff = 0;
     if (i < n) {
         const float4 v = packed[i];
-        const float r[3] = {v.x, v.y, v.z};
-        int k[3], sub[3];
-        bool outside = false, far = false;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float L = p.g.L[d];
-            outside |= !(r[d] >= 0.0f && r[d] < L);
-            far |= !(r[d] >= -L && r[d] < L);
-            ff |= (r[d] < -0.499f * L ? kFrameLow : 0u) | (r[d] < -0.749f * L ? kFrameVeryLow : 0u) |
-                  (r[d] >= 0.749f * L ? kFrameHigh : 0u);
-            const float w = r[d] - L * floorf(r[d] / L);
-            const float t = w * ((float)p.nc[d] / L);
-            int c = (int)t;
-            c = c < 0 ? 0 : (c >= p.nc[d] ? p.nc[d] - 1 : c);
-            k[d] = c;
-            const int sc = (int)((t - (float)c) * (float)p.sub[d]);
-            sub[d] = sc < 0 ? 0 : (sc >= p.sub[d] ? p.sub[d] - 1 : sc);  // also catches NaN coordinates (sc = 0)
-        }
-        const int c = (k[0] * p.nc[1] + k[1]) * p.nc[2] + k[2];
-        const int key = c * p.nsub + (sub[0] * p.sub[1] + sub[1]) * p.sub[2] + sub[2];
+        const AtomCell c = place(v, p);
+        ff = c.frame;
         // A species outside 0..nsp-1 can only come from a frame already flagged as bad data: not placed.
         const bool ok = __float_as_uint(v.w) < (unsigned)p.g.nsp;
-        akey[i] = ok ? key : -1;
-        if (ok) aslot[i] = atomicAdd(&fcount[key], 1);
-        // bit 0: a coordinate outside [0, L) (pairs of the cell need the minimum image);
-        // bit 1: a coordinate outside [-L, L) or NaN (its wrapped value is not x or x + L: no cull)
-        if (outside) atomicOr(&cflag[c], far ? 3 : 1);
+        akey[i] = ok ? c.key : -1;
+        if (ok) aslot[i] = atomicAdd(&fcount[c.key], 1);
+        if (c.flag) atomicOr(&cflag[c.cell], c.flag);
     }
     ff = __reduce_or_sync(0xffffffffu, ff);
     if ((threadIdx.x & 31) == 0 && (ff & ~*(volatile unsigned*)fflag)) atomicOr(fflag, ff);
@@ -721,40 +760,157 @@ __global__ void __launch_bounds__(256) group_offsets_kernel(const int32_t* __res
     if (k < nkey) fstart[k] = base + wsum[warp] + x - v;
 }
 
+// Sum over a block of v (FP64, fixed order): warp shuffles, then warps in order; thread 0 has it.
+__device__ __forceinline__ double block_sum(double v, double* red) {
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v += red[w];
+    return v;
+}
+
+// q2[block]: sum of the block's squared charges (frames with charges).
 __global__ void cell_scatter_kernel(const float4* __restrict__ packed, int64_t n,
                                     const int32_t* __restrict__ akey, const int32_t* __restrict__ aslot,
                                     const int32_t* __restrict__ fstart, unsigned wscale, float4* __restrict__ sorted,
-                                    const float* __restrict__ q, float* __restrict__ sorted_q) {
+                                    const float* __restrict__ q, float* __restrict__ sorted_q,
+                                    double* __restrict__ q2) {
+    __shared__ double red[32];
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int key = akey[i];
-    if (key < 0) return;
-    const int64_t d = fstart[key] + aslot[i];
-    float4 v = packed[i];
-    v.w = __uint_as_float(__float_as_uint(v.w) * wscale);  // species as the pair kernel adds it to addresses
-    sorted[d] = v;
-    if (q) sorted_q[d] = q[i];
+    const int key = i < n ? akey[i] : -1;
+    const float qi = q && i < n ? q[i] : 0.f;
+    if (key >= 0) {
+        const int64_t d = fstart[key] + aslot[i];
+        float4 v = packed[i];
+        v.w = __uint_as_float(__float_as_uint(v.w) * wscale);  // species as the pair kernel adds it to addresses
+        sorted[d] = v;
+        if (q) sorted_q[d] = qi;
+    }
+    if (q) {
+        const double s = block_sum((double)qi * (double)qi, red);
+        if (threadIdx.x == 0) q2[blockIdx.x] = s;
+    }
+}
+
+// The whole cell sort of a small frame in one CTA, counts in shared memory: one launch instead of a memset and
+// three kernels, which between them cost more than the sort.  Each thread keeps its atoms' keys in registers.
+constexpr int kSmallThreads = 1024, kSmallRounds = 8;
+constexpr int kSmallAtoms = kSmallThreads * kSmallRounds;
+constexpr int kSmallKeys = 4096;  // most groups, and most cells, of a frame sorted this way
+__global__ void __launch_bounds__(kSmallThreads) cell_sort_small_kernel(
+    const float4* __restrict__ packed, int n, const __grid_constant__ RdfParams p, int ncell, int nkey, unsigned wscale,
+    unsigned* __restrict__ work, unsigned* __restrict__ fflag, int32_t* __restrict__ cflag, int32_t* __restrict__ fcount,
+    int32_t* __restrict__ fstart, float4* __restrict__ sorted, const float* __restrict__ q,
+    float* __restrict__ sorted_q, double* __restrict__ q2) {
+    __shared__ double red[32];
+    __shared__ int cnt[kSmallKeys], flag[kSmallKeys], wsum[32];
+    __shared__ unsigned frame;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int k = tid; k < nkey; k += kSmallThreads) cnt[k] = 0;
+    for (int k = tid; k < ncell; k += kSmallThreads) flag[k] = 0;
+    if (tid == 0) frame = 0u;
+    __syncthreads();
+    int key[kSmallRounds], slot[kSmallRounds];
+    unsigned ff = 0;
+#pragma unroll
+    for (int r = 0; r < kSmallRounds; ++r) {
+        const int i = r * kSmallThreads + tid;
+        key[r] = -1;
+        if (i < n) {
+            const float4 v = packed[i];
+            const AtomCell c = place(v, p);
+            ff |= c.frame;
+            if (__float_as_uint(v.w) < (unsigned)p.g.nsp) {
+                key[r] = c.key;
+                slot[r] = atomicAdd(&cnt[c.key], 1);
+            }
+            if (c.flag) atomicOr(&flag[c.cell], c.flag);
+        }
+    }
+    if (ff) atomicOr(&frame, ff);
+    __syncthreads();
+    // starts: every thread scans kSmallKeys / kSmallThreads consecutive keys
+    constexpr int kPer = kSmallKeys / kSmallThreads;
+    int v[kPer], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int g = tid * kPer + k;
+        v[k] = g < nkey ? cnt[g] : 0;
+        sum += v[k];
+    }
+    int x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    int w = wsum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += y;
+    }
+    const int before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+    int run = (warp > 0 ? before : 0) + x - sum;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int g = tid * kPer + k;
+        if (g < nkey) {
+            fstart[g] = run;
+            fcount[g] = v[k];
+            cnt[g] = run;
+        }
+        run += v[k];
+    }
+    for (int k = tid; k < ncell; k += kSmallThreads) cflag[k] = flag[k];
+    if (tid == 0) {
+        *work = 0u;
+        *fflag = frame;
+    }
+    __syncthreads();
+    double s2 = 0.0;
+#pragma unroll
+    for (int r = 0; r < kSmallRounds; ++r) {
+        const int i = r * kSmallThreads + tid;
+        const float qi = q && i < n ? q[i] : 0.f;
+        s2 += (double)qi * (double)qi;
+        if (key[r] >= 0) {
+            const int d = cnt[key[r]] + slot[r];
+            float4 a = packed[i];
+            a.w = __uint_as_float(__float_as_uint(a.w) * wscale);
+            sorted[d] = a;
+            if (q) sorted_q[d] = qi;
+        }
+    }
+    if (q) {
+        s2 = block_sum(s2, red);
+        if (tid == 0) q2[0] = s2;
+    }
 }
 
 // One block, after the pair kernel: avq2 = sum(q^2)/N in FP64 rounded to FP32 (rdf.cuf:272, where
-// avq2 is a default-real variable), then gqq += gqq_frame/avq2 (rdf.cuf:273).  The reduction order
-// is fixed, so avq2 does not depend on scheduling.
-__global__ void gqq_finish_kernel(const float* __restrict__ q, int64_t n, const double* __restrict__ gqq_frame,
-                                  int lsmax, double* __restrict__ gqq) {
-    __shared__ double part[1024];
+// avq2 is a default-real variable) from the sorting blocks' sums, then gqq += gqq_frame/avq2 (rdf.cuf:273).
+// The order is fixed, so avq2 does not depend on scheduling.
+__global__ void __launch_bounds__(1024) gqq_finish_kernel(const double* __restrict__ q2, int nparts, int64_t n,
+                                                          const double* __restrict__ gqq_frame, int lsmax,
+                                                          double* __restrict__ gqq) {
+    __shared__ double red[32], total;
     double s = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const double v = (double)q[i];
-        s += v * v;
-    }
-    part[threadIdx.x] = s;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nparts; i += 1024) s += q2[i];
+    s = block_sum(s, red);
+    if (threadIdx.x == 0) total = s;
     __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-        if ((int)threadIdx.x < off) part[threadIdx.x] += part[threadIdx.x + off];
-        __syncthreads();
-    }
-    const float avq2 = (float)(part[0] / (double)n);
-    for (int k = threadIdx.x; k < lsmax; k += blockDim.x) gqq[k] += gqq_frame[k] / (double)avq2;
+    const float avq2 = (float)(total / (double)n);
+    for (int k = threadIdx.x; k < lsmax; k += 1024) gqq[k] += gqq_frame[k] / (double)avq2;
+}
+
+// The squared charge of a one-atom frame, which has no pairs and is not sorted.
+__global__ void one_charge_kernel(const float* __restrict__ q, double* __restrict__ q2) {
+    q2[0] = (double)q[0] * (double)q[0];
 }
 
 // Number fluctuations (s2D3_sh, rdf.cuf:489-553): block b draws one point uniformly in the box with
@@ -1028,6 +1184,7 @@ struct trj_rdf_plan {
     int cells_valid = 0;        // sorted, fstart and the counts hold the last accumulated frame
     float box_last[3] = {0.f, 0.f, 0.f};
     double* gqq_frame = nullptr;  // lsmax: this frame's charge-product sums
+    double* q2_part = nullptr;    // one per sorting block: sums of squared charges
     int64_t scratch_bytes = 0;
     trj_kernel_timer timer;
 };
@@ -1094,6 +1251,17 @@ static void fill_geom(PairGeom& g, const float box[3], float side2, float deltar
     g.row_words = lsmax + 2;
     g.want_edge = want_edge;
     g.one = 1.0f;
+}
+
+static FastDiv make_fast_div(int d) {
+    FastDiv f = {(unsigned)d, 0u, 0};
+    if (d > 1) {
+        int l = 0;
+        while ((1ll << l) < d) ++l;
+        f.mul = (unsigned)((((unsigned long long)1 << (31 + l)) + d - 1) / d);
+        f.shift = l - 1;
+    }
+    return f;
 }
 
 // Volume (2D: area) of the region within r of a box of edges e: what the homes of one group are tested against.
@@ -1325,12 +1493,14 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
     cudaStream_t s = (cudaStream_t)stream;
     if (charged && !plan->sorted_q) {
         const size_t nq = (size_t)std::max<int64_t>(plan->n_max, 1);
-        const size_t qbytes = ((nq * sizeof(float) + 255) & ~(size_t)255) + sizeof(double) * (size_t)plan->lsmax;
+        const size_t charges = (nq * sizeof(float) + 255) & ~(size_t)255, blocks = (nq + 255) / 256;
+        const size_t qbytes = charges + sizeof(double) * ((size_t)plan->lsmax + blocks);
         char* qb = nullptr;
         if (trj_dev_alloc(ctx, (void**)&qb, qbytes) != cudaSuccess)
             return trj_fail(ctx, TRJ_ERR_NOMEM, "rdf accumulate: %zu bytes of charge scratch", qbytes);
         plan->sorted_q = reinterpret_cast<float*>(qb);
-        plan->gqq_frame = reinterpret_cast<double*>(qb + ((nq * sizeof(float) + 255) & ~(size_t)255));
+        plan->gqq_frame = reinterpret_cast<double*>(qb + charges);
+        plan->q2_part = plan->gqq_frame + plan->lsmax;
         plan->scratch_bytes += (int64_t)qbytes;
     }
     plan->cells_valid = 0;
@@ -1338,8 +1508,9 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
         // No pair; gqq still receives 0/avq2 per bin, as the reference adds gqq_d/avq2 every frame.
         if (charged && n == 1) {
             TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->gqq_frame, 0, sizeof(double) * plan->lsmax, s));
-            gqq_finish_kernel<<<1, 1024, 0, s>>>(charge_dev, n, plan->gqq_frame, plan->lsmax, gqq_dev);
-            ctx->launches += 1;
+            one_charge_kernel<<<1, 1, 0, s>>>(charge_dev, plan->q2_part);
+            gqq_finish_kernel<<<1, 1024, 0, s>>>(plan->q2_part, 1, n, plan->gqq_frame, plan->lsmax, gqq_dev);
+            ctx->launches += 2;
             TRJ_CUDA_TRY(ctx, cudaGetLastError());
         }
         return TRJ_OK;
@@ -1393,19 +1564,24 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
                 P.off[no][2] = dz;
                 ++no;
             }
-    P.noff = no;
     // Launch shape: as many warps per SM as the histogram leaves room for, with a row per ordered species
     // pair where that costs no warps.
     PairShape shape;
     if (!pair_shape(ctx, plan->nsp, plan->nit, P.g.row_words, charged, &shape))
         return trj_fail(ctx, TRJ_ERR_UNSUPPORTED, "rdf accumulate: histogram too large");
     // Segments: about twelve items per resident warp, so that the last ones end together (six: 62,500 atoms
-    // 485 us instead of 455; twenty-four: 459), but at least six neighbour groups per item.
+    // 485 us instead of 455; twenty-four: 459), but at least two neighbour groups per item.
     const int64_t warps = (int64_t)ctx->sm_count * shape.ctas * shape.warps;
-    const int64_t list = (int64_t)P.noff * P.nsub;
-    P.nseg = (int)std::max<int64_t>(1, std::min<int64_t>((12 * warps + nkey - 1) / nkey, list / 6));
-    P.per_seg = (int)((list + P.nseg - 1) / P.nseg);
-    P.nitems = (unsigned)nkey * (unsigned)P.nseg;  // below 2^32: nseg > 1 only for few keys
+    P.nself = P.nsub / 2 + 1;
+    P.list = P.nself + (no - 1) * P.nsub;
+    P.nseg = (int)std::max<int64_t>(1, std::min<int64_t>((12 * warps + nkey - 1) / nkey, P.list / 2));
+    P.per_seg = (P.list + P.nseg - 1) / P.nseg;
+    P.nseg = (P.list + P.per_seg - 1) / P.per_seg;
+    P.div_nsub = make_fast_div(P.nsub);
+    P.div_nc1 = make_fast_div(P.nc[1]);
+    P.div_nc2 = make_fast_div(P.nc[2]);
+    P.div_nseg = make_fast_div(P.nseg);
+    P.nitems = (unsigned)nkey * (unsigned)P.nseg;  // below 2^31: nseg > 1 only for few keys
 
     const PairKernel kern = pair_kernel(plan->floor_bins, charged, shape.square, edge_dev != nullptr);
     TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem));
@@ -1419,13 +1595,26 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
     plan->fcount_last = fcount;
     plan->nsub = P.nsub;
     for (int d = 0; d < 3; ++d) plan->grid_nc[d] = P.nc[d];
-    TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->zeroed, 0, sizeof(int32_t) * (size_t)(4 + ncell + nkey), s));
-    unsigned nb = (unsigned)((n + 255) / 256);
-    cell_assign_kernel<<<nb, 256, 0, s>>>((const float4*)packed_dev, n, P, fcount, cflag, fflag, plan->akey,
-                                          plan->aslot);
-    group_offsets_kernel<<<(unsigned)((nkey + 255) / 256), 256, 0, s>>>(fcount, nkey, total, plan->fstart);
-    cell_scatter_kernel<<<nb, 256, 0, s>>>((const float4*)packed_dev, n, plan->akey, plan->aslot, plan->fstart,
-                                           shape.square ? 4u * (unsigned)P.g.row_words : 64u, plan->sorted, charged ? charge_dev : nullptr, plan->sorted_q);
+    const unsigned wscale = shape.square ? 4u * (unsigned)P.g.row_words : 64u;
+    const float* q_dev = charged ? charge_dev : nullptr;
+    int q2_parts = 0;  // sums of squared charges, one per sorting block
+    if (n <= kSmallAtoms && nkey <= kSmallKeys) {
+        cell_sort_small_kernel<<<1, kSmallThreads, 0, s>>>((const float4*)packed_dev, (int)n, P, ncell, nkey, wscale, work,
+                                                           fflag, cflag, fcount, plan->fstart, plan->sorted, q_dev,
+                                                           plan->sorted_q, plan->q2_part);
+        q2_parts = 1;
+        ctx->launches += 1;
+    } else {
+        TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->zeroed, 0, sizeof(int32_t) * (size_t)(4 + ncell + nkey), s));
+        const unsigned nb = (unsigned)((n + 255) / 256);
+        cell_assign_kernel<<<nb, 256, 0, s>>>((const float4*)packed_dev, n, P, fcount, cflag, fflag, plan->akey,
+                                              plan->aslot);
+        group_offsets_kernel<<<(unsigned)((nkey + 255) / 256), 256, 0, s>>>(fcount, nkey, total, plan->fstart);
+        cell_scatter_kernel<<<nb, 256, 0, s>>>((const float4*)packed_dev, n, plan->akey, plan->aslot, plan->fstart,
+                                               wscale, plan->sorted, q_dev, plan->sorted_q, plan->q2_part);
+        q2_parts = (int)nb;
+        ctx->launches += 3;
+    }
     if (charged) TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->gqq_frame, 0, sizeof(double) * plan->lsmax, s));
     const int64_t grid = std::min<int64_t>((int64_t)ctx->sm_count * shape.ctas,
                                            ((int64_t)P.nitems + shape.warps - 1) / shape.warps);
@@ -1436,9 +1625,9 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
                                                               charged ? plan->gqq_frame : nullptr);
     plan->timer.end(ctx, s);
     plan->cells_valid = 1;
-    ctx->launches += 4;
+    ctx->launches += 1;
     if (charged) {
-        gqq_finish_kernel<<<1, 1024, 0, s>>>(charge_dev, n, plan->gqq_frame, plan->lsmax, gqq_dev);
+        gqq_finish_kernel<<<1, 1024, 0, s>>>(plan->q2_part, q2_parts, n, plan->gqq_frame, plan->lsmax, gqq_dev);
         ctx->launches += 1;
     }
     TRJ_CUDA_TRY(ctx, cudaGetLastError());
