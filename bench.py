@@ -380,7 +380,7 @@ def run_serving(n_req, seed=5):
                    "fused_turns": srv.fuse_turns - c0[2], "fuse_max_atoms": srv.fuse_max_atoms,
                    "batch_device_bytes": srv.batch.device_bytes if srv.batch is not None else 0,
                    "note": "offline run: requests packed into fused launches, their frames, and the fused "
-                           "launches (each one table copy + five kernels, replayed from a CUDA graph)"}
+                           "launches (each one table copy + eight kernels, replayed from a CUDA graph)"}
 
     def poisson(load, seed_):
         rng = np.random.default_rng(seed_)
@@ -747,7 +747,7 @@ def run_fused(args):
             "higher_is_better": True, "dtype": "f32 terms, f64 sums", "data": "synthetic",
             "config": {"workload": "64 serving requests, N log-uniform [1e3, 16384]", "atoms": int(n.sum()),
                        "kvec": int(nvec.sum()), "l2": "256 MB buffer written between steps"},
-            "fused": {"ms": f_ms, "launches": 5, "copies": 1, "pair_tests_per_s": pairs / (f_ms * 1e-3),
+            "fused": {"ms": f_ms, "launches": 8, "copies": 1, "pair_tests_per_s": pairs / (f_ms * 1e-3),
                       "sq_terms_per_s": terms / (f_ms * 1e-3)},
             "per_request": {"ms": u_ms, "launches": unfused_launches, "frames_per_s": 64.0 / (u_ms * 1e-3)},
             "fused_vs_per_request": u_ms / f_ms, "launches_before_timing": int(launches0)}

@@ -341,8 +341,8 @@ TRJ_API int trj_dyn_plan_destroy(trj_dyn_plan* plan);
  * launch rdf.cuf:240 and SQcalc's sqfnD launch sq.cuf:89).  A batch runs one
  * frame of each of up to max_items requests per turn through one fixed launch
  * sequence: a copy of the turn's descriptor table, frame layout (fold, species
- * order, fixed-point phases; select_ncdfinput), an all-pairs histogram with
- * rdf_sh's arithmetic (rdf.cuf:449-475) and the FP32 direct sum with FP64 shell
+ * order, fixed-point phases; select_ncdfinput), a pair histogram with rdf_sh's
+ * arithmetic (rdf.cuf:449-475) over a cell sort and the FP32 direct sum with FP64 shell
  * sums (the plain method of trj_sq_accumulate), every kernel over the work of
  * all the turn's frames.  The sequence does not depend on what the table holds,
  * so a CUDA graph captured once per staging buffer replays every later turn.
@@ -352,7 +352,7 @@ TRJ_API int trj_dyn_plan_destroy(trj_dyn_plan* plan);
  * executes.  Counts are those of trj_rdf_accumulate and S(Q) sums those of
  * trj_sq_accumulate(TRJ_SQ_PLAIN_FP32) for the same plans, bit for bit.
  * max_atoms: staged atoms per turn; hist_words: the largest nit*lsmax of a
- * pair plan the batch takes (shared memory: 8 bytes per word + 4 KB). */
+ * pair plan the batch takes (shared memory: 8 bytes per word + 20 KB). */
 TRJ_API int trj_batch_create(trj_ctx* ctx, int max_items, int64_t max_atoms, int hist_words, trj_batch** out);
 /* Host staging of buffer buf: xyz[3 * max_atoms] float and species[max_atoms]
  * int32 (0-based species ids), pinned and mapped into the device's address
@@ -362,8 +362,8 @@ TRJ_API int trj_batch_staging(trj_batch* batch, int buf, float** xyz_host, int32
 TRJ_API int trj_batch_begin(trj_batch* batch, int buf);
 /* Adds one frame of one request: atoms [atom_off, atom_off + n) of the
  * staging, items in increasing atom order.  rdf: the request's pair plan (its
- * cutoff, clipped per frame as trj_rdf_accumulate does, bins and species; its
- * cell arrays are not used, so it may be created with n_max 0) or NULL; sq: its
+ * cutoff, clipped per frame as trj_rdf_accumulate does, bins and species; the
+ * batch has cell arrays of its own, so it may be created with n_max 0) or NULL; sq: its
  * S(Q) plan (uncharged; species counts summing to n; its partial-sum scratch is
  * used) or NULL.  Accumulates into hist_dev ([nit][lsmax] uint64), edge_dev
  * (TRJ_EDGE_* counters, may be NULL) and sq_out_dev ([nbins][nit] double) as
@@ -372,9 +372,9 @@ TRJ_API int trj_batch_begin(trj_batch* batch, int buf);
 TRJ_API int trj_batch_add(trj_batch* batch, int buf, trj_rdf_plan* rdf, trj_sq_plan* sq, int64_t atom_off,
                           int64_t n, const float box[3], uint64_t* hist_dev, uint64_t* edge_dev,
                           double* sq_out_dev);
-/* Enqueues the turn of buffer buf on stream: one table copy and five kernels. */
+/* Enqueues the turn of buffer buf on stream: one table copy, one clear and eight kernels. */
 TRJ_API int trj_batch_launch(trj_batch* batch, int buf, void* stream);
-/* Items and work units (layout, pair tiles, direct-sum blocks, shell bins) of
+/* Items and work units (layout, pair items, direct-sum blocks, shell bins) of
  * buffer buf's turn; device memory the batch holds. */
 TRJ_API int trj_batch_info(const trj_batch* batch, int buf, int* nitems, int64_t units[4], int64_t* device_bytes);
 /* Duration (ms) of the last launched turn's kernels; needs timing enabled. */

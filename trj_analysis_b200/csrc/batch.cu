@@ -7,7 +7,7 @@
 // turn and runs the same fixed sequence of launches for all of them:
 //
 //   copy of the pinned descriptor table -> layout count -> layout scatter (fold, species order,
-//   fixed-point phases) -> all-pairs histogram -> direct sum -> shell reduction
+//   fixed-point phases) -> cell sort -> pair histogram -> direct sum -> shell reduction
 //
 // Grids and arguments depend only on the batch's capacity, so a CUDA graph captured once per staging
 // buffer replays any mix of requests: the host rewrites the table and the staged atoms between turns.
@@ -36,6 +36,9 @@ struct trj_batch {
         uint4* phase = nullptr;               // device: fixed-point phase entries
         int32_t* chunk_counts = nullptr;      // device: species counts per layout unit
         int64_t atoms_end = 0;                // end of the last item's atoms
+        BatchSort sort = {};                  // device: cell sort of the pair histogram (sorted shares `raw`)
+        size_t zero_bytes = 0;                // of sort.state, fcount and cflag
+        int64_t key_cap = 0;
         int64_t chunk_cap = 0;
         BatchHeader* hdr() { return reinterpret_cast<BatchHeader*>(table_host); }
         BatchItem* items() { return reinterpret_cast<BatchItem*>(table_host + sizeof(BatchHeader)); }
@@ -72,8 +75,11 @@ extern "C" int trj_batch_create(trj_ctx* ctx, int max_items, int64_t max_atoms, 
     auto a256 = [](size_t x) { return (x + 255) & ~(size_t)255; };
     for (auto& B : b->buf) {
         B.chunk_cap = (max_atoms + kBatchChunk - 1) / kBatchChunk + max_items;
+        B.key_cap = max_atoms / 8 + (int64_t)max_items * (64 + 32);
+        B.zero_bytes = sizeof(unsigned) * 4 * (size_t)max_items + 2 * sizeof(int32_t) * (size_t)B.key_cap;
         const size_t dev = a256(b->table_bytes) + 3 * a256(sizeof(float4) * (size_t)max_atoms) +
-                           a256(sizeof(int32_t) * kBatchMaxSpecies * (size_t)B.chunk_cap);
+                           a256(sizeof(int32_t) * kBatchMaxSpecies * (size_t)B.chunk_cap) + a256(B.zero_bytes) +
+                           a256(sizeof(int32_t) * (size_t)B.key_cap) + 2 * a256(sizeof(int32_t) * (size_t)max_atoms);
         if (cudaHostAlloc((void**)&B.table_host, b->table_bytes, cudaHostAllocDefault) != cudaSuccess ||
             cudaHostAlloc((void**)&B.xyz_host, sizeof(float) * 3 * (size_t)max_atoms,
                           cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
@@ -99,6 +105,17 @@ extern "C" int trj_batch_create(trj_ctx* ctx, int max_items, int64_t max_atoms, 
         B.phase = reinterpret_cast<uint4*>(p);
         p += a256(sizeof(float4) * (size_t)max_atoms);
         B.chunk_counts = reinterpret_cast<int32_t*>(p);
+        p += a256(sizeof(int32_t) * kBatchMaxSpecies * (size_t)B.chunk_cap);
+        B.sort.state = reinterpret_cast<unsigned*>(p);
+        B.sort.fcount = reinterpret_cast<int32_t*>(B.sort.state + 4 * (size_t)max_items);
+        B.sort.cflag = B.sort.fcount + B.key_cap;
+        p += a256(B.zero_bytes);
+        B.sort.fstart = reinterpret_cast<int32_t*>(p);
+        p += a256(sizeof(int32_t) * (size_t)B.key_cap);
+        B.sort.akey = reinterpret_cast<int32_t*>(p);
+        p += a256(sizeof(int32_t) * (size_t)max_atoms);
+        B.sort.aslot = reinterpret_cast<int32_t*>(p);
+        B.sort.sorted = B.raw;  // the staged atoms are read for the last time by the layout
         b->device_bytes += (int64_t)dev;
         memset(B.table_host, 0, b->table_bytes);
     }
@@ -174,6 +191,7 @@ extern "C" int trj_batch_add(trj_batch* b, int buf, trj_rdf_plan* rdf, trj_sq_pl
     for (int d = 0; d < 3; ++d) it.L[d] = box[d];
     for (int a = 0; a <= kBatchMaxSpecies; ++a) it.sp_off[a] = -1;  // g(r) only: atoms keep their order
     int nsp = 0;
+    int64_t nkey = 0;
     if (sq) {
         int rc = trj_batch_fill_sq(sq, n, &it);
         if (rc != TRJ_OK) return rc;
@@ -182,7 +200,7 @@ extern "C" int trj_batch_add(trj_batch* b, int buf, trj_rdf_plan* rdf, trj_sq_pl
     }
     if (rdf) {
         int p_nsp = 0;
-        int rc = trj_batch_fill_rdf(rdf, box, b->hist_words, &it, &p_nsp);
+        int rc = trj_batch_fill_rdf(rdf, n, box, b->hist_words, edge_dev != nullptr, &it, &p_nsp, &nkey);
         if (rc != TRJ_OK) return rc;
         if (sq && p_nsp != nsp)
             return trj_fail(ctx, TRJ_ERR_INVALID, "batch: pair plan has %d species, S(Q) plan %d", p_nsp, nsp);
@@ -192,15 +210,19 @@ extern "C" int trj_batch_add(trj_batch* b, int buf, trj_rdf_plan* rdf, trj_sq_pl
     }
     it.nsp = nsp;
     it.nchunk = (int32_t)((n + kBatchChunk - 1) / kBatchChunk);
-    it.ntile = rdf && n >= 2 ? (int32_t)((n + kBatchTile - 1) / kBatchTile) : 0;
     it.chunk_begin = h->total_chunk;
     it.pair_begin = h->total_pair;
     it.sq_begin = h->total_sq;
     it.red_begin = h->total_red;
+    it.key_begin = h->total_key;
     if (h->total_chunk + it.nchunk > B.chunk_cap)
         return trj_fail(ctx, TRJ_ERR_CAPACITY, "batch: layout units exceed %lld", (long long)B.chunk_cap);
+    nkey = (nkey + 31) / 32 * 32;
+    if (h->total_key + nkey > B.key_cap)
+        return trj_fail(ctx, TRJ_ERR_CAPACITY, "batch: pair groups exceed %lld", (long long)B.key_cap);
     h->total_chunk += it.nchunk;
-    h->total_pair += (int64_t)it.ntile * (it.ntile + 1) / 2;
+    h->total_key += nkey;
+    h->total_pair += it.pair.nitems;
     if (sq && it.nvec > 0) {
         h->total_sq += (int64_t)it.nvblk * it.nsplit * it.parts;
         h->total_red += it.nbins;
@@ -227,10 +249,11 @@ extern "C" int trj_batch_launch(trj_batch* b, int buf, void* stream) {
     b->timer.begin(ctx, s);
     trj_batch_launch_layout(hdr, items, B.xyz_map, B.sp_map, B.raw, B.chunk_counts, B.packed, B.phase,
                             ctx->status_dev, b->grid_layout, s);
-    trj_batch_launch_pairs(hdr, items, B.packed, b->hist_words, b->grid_pairs, s);
+    if (trj_batch_launch_pairs(hdr, items, B.packed, B.sort, B.zero_bytes, b->hist_words, b->grid_layout, b->grid_pairs, s))
+        return trj_fail(ctx, TRJ_ERR_CUDA, "batch: clearing the cell sort failed");
     trj_batch_launch_sq(hdr, items, B.phase, ctx->turn_dev, b->grid_sq, b->grid_red, s);
     b->timer.end(ctx, s);
-    ctx->launches += 5;
+    ctx->launches += 8;
     TRJ_CUDA_TRY(ctx, cudaGetLastError());
     return TRJ_OK;
 }

@@ -8,10 +8,10 @@
 // start at its *_begin offset (exclusive prefix over the items before it).
 #pragma once
 
+#include "pairs.cuh"
 #include "trj_common.cuh"
 
 constexpr int kBatchChunk = 1024;        // atoms per layout unit
-constexpr int kBatchTile = 256;          // atoms per side of a pair tile (one home atom per thread)
 constexpr int kBatchThreads = 256;
 constexpr int kBatchMaxSpecies = 16;
 constexpr int kBatchCounters = 4;        // dynamic work counters: pairs, direct sum, reduction, spare
@@ -22,14 +22,11 @@ struct __align__(16) BatchItem {
     int32_t n, nsp;
     float L[3];
     int32_t nchunk;                      // layout units: ceil(n / kBatchChunk)
-    int32_t ntile;                       // pair tiles per side: ceil(n / kBatchTile)
-    int32_t nit;
+    int32_t square;                      // pair rows by ordered species pair (else by ind_ij through a table)
     int64_t sp_off[kBatchMaxSpecies + 1];  // species offsets of the S(Q) plan within the frame
-    // pair histogram (the rdf plan's geometry after the per-frame clip)
-    float h1[3], h2[3], pad_h[3];        // minimum-image thresholds (rdf.cu min_image)
-    float side2, side2_lo, side2_hi, deltar, inv_deltar;
-    int32_t lsmax, floor_bins;
-    unsigned long long* hist;            // [nit][lsmax] accumulator
+    // pair histogram (the rdf plan's geometry after the per-frame clip); pair.nitems work items
+    RdfParams pair;
+    unsigned long long* hist;            // [nit][lsmax] accumulator, null: no pair plan
     unsigned long long* edge;            // edge counters (ulp, fma, counted) or null
     // S(Q) direct sum over the plan's vectors (the plain method of trj_sq_accumulate)
     const int4* vecs;
@@ -45,13 +42,14 @@ struct __align__(16) BatchItem {
     int32_t parts, tv, tg;               // rest of its shape (sq.cu PlainShape)
     // first work unit of the item in each kernel's list
     int64_t chunk_begin, pair_begin, sq_begin, red_begin;
+    int64_t key_begin;                   // first group of the item in the sort's arrays: a multiple of 32
 };
 
 struct __align__(16) BatchHeader {
     unsigned long long counter[kBatchCounters];  // zero in every turn's copy of the table
     int32_t nitems, pad0;
-    int64_t total_chunk, total_pair, total_sq, total_red, total_atoms;
-    int64_t pad1[2];
+    int64_t total_chunk, total_pair, total_sq, total_red, total_atoms, total_key;
+    int64_t pad1[1];
 };
 static_assert(sizeof(BatchHeader) % 16 == 0, "table alignment");
 static_assert(sizeof(BatchItem) % 16 == 0, "table alignment");
@@ -68,13 +66,28 @@ __device__ __forceinline__ int batch_item_of(const BatchItem* __restrict__ items
     return lo;
 }
 
+// Device arrays of the turn's cell sort.  Zeroed together at the start of a turn's pair work: state (per item:
+// pair work counter, atoms placed, frame flags, spare), fcount and cflag.
+struct BatchSort {
+    unsigned* state;
+    int32_t *fcount, *cflag, *fstart;    // per group (cflag: per cell), an item's at its key_begin
+    int32_t *akey, *aslot;               // per atom
+    float4* sorted;                      // per atom: an item's atoms by group
+};
+
+// Most groups of an item of n atoms (choose_groups keeps to it), and the shared-memory words of the pair kernel's
+// bin rows: triangular rows always fit (hist_words plus two words for each of up to 136 rows), square rows are
+// taken where they do.
+inline int64_t batch_keys_most(int64_t n) { return n / 8 + 64; }
+__host__ __device__ inline int batch_hist_smem_words(int hist_words) { return 2 * hist_words + 272; }
+
 // Kernel launchers of the fused turn, each defined beside the single-request kernels whose
 // arithmetic it shares.  grid: CTAs of the fixed-size launch.
 void trj_batch_launch_layout(const BatchHeader* hdr, const BatchItem* items, const float* xyz_staged,
                              const int32_t* sp_staged, float4* raw, int32_t* chunk_counts, float4* packed,
                              uint4* phase, unsigned* status, int grid, cudaStream_t s);        // ctx.cu
-void trj_batch_launch_pairs(BatchHeader* hdr, const BatchItem* items, const float4* packed, int hist_words,
-                            int grid, cudaStream_t s);                                        // rdf.cu
+int trj_batch_launch_pairs(BatchHeader* hdr, const BatchItem* items, const float4* packed, const BatchSort& st,
+                           size_t zero_bytes, int hist_words, int grid_layout, int grid, cudaStream_t s);  // rdf.cu
 size_t trj_batch_pairs_smem(int hist_words);                                                  // rdf.cu
 int trj_batch_pairs_prepare(int hist_words);                                                  // rdf.cu
 int trj_batch_pairs_occupancy(int hist_words, int* per_sm);                                   // rdf.cu
@@ -85,5 +98,6 @@ struct trj_rdf_plan;
 struct trj_sq_plan;
 // Fill the pair part of an item from a plan after the per-frame clip (rdf.cu), and the S(Q) part
 // (sq.cu); non-zero: the plan cannot run in a fused launch (the message is on the context).
-int trj_batch_fill_rdf(trj_rdf_plan* plan, const float box[3], int hist_words, BatchItem* it, int* nsp);
+int trj_batch_fill_rdf(trj_rdf_plan* plan, int64_t n, const float box[3], int hist_words, bool want_edge, BatchItem* it,
+                       int* nsp, int64_t* nkey);
 int trj_batch_fill_sq(trj_sq_plan* plan, int64_t n, BatchItem* it);

@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "batch.cuh"
+#include "pairs.cuh"
 #include "trj_common.cuh"
 
 namespace {
@@ -35,7 +36,6 @@ constexpr double kGroupFill = 28.0;   // average atoms per group aimed at: few g
 constexpr int kRing = 128;            // surviving neighbours buffered per warp (arrays x, y, z, w)
 constexpr int kRingRun = 64;          // survivors tested per run
 constexpr int kMaxWarps = 32;         // per SM: 64 registers a thread (24 warps of 80 registers: 4 % slower at 1e6 atoms)
-constexpr int kMaxOffsets = 14;
 
 typedef unsigned long long u64;
 
@@ -43,52 +43,9 @@ typedef unsigned long long u64;
 // whether |d| < 3L/2 holds for every pair of the frame (see frame_within).
 enum : unsigned { kFrameLow = 1u, kFrameVeryLow = 2u, kFrameHigh = 4u };
 
-// What one pair's test and bin need.
-struct PairGeom {
-    float L[3];
-    float inv_L[3];
-    float h1[3], h2[3];         // |dx| < h1: nint(dx/L) = 0; h1 <= |dx| < h2: +-1; else the division
-    float side2, side2_lo, side2_hi;
-    float side2_win;            // side2_hi - side2, the larger half of that window
-    float deltar, inv_deltar;
-    float edge_thr;             // distance of q from the nearest integer above which a bin edge may be near
-    int lsmax, nsp;
-    int floor_bins;             // 0: bin nint(r/deltar) (reference); 1: bin floor(r/deltar)+1
-    int row_words;              // words of a shared histogram row: lsmax + 2 (first and last: not counted)
-    int want_edge;              // edge statistics are collected
-    float one;                  // 1.0f, from the host: not a constant the assembler could fold
-};
-
-// Division of n < 2^31 by a launch constant: n * ceil(2^(31+l) / d) >> (31+l), l = ceil(log2 d).
-struct FastDiv {
-    unsigned d, mul;
-    int shift;
-};
 __device__ __forceinline__ int fast_div(int n, const FastDiv& f) {
     return f.d == 1u ? n : (int)(__umulhi((unsigned)n, f.mul) >> f.shift);
 }
-
-struct RdfParams {
-    PairGeom g;
-    int nit;
-    int nc[3];                  // cells per axis (1: the axis is not split)
-    int sub[3], nsub;           // groups per cell: sub[0] x sub[1] x sub[2] boxes, z fastest
-    float inv_sub[3];           // 1 / sub
-    float edge[3];              // cell edge
-    float half[3];              // half edge of a group's box, with the cull pad
-    FastDiv div_nsub, div_nc1, div_nc2, div_nseg;
-    // A home group's neighbour list: its own cell's groups at distance 0 .. nsub / 2 after it (cyclically, so
-    // that every group has the same share), then all groups of each further stencil cell.
-    int nself, list;            // entries of the own cell, of the list
-    int nseg, per_seg;          // segments of the list (one work item each); their length
-    int split_all;              // every axis of the geometry is split (in two dimensions: x and y)
-    float cull2;                // (cutoff * (1 + 2^-10))^2: neighbours farther from the homes' box are skipped
-    float cull_pad;             // added to half-widths: covers the FP32 rounding of the cull test
-    long long wait_clocks;      // limit of the stall test's wait
-    int stall_test;             // 1: every warp waits on a barrier nothing arrives on (timeout test)
-    int off[kMaxOffsets][3];
-    unsigned nitems;
-};
 
 // ---- packed FP32 (two independent IEEE operations per instruction, each rounded to nearest once) ----
 __device__ __forceinline__ u64 add2(u64 a, u64 b) {
@@ -385,12 +342,11 @@ __device__ __forceinline__ float axis_gap(float b, float c, float h, float L) {
     return fmaxf(t - h, 0.f);
 }
 
-// The warp's home atoms' bounding box along one axis (wrapped coordinates, in [0, L]: their bit patterns
-// order like the values; + 0 turns -0 into +0).
-__device__ __forceinline__ void axis_box(float v, bool has, float pad, float& c, float& h) {
-    const unsigned b = __float_as_uint(v + 0.0f);
-    const float mn = __uint_as_float(__reduce_min_sync(0xffffffffu, has ? b : 0x7f800000u));
-    const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, has ? b : 0u));
+// A group's bounding box along one axis from the lanes' least and largest wrapped coordinates (in [0, L]: their
+// bit patterns order like the values).
+__device__ __forceinline__ void axis_box(unsigned lo, unsigned hi, float pad, float& c, float& h) {
+    const float mn = __uint_as_float(__reduce_min_sync(0xffffffffu, lo));
+    const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, hi));
     c = 0.5f * (mn + mx);
     h = 0.5f * (mx - mn) + pad;
 }
@@ -399,6 +355,239 @@ __device__ __forceinline__ void axis_box(float v, bool has, float pad, float& c,
 // reaches 0.749 L (frames centred on the origin).  (Coordinates outside [-L, L) are flagged per cell.)
 __device__ __forceinline__ bool frame_within(unsigned f) {
     return !(f & kFrameLow) || !(f & (kFrameVeryLow | kFrameHigh));
+}
+
+// One work item of a frame: home group key = item / nseg against segment item % nseg of its neighbour list.
+// hist: shared-memory address of the bin rows (SQUARE), rowtab: of the row table (otherwise).
+template <bool FLOOR, bool QMODE, bool SQUARE, bool EDGE>
+__device__ __forceinline__ void pair_item(const RdfParams& p, int item, const float4* __restrict__ sorted,
+                                          const int32_t* __restrict__ fstart, const int32_t* __restrict__ fcount,
+                                          const int32_t* __restrict__ cflag, bool frame_ok,
+                                          const float* __restrict__ sorted_q, float* ring, double* ring_q,
+                                          unsigned hist_base, unsigned rowtab, double* qhist, PairCounters& pc,
+                                          u64& n_tested) {
+    const PairGeom& g = p.g;
+    const int lane = (int)(threadIdx.x & 31u);
+    const unsigned lt = (1u << lane) - 1u;
+    const int key = fast_div((int)item, p.div_nseg), seg = (int)item - key * p.nseg;
+    const int hbeg = fstart[key], hend = hbeg + fcount[key];
+    if (hbeg >= hend) return;
+    const int c = fast_div(key, p.div_nsub), own = key - c * p.nsub;
+    const int cxy = fast_div(c, p.div_nc2), cz = c - cxy * p.nc[2];
+    const int cx = fast_div(cxy, p.div_nc1), cy = cxy - cx * p.nc[1];
+    const int fl = cflag[c];
+    const int t0 = seg * p.per_seg, t1 = min(p.list, t0 + p.per_seg);
+    // The group's box: centre and half-widths (of all its atoms, so that the pairs tested do not depend on their
+    // order; + 0 turns -0 into +0).
+    float bx, by, bz, wx, wy, wz;
+    {
+        unsigned lo[3] = {0x7f800000u, 0x7f800000u, 0x7f800000u}, hi[3] = {0u, 0u, 0u};
+        for (int i = hbeg + lane; i < hend; i += kGroup) {
+            const float4 a = sorted[i];
+            const unsigned v[3] = {__float_as_uint(wrap_cull(a.x, g.L[0]) + 0.0f),
+                                   __float_as_uint(wrap_cull(a.y, g.L[1]) + 0.0f),
+                                   __float_as_uint(wrap_cull(a.z, g.L[2]) + 0.0f)};
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                lo[d] = min(lo[d], v[d]);
+                hi[d] = max(hi[d], v[d]);
+            }
+        }
+        axis_box(lo[0], hi[0], p.cull_pad, bx, wx);
+        axis_box(lo[1], hi[1], p.cull_pad, by, wy);
+        axis_box(lo[2], hi[2], p.cull_pad, bz, wz);
+    }
+    for (int h0 = hbeg; h0 < hend; h0 += kGroup) {
+        const int nh = min(kGroup, hend - h0);
+        const bool has = lane < nh;
+        const float4 a = has ? sorted[h0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        Home h;
+        h.nx = -a.x;
+        h.ny = -a.y;
+        h.nz = -a.z;
+        h.q = (QMODE && has) ? sorted_q[h0 + lane] : 0.f;
+        const unsigned wa = __float_as_uint(a.w);  // species * row bytes (64 with the row table)
+        h.hist = SQUARE ? hist_base + wa * (unsigned)g.nsp - 4u * kBinBias : rowtab + (wa >> 4);
+        for (int t = t0; t < t1;) {
+            // entries [e_lo, e_hi) of offset o: group e, or (own cell) the e-th after the homes' own
+            const int o = t < p.nself ? 0 : 1 + fast_div(t - p.nself, p.div_nsub);
+            const int first = o == 0 ? 0 : p.nself + (o - 1) * p.nsub;
+            const int e_lo = t - first, e_hi = min(o == 0 ? p.nself : p.nsub, t1 - first);
+            t = first + e_hi;
+            const int ex = cx + p.off[o][0], ey = cy + p.off[o][1], ez = cz + p.off[o][2];
+            const int c2 = (wrapc(ex, p.nc[0]) * p.nc[1] + wrapc(ey, p.nc[1])) * p.nc[2] + wrapc(ez, p.nc[2]);
+            const int f2 = fl | cflag[c2];
+            const bool far = f2 & 2;
+            const float ix = ex < 0 ? -g.L[0] : (ex >= p.nc[0] ? g.L[0] : 0.f);
+            const float iy = ey < 0 ? -g.L[1] : (ey >= p.nc[1] ? g.L[1] : 0.f);
+            const float iz = ez < 0 ? -g.L[2] : (ez >= p.nc[2] ? g.L[2] : 0.f);
+            const bool plain = p.split_all && !(f2 & 1);  // image known from the cells
+            const int mode = plain ? ((ix != 0.f || iy != 0.f || iz != 0.f) ? kImgShift : kImgNone)
+                                   : far ? kImgAny : p.split_all ? kImgRound : frame_ok ? kImgFold : kImgAny;
+            const int kb = c2 * p.nsub;
+            int head = 0, tail = 0;
+            auto append = [&](const float4& b, float qb, bool keep) {
+                const unsigned m = __ballot_sync(0xffffffffu, keep);
+                if (keep) {
+                    const int e = (tail + __popc(m & lt)) & (kRing - 1);
+                    ring[e] = b.x;
+                    ring[kRing + e] = b.y;
+                    ring[2 * kRing + e] = b.z;
+                    ring[3 * kRing + e] = b.w;
+                    if (QMODE) ring_q[e] = (double)qb;
+                }
+                tail += __popc(m);
+            };
+            // Fills the buffer up to a multiple of four with NaN entries (in no range, near no edge).
+            auto pad = [&]() {
+                const int n = tail - head, up = (n + 3) & ~3;
+                if (lane < up - n) {
+                    const int e = (tail + lane) & (kRing - 1);
+                    ring[e] = ring[kRing + e] = ring[2 * kRing + e] = NAN;
+                    ring[3 * kRing + e] = 0.f;
+                    if (QMODE) ring_q[e] = 0.0;
+                }
+                return up >> 2;
+            };
+#define TRJ_RUN(M, S, N4) test_run<M, S, FLOOR, QMODE, SQUARE, EDGE>(ring, ring_q, head, N4, h, has, ix, iy, iz, g, pc, qhist)
+            if (o == 0 && e_lo == 0) {
+                // pairs j > i of the round's own atoms, through the buffer in lane order
+                append(a, h.q, has);
+                const int n4 = pad();
+                __syncwarp();
+                if (plain) TRJ_RUN(kImgNone, true, n4);
+                else if (mode == kImgRound) TRJ_RUN(kImgRound, true, n4);
+                else if (mode == kImgFold) TRJ_RUN(kImgFold, true, n4);
+                else TRJ_RUN(kImgAny, true, n4);
+                __syncwarp();
+                if (EDGE && has) n_tested += (unsigned)(nh - 1 - lane);
+                tail = 0;
+            }
+            int e0 = e_lo - 32, j = 0, je = 0, gs = 0, gn = 0;  // gs, gn: start and atoms of lane's group
+            unsigned m = 0;
+            bool more = true;
+            do {
+                // survivors into the buffer until a run is full or the segment's groups are used up
+                while (tail - head < kRingRun) {
+                    if (j >= je) {
+                        if (!m) {
+                            e0 += 32;
+                            if (e0 >= e_hi) {
+                                more = false;
+                                break;
+                            }
+                            // lanes over the neighbour groups: which can hold an atom in range of the homes' box
+                            const int e = e0 + lane;
+                            int s = o == 0 ? own + e : e;
+                            if (s >= p.nsub) s -= p.nsub;
+                            // half-way round an even number of groups each pair is met twice: the lower has it
+                            bool near = e < e_hi && (o > 0 || 2 * e != p.nsub || 2 * own < p.nsub);
+                            if (near && !far) {
+                                const int q = (int)(((float)s + 0.5f) * p.inv_sub[2]), sz = s - q * p.sub[2];
+                                const int sx = (int)(((float)q + 0.5f) * p.inv_sub[1]), sy = q - sx * p.sub[1];
+                                const float gx = ((float)ex + ((float)sx + 0.5f) * p.inv_sub[0]) * p.edge[0];
+                                const float gy = ((float)ey + ((float)sy + 0.5f) * p.inv_sub[1]) * p.edge[1];
+                                const float gz = ((float)ez + ((float)sz + 0.5f) * p.inv_sub[2]) * p.edge[2];
+                                float dx, dy, dz;
+                                if (p.split_all) {
+                                    dx = axis_gap<false>(gx, bx, wx + p.half[0], 0.f);
+                                    dy = axis_gap<false>(gy, by, wy + p.half[1], 0.f);
+                                    dz = axis_gap<false>(gz, bz, wz + p.half[2], 0.f);
+                                } else {
+                                    dx = axis_gap<true>(gx - ix, bx, wx + p.half[0], g.L[0]);
+                                    dy = axis_gap<true>(gy - iy, by, wy + p.half[1], g.L[1]);
+                                    dz = axis_gap<true>(gz - iz, bz, wz + p.half[2], g.L[2]);
+                                }
+                                near = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
+                            }
+                            if (near) {
+                                gs = fstart[kb + s];
+                                gn = fcount[kb + s];
+                            }
+                            m = __ballot_sync(0xffffffffu, near);
+                            continue;
+                        }
+                        const int k = __ffs(m) - 1;
+                        m &= m - 1u;
+                        j = __shfl_sync(0xffffffffu, gs, k);
+                        je = j + __shfl_sync(0xffffffffu, gn, k);
+                        if (o == 0 && e0 + k == 0) j = h0 + nh;  // the round's own atoms are done
+                        continue;
+                    }
+                    bool keep = j + lane < je;
+                    const float4 b = keep ? sorted[j + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float qb = (QMODE && keep) ? sorted_q[j + lane] : 0.f;
+                    j += 32;
+                    if (keep && !far) {
+                        float dx, dy, dz;
+                        if (plain) {
+                            dx = axis_gap<false>(b.x, bx - ix, wx, 0.f);
+                            dy = axis_gap<false>(b.y, by - iy, wy, 0.f);
+                            dz = axis_gap<false>(b.z, bz - iz, wz, 0.f);
+                        } else {
+                            dx = axis_gap<true>(wrap_cull(b.x, g.L[0]), bx, wx, g.L[0]);
+                            dy = axis_gap<true>(wrap_cull(b.y, g.L[1]), by, wy, g.L[1]);
+                            dz = axis_gap<true>(wrap_cull(b.z, g.L[2]), bz, wz, g.L[2]);
+                        }
+                        keep = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
+                    }
+                    const int before = tail;
+                    append(b, qb, keep);
+                    if (EDGE && has) n_tested += (unsigned)(tail - before);
+                }
+                const int n4 = tail - head >= kRingRun ? kRingRun / 4 : pad();
+                __syncwarp();  // the other lanes' entries
+                if (mode == kImgNone) TRJ_RUN(kImgNone, false, n4);
+                else if (mode == kImgShift) TRJ_RUN(kImgShift, false, n4);
+                else if (mode == kImgRound) TRJ_RUN(kImgRound, false, n4);
+                else if (mode == kImgFold) TRJ_RUN(kImgFold, false, n4);
+                else TRJ_RUN(kImgAny, false, n4);
+                __syncwarp();
+                head += 4 * n4;
+            } while (more);
+#undef TRJ_RUN
+        }
+    }
+}
+
+// The CTA's rows into the frame's uint64 histogram (their total is the counted pairs).
+template <bool SQUARE>
+__device__ __forceinline__ void merge_rows(const RdfParams& p, const unsigned* hist, u64* __restrict__ hist_g,
+                                           PairCounters& pc) {
+    const int nsp = p.g.nsp, rw = p.g.row_words, lsmax = p.g.lsmax, hsz = p.nit * lsmax;
+    int row = 0, sa = 0, sb = 0;  // species of the row of element k
+    for (int k = threadIdx.x; k < hsz; k += blockDim.x) {
+        while (row < k / lsmax) {
+            ++row;
+            if (++sb == nsp) sb = ++sa;
+        }
+        const int bin = k - row * lsmax + 1;
+        u64 s;
+        if (SQUARE) {
+            s = hist[(sa * nsp + sb) * rw + bin];
+            if (sa != sb) s += hist[(sb * nsp + sa) * rw + bin];
+        } else {
+            s = hist[row * rw + bin];
+        }
+        if (s) atomicAdd(&hist_g[k], s);
+        pc.counted += s;
+    }
+}
+
+__device__ __forceinline__ void add_edges(u64* __restrict__ edge_g, const PairCounters& pc, u64 n_tested) {
+    u64 n_ulp = pc.ulp, n_fma = pc.fma, n_counted = pc.counted;
+    for (int off = 16; off > 0; off >>= 1) {
+        n_ulp += __shfl_down_sync(0xffffffffu, n_ulp, off);
+        n_fma += __shfl_down_sync(0xffffffffu, n_fma, off);
+        n_counted += __shfl_down_sync(0xffffffffu, n_counted, off);
+        n_tested += __shfl_down_sync(0xffffffffu, n_tested, off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (n_ulp) atomicAdd(&edge_g[TRJ_EDGE_ULP], n_ulp);
+        if (n_fma) atomicAdd(&edge_g[TRJ_EDGE_FMA], n_fma);
+        if (n_counted) atomicAdd(&edge_g[TRJ_EDGE_COUNTED], n_counted);
+        if (n_tested) atomicAdd(&edge_g[TRJ_EDGE_TESTED], n_tested);
+    }
 }
 
 // Work item = (home group, segment of its neighbour list), taken from a global counter by one warp at a
@@ -453,7 +642,6 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     __syncthreads();
     if (stalled) return;
 
-    const unsigned lt = (1u << lane) - 1u;
     const bool frame_ok = frame_within(*fflag);
     PairCounters pc;
     u64 n_tested = 0;
@@ -462,211 +650,18 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
         if (lane == 0) item = atomicAdd(work, 1u);
         item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= p.nitems) break;
-        const int key = fast_div((int)item, p.div_nseg), seg = (int)item - key * p.nseg;
-        const int hbeg = fstart[key], hend = hbeg + fcount[key];
-        if (hbeg >= hend) continue;
-        const int c = fast_div(key, p.div_nsub), own = key - c * p.nsub;
-        const int cxy = fast_div(c, p.div_nc2), cz = c - cxy * p.nc[2];
-        const int cx = fast_div(cxy, p.div_nc1), cy = cxy - cx * p.nc[1];
-        const int fl = cflag[c];
-        const int t0 = seg * p.per_seg, t1 = min(p.list, t0 + p.per_seg);
-        for (int h0 = hbeg; h0 < hend; h0 += kGroup) {
-            const int nh = min(kGroup, hend - h0);
-            const bool has = lane < nh;
-            const float4 a = has ? sorted[h0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-            Home h;
-            h.nx = -a.x;
-            h.ny = -a.y;
-            h.nz = -a.z;
-            h.q = (QMODE && has) ? sorted_q[h0 + lane] : 0.f;
-            const unsigned wa = __float_as_uint(a.w);  // species * row bytes (64 with the row table)
-            h.hist = SQUARE ? hist_base + wa * (unsigned)nsp - 4u * kBinBias : trj_smem_addr(rowtab) + (wa >> 4);
-            float bx, by, bz, wx, wy, wz;  // the homes' box: centre and half-widths
-            axis_box(wrap_cull(a.x, g.L[0]), has, p.cull_pad, bx, wx);
-            axis_box(wrap_cull(a.y, g.L[1]), has, p.cull_pad, by, wy);
-            axis_box(wrap_cull(a.z, g.L[2]), has, p.cull_pad, bz, wz);
-            for (int t = t0; t < t1;) {
-                // entries [e_lo, e_hi) of offset o: group e, or (own cell) the e-th after the homes' own
-                const int o = t < p.nself ? 0 : 1 + fast_div(t - p.nself, p.div_nsub);
-                const int first = o == 0 ? 0 : p.nself + (o - 1) * p.nsub;
-                const int e_lo = t - first, e_hi = min(o == 0 ? p.nself : p.nsub, t1 - first);
-                t = first + e_hi;
-                const int ex = cx + p.off[o][0], ey = cy + p.off[o][1], ez = cz + p.off[o][2];
-                const int c2 = (wrapc(ex, p.nc[0]) * p.nc[1] + wrapc(ey, p.nc[1])) * p.nc[2] + wrapc(ez, p.nc[2]);
-                const int f2 = fl | cflag[c2];
-                const bool far = f2 & 2;
-                const float ix = ex < 0 ? -g.L[0] : (ex >= p.nc[0] ? g.L[0] : 0.f);
-                const float iy = ey < 0 ? -g.L[1] : (ey >= p.nc[1] ? g.L[1] : 0.f);
-                const float iz = ez < 0 ? -g.L[2] : (ez >= p.nc[2] ? g.L[2] : 0.f);
-                const bool plain = p.split_all && !(f2 & 1);  // image known from the cells
-                const int mode = plain ? ((ix != 0.f || iy != 0.f || iz != 0.f) ? kImgShift : kImgNone)
-                                       : far ? kImgAny : p.split_all ? kImgRound : frame_ok ? kImgFold : kImgAny;
-                const int kb = c2 * p.nsub;
-                int head = 0, tail = 0;
-                auto append = [&](const float4& b, float qb, bool keep) {
-                    const unsigned m = __ballot_sync(0xffffffffu, keep);
-                    if (keep) {
-                        const int e = (tail + __popc(m & lt)) & (kRing - 1);
-                        ring[e] = b.x;
-                        ring[kRing + e] = b.y;
-                        ring[2 * kRing + e] = b.z;
-                        ring[3 * kRing + e] = b.w;
-                        if (QMODE) ring_q[e] = (double)qb;
-                    }
-                    tail += __popc(m);
-                };
-                // Fills the buffer up to a multiple of four with NaN entries (in no range, near no edge).
-                auto pad = [&]() {
-                    const int n = tail - head, up = (n + 3) & ~3;
-                    if (lane < up - n) {
-                        const int e = (tail + lane) & (kRing - 1);
-                        ring[e] = ring[kRing + e] = ring[2 * kRing + e] = NAN;
-                        ring[3 * kRing + e] = 0.f;
-                        if (QMODE) ring_q[e] = 0.0;
-                    }
-                    return up >> 2;
-                };
-#define TRJ_RUN(M, S, N4) test_run<M, S, FLOOR, QMODE, SQUARE, EDGE>(ring, ring_q, head, N4, h, has, ix, iy, iz, g, pc, qhist)
-                if (o == 0 && e_lo == 0) {
-                    // pairs j > i of the round's own atoms, through the buffer in lane order
-                    append(a, h.q, has);
-                    const int n4 = pad();
-                    __syncwarp();
-                    if (plain) TRJ_RUN(kImgNone, true, n4);
-                    else if (mode == kImgRound) TRJ_RUN(kImgRound, true, n4);
-                    else if (mode == kImgFold) TRJ_RUN(kImgFold, true, n4);
-                    else TRJ_RUN(kImgAny, true, n4);
-                    __syncwarp();
-                    if (EDGE && has) n_tested += (unsigned)(nh - 1 - lane);
-                    tail = 0;
-                }
-                int e0 = e_lo - 32, j = 0, je = 0, gs = 0, gn = 0;  // gs, gn: start and atoms of lane's group
-                unsigned m = 0;
-                bool more = true;
-                do {
-                    // survivors into the buffer until a run is full or the segment's groups are used up
-                    while (tail - head < kRingRun) {
-                        if (j >= je) {
-                            if (!m) {
-                                e0 += 32;
-                                if (e0 >= e_hi) {
-                                    more = false;
-                                    break;
-                                }
-                                // lanes over the neighbour groups: which can hold an atom in range of the homes' box
-                                const int e = e0 + lane;
-                                int s = o == 0 ? own + e : e;
-                                if (s >= p.nsub) s -= p.nsub;
-                                // half-way round an even number of groups each pair is met twice: the lower has it
-                                bool near = e < e_hi && (o > 0 || 2 * e != p.nsub || 2 * own < p.nsub);
-                                if (near && !far) {
-                                    const int q = (int)(((float)s + 0.5f) * p.inv_sub[2]), sz = s - q * p.sub[2];
-                                    const int sx = (int)(((float)q + 0.5f) * p.inv_sub[1]), sy = q - sx * p.sub[1];
-                                    const float gx = ((float)ex + ((float)sx + 0.5f) * p.inv_sub[0]) * p.edge[0];
-                                    const float gy = ((float)ey + ((float)sy + 0.5f) * p.inv_sub[1]) * p.edge[1];
-                                    const float gz = ((float)ez + ((float)sz + 0.5f) * p.inv_sub[2]) * p.edge[2];
-                                    float dx, dy, dz;
-                                    if (p.split_all) {
-                                        dx = axis_gap<false>(gx, bx, wx + p.half[0], 0.f);
-                                        dy = axis_gap<false>(gy, by, wy + p.half[1], 0.f);
-                                        dz = axis_gap<false>(gz, bz, wz + p.half[2], 0.f);
-                                    } else {
-                                        dx = axis_gap<true>(gx - ix, bx, wx + p.half[0], g.L[0]);
-                                        dy = axis_gap<true>(gy - iy, by, wy + p.half[1], g.L[1]);
-                                        dz = axis_gap<true>(gz - iz, bz, wz + p.half[2], g.L[2]);
-                                    }
-                                    near = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
-                                }
-                                if (near) {
-                                    gs = fstart[kb + s];
-                                    gn = fcount[kb + s];
-                                }
-                                m = __ballot_sync(0xffffffffu, near);
-                                continue;
-                            }
-                            const int k = __ffs(m) - 1;
-                            m &= m - 1u;
-                            j = __shfl_sync(0xffffffffu, gs, k);
-                            je = j + __shfl_sync(0xffffffffu, gn, k);
-                            if (o == 0 && e0 + k == 0) j = h0 + nh;  // the round's own atoms are done
-                            continue;
-                        }
-                        bool keep = j + lane < je;
-                        const float4 b = keep ? sorted[j + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-                        const float qb = (QMODE && keep) ? sorted_q[j + lane] : 0.f;
-                        j += 32;
-                        if (keep && !far) {
-                            float dx, dy, dz;
-                            if (plain) {
-                                dx = axis_gap<false>(b.x, bx - ix, wx, 0.f);
-                                dy = axis_gap<false>(b.y, by - iy, wy, 0.f);
-                                dz = axis_gap<false>(b.z, bz - iz, wz, 0.f);
-                            } else {
-                                dx = axis_gap<true>(wrap_cull(b.x, g.L[0]), bx, wx, g.L[0]);
-                                dy = axis_gap<true>(wrap_cull(b.y, g.L[1]), by, wy, g.L[1]);
-                                dz = axis_gap<true>(wrap_cull(b.z, g.L[2]), bz, wz, g.L[2]);
-                            }
-                            keep = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
-                        }
-                        const int before = tail;
-                        append(b, qb, keep);
-                        if (EDGE && has) n_tested += (unsigned)(tail - before);
-                    }
-                    const int n4 = tail - head >= kRingRun ? kRingRun / 4 : pad();
-                    __syncwarp();  // the other lanes' entries
-                    if (mode == kImgNone) TRJ_RUN(kImgNone, false, n4);
-                    else if (mode == kImgShift) TRJ_RUN(kImgShift, false, n4);
-                    else if (mode == kImgRound) TRJ_RUN(kImgRound, false, n4);
-                    else if (mode == kImgFold) TRJ_RUN(kImgFold, false, n4);
-                    else TRJ_RUN(kImgAny, false, n4);
-                    __syncwarp();
-                    head += 4 * n4;
-                } while (more);
-#undef TRJ_RUN
-            }
-        }
+        pair_item<FLOOR, QMODE, SQUARE, EDGE>(p, (int)item, sorted, fstart, fcount, cflag, frame_ok, sorted_q, ring,
+                                              ring_q, hist_base, trj_smem_addr(rowtab), qhist, pc, n_tested);
     }
     __syncthreads();
-    // Merge into the global uint64 histogram (the total is the counted pairs).
-    const int hsz = p.nit * g.lsmax;
-    int row = 0, sa = 0, sb = 0;  // species of the row of element k
-    for (int k = tid; k < hsz; k += blockDim.x) {
-        while (row < k / g.lsmax) {
-            ++row;
-            if (++sb == nsp) sb = ++sa;
-        }
-        const int bin = k - row * g.lsmax + 1;
-        u64 s;
-        if (SQUARE) {
-            s = hist[(sa * nsp + sb) * rw + bin];
-            if (sa != sb) s += hist[(sb * nsp + sa) * rw + bin];
-        } else {
-            s = hist[row * rw + bin];
-        }
-        if (s) atomicAdd(&hist_g[k], s);
-        pc.counted += s;
-    }
+    merge_rows<SQUARE>(p, hist, hist_g, pc);
     if (QMODE) {
         for (int k = tid; k < g.lsmax; k += blockDim.x) {
             const double s = qhist[k + 1];
             if (s != 0.0) atomicAdd(&gqq_frame[k], s);
         }
     }
-    if (edge_g) {
-        u64 n_ulp = pc.ulp, n_fma = pc.fma, n_counted = pc.counted;
-        for (int off = 16; off > 0; off >>= 1) {
-            n_ulp += __shfl_down_sync(0xffffffffu, n_ulp, off);
-            n_fma += __shfl_down_sync(0xffffffffu, n_fma, off);
-            n_counted += __shfl_down_sync(0xffffffffu, n_counted, off);
-            n_tested += __shfl_down_sync(0xffffffffu, n_tested, off);
-        }
-        if (lane == 0) {
-            if (n_ulp) atomicAdd(&edge_g[TRJ_EDGE_ULP], n_ulp);
-            if (n_fma) atomicAdd(&edge_g[TRJ_EDGE_FMA], n_fma);
-            if (n_counted) atomicAdd(&edge_g[TRJ_EDGE_COUNTED], n_counted);
-            if (n_tested) atomicAdd(&edge_g[TRJ_EDGE_TESTED], n_tested);
-        }
-    }
+    if (edge_g) add_edges(edge_g, pc, n_tested);
 }
 
 // Group of a folded coordinate along one axis: cell, then box within the cell (NaN: the first ones).
@@ -988,172 +983,160 @@ __global__ void s2n_kernel(const float4* __restrict__ sorted, const int32_t* __r
 }
 
 
-// ---- fused multi-request launch: all-pairs histogram of every packed frame ---------------------
+// ---- fused multi-request launch: pair histogram of every packed frame --------------------------
 //
-// Unit = (item, tile pair bi <= bj) of kBatchTile x kBatchTile atoms of one frame: home atom
-// i = bi * 256 + thread against the staged tile bj (j > i on the diagonal tile), each pair through the
-// general path of the cell kernel (reference minimum image, exact binning near edges), so the counts
-// are those of the reference's all-pairs sweep (rdf.cuf:449-475).  Units come from a global counter;
-// a CTA keeps the counts of one item in two shared replicas (even and odd warps) and merges them into
-// that item's uint64 histogram when its next unit belongs to another item, and at exit.
-template <bool FLOOR>
-__device__ __forceinline__ void bin_pair(float rr2, float x2, float dy, float dz, int row, const PairGeom& p,
-                                         unsigned* myhist, PairCounters& pc) {
-    const float q = rr2 * rsqrtf(rr2) * p.inv_deltar;
-    // Nearest integer of q by adding and removing 1.5*2^23 (q < 2^22): qb holds it in its low
-    // mantissa bits; d = q - r in [-1/2, 1/2] exactly.
-    const float qb = __fadd_rn(q, 12582912.0f);
-    const float d = __fsub_rn(q, __fsub_rn(qb, 12582912.0f));
-    const float win = fmaf(q, 1.9073486e-6f, 9.5367432e-7f);  // q*2^-19 + 2^-20
-    // distance of q from the nearest bin edge: integers (floor bins) or half-integers (nint bins)
-    const float edge = FLOOR ? fabsf(d) : 0.5f - fabsf(d);
-    int ind;
-    if (rr2 >= p.side2_lo || !(edge > win)) {  // NaN (rr2 == 0) takes this path too
-        const int e = exact_bin(rr2, x2, dy, dz, p.side2, p.deltar, p.lsmax, p.floor_bins);
-        pc.ulp += (e >> 29) & 1;
-        pc.fma += (e >> 30) & 1;
-        ind = e & ((1 << 29) - 1);
-    } else {
-        // Away from an edge, round-to-nearest-even and NINT agree, and floor(q) = r - (d < 0).
-        const int r = __float_as_int(qb) - 0x4B400000;
-        ind = FLOOR ? r + (d > 0.f ? 1 : 0) : r;
-        if (ind > p.lsmax) ind = 0;
-    }
-    if (ind > 0) atomicAdd(&myhist[row * p.lsmax + ind - 1], 1u);
-}
-
-template <bool FLOOR>
-__device__ __forceinline__ void pair(const float4& a, const float4& b, bool valid, int si, const PairGeom& p,
-                                     const int* rowtab, unsigned* myhist, PairCounters& pc) {
-    float dx = __fsub_rn(b.x, a.x);
-    float dy = __fsub_rn(b.y, a.y);
-    float dz = __fsub_rn(b.z, a.z);
-    dx = min_image(dx, p.L[0], p.h1[0], p.h2[0]);
-    dy = min_image(dy, p.L[1], p.h1[1], p.h2[1]);
-    dz = min_image(dz, p.L[2], p.h1[2], p.h2[2]);
-    const float x2 = __fmul_rn(dx, dx);
-    const float rr2 = __fadd_rn(__fadd_rn(x2, __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-    if (valid && rr2 < p.side2_hi) {
-        const int sj = __float_as_int(b.w);
-        if ((unsigned)sj < (unsigned)p.nsp)
-            bin_pair<FLOOR>(rr2, x2, dy, dz, rowtab[si * p.nsp + sj], p, myhist, pc);
-    }
-}
-
-template <bool FLOOR>
-__device__ __forceinline__ unsigned batch_tile_pairs(const float4* __restrict__ tile, int jcount, const float4& a,
-                                                     bool has_a, int il, bool diag, int si, const PairGeom& P,
-                                                     const int* rowtab, unsigned* myhist, PairCounters& pc) {
-    unsigned tested = 0;
-    for (int jj = 0; jj < jcount; ++jj) {
-        const bool valid = has_a && (!diag || jj > il);
-        tested += valid ? 1u : 0u;
-        pair<FLOOR>(a, tile[jj], valid, si, P, rowtab, myhist, pc);
-    }
-    return tested;
-}
-
-__device__ __forceinline__ void batch_pairs_flush(const BatchItem& it, unsigned* hist, int hist_words,
-                                                  PairCounters& pc, unsigned long long& tested) {
-    const int hsz = it.nit * it.lsmax;
-    for (int k = threadIdx.x; k < hsz; k += kBatchThreads) {
-        const unsigned long long v = (unsigned long long)hist[k] + hist[hist_words + k];
-        if (v) atomicAdd(&it.hist[k], v);
-        pc.counted += v;
-        hist[k] = 0u;
-        hist[hist_words + k] = 0u;
-    }
-    if (it.edge) {
-        unsigned long long n_ulp = pc.ulp, n_fma = pc.fma, n_counted = pc.counted, n_tested = tested;
-        for (int off = 16; off > 0; off >>= 1) {
-            n_ulp += __shfl_down_sync(0xffffffffu, n_ulp, off);
-            n_fma += __shfl_down_sync(0xffffffffu, n_fma, off);
-            n_counted += __shfl_down_sync(0xffffffffu, n_counted, off);
-            n_tested += __shfl_down_sync(0xffffffffu, n_tested, off);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            if (n_ulp) atomicAdd(&it.edge[TRJ_EDGE_ULP], n_ulp);
-            if (n_fma) atomicAdd(&it.edge[TRJ_EDGE_FMA], n_fma);
-            if (n_counted) atomicAdd(&it.edge[TRJ_EDGE_COUNTED], n_counted);
-            if (n_tested) atomicAdd(&it.edge[TRJ_EDGE_TESTED], n_tested);
-        }
-    }
-    pc = PairCounters();
-    tested = 0;
-}
-
-__global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(BatchHeader* __restrict__ hdr,
-                                                                    const BatchItem* __restrict__ items,
-                                                                    const float4* __restrict__ packed,
-                                                                    int hist_words) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    float4* tile = reinterpret_cast<float4*>(smem);                              // [kBatchTile]
-    unsigned* hist = reinterpret_cast<unsigned*>(smem + kBatchTile * sizeof(float4));  // [2][hist_words]
-    __shared__ int rowtab[kBatchMaxSpecies * kBatchMaxSpecies];
-    __shared__ long long unit_s;
-    const int tid = threadIdx.x;
-    unsigned* myhist = hist + ((tid >> 5) & 1) * hist_words;
-    for (int k = tid; k < 2 * hist_words; k += kBatchThreads) hist[k] = 0u;
-    const int nitems = hdr->nitems;
-    const int64_t total = hdr->total_pair;
+// The cell sort and the work items of the single-frame path for all frames of the turn at once: keys and counts
+// of every atom, group offsets (each item's groups start at its key_begin, a multiple of 32), placing, and one
+// pair kernel whose CTAs each work on one frame at a time, merge its counts and move on to the next frame that
+// has items left.
+__global__ void __launch_bounds__(kBatchThreads) batch_keys_kernel(const BatchHeader* __restrict__ hdr,
+                                                                   const BatchItem* __restrict__ items,
+                                                                   const float4* __restrict__ packed, BatchSort st) {
+    __shared__ RdfParams p;
+    const int64_t total = hdr->total_chunk;
     int cur = -1;
-    PairGeom P;
-    int n = 0, ntile = 0;
-    int64_t off = 0;
-    PairCounters pc;
-    unsigned long long tested = 0;
-    while (true) {
-        if (tid == 0) unit_s = (long long)atomicAdd(&hdr->counter[0], 1ull);
-        __syncthreads();
-        const int64_t u = unit_s;
-        const int r = u < total ? batch_item_of<&BatchItem::pair_begin>(items, nitems, u) : -1;
-        if (r != cur) {  // block-uniform
-            if (cur >= 0) batch_pairs_flush(items[cur], hist, hist_words, pc, tested);
-            cur = r;
-            if (r >= 0) {
-                const BatchItem& it = items[r];
-                for (int d = 0; d < 3; ++d) {
-                    P.L[d] = it.L[d];
-                    P.h1[d] = it.h1[d];
-                    P.h2[d] = it.h2[d];
-                }
-                P.side2 = it.side2;
-                P.side2_lo = it.side2_lo;
-                P.side2_hi = it.side2_hi;
-                P.deltar = it.deltar;
-                P.inv_deltar = it.inv_deltar;
-                P.lsmax = it.lsmax;
-                P.nsp = it.nsp;
-                P.floor_bins = it.floor_bins;
-                n = it.n;
-                ntile = it.ntile;
-                off = it.atom_off;
-                for (int k = tid; k < P.nsp * P.nsp; k += kBatchThreads)
-                    rowtab[k] = trj_pair_row(k / P.nsp, k % P.nsp, P.nsp);
-            }
+    for (int64_t u = blockIdx.x; u < total; u += gridDim.x) {
+        const int r = batch_item_of<&BatchItem::chunk_begin>(items, hdr->nitems, u);
+        const BatchItem& it = items[r];
+        if (!it.hist) continue;  // block-uniform
+        if (r != cur) {
             __syncthreads();
+            for (int k = threadIdx.x; k < (int)(sizeof(RdfParams) / 4); k += kBatchThreads)
+                reinterpret_cast<unsigned*>(&p)[k] = reinterpret_cast<const unsigned*>(&it.pair)[k];
+            __syncthreads();
+            cur = r;
         }
-        if (r < 0) break;
-        // tile pair (bi, bj), bi <= bj, of triangle index t (row bi holds ntile - bi pairs)
-        const int64_t t = u - items[r].pair_begin;
-        const double b2 = 2.0 * ntile + 1.0;
-        int bi = (int)((b2 - sqrt(b2 * b2 - 8.0 * (double)t)) * 0.5);
-        auto row_start = [&](int b) { return (int64_t)b * ntile - (int64_t)b * (b - 1) / 2; };
-        while (bi > 0 && row_start(bi) > t) --bi;
-        while (bi + 1 < ntile && row_start(bi + 1) <= t) ++bi;
-        const int bj = bi + (int)(t - row_start(bi));
-        const int j = bj * kBatchTile + tid;
-        tile[tid] = j < n ? packed[off + j] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-        const int i = bi * kBatchTile + tid;
-        const float4 a = i < n ? packed[off + i] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-        const int si = __float_as_int(a.w);
-        const bool has_a = i < n && (unsigned)si < (unsigned)P.nsp;
-        const int jcount = min(kBatchTile, n - bj * kBatchTile);
+        const int64_t c = u - it.chunk_begin;
+        for (int k = threadIdx.x; k < kBatchChunk; k += kBatchThreads) {
+            const int64_t i = c * kBatchChunk + k;
+            unsigned ff = 0;
+            if (i < it.n) {
+                const float4 v = packed[it.atom_off + i];
+                const AtomCell a = place(v, p);
+                ff = a.frame;
+                const bool ok = __float_as_uint(v.w) < (unsigned)p.g.nsp;  // else flagged as bad data: not placed
+                st.akey[it.atom_off + i] = ok ? a.key : -1;
+                if (ok) st.aslot[it.atom_off + i] = atomicAdd(&st.fcount[it.key_begin + a.key], 1);
+                if (a.flag) atomicOr(&st.cflag[it.key_begin + a.cell], a.flag);
+            }
+            ff = __reduce_or_sync(0xffffffffu, ff);
+            if ((threadIdx.x & 31) == 0 && ff) atomicOr(&st.state[4 * r + 2], ff);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kBatchThreads) batch_offsets_kernel(const BatchHeader* __restrict__ hdr,
+                                                                      const BatchItem* __restrict__ items, BatchSort st) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t k0 = ((int64_t)blockIdx.x * kBatchThreads + threadIdx.x) & ~31ll; k0 < hdr->total_key;
+         k0 += (int64_t)gridDim.x * kBatchThreads) {
+        const int r = batch_item_of<&BatchItem::key_begin>(items, hdr->nitems, k0);
+        const int v = st.fcount[k0 + lane];
+        int x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        int base = 0;
+        if (lane == 31) base = (int)atomicAdd(&st.state[4 * r + 1], (unsigned)x);
+        base = __shfl_sync(0xffffffffu, base, 31);
+        st.fstart[k0 + lane] = base + x - v;
+    }
+}
+
+__global__ void __launch_bounds__(kBatchThreads) batch_place_kernel(const BatchHeader* __restrict__ hdr,
+                                                                    const BatchItem* __restrict__ items,
+                                                                    const float4* __restrict__ packed, BatchSort st) {
+    const int64_t total = hdr->total_chunk;
+    for (int64_t u = blockIdx.x; u < total; u += gridDim.x) {
+        const BatchItem& it = items[batch_item_of<&BatchItem::chunk_begin>(items, hdr->nitems, u)];
+        if (!it.hist) continue;
+        const unsigned wscale = it.square ? 4u * (unsigned)it.pair.g.row_words : 64u;
+        const int64_t c = u - it.chunk_begin;
+        for (int k = threadIdx.x; k < kBatchChunk; k += kBatchThreads) {
+            const int64_t i = c * kBatchChunk + k;
+            if (i >= it.n) break;
+            const int key = st.akey[it.atom_off + i];
+            if (key < 0) continue;
+            float4 v = packed[it.atom_off + i];
+            v.w = __uint_as_float(__float_as_uint(v.w) * wscale);
+            st.sorted[it.atom_off + st.fstart[it.key_begin + key] + st.aslot[it.atom_off + i]] = v;
+        }
+    }
+}
+
+// What bounds it: instruction issue, as the single-frame kernel.  64 frames of 1,000 to 16,384 atoms: 2.74 ms
+// for an all-pairs sweep with a branch per pair, 0.70 ms so (80 registers a thread; 64, at four CTAs per SM: 0.74).
+__global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const BatchHeader* __restrict__ hdr,
+                                                                       const BatchItem* __restrict__ items, BatchSort st,
+                                                                       int hist_words) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ RdfParams p;
+    __shared__ unsigned rowtab[256];
+    __shared__ int next;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float* ring = reinterpret_cast<float*>(smem) + (size_t)warp * 4 * kRing;
+    unsigned* hist = reinterpret_cast<unsigned*>(smem + (size_t)(kBatchThreads / 32) * 16 * kRing);
+    const unsigned hist_base = trj_smem_addr(hist), rowtab_base = trj_smem_addr(rowtab);
+    for (int k = tid; k < batch_hist_smem_words(hist_words); k += kBatchThreads) hist[k] = 0u;
+    const int nitems = hdr->nitems;
+    if (nitems == 0) return;
+    // CTAs start spread over the turn's work; each then moves on cyclically to frames with items left
+    int r = batch_item_of<&BatchItem::pair_begin>(items, nitems, hdr->total_pair * blockIdx.x / gridDim.x);
+    for (;;) {
+        if (tid == 0) next = nitems;
         __syncthreads();
-        tested += P.floor_bins
-                      ? batch_tile_pairs<true>(tile, jcount, a, has_a, tid, bi == bj, si, P, rowtab, myhist, pc)
-                      : batch_tile_pairs<false>(tile, jcount, a, has_a, tid, bi == bj, si, P, rowtab, myhist, pc);
+        for (int k = tid; k < nitems; k += kBatchThreads) {
+            const int q = r + k < nitems ? r + k : r + k - nitems;
+            if (*(volatile unsigned*)&st.state[4 * q] < items[q].pair.nitems && items[q].hist) {
+                atomicMin(&next, k);
+                break;
+            }
+        }
         __syncthreads();
+        const int k = next;
+        if (k >= nitems) break;
+        r = r + k < nitems ? r + k : r + k - nitems;
+        const BatchItem& it = items[r];
+        for (int q = tid; q < (int)(sizeof(RdfParams) / 4); q += kBatchThreads)
+            reinterpret_cast<unsigned*>(&p)[q] = reinterpret_cast<const unsigned*>(&it.pair)[q];
+        __syncthreads();
+        const bool square = it.square;
+        if (!square)
+            for (int q = tid; q < p.g.nsp * p.g.nsp; q += kBatchThreads)
+                rowtab[(q / p.g.nsp) * 16 + q % p.g.nsp] =
+                    hist_base + (unsigned)(trj_pair_row(q / p.g.nsp, q % p.g.nsp, p.g.nsp) * p.g.row_words * 4) -
+                    4u * kBinBias;
+        __syncthreads();
+        PairCounters pc;
+        u64 n_tested = 0;
+        const bool frame_ok = frame_within(st.state[4 * r + 2]);
+        const float4* sorted = st.sorted + it.atom_off;
+        const int32_t *fstart = st.fstart + it.key_begin, *fcount = st.fcount + it.key_begin,
+                      *cflag = st.cflag + it.key_begin;
+        for (;;) {
+            unsigned item = 0;
+            if (lane == 0) item = atomicAdd(&st.state[4 * r], 1u);
+            item = __shfl_sync(0xffffffffu, item, 0);
+            if (item >= p.nitems) break;
+#define TRJ_ITEM(F, S, E)                                                                                       \
+    pair_item<F, false, S, E>(p, (int)item, sorted, fstart, fcount, cflag, frame_ok, nullptr, ring, nullptr, hist_base, \
+                              rowtab_base, nullptr, pc, n_tested)
+            if (p.g.floor_bins) TRJ_ITEM(true, false, true);
+            else if (!square) TRJ_ITEM(false, false, true);
+            else if (p.g.want_edge) TRJ_ITEM(false, true, true);
+            else TRJ_ITEM(false, true, false);
+#undef TRJ_ITEM
+        }
+        __syncthreads();
+        if (square) merge_rows<true>(p, hist, it.hist, pc);
+        else merge_rows<false>(p, hist, it.hist, pc);
+        if (it.edge) add_edges(it.edge, pc, n_tested);
+        __syncthreads();
+        const int rows = square ? p.g.nsp * p.g.nsp : p.nit;
+        for (int q = tid; q < rows * p.g.row_words; q += kBatchThreads) hist[q] = 0u;
+        r = r + 1 < nitems ? r + 1 : 0;
     }
 }
 
@@ -1283,6 +1266,12 @@ static void choose_groups(int64_t n, const float box[3], double rc, int dim, int
             if (nc[d] >= 3) nc[d] = std::max(3, (int)(nc[d] / f));
         m = (double)n / ((double)nc[0] * nc[1] * nc[2]);
     }
+    // room for the cells themselves: coarser ones where there is not (an axis without a split always works)
+    while ((int64_t)nc[0] * nc[1] * nc[2] > key_cap) {
+        int d = nc[0] >= nc[1] ? (nc[0] >= nc[2] ? 0 : 2) : (nc[1] >= nc[2] ? 1 : 2);
+        nc[d] = nc[d] > 3 ? std::max(3, nc[d] / 2) : 1;
+    }
+    m = (double)n / ((double)nc[0] * nc[1] * nc[2]);
     sub[0] = sub[1] = sub[2] = 1;
     if (m <= kGroupFill) return;
     double e[3], vol = 1.0;
@@ -1310,6 +1299,51 @@ static void choose_groups(int64_t n, const float box[3], double rc, int dim, int
                     sub[2] = c;
                 }
             }
+}
+
+// Cells, groups, stencil and cull of an n-atom frame; P.nc holds the most cells the cutoff allows.
+static void fill_grid(RdfParams& P, int64_t n, const float box[3], float side2, float rc, int dim, int64_t key_cap) {
+    choose_groups(n, box, rc, dim, key_cap, P.nc, P.sub);
+    P.nsub = P.sub[0] * P.sub[1] * P.sub[2];
+    // Cull radius 2^-10 above the cutoff (the exact test needs rr2 < side2*(1 + 2^-20)); the pad,
+    // 2^-16 of the largest edge, exceeds the rounding of the box and gap arithmetic (a few ulps of
+    // coordinates below 2L).
+    P.cull2 = (float)((double)side2 * (1.0 + 1.0 / 1024.0) * (1.0 + 1.0 / 1024.0));
+    P.cull_pad = (float)((double)std::max(box[0], std::max(box[1], box[2])) / 65536.0);
+    for (int d = 0; d < 3; ++d) {
+        P.inv_sub[d] = 1.0f / (float)P.sub[d];
+        P.edge[d] = box[d] / (float)P.nc[d];
+        P.half[d] = 0.5f * P.edge[d] / (float)P.sub[d] + P.cull_pad;
+    }
+    P.split_all = P.nc[0] >= 3 && P.nc[1] >= 3 && (P.nc[2] >= 3 || dim == 2);
+    // Half-shell stencil over the split axes: (0,0,0) first, then offsets > 0 lexicographically.
+    int no = 0;
+    P.off[no][0] = P.off[no][1] = P.off[no][2] = 0;
+    ++no;
+    for (int dx = -1; dx <= 1; ++dx)
+        for (int dy = -1; dy <= 1; ++dy)
+            for (int dz = -1; dz <= 1; ++dz) {
+                if ((dx && P.nc[0] == 1) || (dy && P.nc[1] == 1) || (dz && P.nc[2] == 1)) continue;
+                bool pos = dx > 0 || (dx == 0 && (dy > 0 || (dy == 0 && dz > 0)));
+                if (!pos) continue;
+                P.off[no][0] = dx;
+                P.off[no][1] = dy;
+                P.off[no][2] = dz;
+                ++no;
+            }
+    P.nself = P.nsub / 2 + 1;
+    P.list = P.nself + (no - 1) * P.nsub;
+    P.div_nsub = make_fast_div(P.nsub);
+    P.div_nc1 = make_fast_div(P.nc[1]);
+    P.div_nc2 = make_fast_div(P.nc[2]);
+}
+
+// Work items of nkey home groups with neighbour lists cut into about nseg segments.
+static void set_segments(RdfParams& P, int nseg, int nkey) {
+    P.per_seg = (P.list + nseg - 1) / nseg;
+    P.nseg = (P.list + P.per_seg - 1) / P.per_seg;
+    P.div_nseg = make_fast_div(P.nseg);
+    P.nitems = (unsigned)nkey * (unsigned)P.nseg;  // below 2^31: nseg > 1 only for few keys
 }
 
 struct PairShape {
@@ -1534,36 +1568,9 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
     if (P.nc[0] * P.nc[1] * P.nc[2] > plan->ncell_cap)
         return trj_fail(ctx, TRJ_ERR_CAPACITY, "rdf accumulate: %d cells exceed plan capacity %d",
                         P.nc[0] * P.nc[1] * P.nc[2], plan->ncell_cap);
-    choose_groups(n, box, plan->rcrdf_eff, plan->dim, plan->key_cap, P.nc, P.sub);
+    fill_grid(P, n, box, plan->side2, plan->rcrdf_eff, plan->dim, plan->key_cap);
     const int ncell = P.nc[0] * P.nc[1] * P.nc[2];
-    P.nsub = P.sub[0] * P.sub[1] * P.sub[2];
     const int nkey = ncell * P.nsub;
-    // Cull radius 2^-10 above the cutoff (the exact test needs rr2 < side2*(1 + 2^-20)); the pad,
-    // 2^-16 of the largest edge, exceeds the rounding of the box and gap arithmetic (a few ulps of
-    // coordinates below 2L).
-    P.cull2 = (float)((double)plan->side2 * (1.0 + 1.0 / 1024.0) * (1.0 + 1.0 / 1024.0));
-    P.cull_pad = (float)((double)std::max(box[0], std::max(box[1], box[2])) / 65536.0);
-    for (int d = 0; d < 3; ++d) {
-        P.inv_sub[d] = 1.0f / (float)P.sub[d];
-        P.edge[d] = box[d] / (float)P.nc[d];
-        P.half[d] = 0.5f * P.edge[d] / (float)P.sub[d] + P.cull_pad;
-    }
-    P.split_all = P.nc[0] >= 3 && P.nc[1] >= 3 && (P.nc[2] >= 3 || plan->dim == 2);
-    // Half-shell stencil over the split axes: (0,0,0) first, then offsets > 0 lexicographically.
-    int no = 0;
-    P.off[no][0] = P.off[no][1] = P.off[no][2] = 0;
-    ++no;
-    for (int dx = -1; dx <= 1; ++dx)
-        for (int dy = -1; dy <= 1; ++dy)
-            for (int dz = -1; dz <= 1; ++dz) {
-                if ((dx && P.nc[0] == 1) || (dy && P.nc[1] == 1) || (dz && P.nc[2] == 1)) continue;
-                bool pos = dx > 0 || (dx == 0 && (dy > 0 || (dy == 0 && dz > 0)));
-                if (!pos) continue;
-                P.off[no][0] = dx;
-                P.off[no][1] = dy;
-                P.off[no][2] = dz;
-                ++no;
-            }
     // Launch shape: as many warps per SM as the histogram leaves room for, with a row per ordered species
     // pair where that costs no warps.
     PairShape shape;
@@ -1572,16 +1579,7 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
     // Segments: about twelve items per resident warp, so that the last ones end together (six: 62,500 atoms
     // 485 us instead of 455; twenty-four: 459), but at least two neighbour groups per item.
     const int64_t warps = (int64_t)ctx->sm_count * shape.ctas * shape.warps;
-    P.nself = P.nsub / 2 + 1;
-    P.list = P.nself + (no - 1) * P.nsub;
-    P.nseg = (int)std::max<int64_t>(1, std::min<int64_t>((12 * warps + nkey - 1) / nkey, P.list / 2));
-    P.per_seg = (P.list + P.nseg - 1) / P.nseg;
-    P.nseg = (P.list + P.per_seg - 1) / P.per_seg;
-    P.div_nsub = make_fast_div(P.nsub);
-    P.div_nc1 = make_fast_div(P.nc[1]);
-    P.div_nc2 = make_fast_div(P.nc[2]);
-    P.div_nseg = make_fast_div(P.nseg);
-    P.nitems = (unsigned)nkey * (unsigned)P.nseg;  // below 2^31: nseg > 1 only for few keys
+    set_segments(P, (int)std::max<int64_t>(1, std::min<int64_t>((12 * warps + nkey - 1) / nkey, P.list / 2)), nkey);
 
     const PairKernel kern = pair_kernel(plan->floor_bins, charged, shape.square, edge_dev != nullptr);
     TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem));
@@ -1690,16 +1688,23 @@ extern "C" int trj_rdf_plan_set_wait(trj_rdf_plan* plan, int64_t clocks, int sta
 
 // ---- fused multi-request launch: host side of the pair kernel ----------------------------------
 
-size_t trj_batch_pairs_smem(int hist_words) { return kBatchTile * sizeof(float4) + 2 * (size_t)hist_words * 4; }
+size_t trj_batch_pairs_smem(int hist_words) {
+    return (size_t)(kBatchThreads / 32) * 16 * kRing + 4 * (size_t)batch_hist_smem_words(hist_words);
+}
 
 int trj_batch_pairs_prepare(int hist_words) {
     return cudaFuncSetAttribute(batch_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)trj_batch_pairs_smem(hist_words)) == cudaSuccess ? 0 : -1;
 }
 
-void trj_batch_launch_pairs(BatchHeader* hdr, const BatchItem* items, const float4* packed, int hist_words,
-                            int grid, cudaStream_t s) {
-    batch_pairs_kernel<<<grid, kBatchThreads, trj_batch_pairs_smem(hist_words), s>>>(hdr, items, packed, hist_words);
+int trj_batch_launch_pairs(BatchHeader* hdr, const BatchItem* items, const float4* packed, const BatchSort& st,
+                           size_t zero_bytes, int hist_words, int grid_layout, int grid, cudaStream_t s) {
+    if (cudaMemsetAsync(st.state, 0, zero_bytes, s) != cudaSuccess) return -1;
+    batch_keys_kernel<<<grid_layout, kBatchThreads, 0, s>>>(hdr, items, packed, st);
+    batch_offsets_kernel<<<grid_layout, kBatchThreads, 0, s>>>(hdr, items, st);
+    batch_place_kernel<<<grid_layout, kBatchThreads, 0, s>>>(hdr, items, packed, st);
+    batch_pairs_kernel<<<grid, kBatchThreads, trj_batch_pairs_smem(hist_words), s>>>(hdr, items, st, hist_words);
+    return 0;
 }
 
 int trj_batch_pairs_occupancy(int hist_words, int* per_sm) {
@@ -1707,7 +1712,8 @@ int trj_batch_pairs_occupancy(int hist_words, int* per_sm) {
                                                          trj_batch_pairs_smem(hist_words)) == cudaSuccess ? 0 : -1;
 }
 
-int trj_batch_fill_rdf(trj_rdf_plan* plan, const float box[3], int hist_words, BatchItem* it, int* nsp) {
+int trj_batch_fill_rdf(trj_rdf_plan* plan, int64_t n, const float box[3], int hist_words, bool want_edge, BatchItem* it,
+                       int* nsp, int64_t* nkey) {
     trj_ctx* ctx = plan->ctx;
     if (plan->dim != 3) return trj_fail(ctx, TRJ_ERR_UNSUPPORTED, "batch: two-dimensional pair plans run unfused");
     if (plan->nsp > kBatchMaxSpecies)
@@ -1720,18 +1726,18 @@ int trj_batch_fill_rdf(trj_rdf_plan* plan, const float box[3], int hist_words, B
     plan->rcrdf_eff = fminf(plan->rcrdf_eff, side / 2.0f);
     plan->side2 = plan->rcrdf_eff * plan->rcrdf_eff;
     plan->cells_valid = 0;
-    for (int d = 0; d < 3; ++d) {
-        it->h1[d] = nint_threshold(box[d], 0.5f);
-        it->h2[d] = nint_threshold(box[d], 1.5f);
-    }
-    it->side2 = plan->side2;
-    it->side2_lo = (float)((double)plan->side2 * (1.0 - 1.0 / 1048576.0));
-    it->side2_hi = (float)((double)plan->side2 * (1.0 + 1.0 / 1048576.0));
-    it->deltar = plan->deltar;
-    it->inv_deltar = 1.0f / plan->deltar;
-    it->lsmax = plan->lsmax;
-    it->nit = plan->nit;
-    it->floor_bins = plan->floor_bins;
+    RdfParams& P = it->pair;
+    memset(&P, 0, sizeof(P));
+    fill_geom(P.g, box, plan->side2, plan->deltar, plan->lsmax, plan->nsp, plan->floor_bins, want_edge);
+    P.nit = plan->nit;
+    cells_for(box, plan->side2, P.nc);
+    fill_grid(P, n, box, plan->side2, plan->rcrdf_eff, 3, batch_keys_most(n));
+    *nkey = (int64_t)P.nc[0] * P.nc[1] * P.nc[2] * P.nsub;
+    // about ten neighbour groups per item; one-atom frames have no pairs
+    if (n >= 2) set_segments(P, std::max(1, P.list / 10), (int)*nkey);
+    // a row per ordered species pair where those fit (floor bins: the general layout only)
+    it->square = !plan->floor_bins &&
+                 (int64_t)plan->nsp * plan->nsp * P.g.row_words <= (int64_t)batch_hist_smem_words(hist_words);
     *nsp = plan->nsp;
     return TRJ_OK;
 }

@@ -327,7 +327,7 @@ class Batch:
         check(rc, self.ctx.h, "trj_batch_add")
 
     def info(self, buf: int):
-        """(items, [layout units, pair tiles, direct-sum blocks, shell bins]) of the buffer's turn."""
+        """(items, [layout units, pair items, direct-sum blocks, shell bins]) of the buffer's turn."""
         ni = ctypes.c_int()
         units = (ctypes.c_int64 * 4)()
         check(self.ctx.lib.trj_batch_info(self.h, int(buf), ctypes.byref(ni), units, None), self.ctx.h,
