@@ -31,9 +31,68 @@ namespace {
 
 constexpr int kDynThreads = 256;
 constexpr int kDynVPT = 4;        // vectors per thread
-constexpr int kDynChunk = 1024;   // atoms staged per pass
+constexpr int kDynChunk = 1024;   // least atoms of a slice
+constexpr int kDynStage = 512;    // atoms staged per pass
 constexpr int kDynSub = 64;       // FP32 run length before the FP64 add
+constexpr int kDynCtas = 4;       // blocks of 256 threads per SM the launch shapes count on
 constexpr float kTwoPiOver2_32 = 1.4629180792671596e-09f;
+
+typedef unsigned long long u64;
+
+// Packed FP32: two independent IEEE operations per instruction, each rounded to nearest once.
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ u64 pack2(float lo, float hi) {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// Vectors in launch order: a thread's kDynVPT vectors are consecutive slots.  Slots hold the components with
+// axis `axis` first; shared: the vectors of a thread have that component in common, so its product is formed
+// once per atom.
+struct DynSlots {
+    const int4* slot;  // components, index of the vector (-1: padding)
+    int64_t n;         // slots, a multiple of kDynVPT
+    int axis, shared;
+};
+
+// Components of an atom's phase with the slots' axis first.
+__device__ __forceinline__ uint4 axis_first(const uint4& a, int axis) {
+    return axis == 0 ? a : axis == 1 ? make_uint4(a.y, a.x, a.z, a.w) : make_uint4(a.z, a.x, a.y, a.w);
+}
+
+// Atoms [s0, s1) of slice sl of nsl; a part of it takes runs [r0, r1) of 64 atoms from the slice's start, which
+// fix the FP32 partial sums whatever the launch shape.
+struct DynRuns {
+    int64_t s0, s1, r0, r1;
+};
+__device__ __forceinline__ DynRuns dyn_runs(int64_t n, int row, int nsplit, int parts) {
+    const int sl = row / parts, part = row - sl * parts;
+    DynRuns r;
+    r.s0 = n * sl / nsplit;
+    r.s1 = n * (sl + 1) / nsplit;
+    const int64_t runs = (r.s1 - r.s0 + kDynSub - 1) / kDynSub;
+    r.r0 = runs * part / parts;
+    r.r1 = runs * (part + 1) / parts;
+    return r;
+}
 
 struct DynJob {
     int buf;     // buffer index
@@ -57,82 +116,121 @@ __global__ void dyn_phase_kernel(const float4* __restrict__ packed, int64_t n, d
     u[i] = make_uint4(w[0], w[1], w[2], (unsigned)__float_as_int(v.w));
 }
 
-// Partial rho(k) = sum_j bsc[species_j] e^{i k.r_j} over the atom range of blockIdx.y.
-__global__ void __launch_bounds__(kDynThreads) dyn_rho_kernel(const uint4* __restrict__ u, int64_t n,
-                                                              const float* __restrict__ bsc, int nsp,
-                                                              const int4* __restrict__ vecs, int64_t nvec,
-                                                              int nsplit, double2* __restrict__ part) {
-    __shared__ uint4 atoms[kDynChunk];
-    __shared__ float wts[kDynChunk];
-    const int tid = threadIdx.x;
-    unsigned nx[kDynVPT], ny[kDynVPT], nz[kDynVPT];
-    int64_t vi[kDynVPT];
+// Phases of a thread's vectors for one atom.
+template <bool SHARED>
+__device__ __forceinline__ void dyn_phases(const unsigned (&n0)[kDynVPT], const unsigned (&n1)[kDynVPT],
+                                           const unsigned (&n2)[kDynVPT], const uint4& a, unsigned (&ph)[kDynVPT]) {
+    const unsigned p0 = n0[0] * a.x;
+#pragma unroll
+    for (int q = 0; q < kDynVPT; ++q) ph[q] = (SHARED ? p0 : n0[q] * a.x) + n1[q] * a.y + n2[q] * a.z;
+}
+
+__device__ __forceinline__ void dyn_load_slots(const DynSlots& sl, int64_t first, unsigned (&n0)[kDynVPT],
+                                               unsigned (&n1)[kDynVPT], unsigned (&n2)[kDynVPT]) {
 #pragma unroll
     for (int q = 0; q < kDynVPT; ++q) {
-        vi[q] = (int64_t)blockIdx.x * kDynThreads * kDynVPT + q * kDynThreads + tid;
-        const int4 v = vi[q] < nvec ? vecs[vi[q]] : make_int4(0, 0, 0, 0);
-        nx[q] = (unsigned)v.x;
-        ny[q] = (unsigned)v.y;
-        nz[q] = (unsigned)v.z;
+        const int4 v = first < sl.n ? sl.slot[first + q] : make_int4(0, 0, 0, -1);
+        n0[q] = (unsigned)v.x;
+        n1[q] = (unsigned)v.y;
+        n2[q] = (unsigned)v.z;
     }
-    const int64_t a0 = n * blockIdx.y / nsplit, a1 = n * (blockIdx.y + 1) / nsplit;
+}
+
+// Partial rho(k) = sum_j bsc[species_j] e^{i k.r_j} over the runs of row blockIdx.y, by slot.
+template <bool SHARED>
+__global__ void __launch_bounds__(kDynThreads, kDynCtas) dyn_rho_kernel(const uint4* __restrict__ u, int64_t n,
+                                                                        const float* __restrict__ bsc, int nsp,
+                                                                        DynSlots sl, int nsplit, int parts,
+                                                                        double2* __restrict__ part) {
+    __shared__ uint4 atoms[kDynStage];  // w: the atom's weight
+    const int tid = threadIdx.x;
+    const int64_t first = ((int64_t)blockIdx.x * blockDim.x + tid) * kDynVPT;
+    unsigned n0[kDynVPT], n1[kDynVPT], n2[kDynVPT];
+    dyn_load_slots(sl, first, n0, n1, n2);
+    const DynRuns rr = dyn_runs(n, blockIdx.y, nsplit, parts);
     double accr[kDynVPT], acci[kDynVPT];
 #pragma unroll
     for (int q = 0; q < kDynVPT; ++q) accr[q] = acci[q] = 0.0;
-    for (int64_t c0 = a0; c0 < a1; c0 += kDynChunk) {
-        const int cnt = (int)min((int64_t)kDynChunk, a1 - c0);
+    for (int64_t r = rr.r0; r < rr.r1; r += kDynStage / kDynSub) {
+        const int64_t c0 = rr.s0 + r * kDynSub, c1 = min(rr.s1, rr.s0 + min(r + kDynStage / kDynSub, rr.r1) * kDynSub);
+        const int cnt = (int)(c1 - c0);
         __syncthreads();
-        for (int k = tid; k < cnt; k += kDynThreads) {
-            const uint4 a = u[c0 + k];
-            atoms[k] = a;
+        for (int k = tid; k < cnt; k += (int)blockDim.x) {
+            uint4 a = axis_first(u[c0 + k], sl.axis);
             const int s = (int)a.w;
-            wts[k] = (s >= 0 && s < nsp) ? bsc[s] : 0.f;
+            a.w = __float_as_uint((s >= 0 && s < nsp) ? bsc[s] : 0.f);
+            atoms[k] = a;
         }
         __syncthreads();
         for (int j0 = 0; j0 < cnt; j0 += kDynSub) {
             const int j1 = min(cnt, j0 + kDynSub);
-            float fr[kDynVPT], fi[kDynVPT];
+            u64 fr[kDynVPT / 2], fi[kDynVPT / 2];
 #pragma unroll
-            for (int q = 0; q < kDynVPT; ++q) fr[q] = fi[q] = 0.f;
+            for (int q = 0; q < kDynVPT / 2; ++q) fr[q] = fi[q] = 0ull;
             for (int j = j0; j < j1; ++j) {
                 const uint4 a = atoms[j];
-                const float w = wts[j];
+                const u64 w = pack2(__uint_as_float(a.w), __uint_as_float(a.w));
+                unsigned ph[kDynVPT];
+                dyn_phases<SHARED>(n0, n1, n2, a, ph);
 #pragma unroll
-                for (int q = 0; q < kDynVPT; ++q) {
-                    const unsigned ph = nx[q] * a.x + ny[q] * a.y + nz[q] * a.z;
-                    float sn, cs;
-                    __sincosf(__int2float_rn((int)ph) * kTwoPiOver2_32, &sn, &cs);
-                    fr[q] = fmaf(w, cs, fr[q]);
-                    fi[q] = fmaf(w, sn, fi[q]);
+                for (int q = 0; q < kDynVPT / 2; ++q) {
+                    float x, y, sx, cx, sy, cy;
+                    unpack2(mul2(pack2(__int2float_rn((int)ph[2 * q]), __int2float_rn((int)ph[2 * q + 1])),
+                                 pack2(kTwoPiOver2_32, kTwoPiOver2_32)),
+                            x, y);
+                    __sincosf(x, &sx, &cx);
+                    __sincosf(y, &sy, &cy);
+                    fr[q] = fma2(w, pack2(cx, cy), fr[q]);
+                    fi[q] = fma2(w, pack2(sx, sy), fi[q]);
                 }
             }
 #pragma unroll
-            for (int q = 0; q < kDynVPT; ++q) {
-                accr[q] += (double)fr[q];
-                acci[q] += (double)fi[q];
+            for (int q = 0; q < kDynVPT / 2; ++q) {
+                float x, y;
+                unpack2(fr[q], x, y);
+                accr[2 * q] += (double)x;
+                accr[2 * q + 1] += (double)y;
+                unpack2(fi[q], x, y);
+                acci[2 * q] += (double)x;
+                acci[2 * q + 1] += (double)y;
             }
         }
     }
 #pragma unroll
     for (int q = 0; q < kDynVPT; ++q)
-        if (vi[q] < nvec) part[(int64_t)blockIdx.y * nvec + vi[q]] = make_double2(accr[q], acci[q]);
+        if (first < sl.n) part[(int64_t)blockIdx.y * sl.n + first + q] = make_double2(accr[q], acci[q]);
 }
 
-// rho_t = sum over splits (fixed order); origin buffers keep a copy as their rho(k, t0).
-__global__ void dyn_rho_gather_kernel(const double2* __restrict__ part, int64_t nvec, int nsplit,
-                                      const DynJob* __restrict__ jobs, int njobs, double2* __restrict__ rho_t,
-                                      double2* __restrict__ rho0) {
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nvec) return;
-    double re = 0.0, im = 0.0;
-    for (int s = 0; s < nsplit; ++s) {
-        const double2 p = part[(int64_t)s * nvec + k];
-        re += p.x;
-        im += p.y;
+// rho_t = sum over the rows (fixed order: warp w of eight takes rows w, w + 8, ..., then the warps in order), 32
+// slots per block; origin buffers keep a copy as their rho(k, t0).
+__global__ void __launch_bounds__(256) dyn_rho_gather_kernel(const double2* __restrict__ part,
+                                                             const int4* __restrict__ slot, int64_t nslot,
+                                                             int64_t nvec, int rows, const DynJob* __restrict__ jobs,
+                                                             int njobs, double2* __restrict__ rho_t,
+                                                             double2* __restrict__ rho0) {
+    __shared__ double2 red[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t s = (int64_t)blockIdx.x * 32 + lane;
+    double2 t = make_double2(0.0, 0.0);
+    if (s < nslot) {
+#pragma unroll 8
+        for (int r = warp; r < rows; r += 8) {
+            const double2 p = part[(int64_t)r * nslot + s];
+            t.x += p.x;
+            t.y += p.y;
+        }
     }
-    rho_t[k] = make_double2(re, im);
+    red[warp][lane] = t;
+    __syncthreads();
+    const int k = warp == 0 && s < nslot ? slot[s].w : -1;
+    if (k < 0) return;
+    for (int w = 1; w < 8; ++w) {
+        t.x += red[w][lane].x;
+        t.y += red[w][lane].y;
+    }
+    rho_t[k] = t;
     for (int j = 0; j < njobs; ++j)
-        if (jobs[j].origin) rho0[(int64_t)jobs[j].buf * nvec + k] = make_double2(re, im);
+        if (jobs[j].origin) rho0[(int64_t)jobs[j].buf * nvec + k] = t;
 }
 
 // Origin frames: phases and coordinates of every atom become the buffer's origin state.
@@ -189,103 +287,127 @@ __global__ void dyn_msd_kernel(const float4* __restrict__ packed, int64_t n, flo
     }
 }
 
-// Partial Fs(k) = sum_j cos(k.(r_j(t) - r_j(t0))) over the atom range of blockIdx.y, for job blockIdx.z.
-__global__ void __launch_bounds__(kDynThreads) dyn_self_kernel(const uint4* __restrict__ u,
-                                                               const uint4* __restrict__ u0, int64_t n,
-                                                               const DynJob* __restrict__ jobs,
-                                                               const int4* __restrict__ vecs, int64_t nvec,
-                                                               int nsplit, double* __restrict__ part) {
-    __shared__ uint4 dis[kDynChunk];
+// Partial Fs(k) = sum_j cos(k.(r_j(t) - r_j(t0))) over the runs of row blockIdx.y, for job blockIdx.z, by slot.
+//
+// What bounds it: the special-function unit's cosine (8.4 clocks per warp and scheduler) and, nearly as long, the
+// FMA pipe's integer multiply-adds of the phase, one per atom less for vectors that share a component.  62,500
+// atoms x 5,319 vectors x 10 origins: 1.33 ms with one wave and a bit of equal blocks, 0.96 ms so (floor of the
+// cosines alone 0.76; five blocks per SM or no unrolling: 1.04 to 1.24 at 256 threads, where this took 1.06).
+template <bool SHARED>
+__global__ void __launch_bounds__(kDynThreads, kDynCtas) dyn_self_kernel(const uint4* __restrict__ u,
+                                                                         const uint4* __restrict__ u0, int64_t n,
+                                                                         const DynJob* __restrict__ jobs, DynSlots sl,
+                                                                         int nsplit, int parts,
+                                                                         double* __restrict__ part) {
+    __shared__ uint4 dis[kDynStage];
     const int tid = threadIdx.x;
     const DynJob jb = jobs[blockIdx.z];
     const uint4* __restrict__ org = u0 + (int64_t)jb.buf * n;
-    unsigned nx[kDynVPT], ny[kDynVPT], nz[kDynVPT];
-    int64_t vi[kDynVPT];
-#pragma unroll
-    for (int q = 0; q < kDynVPT; ++q) {
-        vi[q] = (int64_t)blockIdx.x * kDynThreads * kDynVPT + q * kDynThreads + tid;
-        const int4 v = vi[q] < nvec ? vecs[vi[q]] : make_int4(0, 0, 0, 0);
-        nx[q] = (unsigned)v.x;
-        ny[q] = (unsigned)v.y;
-        nz[q] = (unsigned)v.z;
-    }
-    const int64_t a0 = n * blockIdx.y / nsplit, a1 = n * (blockIdx.y + 1) / nsplit;
+    const int64_t first = ((int64_t)blockIdx.x * blockDim.x + tid) * kDynVPT;
+    unsigned n0[kDynVPT], n1[kDynVPT], n2[kDynVPT];
+    dyn_load_slots(sl, first, n0, n1, n2);
+    const DynRuns rr = dyn_runs(n, blockIdx.y, nsplit, parts);
     double acc[kDynVPT];
 #pragma unroll
     for (int q = 0; q < kDynVPT; ++q) acc[q] = 0.0;
-    for (int64_t c0 = a0; c0 < a1; c0 += kDynChunk) {
-        const int cnt = (int)min((int64_t)kDynChunk, a1 - c0);
+    for (int64_t r = rr.r0; r < rr.r1; r += kDynStage / kDynSub) {
+        const int64_t c0 = rr.s0 + r * kDynSub, c1 = min(rr.s1, rr.s0 + min(r + kDynStage / kDynSub, rr.r1) * kDynSub);
+        const int cnt = (int)(c1 - c0);
         __syncthreads();
-        for (int k = tid; k < cnt; k += kDynThreads) {
+        for (int k = tid; k < cnt; k += (int)blockDim.x) {
             const uint4 a = u[c0 + k], b = org[c0 + k];
-            dis[k] = make_uint4(a.x - b.x, a.y - b.y, a.z - b.z, 0u);  // displacement, exact mod 1 box
+            // displacement, exact mod 1 box
+            dis[k] = axis_first(make_uint4(a.x - b.x, a.y - b.y, a.z - b.z, 0u), sl.axis);
         }
         __syncthreads();
         for (int j0 = 0; j0 < cnt; j0 += kDynSub) {
             const int j1 = min(cnt, j0 + kDynSub);
-            float f[kDynVPT];
+            u64 f[kDynVPT / 2];
 #pragma unroll
-            for (int q = 0; q < kDynVPT; ++q) f[q] = 0.f;
+            for (int q = 0; q < kDynVPT / 2; ++q) f[q] = 0ull;
+#pragma unroll 2
             for (int j = j0; j < j1; ++j) {
-                const uint4 d = dis[j];
+                unsigned ph[kDynVPT];
+                dyn_phases<SHARED>(n0, n1, n2, dis[j], ph);
 #pragma unroll
-                for (int q = 0; q < kDynVPT; ++q) {
-                    const unsigned ph = nx[q] * d.x + ny[q] * d.y + nz[q] * d.z;
-                    f[q] += __cosf(__int2float_rn((int)ph) * kTwoPiOver2_32);
+                for (int q = 0; q < kDynVPT / 2; ++q) {
+                    float x, y;
+                    unpack2(mul2(pack2(__int2float_rn((int)ph[2 * q]), __int2float_rn((int)ph[2 * q + 1])),
+                                 pack2(kTwoPiOver2_32, kTwoPiOver2_32)),
+                            x, y);
+                    f[q] = add2(f[q], pack2(__cosf(x), __cosf(y)));
                 }
             }
 #pragma unroll
-            for (int q = 0; q < kDynVPT; ++q) acc[q] += (double)f[q];
+            for (int q = 0; q < kDynVPT / 2; ++q) {
+                float x, y;
+                unpack2(f[q], x, y);
+                acc[2 * q] += (double)x;
+                acc[2 * q + 1] += (double)y;
+            }
         }
     }
 #pragma unroll
     for (int q = 0; q < kDynVPT; ++q)
-        if (vi[q] < nvec) part[((int64_t)blockIdx.z * nsplit + blockIdx.y) * nvec + vi[q]] = acc[q];
+        if (first < sl.n) part[((int64_t)blockIdx.z * nsplit * parts + blockIdx.y) * sl.n + first + q] = acc[q];
+}
+
+// Per job and vector: the self term's rows added up (fixed order, as for rho).
+__global__ void dyn_self_gather_kernel(const double* __restrict__ part, const int4* __restrict__ slot, int64_t nslot,
+                                       int64_t nvec, int rows, double* __restrict__ self) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nslot) return;
+    const int k = slot[s].w;
+    if (k < 0) return;
+    const double* p = part + (int64_t)blockIdx.y * rows * nslot + s;
+    double t[8] = {};
+    for (int r = 0; r < rows; r += 8)
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+            if (r + c < rows) t[c] += p[(int64_t)(r + c) * nslot];
+    double sum = 0.0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) sum += t[c];
+    self[(int64_t)blockIdx.y * nvec + k] = sum;
+}
+
+// Block sum of v in a fixed order (warp shuffles, warps in order); thread 0 has it.
+__device__ __forceinline__ double dyn_block_sum(double v, double* red) {
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v += red[w];
+    return v;
 }
 
 // One block per (bin, job): the bin's vectors in a fixed order; bin 0's block also adds the MSD.
-__global__ void dyn_reduce_kernel(const double* __restrict__ self_part, const double2* __restrict__ rho_t,
-                                  const double2* __restrict__ rho0, const int32_t* __restrict__ bin_start,
-                                  const int32_t* __restrict__ bin_vec, int64_t nvec, int nsplit, int nbins,
-                                  int ndyn, const DynJob* __restrict__ jobs, const double* __restrict__ msd_part,
-                                  int msd_blocks, int64_t n, double* __restrict__ fc, double* __restrict__ fs,
-                                  double* __restrict__ msd) {
-    __shared__ double red[2][kDynThreads / 32];
+__global__ void __launch_bounds__(kDynThreads) dyn_reduce_kernel(
+    const double* __restrict__ self, const double2* __restrict__ rho_t, const double2* __restrict__ rho0,
+    const int32_t* __restrict__ bin_start, const int32_t* __restrict__ bin_vec, int64_t nvec, int nbins, int ndyn,
+    const DynJob* __restrict__ jobs, const double* __restrict__ msd_part, int msd_blocks, int64_t n,
+    double* __restrict__ fc, double* __restrict__ fs, double* __restrict__ msd) {
+    __shared__ double red[3][kDynThreads / 32];
     const int bin = blockIdx.x, j = blockIdx.y;
     const DynJob jb = jobs[j];
     const int v0 = bin_start[bin], v1 = bin_start[bin + 1];
-    double sc = 0.0, ss = 0.0;
-    for (int t = v0 + threadIdx.x; t < v1; t += blockDim.x) {
+    double sc = 0.0, ss = 0.0, m = 0.0;
+    for (int t = v0 + threadIdx.x; t < v1; t += kDynThreads) {
         const int k = bin_vec[t];
         const double2 a = rho0[(int64_t)jb.buf * nvec + k], b = rho_t[k];
         sc += a.x * b.x + a.y * b.y;
-        double s = 0.0;
-        for (int p = 0; p < nsplit; ++p) s += self_part[((int64_t)j * nsplit + p) * nvec + k];
-        ss += s;
+        ss += self[(int64_t)j * nvec + k];
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        sc += __shfl_down_sync(0xffffffffu, sc, off);
-        ss += __shfl_down_sync(0xffffffffu, ss, off);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        red[0][threadIdx.x >> 5] = sc;
-        red[1][threadIdx.x >> 5] = ss;
-    }
-    __syncthreads();
+    if (bin == 0)
+        for (int b = threadIdx.x; b < msd_blocks; b += kDynThreads) m += msd_part[(int64_t)j * msd_blocks + b];
+    sc = dyn_block_sum(sc, red[0]);
+    ss = dyn_block_sum(ss, red[1]);
+    m = dyn_block_sum(m, red[2]);
     if (threadIdx.x == 0) {
-        double tc = 0.0, ts = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            tc += red[0][w];
-            ts += red[1][w];
-        }
         const int64_t o = ((int64_t)jb.buf * ndyn + jb.lag) * nbins + bin;
-        fc[o] += tc;
-        fs[o] += ts;
-        if (bin == 0) {
-            double m = 0.0;
-            for (int b = 0; b < msd_blocks; ++b) m += msd_part[(int64_t)j * msd_blocks + b];
-            msd[(int64_t)jb.buf * ndyn + jb.lag] += m / (double)n;
-        }
+        fc[o] += sc;
+        fs[o] += ss;
+        if (bin == 0) msd[(int64_t)jb.buf * ndyn + jb.lag] += m / (double)n;
     }
 }
 
@@ -324,10 +446,13 @@ struct trj_dyn_plan {
     trj_ctx* ctx = nullptr;
     int nsp = 0, nbuf = 0, ndyn = 0, nbins = 0;
     int64_t n = 0, nvec = 0;
-    int gx = 1;              // vector blocks of the rho/self kernels
-    int nsplit_rho = 1;
-    int nsplit_cap = 1;      // self-part rows: nsplit * jobs <= nsplit_cap
-    int4* vecs = nullptr;
+    int gx = 1;              // vector blocks the slice counts go by
+    int nsplit_rho = 1;      // slices: they fix the FP32 partial sums
+    int nsplit_cap = 1;      // slices of the self term: nsplit * jobs <= nsplit_cap
+    int parts_rho = 1;       // parts of a slice
+    int gslot = 1, tslot = kDynThreads;  // slot blocks of the rho/self kernels, threads of one
+    DynSlots slots = {};
+    int4* slot_dev = nullptr;
     int32_t* bin_start = nullptr;  // nbins + 1
     int32_t* bin_vec = nullptr;    // vectors of each bin
     float* bsc = nullptr;
@@ -335,10 +460,11 @@ struct trj_dyn_plan {
     uint4* u0 = nullptr;           // nbuf * n
     float4* r0 = nullptr;          // nbuf * n
     float4* rt = nullptr;          // nbuf * n
-    double2* rho_part = nullptr;   // nsplit_rho * nvec
+    double2* rho_part = nullptr;   // rows x slots
     double2* rho_t = nullptr;      // nvec
     double2* rho0 = nullptr;       // nbuf * nvec
-    double* self_part = nullptr;   // nsplit_cap * nvec
+    double* self_part = nullptr;   // rows x jobs x slots
+    double* self = nullptr;        // nbuf * nvec
     double* msd_part = nullptr;    // nbuf * msd_blocks
     double* fc = nullptr;          // nbuf * ndyn * nbins
     double* fs = nullptr;          // nbuf * ndyn * nbins
@@ -366,6 +492,34 @@ static bool dyn_alloc(trj_dyn_plan* p, T** out, size_t count) {
     p->scratch_bytes += (int64_t)bytes;
     *out = reinterpret_cast<T*>(q);
     return true;
+}
+
+// Slices of the self term for nj jobs.
+static int self_split(const trj_dyn_plan* p, int nj) {
+    const int64_t target = (int64_t)p->ctx->sm_count * 8;
+    const int64_t by_atoms = std::max<int64_t>(1, p->n / kDynChunk);
+    const int64_t blocks = (int64_t)p->gx * nj;
+    const int nsplit = (int)std::min<int64_t>(by_atoms, std::max<int64_t>(1, (target + blocks - 1) / blocks));
+    return std::max(1, std::min(nsplit, p->nsplit_cap / nj));
+}
+
+// Parts of a slice: the number that wastes least of the last wave of equal blocks (up to six waves), within the
+// slice's runs and 256 MB of partials.
+static int dyn_parts(const trj_dyn_plan* p, int64_t blocks, int nsplit, int64_t row_bytes) {
+    const double slots = (double)p->ctx->sm_count * (kDynCtas * kDynThreads / p->tslot);
+    const int64_t runs = std::max<int64_t>(1, p->n / ((int64_t)nsplit * kDynSub));
+    const int64_t room = std::max<int64_t>(1, ((int64_t)256 << 20) / std::max<int64_t>(1, row_bytes));
+    const int64_t most = std::max<int64_t>(1, std::min(std::min(runs, room), (int64_t)(6.0 * slots / (double)blocks)));
+    double best = 0.0;
+    int parts = 1;
+    for (int64_t k = 1; k <= most; ++k) {
+        const double waves = (double)(blocks * k) / slots, use = waves / ceil(waves);
+        if (use > best + 0.01) {
+            best = use;
+            parts = (int)k;
+        }
+    }
+    return parts;
 }
 
 extern "C" int trj_dyn_plan_create(trj_ctx* ctx, int nsp, int64_t n, int nbuffer, int ndyn, int64_t nvec,
@@ -400,11 +554,62 @@ extern "C" int trj_dyn_plan_create(trj_ctx* ctx, int nsp, int64_t n, int nbuffer
     const int64_t split_max = std::min<int64_t>(by_atoms, target);
     const int64_t rows_budget = std::max<int64_t>(nbuffer, ((int64_t)256 << 20) / (8 * std::max<int64_t>(nvec, 1)));
     p->nsplit_cap = (int)std::min<int64_t>((int64_t)nbuffer * split_max, std::max<int64_t>(rows_budget, nbuffer));
-    std::vector<int4> vecs(nvec);
     std::vector<int32_t> start(nbins + 1, 0), bv(nvec);
-    for (int64_t v = 0; v < nvec; ++v) {
-        vecs[v] = make_int4(vec_host[3 * v], vec_host[3 * v + 1], vec_host[3 * v + 2], bin_host[v]);
-        start[bin_host[v] + 1] += 1;
+    for (int64_t v = 0; v < nvec; ++v) start[bin_host[v] + 1] += 1;
+    // Slots: vectors by the component of one axis, padded so that no thread's vectors differ in it, for the axis
+    // that needs the least padding; in the caller's order where that is more than 6 % (the phase's first product
+    // is then formed per vector).
+    std::vector<int4> slots;
+    {
+        int best = -1;
+        int64_t best_n = nvec + nvec / 16 + kDynVPT;
+        std::vector<int64_t> order(nvec);
+        for (int ax = 0; ax < 3; ++ax) {
+            for (int64_t v = 0; v < nvec; ++v) order[v] = v;
+            std::stable_sort(order.begin(), order.end(),
+                             [&](int64_t x, int64_t y) { return vec_host[3 * x + ax] < vec_host[3 * y + ax]; });
+            int64_t total = 0;
+            for (int64_t i = 0, j = 0; i < nvec; i = j) {
+                while (j < nvec && vec_host[3 * order[j] + ax] == vec_host[3 * order[i] + ax]) ++j;
+                total += (j - i + kDynVPT - 1) / kDynVPT * kDynVPT;
+            }
+            if (total < best_n) {
+                best_n = total;
+                best = ax;
+            }
+        }
+        const int ax = best >= 0 ? best : 0, a1 = ax == 0 ? 1 : 0, a2 = ax == 2 ? 1 : 2;
+        p->slots.axis = ax;
+        p->slots.shared = best >= 0;
+        for (int64_t v = 0; v < nvec; ++v) order[v] = v;
+        if (best >= 0)
+            std::stable_sort(order.begin(), order.end(),
+                             [&](int64_t x, int64_t y) { return vec_host[3 * x + ax] < vec_host[3 * y + ax]; });
+        auto pad = [&](int c) {
+            while (slots.size() % kDynVPT) slots.push_back(make_int4(c, 0, 0, -1));
+        };
+        for (int64_t i = 0; i < nvec; ++i) {
+            const int32_t* v = vec_host + 3 * order[i];
+            if (best >= 0 && !slots.empty() && slots.back().x != v[ax]) pad(slots.back().x);
+            slots.push_back(make_int4(v[ax], v[a1], v[a2], (int)order[i]));
+        }
+        if (!slots.empty()) pad(slots.back().x);
+    }
+    p->slots.n = (int64_t)slots.size();
+    // block size with the fewest idle threads
+    for (int t = kDynThreads; t >= kDynThreads / 2; t -= 32) {
+        const int64_t quads = p->slots.n / kDynVPT, blocks = std::max<int64_t>(1, (quads + t - 1) / t);
+        if (t == kDynThreads || blocks * t < (int64_t)p->gslot * p->tslot) {
+            p->gslot = (int)blocks;
+            p->tslot = t;
+        }
+    }
+    p->parts_rho = dyn_parts(p, (int64_t)p->gslot * p->nsplit_rho, p->nsplit_rho, 16 * p->slots.n * p->nsplit_rho);
+    int64_t self_rows = 0;  // of every job together, the most for any number of jobs
+    for (int nj = 1; nj <= nbuffer; ++nj) {
+        const int ns = self_split(p, nj);
+        self_rows = std::max<int64_t>(self_rows, (int64_t)nj * ns * dyn_parts(p, (int64_t)p->gslot * ns * nj, ns,
+                                                                              8 * p->slots.n * ns * nj));
     }
     for (int b = 0; b < nbins; ++b) start[b + 1] += start[b];
     {
@@ -414,13 +619,14 @@ extern "C" int trj_dyn_plan_create(trj_ctx* ctx, int nsp, int64_t n, int nbuffer
     trj_device_guard g(ctx->device);
     const int msd_blocks = (int)((n + kDynThreads - 1) / kDynThreads);
     const int64_t rows = (int64_t)nbuffer * ndyn;
-    bool ok = dyn_alloc(p, &p->vecs, nvec) && dyn_alloc(p, &p->bin_start, nbins + 1) &&
+    bool ok = dyn_alloc(p, &p->slot_dev, slots.size()) && dyn_alloc(p, &p->bin_start, nbins + 1) &&
               dyn_alloc(p, &p->bin_vec, nvec) && dyn_alloc(p, &p->bsc, nsp) && dyn_alloc(p, &p->u, n) &&
               dyn_alloc(p, &p->u0, (size_t)nbuffer * n) && dyn_alloc(p, &p->r0, (size_t)nbuffer * n) &&
               dyn_alloc(p, &p->rt, (size_t)nbuffer * n) &&
-              dyn_alloc(p, &p->rho_part, (size_t)p->nsplit_rho * nvec) && dyn_alloc(p, &p->rho_t, nvec) &&
+              dyn_alloc(p, &p->rho_part, (size_t)p->nsplit_rho * p->parts_rho * slots.size()) && dyn_alloc(p, &p->rho_t, nvec) &&
               dyn_alloc(p, &p->rho0, (size_t)nbuffer * nvec) &&
-              dyn_alloc(p, &p->self_part, (size_t)p->nsplit_cap * nvec) &&
+              dyn_alloc(p, &p->self_part, (size_t)self_rows * slots.size()) &&
+              dyn_alloc(p, &p->self, (size_t)nbuffer * nvec) &&
               dyn_alloc(p, &p->msd_part, (size_t)nbuffer * msd_blocks) &&
               dyn_alloc(p, &p->fc, (size_t)rows * nbins) && dyn_alloc(p, &p->fs, (size_t)rows * nbins) &&
               dyn_alloc(p, &p->msd, rows) && dyn_alloc(p, &p->jobs_dev, nbuffer) &&
@@ -433,7 +639,8 @@ extern "C" int trj_dyn_plan_create(trj_ctx* ctx, int nsp, int64_t n, int nbuffer
     }
     cudaError_t e = cudaSuccess;
     if (nvec) {
-        e = cudaMemcpy(p->vecs, vecs.data(), sizeof(int4) * nvec, cudaMemcpyHostToDevice);
+        e = cudaMemcpy(p->slot_dev, slots.data(), sizeof(int4) * slots.size(), cudaMemcpyHostToDevice);
+        p->slots.slot = p->slot_dev;
         if (e == cudaSuccess) e = cudaMemcpy(p->bin_vec, bv.data(), sizeof(int32_t) * nvec, cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess)
@@ -492,10 +699,11 @@ extern "C" int trj_dyn_accumulate(trj_dyn_plan* p, const float* packed_dev, int6
                                                  (double)box[2], p->u);
     int launches = 1;
     if (p->nvec > 0) {
-        dyn_rho_kernel<<<dim3(p->gx, p->nsplit_rho), kDynThreads, 0, s>>>(p->u, n, p->bsc, p->nsp, p->vecs, p->nvec,
-                                                                          p->nsplit_rho, p->rho_part);
-        dyn_rho_gather_kernel<<<(unsigned)((p->nvec + 255) / 256), 256, 0, s>>>(p->rho_part, p->nvec, p->nsplit_rho,
-                                                                               p->jobs_dev, nj, p->rho_t, p->rho0);
+        const int rows = p->nsplit_rho * p->parts_rho;
+        (p->slots.shared ? dyn_rho_kernel<true> : dyn_rho_kernel<false>)<<<dim3(p->gslot, rows), p->tslot, 0, s>>>(
+            p->u, n, p->bsc, p->nsp, p->slots, p->nsplit_rho, p->parts_rho, p->rho_part);
+        dyn_rho_gather_kernel<<<(unsigned)((p->slots.n + 31) / 32), 256, 0, s>>>(p->rho_part, p->slot_dev, p->slots.n, p->nvec, rows, p->jobs_dev, nj,
+                                                 p->rho_t, p->rho0);
         launches += 2;
     }
     dyn_origin_kernel<<<dim3(nb, nj), kDynThreads, 0, s>>>((const float4*)packed_dev, p->u, n, p->jobs_dev, p->u0,
@@ -503,22 +711,21 @@ extern "C" int trj_dyn_accumulate(trj_dyn_plan* p, const float* packed_dev, int6
     dyn_msd_kernel<<<dim3(nb, nj), kDynThreads, 0, s>>>((const float4*)packed_dev, n, box[0], box[1], box[2],
                                                        p->jobs_dev, p->r0, p->rt, p->msd_part);
     launches += 2;
-    const int64_t target = (int64_t)ctx->sm_count * 8;
-    const int64_t by_atoms = std::max<int64_t>(1, n / kDynChunk);
-    int nsplit = (int)std::min<int64_t>(by_atoms, std::max<int64_t>(1, (target + (int64_t)p->gx * nj - 1) /
-                                                                          ((int64_t)p->gx * nj)));
-    nsplit = std::max(1, std::min(nsplit, p->nsplit_cap / nj));
     if (p->nvec > 0) {
+        const int nsplit = self_split(p, nj);
+        const int parts = dyn_parts(p, (int64_t)p->gslot * nsplit * nj, nsplit, 8 * p->slots.n * nsplit * nj);
+        const int rows = nsplit * parts;
         p->timer.begin(ctx, s);
-        dyn_self_kernel<<<dim3(p->gx, nsplit, nj), kDynThreads, 0, s>>>(p->u, p->u0, n, p->jobs_dev, p->vecs,
-                                                                        p->nvec, nsplit, p->self_part);
+        (p->slots.shared ? dyn_self_kernel<true> : dyn_self_kernel<false>)<<<dim3(p->gslot, rows, nj), p->tslot, 0, s>>>(
+            p->u, p->u0, n, p->jobs_dev, p->slots, nsplit, parts, p->self_part);
         p->timer.end(ctx, s);
-        launches += 1;
+        dyn_self_gather_kernel<<<dim3((unsigned)((p->slots.n + 255) / 256), nj), 256, 0, s>>>(
+            p->self_part, p->slot_dev, p->slots.n, p->nvec, rows, p->self);
+        launches += 2;
     }
-    dyn_reduce_kernel<<<dim3(p->nbins, nj), kDynThreads, 0, s>>>(p->self_part, p->rho_t, p->rho0, p->bin_start,
-                                                                 p->bin_vec, p->nvec, nsplit, p->nbins, p->ndyn,
-                                                                 p->jobs_dev, p->msd_part, (int)nb, n, p->fc, p->fs,
-                                                                 p->msd);
+    dyn_reduce_kernel<<<dim3(p->nbins, nj), kDynThreads, 0, s>>>(p->self, p->rho_t, p->rho0, p->bin_start, p->bin_vec,
+                                                                 p->nvec, p->nbins, p->ndyn, p->jobs_dev, p->msd_part,
+                                                                 (int)nb, n, p->fc, p->fs, p->msd);
     launches += 1;
     ctx->launches += launches;
     TRJ_CUDA_TRY(ctx, cudaGetLastError());
