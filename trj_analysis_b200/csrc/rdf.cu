@@ -191,6 +191,22 @@ struct Home {
     float q;            // charge
 };
 
+// What a warp keeps between the culling and the tests, in shared memory so that neither loop holds the other's
+// registers.
+struct WarpState {
+    float4 home[kGroup];        // negated coordinates, Home::hist (bits) of every lane
+    int gs[32], gn[32];         // start and atoms of the neighbour groups of the current 32
+    float home_q[kGroup];
+    float4 box, half;           // the group's box: centre and half-widths
+    float4 cut;                 // its centre less the neighbour cell's image
+    float4 img;
+    int4 walk;                  // j, je, m, e0 of the neighbour walk
+    int4 outer;                 // position in the neighbour list, cell of the homes and its flags, first home
+    int nh;
+};
+
+constexpr size_t kWarpBytes = 16 * kRing + (sizeof(WarpState) + 15) / 16 * 16;  // buffer and state of a warp
+
 // Tests `n4` blocks of four survivors from ring position `head` (SELF: the round's own atoms in lane order
 // from position 0, pairs j > i).  w of a survivor: bytes to add to Home::hist (square layout: species * row
 // bytes; triangular layout: species * 64, a row of the 16 x 16 table).
@@ -205,12 +221,32 @@ struct Home {
 // window of an edge (or, with EDGE, within 2^-20 of the cutoff, where one-ulp changes decide) is looked at
 // again and the few wrong counts are moved.  QMODE instead leaves those out of the first count, since a
 // charge product cannot be taken back exactly.
-template <int MODE, bool SELF, bool FLOOR, bool QMODE, bool SQUARE, bool EDGE>
+template <int MODE, bool SELF, bool FLOOR, bool QMODE, bool SQUARE, bool EDGE, int UNROLL>
 __device__ __forceinline__ void test_run(const float* __restrict__ ring, const double* __restrict__ ring_q, int head,
-                                         int n4, const Home& h, bool has, float ix, float iy, float iz,
-                                         const PairGeom& g, PairCounters& pc, double* myq) {
-    const float cx = MODE == kImgRound ? g.inv_L[0] : ix, cy = MODE == kImgRound ? g.inv_L[1] : iy,
-                cz = MODE == kImgRound ? g.inv_L[2] : iz;
+                                         int n4, const WarpState* __restrict__ ws, const PairGeom& g,
+                                         PairCounters& pc, double* myq) {
+    const int lane = (int)(threadIdx.x & 31u);
+    Home h;
+    {
+        const float4 a = ws->home[lane];
+        h.nx = a.x;
+        h.ny = a.y;
+        h.nz = a.z;
+        h.hist = __float_as_uint(a.w);
+        if (QMODE) h.q = ws->home_q[lane];
+    }
+    const bool has = lane < ws->nh;
+    float cx = 0.f, cy = 0.f, cz = 0.f;
+    if (MODE == kImgShift) {
+        const float4 v = ws->img;
+        cx = v.x;
+        cy = v.y;
+        cz = v.z;
+    } else if (MODE == kImgRound) {
+        cx = g.inv_L[0];
+        cy = g.inv_L[1];
+        cz = g.inv_L[2];
+    }
     const u64 nx = pack2(h.nx, h.nx), ny = pack2(h.ny, h.ny), nz = pack2(h.nz, h.nz);
     const u64 jx = pack2(cx, cx), jy = pack2(cy, cy), jz = pack2(cz, cz);
     const u64 inv = pack2(g.inv_deltar, g.inv_deltar);
@@ -219,8 +255,7 @@ __device__ __forceinline__ void test_run(const float* __restrict__ ring, const d
     const u64 neg1 = pack2(-1.0f, -1.0f), half = pack2(0.5f, 0.5f);
     const float thr = g.edge_thr;
     const float lo = has ? (QMODE ? g.side2_lo : g.side2) : 0.0f, hi = has ? g.side2_hi : 0.0f;
-    const int lane = (int)(threadIdx.x & 31u);
-#pragma unroll 1
+#pragma unroll UNROLL
     for (int k = 0; k < n4; ++k) {
         const int e = (head + 4 * k) & (kRing - 1);
         const ulonglong2 X = *reinterpret_cast<const ulonglong2*>(ring + e);
@@ -359,13 +394,13 @@ __device__ __forceinline__ bool frame_within(unsigned f) {
 
 // One work item of a frame: home group key = item / nseg against segment item % nseg of its neighbour list.
 // hist: shared-memory address of the bin rows (SQUARE), rowtab: of the row table (otherwise).
-template <bool FLOOR, bool QMODE, bool SQUARE, bool EDGE>
+template <bool FLOOR, bool QMODE, bool SQUARE, bool EDGE, int UNROLL>
 __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const float4* __restrict__ sorted,
                                           const int32_t* __restrict__ fstart, const int32_t* __restrict__ fcount,
                                           const int32_t* __restrict__ cflag, bool frame_ok,
                                           const float* __restrict__ sorted_q, float* ring, double* ring_q,
-                                          unsigned hist_base, unsigned rowtab, double* qhist, PairCounters& pc,
-                                          u64& n_tested) {
+                                          WarpState* ws, unsigned hist_base, unsigned rowtab, double* qhist,
+                                          PairCounters& pc, u64& n_tested) {
     const PairGeom& g = p.g;
     const int lane = (int)(threadIdx.x & 31u);
     const unsigned lt = (1u << lane) - 1u;
@@ -379,7 +414,6 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const fl
     const int t0 = seg * p.per_seg, t1 = min(p.list, t0 + p.per_seg);
     // The group's box: centre and half-widths (of all its atoms, so that the pairs tested do not depend on their
     // order; + 0 turns -0 into +0).
-    float bx, by, bz, wx, wy, wz;
     {
         unsigned lo[3] = {0x7f800000u, 0x7f800000u, 0x7f800000u}, hi[3] = {0u, 0u, 0u};
         for (int i = hbeg + lane; i < hend; i += kGroup) {
@@ -393,47 +427,65 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const fl
                 hi[d] = max(hi[d], v[d]);
             }
         }
-        axis_box(lo[0], hi[0], p.cull_pad, bx, wx);
-        axis_box(lo[1], hi[1], p.cull_pad, by, wy);
-        axis_box(lo[2], hi[2], p.cull_pad, bz, wz);
+        float4 c, w;
+        c.w = w.w = 0.f;
+        axis_box(lo[0], hi[0], p.cull_pad, c.x, w.x);
+        axis_box(lo[1], hi[1], p.cull_pad, c.y, w.y);
+        axis_box(lo[2], hi[2], p.cull_pad, c.z, w.z);
+        if (lane == 0) {
+            ws->box = c;
+            ws->half = w;
+        }
     }
     for (int h0 = hbeg; h0 < hend; h0 += kGroup) {
-        const int nh = min(kGroup, hend - h0);
-        const bool has = lane < nh;
-        const float4 a = has ? sorted[h0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-        Home h;
-        h.nx = -a.x;
-        h.ny = -a.y;
-        h.nz = -a.z;
-        h.q = (QMODE && has) ? sorted_q[h0 + lane] : 0.f;
-        const unsigned wa = __float_as_uint(a.w);  // species * row bytes (64 with the row table)
-        h.hist = SQUARE ? hist_base + wa * (unsigned)g.nsp - 4u * kBinBias : rowtab + (wa >> 4);
+        {
+            const int nh = min(kGroup, hend - h0);
+            const bool has = lane < nh;
+            float4 a = has ? sorted[h0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const unsigned wa = __float_as_uint(a.w);  // species * row bytes (64 with the row table)
+            a.x = -a.x;
+            a.y = -a.y;
+            a.z = -a.z;
+            a.w = __uint_as_float(SQUARE ? hist_base + wa * (unsigned)g.nsp - 4u * kBinBias : rowtab + (wa >> 4));
+            ws->home[lane] = a;
+            if (QMODE) ws->home_q[lane] = has ? sorted_q[h0 + lane] : 0.f;
+            if (lane == 0) ws->nh = nh;
+        }
         for (int t = t0; t < t1;) {
             // entries [e_lo, e_hi) of offset o: group e, or (own cell) the e-th after the homes' own
             const int o = t < p.nself ? 0 : 1 + fast_div(t - p.nself, p.div_nsub);
             const int first = o == 0 ? 0 : p.nself + (o - 1) * p.nsub;
             const int e_lo = t - first, e_hi = min(o == 0 ? p.nself : p.nsub, t1 - first);
-            t = first + e_hi;
             const int ex = cx + p.off[o][0], ey = cy + p.off[o][1], ez = cz + p.off[o][2];
             const int c2 = (wrapc(ex, p.nc[0]) * p.nc[1] + wrapc(ey, p.nc[1])) * p.nc[2] + wrapc(ez, p.nc[2]);
             const int f2 = fl | cflag[c2];
             const bool far = f2 & 2;
-            const float ix = ex < 0 ? -g.L[0] : (ex >= p.nc[0] ? g.L[0] : 0.f);
-            const float iy = ey < 0 ? -g.L[1] : (ey >= p.nc[1] ? g.L[1] : 0.f);
-            const float iz = ez < 0 ? -g.L[2] : (ez >= p.nc[2] ? g.L[2] : 0.f);
             const bool plain = p.split_all && !(f2 & 1);  // image known from the cells
-            const int mode = plain ? ((ix != 0.f || iy != 0.f || iz != 0.f) ? kImgShift : kImgNone)
-                                   : far ? kImgAny : p.split_all ? kImgRound : frame_ok ? kImgFold : kImgAny;
-            const int kb = c2 * p.nsub;
+            int mode;
+            {
+                const float4 img = make_float4(ex < 0 ? -g.L[0] : (ex >= p.nc[0] ? g.L[0] : 0.f),
+                                               ey < 0 ? -g.L[1] : (ey >= p.nc[1] ? g.L[1] : 0.f),
+                                               ez < 0 ? -g.L[2] : (ez >= p.nc[2] ? g.L[2] : 0.f), 0.f);
+                mode = plain ? ((img.x != 0.f || img.y != 0.f || img.z != 0.f) ? kImgShift : kImgNone)
+                             : far ? kImgAny : p.split_all ? kImgRound : frame_ok ? kImgFold : kImgAny;
+                __syncwarp();  // the group's box, homes and the last offset's readers
+                if (lane == 0) {
+                    const float4 c = ws->box;
+                    ws->img = img;
+                    ws->cut = plain ? make_float4(c.x - img.x, c.y - img.y, c.z - img.z, 0.f) : c;
+                    ws->outer = make_int4(first + e_hi, c2 * p.nsub, own, h0);
+                }
+                __syncwarp();
+            }
             int head = 0, tail = 0;
-            auto append = [&](const float4& b, float qb, bool keep) {
+            auto append = [&](float x, float y, float z, float w, float qb, bool keep) {
                 const unsigned m = __ballot_sync(0xffffffffu, keep);
                 if (keep) {
                     const int e = (tail + __popc(m & lt)) & (kRing - 1);
-                    ring[e] = b.x;
-                    ring[kRing + e] = b.y;
-                    ring[2 * kRing + e] = b.z;
-                    ring[3 * kRing + e] = b.w;
+                    ring[e] = x;
+                    ring[kRing + e] = y;
+                    ring[2 * kRing + e] = z;
+                    ring[3 * kRing + e] = w;
                     if (QMODE) ring_q[e] = (double)qb;
                 }
                 tail += __popc(m);
@@ -449,10 +501,12 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const fl
                 }
                 return up >> 2;
             };
-#define TRJ_RUN(M, S, N4) test_run<M, S, FLOOR, QMODE, SQUARE, EDGE>(ring, ring_q, head, N4, h, has, ix, iy, iz, g, pc, qhist)
+#define TRJ_RUN(M, S, N4) test_run<M, S, FLOOR, QMODE, SQUARE, EDGE, UNROLL>(ring, ring_q, head, N4, ws, g, pc, qhist)
             if (o == 0 && e_lo == 0) {
                 // pairs j > i of the round's own atoms, through the buffer in lane order
-                append(a, h.q, has);
+                const int nh = ws->nh;
+                const float4 a = lane < nh ? sorted[h0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+                append(a.x, a.y, a.z, a.w, QMODE ? ws->home_q[lane] : 0.f, lane < nh);
                 const int n4 = pad();
                 __syncwarp();
                 if (plain) TRJ_RUN(kImgNone, true, n4);
@@ -460,10 +514,10 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const fl
                 else if (mode == kImgFold) TRJ_RUN(kImgFold, true, n4);
                 else TRJ_RUN(kImgAny, true, n4);
                 __syncwarp();
-                if (EDGE && has) n_tested += (unsigned)(nh - 1 - lane);
+                if (EDGE && lane < nh) n_tested += (unsigned)(nh - 1 - lane);
                 tail = 0;
             }
-            int e0 = e_lo - 32, j = 0, je = 0, gs = 0, gn = 0;  // gs, gn: start and atoms of lane's group
+            int e0 = e_lo - 32, j = 0, je = 0;
             unsigned m = 0;
             bool more = true;
             do {
@@ -477,12 +531,14 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const fl
                                 break;
                             }
                             // lanes over the neighbour groups: which can hold an atom in range of the homes' box
+                            const int4 out = ws->outer;
                             const int e = e0 + lane;
-                            int s = o == 0 ? own + e : e;
+                            int s = o == 0 ? out.z + e : e;
                             if (s >= p.nsub) s -= p.nsub;
                             // half-way round an even number of groups each pair is met twice: the lower has it
-                            bool near = e < e_hi && (o > 0 || 2 * e != p.nsub || 2 * own < p.nsub);
+                            bool near = e < e_hi && (o > 0 || 2 * e != p.nsub || 2 * out.z < p.nsub);
                             if (near && !far) {
+                                const float4 b = ws->box, w = ws->half, img = ws->img;
                                 const int q = (int)(((float)s + 0.5f) * p.inv_sub[2]), sz = s - q * p.sub[2];
                                 const int sx = (int)(((float)q + 0.5f) * p.inv_sub[1]), sy = q - sx * p.sub[1];
                                 const float gx = ((float)ex + ((float)sx + 0.5f) * p.inv_sub[0]) * p.edge[0];
@@ -490,28 +546,29 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const fl
                                 const float gz = ((float)ez + ((float)sz + 0.5f) * p.inv_sub[2]) * p.edge[2];
                                 float dx, dy, dz;
                                 if (p.split_all) {
-                                    dx = axis_gap<false>(gx, bx, wx + p.half[0], 0.f);
-                                    dy = axis_gap<false>(gy, by, wy + p.half[1], 0.f);
-                                    dz = axis_gap<false>(gz, bz, wz + p.half[2], 0.f);
+                                    dx = axis_gap<false>(gx, b.x, w.x + p.half[0], 0.f);
+                                    dy = axis_gap<false>(gy, b.y, w.y + p.half[1], 0.f);
+                                    dz = axis_gap<false>(gz, b.z, w.z + p.half[2], 0.f);
                                 } else {
-                                    dx = axis_gap<true>(gx - ix, bx, wx + p.half[0], g.L[0]);
-                                    dy = axis_gap<true>(gy - iy, by, wy + p.half[1], g.L[1]);
-                                    dz = axis_gap<true>(gz - iz, bz, wz + p.half[2], g.L[2]);
+                                    dx = axis_gap<true>(gx - img.x, b.x, w.x + p.half[0], g.L[0]);
+                                    dy = axis_gap<true>(gy - img.y, b.y, w.y + p.half[1], g.L[1]);
+                                    dz = axis_gap<true>(gz - img.z, b.z, w.z + p.half[2], g.L[2]);
                                 }
                                 near = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
                             }
-                            if (near) {
-                                gs = fstart[kb + s];
-                                gn = fcount[kb + s];
-                            }
                             m = __ballot_sync(0xffffffffu, near);
+                            if (near) {
+                                ws->gs[lane] = fstart[out.y + s];
+                                ws->gn[lane] = fcount[out.y + s];
+                            }
+                            __syncwarp();
                             continue;
                         }
                         const int k = __ffs(m) - 1;
                         m &= m - 1u;
-                        j = __shfl_sync(0xffffffffu, gs, k);
-                        je = j + __shfl_sync(0xffffffffu, gn, k);
-                        if (o == 0 && e0 + k == 0) j = h0 + nh;  // the round's own atoms are done
+                        j = ws->gs[k];
+                        je = j + ws->gn[k];
+                        if (o == 0 && e0 + k == 0) j = ws->outer.w + ws->nh;  // the round's own atoms are done
                         continue;
                     }
                     bool keep = j + lane < je;
@@ -519,33 +576,42 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const fl
                     const float qb = (QMODE && keep) ? sorted_q[j + lane] : 0.f;
                     j += 32;
                     if (keep && !far) {
+                        const float4 c = ws->cut, w = ws->half;
                         float dx, dy, dz;
                         if (plain) {
-                            dx = axis_gap<false>(b.x, bx - ix, wx, 0.f);
-                            dy = axis_gap<false>(b.y, by - iy, wy, 0.f);
-                            dz = axis_gap<false>(b.z, bz - iz, wz, 0.f);
+                            dx = axis_gap<false>(b.x, c.x, w.x, 0.f);
+                            dy = axis_gap<false>(b.y, c.y, w.y, 0.f);
+                            dz = axis_gap<false>(b.z, c.z, w.z, 0.f);
                         } else {
-                            dx = axis_gap<true>(wrap_cull(b.x, g.L[0]), bx, wx, g.L[0]);
-                            dy = axis_gap<true>(wrap_cull(b.y, g.L[1]), by, wy, g.L[1]);
-                            dz = axis_gap<true>(wrap_cull(b.z, g.L[2]), bz, wz, g.L[2]);
+                            dx = axis_gap<true>(wrap_cull(b.x, g.L[0]), c.x, w.x, g.L[0]);
+                            dy = axis_gap<true>(wrap_cull(b.y, g.L[1]), c.y, w.y, g.L[1]);
+                            dz = axis_gap<true>(wrap_cull(b.z, g.L[2]), c.z, w.z, g.L[2]);
                         }
                         keep = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
                     }
                     const int before = tail;
-                    append(b, qb, keep);
-                    if (EDGE && has) n_tested += (unsigned)(tail - before);
+                    append(b.x, b.y, b.z, b.w, qb, keep);
+                    if (EDGE && lane < ws->nh) n_tested += (unsigned)(tail - before);
                 }
                 const int n4 = tail - head >= kRingRun ? kRingRun / 4 : pad();
+                if (lane == 0) ws->walk = make_int4(j, je, (int)m, e0);
                 __syncwarp();  // the other lanes' entries
                 if (mode == kImgNone) TRJ_RUN(kImgNone, false, n4);
                 else if (mode == kImgShift) TRJ_RUN(kImgShift, false, n4);
                 else if (mode == kImgRound) TRJ_RUN(kImgRound, false, n4);
                 else if (mode == kImgFold) TRJ_RUN(kImgFold, false, n4);
                 else TRJ_RUN(kImgAny, false, n4);
-                __syncwarp();
+                const int4 walk = ws->walk;
+                __syncwarp();  // before the buffer and the state are written again
+                j = walk.x;
+                je = walk.y;
+                m = (unsigned)walk.z;
+                e0 = walk.w;
                 head += 4 * n4;
             } while (more);
 #undef TRJ_RUN
+            t = ws->outer.x;
+            __syncwarp();
         }
     }
 }
@@ -595,12 +661,15 @@ __device__ __forceinline__ void add_edges(u64* __restrict__ edge_g, const PairCo
 // the warps' buffers.  SQUARE: a bin row per ordered species pair, so that a pair's row address is a sum of
 // two registers; otherwise the rows of ind_ij through a 16 x 16 table of addresses.
 //
-// What bounds it: instruction issue (76 % of the slots at 62,500 atoms), not the 22 MB it moves.  At 1e6
-// atoms (3 species, 0.86e9 pairs in range) 1.75e9 pairs are tested, in 17.6e6 blocks of four survivors x 32
-// homes of about 100 instructions each, and 4.6e6 neighbour groups read and culled, together a quarter of
-// the time.  Measured: 7.25 -> 2.9 ms at 1e6 atoms, 1.62 -> 0.41 ms at 62,500 (cutoff 10, four cells per
-// axis), 19.3 -> 6.0 ms for the 4e6-atom slab, against 64-atom homes (two per lane) that a CTA walks over
-// staged neighbour cells with a branch per pair.
+// What bounds it: instruction issue, not the 22 MB it moves.  At 1e6 atoms (3 species, 0.86e9 pairs in range)
+// 1.75e9 pairs are tested, in 17.6e6 blocks of four survivors x 32 homes of about 75 instructions each (packed
+// FP32 alone takes 63 of the 80 issue slots of such a block), and 4.6e6 neighbour groups read and culled,
+// together a quarter of the time.  With the culling's variables in registers across the tests 64 registers do
+// not hold both (100 bytes spilled in the inner loop, 97 instructions a block): 2.95 ms at 1e6 atoms, 0.437 ms
+// at 62,500 (cutoff 10, four cells per axis), 6.08 ms for the 4e6-atom slab, 1.83 ms for 256,000 ions; with
+// them in WarpState and two blocks per turn of the loop 2.64, 0.394, 5.50 and 1.63 ms.  (The ions' loop keeps
+// one block per turn: two take 1.97 ms.)  64-atom homes, two per lane, that a CTA walks over staged neighbour
+// cells with a branch per pair: 7.37, 1.69, 19.5 and 3.75 ms.
 template <bool FLOOR, bool QMODE, bool SQUARE, bool EDGE>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     rdf_pairs_kernel(const __grid_constant__ RdfParams p, const float4* __restrict__ sorted,
@@ -616,10 +685,11 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     const PairGeom& g = p.g;
     const int nsp = g.nsp, rw = g.row_words;
     const int nrow = SQUARE ? nsp * nsp : p.nit;
-    // [warps' buffers][QMODE: warps' charge buffers, FP64 rows][count rows]
-    float* ring = reinterpret_cast<float*>(smem) + (size_t)warp * 4 * kRing;
-    double* ring_q = reinterpret_cast<double*>(smem + (size_t)nwarp * 16 * kRing) + (QMODE ? warp * kRing : 0);
-    double* qhist = reinterpret_cast<double*>(smem + (size_t)nwarp * 16 * kRing) + (QMODE ? nwarp * kRing : 0);
+    // [warps' buffers and states][QMODE: warps' charge buffers, FP64 rows][count rows]
+    float* ring = reinterpret_cast<float*>(smem + (size_t)warp * kWarpBytes);
+    WarpState* ws = reinterpret_cast<WarpState*>(smem + (size_t)warp * kWarpBytes + 16 * kRing);
+    double* ring_q = reinterpret_cast<double*>(smem + (size_t)nwarp * kWarpBytes) + (QMODE ? warp * kRing : 0);
+    double* qhist = reinterpret_cast<double*>(smem + (size_t)nwarp * kWarpBytes) + (QMODE ? nwarp * kRing : 0);
     unsigned* hist = reinterpret_cast<unsigned*>(qhist + (QMODE ? rw : 0));
     for (int k = tid; k < nrow * rw; k += blockDim.x) hist[k] = 0u;
     if (QMODE)
@@ -650,8 +720,9 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
         if (lane == 0) item = atomicAdd(work, 1u);
         item = __shfl_sync(0xffffffffu, item, 0);
         if (item >= p.nitems) break;
-        pair_item<FLOOR, QMODE, SQUARE, EDGE>(p, (int)item, sorted, fstart, fcount, cflag, frame_ok, sorted_q, ring,
-                                              ring_q, hist_base, trj_smem_addr(rowtab), qhist, pc, n_tested);
+        pair_item<FLOOR, QMODE, SQUARE, EDGE, QMODE ? 1 : 2>(p, (int)item, sorted, fstart, fcount, cflag, frame_ok,
+                                                             sorted_q, ring, ring_q, ws, hist_base,
+                                                             trj_smem_addr(rowtab), qhist, pc, n_tested);
     }
     __syncthreads();
     merge_rows<SQUARE>(p, hist, hist_g, pc);
@@ -1067,7 +1138,8 @@ __global__ void __launch_bounds__(kBatchThreads) batch_place_kernel(const BatchH
 }
 
 // What bounds it: instruction issue, as the single-frame kernel.  64 frames of 1,000 to 16,384 atoms: 2.74 ms
-// for an all-pairs sweep with a branch per pair, 0.70 ms so (80 registers a thread; 64, at four CTAs per SM: 0.74).
+// for an all-pairs sweep with a branch per pair, 0.70 ms so (80 registers a thread; 64, at four CTAs per SM: 0.73;
+// two blocks of survivors per turn of the loop: 0.76, runs are short in small frames).
 __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const BatchHeader* __restrict__ hdr,
                                                                        const BatchItem* __restrict__ items, BatchSort st,
                                                                        int hist_words) {
@@ -1076,8 +1148,9 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
     __shared__ unsigned rowtab[256];
     __shared__ int next;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    float* ring = reinterpret_cast<float*>(smem) + (size_t)warp * 4 * kRing;
-    unsigned* hist = reinterpret_cast<unsigned*>(smem + (size_t)(kBatchThreads / 32) * 16 * kRing);
+    float* ring = reinterpret_cast<float*>(smem + (size_t)warp * kWarpBytes);
+    WarpState* ws = reinterpret_cast<WarpState*>(smem + (size_t)warp * kWarpBytes + 16 * kRing);
+    unsigned* hist = reinterpret_cast<unsigned*>(smem + (size_t)(kBatchThreads / 32) * kWarpBytes);
     const unsigned hist_base = trj_smem_addr(hist), rowtab_base = trj_smem_addr(rowtab);
     for (int k = tid; k < batch_hist_smem_words(hist_words); k += kBatchThreads) hist[k] = 0u;
     const int nitems = hdr->nitems;
@@ -1121,8 +1194,8 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
             item = __shfl_sync(0xffffffffu, item, 0);
             if (item >= p.nitems) break;
 #define TRJ_ITEM(F, S, E)                                                                                       \
-    pair_item<F, false, S, E>(p, (int)item, sorted, fstart, fcount, cflag, frame_ok, nullptr, ring, nullptr, hist_base, \
-                              rowtab_base, nullptr, pc, n_tested)
+    pair_item<F, false, S, E, 1>(p, (int)item, sorted, fstart, fcount, cflag, frame_ok, nullptr, ring, nullptr, ws, \
+                                 hist_base, rowtab_base, nullptr, pc, n_tested)
             if (p.g.floor_bins) TRJ_ITEM(true, false, true);
             else if (!square) TRJ_ITEM(false, false, true);
             else if (p.g.want_edge) TRJ_ITEM(false, true, true);
@@ -1362,7 +1435,7 @@ static bool pair_shape(const trj_ctx* ctx, int nsp, int nit, int row_words, bool
     for (int i = 0; i < 7; ++i)
         for (int square = 1; square >= 0; --square) {
             const size_t rows = square ? (size_t)nsp * nsp : (size_t)nit;
-            const size_t smem = (size_t)kWarps[i] * kRing * (16 + (charged ? 8 : 0)) +
+            const size_t smem = (size_t)kWarps[i] * (kWarpBytes + (charged ? 8 * kRing : 0)) +
                                 (size_t)row_words * (4 * rows + (charged ? 8 : 0)) + 16;
             // the driver's reserve and the static shared memory of a CTA
             if (smem + 1200 > optin || (smem + 1024 + 1200) * kCtas[i] > per_sm) continue;
@@ -1689,7 +1762,7 @@ extern "C" int trj_rdf_plan_set_wait(trj_rdf_plan* plan, int64_t clocks, int sta
 // ---- fused multi-request launch: host side of the pair kernel ----------------------------------
 
 size_t trj_batch_pairs_smem(int hist_words) {
-    return (size_t)(kBatchThreads / 32) * 16 * kRing + 4 * (size_t)batch_hist_smem_words(hist_words);
+    return (size_t)(kBatchThreads / 32) * kWarpBytes + 4 * (size_t)batch_hist_smem_words(hist_words);
 }
 
 int trj_batch_pairs_prepare(int hist_words) {
