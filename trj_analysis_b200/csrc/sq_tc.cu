@@ -10,8 +10,7 @@
 // hi*hi + hi*lo + lo*hi (three tcgen05.mma kind::f16 per K-step into one FP32 TMEM accumulator).
 //
 // Operands: A is built by the producer warps straight into tensor memory (the tcgen05.mma form
-// with A in TMEM), in two alternating half-stage buffers of 16 atoms, so shared-memory bandwidth
-// goes to the B operand only.  B (the split Z factors) is a per-frame table, blocked by 32-atom stage
+// with A in TMEM), in a ring of 32-atom buffers, so shared-memory bandwidth goes to the B operand only.  B (the split Z factors) is a per-frame table, blocked by 32-atom stage
 // ([stage][row][32 atoms x (re, im)], so one stage's rows are contiguous), read with 2-D TMA loads
 // (128-byte swizzle, no multicast) through a ring of 32-atom stages; each stage also carries the
 // atoms' x/y phases, from which the producers evaluate the X and Y factors of the tile in shared
@@ -29,15 +28,20 @@
 // factor at FP32 accuracy.
 //
 // Work item = (tile, chunk of one species' atoms).  Persistent CTAs walk their items chunk-major.
-// Roles per CTA (704 threads), handing stages to each other through mbarriers only: warps 8-11
-// evaluate the X/Y factors of a stage into one of two shared-memory buffers; warps 0-7 form the
-// products, split them and store them into the A buffers in TMEM (the two warps of one TMEM lane
-// quarter split a half-stage's 16 atoms); warps 12-19 drain the accumulator (two warps per lane
-// quarter, alternating 16-column chunks); warp 20 issues the TMA loads; warp 21 allocates TMEM and
-// one of its lanes issues the MMAs.  Each role runs at its own pace: a warp arrives on a barrier and
-// moves on (two forms that tied the roles closer were slower at c3: the builders evaluating the
-// factors themselves and issuing the MMAs, 16.2 ms, and the builders issuing the MMAs after a named
-// barrier per half-stage, 13.5 ms, against 10.9 ms).  Every mbarrier wait is bounded and raises TRJ_DEV_TIMEOUT instead of hanging.
+// Roles per CTA (864 threads), handing stages to each other through mbarriers only: warps 0-7 form the
+// products X * Y, split them and store them into the A ring in TMEM (the two warps of one TMEM lane
+// quarter split a stage's atoms); warps 8-23 drain the accumulator; warp 24 loads the B rows, warp 25 the
+// X/Y factor blocks; warp 26 allocates TMEM and issues the MMAs.  Each role runs at its own pace: a warp
+// arrives on a barrier and moves on.  Every mbarrier wait is bounded and raises TRJ_DEV_TIMEOUT instead of
+// hanging.  (The CTA-pair form has its own roles, with the factors evaluated by four warps of each CTA.)
+//
+// What bounds it: the chain of the issuing warp.  With all loads, products, stores and drains taken out it
+// still took 8.4 of 9.98 ms at 1e6 atoms, hardly less with 64-column tiles, as long as `if (lane == 0)` picked
+// the issuing thread: one that the compiler cannot know to be alone has its descriptors brought over
+// lane by lane.  So the issuing warps walk the stages as a whole, on values known to be the same in all
+// lanes (the warp's number and the TMEM address through a shuffle), and an elected lane issues: 7.67 ms.
+// One handoff per stage instead of two: 7.41.  A first try of a barrier without its clock: 7.2.
+// 62,500 atoms: 370 -> 208 us.  Of the 7.2 ms the MMAs alone, without data, are 6.0.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -48,9 +52,7 @@
 
 namespace {
 
-// Builders: two warps per TMEM lane quarter, each taking 8 atoms of a half-stage.  Measured at c3
-// against other layouts of the same roles: four warps per quarter (4 atoms each) 11.46 ms, against
-// 10.88 ms for two.
+// Builders: two warps per TMEM lane quarter, each taking 8 atoms of each half of a stage.
 constexpr int kBuildWarps = 8;                     // warps 0-7: A products into TMEM
 constexpr int kXyWarps = 4;                        // warps 8-11: X/Y factors into shared memory
 constexpr int kEpiWarps = 8;                       // warps 12-19: accumulator drains
@@ -74,7 +76,7 @@ constexpr int k1Threads = (k1MmaWarp + 1) * 32;     // 864
 constexpr int k1RegChunks = 6;
 constexpr int k1TailCol = 8 * 4 * k1RegChunks;      // 192
 constexpr int k1TailBytes = k1EpiWarps * 8 * 32 * 4;  // 16 KB
-constexpr int k1MaxABufs = 9;                       // A half-stage buffers of 32 TMEM columns
+constexpr int k1MaxABufs = 7;                       // A buffers (32 atoms) of 64 TMEM columns
 constexpr int kXyStages = 6;                        // X/Y factor-block ring
 static_assert(k1TailCol + 32 >= 224, "running-sum chunks cover the widest tile");
 constexpr int kStageSlots = 32;  // atoms per stage: K = 64 bf16 = one 128-byte swizzle row of B
@@ -88,16 +90,19 @@ constexpr int kXBytes = kXyRow * kTcTileNx * 8;  // X factors [16 nx][kXyRow] as
 constexpr int kYBytes = kXyRow * kTcTileNy * 8;  // Y factors [8 ny][kXyRow] as (yr, yi)
 constexpr int kXyBytes = kXBytes + kYBytes;           // one of the two X/Y buffers
 constexpr int kUxyBytes = kStageSlots * 8;            // 32 atoms x (ux, uy)
-// Factor blocks of one stage in the one-CTA form: [16 atom pairs][16 nx (8 ny)] x (re, im) of the pair's
-// two atoms, the order in which the builders read them.
+// Factor blocks of one stage in the one-CTA form: [4 groups of 4 atom pairs][16 nx (8 ny)][pair] x (re, im) of
+// the pair's two atoms, the order in which the builders read them.
 constexpr int kXBlockBytes = kStageSlots / 2 * kTcTileNx * 16;  // 4096
 constexpr int kYBlockBytes = kStageSlots / 2 * kTcTileNy * 16;  // 2048
 constexpr int kMaxStages = 8;
 constexpr int kChunkAtoms = 12288;  // atom slots per chunk: the Z-table rows of one chunk are ~10 MB
 constexpr int kMaxTileCols = 224;
 // TMEM columns of the one-CTA form (512 allocated): the accumulator at 0 (bmax columns, the widest
-// tile), then from the next multiple of 32 as many A half-stage buffers of 32 columns (16 of packed
-// bf16 pairs for hi, then 16 for lo) as fit, up to k1MaxABufs: 9 for every bmax <= 224.
+// tile), then from the next multiple of 32 as many A buffers of 64 columns (one stage: 32 of packed
+// bf16 pairs for hi, then 32 for lo) as fit, up to k1MaxABufs: 4 for bmax above 192.  Four whole stages take
+// the place of nine half-stages: half the barriers per stage are worth more than the finer ring (7.67 -> 7.41 ms).
+// Two accumulators, drained in turn, would leave three half-stages beside 208 columns: no gain at 1e6 atoms
+// (8.18 against 8.19 ms), 2 % at 62,500.
 constexpr uint32_t kTmemCols = 512;
 // CTA-pair form: accumulator at 0, four full-stage A buffers (32 columns hi, 32 lo) from 224; its
 // FP32 running sum lives in shared memory.
@@ -132,7 +137,7 @@ struct TcParams {
     int bmax;  // B rows of a stage buffer
     int table_rows;  // Z-table rows per 32-slot block
     uint32_t a_col;  // TMEM column of the first A buffer
-    int nabuf;       // A half-stage buffers
+    int nabuf;       // A buffers
     const float4* xtab;       // X factor blocks [stage][nx block][pair][16]
     const float4* ytab;       // Y factor blocks [stage][ny block][pair][8]
     int nxb, nyb, nx0min, ny0min;
@@ -188,7 +193,7 @@ struct TcState {
     int64_t acc_stride = 0;
     CUtensorMap map_hi, map_lo, map_hi64, map_lo64;  // 16-row and 64-row boxes
     int nstages = 2, stage_bytes = 0, smem_bytes = 0, bmax = 0;
-    int nabuf = 2;  // A half-stage buffers in TMEM
+    int nabuf = 2;  // A buffers in TMEM
     int a_col = 0;  // TMEM column of the first A buffer
     int flush_stages = 8;  // 256 atoms per FP32 tensor-core run between drains
     int grid = 0;
@@ -354,6 +359,30 @@ __device__ __forceinline__ bool timed_wait(uint64_t* bar, unsigned parity, unsig
     return false;
 }
 
+// A wait of a whole warp, with one answer for its lanes; the clock of the limit is read only when the first
+// try fails (the issuing warp's usual wait is over before it starts).
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, unsigned parity, unsigned* status) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(trj_smem_addr(bar)), "r"(parity), "r"(TRJ_SUSPEND_NS)
+        : "memory");
+    if (__all_sync(0xffffffffu, done)) return true;
+    if (__all_sync(0xffffffffu, trj_mbar_wait(bar, parity))) return true;
+    trj_raise(status, TRJ_DEV_TIMEOUT);
+    return false;
+}
+
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 // ---- per-frame table ---------------------------------------------------------
 // slot -> atom of the species-padded layout; padding slots carry zero factors.  Within a species
 // the slots visit the atoms in the order local * mul[a] mod n_a (mul coprime with n_a, near the
@@ -408,8 +437,8 @@ __global__ void tc_ztable_kernel(const uint4* __restrict__ phase, const int64_t*
 }
 
 // X and Y factors of every 32-slot stage, per block of 16 nx (8 ny) values of the tiles, in the order
-// the builders read them: [stage][block][atom pair][value of the block] x (re, im) of the pair's two
-// atoms.  Consecutive threads take consecutive values of one pair: the stores of a warp are contiguous.
+// the builders read them: [stage][block][4 atom pairs][value of the block][pair] x (re, im) of the pair's
+// two atoms.  Consecutive threads take consecutive entries: the stores of a warp are contiguous.
 // A CTA has one stage, a thread one value and pair of every block (of every other block of ny), so that its
 // two phases grow by a constant and nothing is divided.  At 1e6 atoms 0.43 -> 0.225 ms (62,500: 21.6 -> 13.0
 // us) against one entry per thread, found by two 64-bit divisions; what is left is the stores and sincospif.
@@ -422,8 +451,8 @@ __global__ void __launch_bounds__(kXyThreads)
     const uint2* u = uxy + stage * kStageSlots;
     const int tid = threadIdx.x;
     {
-        const int pair = tid / kTcTileNx;
-        const unsigned n = (unsigned)(nx0min + tid % kTcTileNx), u0 = u[2 * pair].x, u1 = u[2 * pair + 1].x;
+        const int pair = tid / (4 * kTcTileNx) * 4 + tid % 4;
+        const unsigned n = (unsigned)(nx0min + tid / 4 % kTcTileNx), u0 = u[2 * pair].x, u1 = u[2 * pair + 1].x;
         unsigned p0 = n * u0, p1 = n * u1;
         float4* out = xtab + stage * nxb * kXyThreads + tid;
         for (int b = 0; b < nxb; ++b) {
@@ -435,8 +464,8 @@ __global__ void __launch_bounds__(kXyThreads)
     }
     {
         constexpr int kHalf = kXyThreads / 2;
-        const int pair = tid % kHalf / kTcTileNy, b0 = tid / kHalf;
-        const unsigned n = (unsigned)(ny0min + kTcTileNy * b0 + tid % kTcTileNy);
+        const int pair = tid % kHalf / (4 * kTcTileNy) * 4 + tid % 4, b0 = tid / kHalf;
+        const unsigned n = (unsigned)(ny0min + kTcTileNy * b0 + tid / 4 % kTcTileNy);
         const unsigned u0 = u[2 * pair].y, u1 = u[2 * pair + 1].y;
         unsigned p0 = n * u0, p1 = n * u1;
         float4* out = ytab + stage * nyb * kHalf + tid;
@@ -449,17 +478,35 @@ __global__ void __launch_bounds__(kXyThreads)
     }
 }
 
-// The hi and lo BF16 pairs of A for row (nxl, nyl) and the 8 atoms of pairs p0 .. p0 + 3 from a stage's
-// factor blocks (lanes of one quarter-warp read consecutive 16-byte entries: no bank conflicts).
-__device__ __forceinline__ void build_row_tab(const float4* xb, const float4* yb, int nxl, int nyl, int p0,
+// The hi and lo BF16 pairs of A for the 32 rows of a lane quarter (16 nx x the two ny from y0) and the 8 atoms
+// of the pair group `pq`, as the 16x256b fragments of tcgen05.st: words 0-3 for TMEM lanes 0-15 (the first ny),
+// 4-7 for lanes 16-31; of each four, two atoms of row lane / 4 and two of row lane / 4 + 8.  A lane then has 2 nx
+// and 2 ny of one atom pair, four 16-byte reads for 8 products (lanes read consecutive entries: no bank
+// conflicts), half of what a lane per row reads.
+__device__ __forceinline__ void build_quarter(const float4* xb, const float4* yb, int lane, int y0, int pq,
                                               uint32_t (&hw)[8], uint32_t (&lw)[8]) {
+    const float4* xp = xb + pq * 4 * kTcTileNx + lane;
+    const float4* yp = yb + (pq * kTcTileNy + y0) * 4 + (lane & 3);
+    const float4 x[2] = {xp[0], xp[32]}, y[2] = {yp[0], yp[4]};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float4 x = xb[(p0 + k) * kTcTileNx + nxl], y = yb[(p0 + k) * kTcTileNy + nyl];
-        product_split(x.x, x.y, y.x, y.y, hw[2 * k], lw[2 * k]);
-        product_split(x.z, x.w, y.z, y.w, hw[2 * k + 1], lw[2 * k + 1]);
-    }
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int w = 4 * i + 2 * k;
+            product_split(x[k].x, x[k].y, y[i].x, y[i].y, hw[w], lw[w]);
+            product_split(x[k].z, x[k].w, y[i].z, y[i].w, hw[w + 1], lw[w + 1]);
+        }
 }
+
+// Stores build_quarter's words: 8 columns of the warp's 32 TMEM lanes.
+__device__ __forceinline__ void tmem_st_quarter(uint32_t taddr, const uint32_t (&w)[8]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+        asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr + (uint32_t)(i << 20)),
+                     "r"(w[4 * i]), "r"(w[4 * i + 1]), "r"(w[4 * i + 2]), "r"(w[4 * i + 3])
+                     : "memory");
+}
+static_assert(kHalfAtoms == 8 && kTcTileNx == 16, "a builder warp's half of a stage");
 
 // ---- the contraction kernel ------------------------------------------------
 
@@ -474,7 +521,8 @@ __global__ void __launch_bounds__(k1Threads, 1)
     __shared__ int abort_flag_s;
     volatile int& abort_flag = abort_flag_s;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be the same in all lanes
     const int NS = p.nstages;
     const int NA = p.nabuf;
     const int F = p.flush_stages;
@@ -514,40 +562,43 @@ __global__ void __launch_bounds__(k1Threads, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
     if (warp == k1TmaWarp) {
-        if (lane == 0) {
+        {
             // ring position of the next stage (slot, phase) kept incrementally: no divisions per stage
             int slot = 0, issued = 0;
             unsigned phase = 0;
-            for (int li = item0; li < item1 && !abort_flag; ++li) {
+            for (int li = item0; li < item1 && !__any_sync(0xffffffffu, abort_flag); ++li) {
                 const int it = p.cta_items[li];
                 const TcTile T = p.tiles[it % p.ntiles];
                 const TcChunk C = p.chunks[it / p.ntiles];
-                const int nst = (C.slot1 - C.slot0) / kStageSlots;
+                const int nst = __shfl_sync(0xffffffffu, (C.slot1 - C.slot0) / kStageSlots, 0);
                 const unsigned bytes = (unsigned)(2 * T.ncols * 128);
                 const int n64 = T.ncols / 64;  // B rows as 64-row boxes, then 16-row boxes
                 for (int s = 0; s < nst; ++s) {
-                    if (!timed_wait(&empty_b[slot], phase ^ 1, p.status)) {
+                    if (!warp_wait(&empty_b[slot], phase ^ 1, p.status)) {
                         abort_flag = 1;
                         break;
                     }
                     uint8_t* bh = stage_ptr(slot);
                     uint8_t* bl = bh + p.bmax * 128;
-                    trj_mbar_arrive_expect_tx(&full_b[slot], bytes);
                     const int slot0 = C.slot0 + s * kStageSlots;
                     // rows of this stage's 32-slot block: contiguous 128-byte rows from row0
                     const int row0 = (slot0 / kStageSlots) * p.table_rows + T.brow;
-                    int r = 0;
-                    for (int b = 0; b < n64; ++b, r += 64) {
-                        tma_load_2d(bh + r * 128, &map_hi64, 0, row0 + r, &full_b[slot]);
-                        tma_load_2d(bl + r * 128, &map_lo64, 0, row0 + r, &full_b[slot]);
+                    if (elect_one()) {
+                        trj_mbar_arrive_expect_tx(&full_b[slot], bytes);
+                        int r = 0;
+                        for (int b = 0; b < n64; ++b, r += 64) {
+                            tma_load_2d(bh + r * 128, &map_hi64, 0, row0 + r, &full_b[slot]);
+                            tma_load_2d(bl + r * 128, &map_lo64, 0, row0 + r, &full_b[slot]);
+                        }
+                        for (; r < T.ncols; r += 16) {
+                            tma_load_2d(bh + r * 128, &map_hi, 0, row0 + r, &full_b[slot]);
+                            tma_load_2d(bl + r * 128, &map_lo, 0, row0 + r, &full_b[slot]);
+                        }
                     }
-                    for (; r < T.ncols; r += 16) {
-                        tma_load_2d(bh + r * 128, &map_hi, 0, row0 + r, &full_b[slot]);
-                        tma_load_2d(bl + r * 128, &map_lo, 0, row0 + r, &full_b[slot]);
-                    }
+                    __syncwarp();
                     ++issued;
                     if (++slot == NS) {
                         slot = 0;
@@ -566,27 +617,30 @@ __global__ void __launch_bounds__(k1Threads, 1)
             }
         }
     } else if (warp == k1XyWarp) {
-        if (lane == 0) {
+        {
             // X and Y factor blocks of every stage, released by the builders once they have read them
             int slot = 0, issued = 0;
             unsigned phase = 0;
-            for (int li = item0; li < item1 && !abort_flag; ++li) {
+            for (int li = item0; li < item1 && !__any_sync(0xffffffffu, abort_flag); ++li) {
                 const int it = p.cta_items[li];
                 const TcTile T = p.tiles[it % p.ntiles];
                 const TcChunk C = p.chunks[it / p.ntiles];
-                const int nst = (C.slot1 - C.slot0) / kStageSlots;
+                const int nst = __shfl_sync(0xffffffffu, (C.slot1 - C.slot0) / kStageSlots, 0);
                 const int bx = (T.nx0 - p.nx0min) / kTcTileNx, by = (T.ny0 - p.ny0min) / kTcTileNy;
                 for (int s = 0; s < nst; ++s) {
-                    if (!timed_wait(&empty_xy[slot], phase ^ 1, p.status)) {
+                    if (!warp_wait(&empty_xy[slot], phase ^ 1, p.status)) {
                         abort_flag = 1;
                         break;
                     }
                     uint8_t* xf = xy_ptr(slot);
-                    trj_mbar_arrive_expect_tx(&full_xy[slot], (unsigned)(kXBlockBytes + kYBlockBytes));
-                    const int64_t stg = (C.slot0 + s * kStageSlots) / kStageSlots;
-                    trj_bulk_g2s(xf, p.xtab + (stg * p.nxb + bx) * (kXBlockBytes / 16), kXBlockBytes, &full_xy[slot]);
-                    trj_bulk_g2s(xf + kXBlockBytes, p.ytab + (stg * p.nyb + by) * (kYBlockBytes / 16), kYBlockBytes,
-                                 &full_xy[slot]);
+                    if (elect_one()) {
+                        trj_mbar_arrive_expect_tx(&full_xy[slot], (unsigned)(kXBlockBytes + kYBlockBytes));
+                        const int64_t stg = (C.slot0 + s * kStageSlots) / kStageSlots;
+                        trj_bulk_g2s(xf, p.xtab + (stg * p.nxb + bx) * (kXBlockBytes / 16), kXBlockBytes, &full_xy[slot]);
+                        trj_bulk_g2s(xf + kXBlockBytes, p.ytab + (stg * p.nyb + by) * (kYBlockBytes / 16), kYBlockBytes,
+                                     &full_xy[slot]);
+                    }
+                    __syncwarp();
                     ++issued;
                     if (++slot == kXyStages) {
                         slot = 0;
@@ -603,7 +657,8 @@ __global__ void __launch_bounds__(k1Threads, 1)
             }
         }
     } else if (warp == k1MmaWarp) {
-        if (lane == 0) {
+        {
+            // the warp walks the stages as a whole, one elected lane issues (see the top of the file)
             // B descriptor of stage slot 0; slot k sits k * stage_bytes further (the start-address
             // field holds addr >> 4 in 14 bits, which covers all of shared memory, so the offset adds
             // without carry).  A K-step of 16 bf16 (32 bytes) adds 2; the lo operand of B sits bmax
@@ -612,57 +667,52 @@ __global__ void __launch_bounds__(k1Threads, 1)
             const uint64_t b_lo = (uint64_t)((p.bmax * 128) >> 4);
             const uint64_t b_step = (uint64_t)(p.stage_bytes >> 4);
             int slot = 0, fg = 0, ab = 0;
-            unsigned phase = 0, aphase = 0;  // B ring phase; A ring (NA half-stage buffers) phase
+            unsigned phase = 0, aphase = 0;  // B ring phase; A ring (NA buffers) phase
             uint64_t bh = b0desc;            // B descriptor of the current slot
-            for (int li = item0; li < item1 && !abort_flag; ++li) {
+            for (int li = item0; li < item1 && !__any_sync(0xffffffffu, abort_flag); ++li) {
                 const int it = p.cta_items[li];
                 const TcTile T = p.tiles[it % p.ntiles];
                 const TcChunk C = p.chunks[it / p.ntiles];
-                const int nst = (C.slot1 - C.slot0) / kStageSlots;
-                const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(T.ncols >> 3) << 17) |
+                const int nst = __shfl_sync(0xffffffffu, (C.slot1 - C.slot0) / kStageSlots, 0);
+                const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(__shfl_sync(0xffffffffu, T.ncols, 0) >> 3) << 17) |
                                        ((uint32_t)(128 >> 4) << 24);
                 int rs = 0;  // stage within the current run
                 for (int s = 0; s < nst; ++s) {
                     const bool first = rs == 0;
                     // the epilogue must have read the previous run out of the accumulator
-                    if (first && fg >= 1 && !timed_wait(&acc_empty, (fg - 1) & 1, p.status)) {
+                    if (first && fg >= 1 && !warp_wait(&acc_empty, (fg - 1) & 1, p.status)) {
                         abort_flag = 1;
                         break;
                     }
-                    if (!timed_wait(&full_b[slot], phase, p.status)) {
+                    if (!warp_wait(&full_b[slot], phase, p.status)) {
                         abort_flag = 1;
                         break;
                     }
                     const uint64_t bl = bh + b_lo;
-                    bool ok = true;
-                    for (int hh = 0; hh < 2 && ok; ++hh) {
-                        const int hb = ab;
-                        if (!timed_wait(&full_a[hb], aphase, p.status)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint32_t ah = tmem + p.a_col + (uint32_t)(32 * hb), al = ah + 16;
-#pragma unroll
-                        for (int k2 = 0; k2 < 2; ++k2) {
-                            const int kk = 2 * hh + k2;
-                            mma_ts(tmem, ah + 8 * k2, bh + 2 * kk, idesc, (first && kk == 0) ? 0u : 1u);
-                            mma_ts(tmem, ah + 8 * k2, bl + 2 * kk, idesc, 1u);
-                            mma_ts(tmem, al + 8 * k2, bh + 2 * kk, idesc, 1u);
-                        }
-                        mma_commit(&empty_a[hb]);
-                        if (++ab == NA) {
-                            ab = 0;
-                            aphase ^= 1;
-                        }
-                    }
-                    if (!ok) {
+                    if (!warp_wait(&full_a[ab], aphase, p.status)) {
                         abort_flag = 1;
                         break;
                     }
-                    mma_commit(&empty_b[slot]);
-                    if (++rs == F || s == nst - 1) {
-                        mma_commit(&acc_full);
+                    tc_fence_after();
+                    const bool flush = ++rs == F || s == nst - 1;
+                    if (elect_one()) {
+                        const uint32_t ah = tmem + p.a_col + (uint32_t)(2 * kStageSlots * ab), al = ah + kStageSlots;
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) {
+                            mma_ts(tmem, ah + 8 * kk, bh + 2 * kk, idesc, (first && kk == 0) ? 0u : 1u);
+                            mma_ts(tmem, ah + 8 * kk, bl + 2 * kk, idesc, 1u);
+                            mma_ts(tmem, al + 8 * kk, bh + 2 * kk, idesc, 1u);
+                        }
+                        mma_commit(&empty_a[ab]);
+                        mma_commit(&empty_b[slot]);
+                        if (flush) mma_commit(&acc_full);
+                    }
+                    __syncwarp();
+                    if (++ab == NA) {
+                        ab = 0;
+                        aphase ^= 1;
+                    }
+                    if (flush) {
                         ++fg;
                         rs = 0;
                     }
@@ -675,8 +725,10 @@ __global__ void __launch_bounds__(k1Threads, 1)
                 }
             }
             // every MMA of this CTA has completed before TMEM is released
-            mma_commit(&mma_done);
+            if (elect_one()) mma_commit(&mma_done);
+            __syncwarp();
             trj_mbar_wait(&mma_done, 0);
+            __syncwarp();
         }
     } else if (warp >= k1EpiWarp0) {
         // ---- epilogue: each run of the accumulator is added (round to nearest) into an FP32 running
@@ -749,14 +801,12 @@ __global__ void __launch_bounds__(k1Threads, 1)
             }
         }
     } else {
-        // ---- A builders (warps 0-7): warp w writes TMEM lanes 32*(w%4).. (A rows m) and, in each
-        //      half-stage buffer, the K-columns of atoms [kHalfAtoms*(w/4), kHalfAtoms*(w/4 + 1)) ----
+        // ---- A builders (warps 0-7): warp w writes TMEM lanes 32*(w%4).. (A rows) and, in each half of
+        //      a buffer, the K-columns of atoms [kHalfAtoms*(w/4), kHalfAtoms*(w/4 + 1)) ----
         const int q = warp & 3, g = warp >> 2;
-        const int m = 32 * q + lane;
-        const int nxl = m & 15, nyl = m >> 4;
         const uint32_t lanes = (uint32_t)(32 * q) << 16;
         int ab = 0, slot = 0;
-        unsigned aphase = 0, phase = 0;  // A ring (NA half-stage buffers) in the MMA warp's order; X/Y ring
+        unsigned aphase = 0, phase = 0;  // A ring (NA buffers) in the MMA warp's order; X/Y ring
         bool stop = false;
         for (int li = item0; li < item1 && !stop; ++li) {
             const int it = p.cta_items[li];
@@ -773,54 +823,34 @@ __global__ void __launch_bounds__(k1Threads, 1)
                 }
                 const float4* xf = reinterpret_cast<const float4*>(xy_ptr(slot));
                 const float4* yf = xf + kXBlockBytes / 16;
-                // Half-stage 0 is built and stored, half-stage 1 built while those stores drain; then
-                // each half is released to the MMA warp once its own stores are complete.
-                const int hb0 = ab;
-                if (!__all_sync(0xffffffffu, trj_mbar_wait(&empty_a[hb0], aphase ^ 1))) {
+                if (!__all_sync(0xffffffffu, trj_mbar_wait(&empty_a[ab], aphase ^ 1))) {
                     if (lane == 0) trj_raise(p.status, TRJ_DEV_TIMEOUT);
                     abort_flag = 1;
                     stop = true;
                     break;
                 }
-                if (++ab == NA) {
-                    ab = 0;
-                    aphase ^= 1;
-                }
                 tc_fence_after();
+                // the second 8 atoms are built while the stores of the first drain
+                const uint32_t ta = tmem + lanes + p.a_col + (uint32_t)(2 * kStageSlots * ab + kHalfAtoms * g);
                 uint32_t hw[kHalfAtoms], lw[kHalfAtoms];
-                build_row_tab(xf, yf, nxl, nyl, (kHalfAtoms * g) / 2, hw, lw);
-                const uint32_t ta0 = tmem + lanes + p.a_col + (uint32_t)(32 * hb0 + kHalfAtoms * g);
-                tmem_st_cols<kHalfAtoms>(ta0, hw);
-                tmem_st_cols<kHalfAtoms>(ta0 + 16, lw);
-                const int hb1 = ab;
-                const bool ok1 = trj_mbar_wait(&empty_a[hb1], aphase ^ 1);
-                if (++ab == NA) {
-                    ab = 0;
-                    aphase ^= 1;
-                }
+                build_quarter(xf, yf, lane, 2 * q, g, hw, lw);
+                tmem_st_quarter(ta, hw);
+                tmem_st_quarter(ta + kStageSlots, lw);
                 uint32_t hw1[kHalfAtoms], lw1[kHalfAtoms];
-                build_row_tab(xf, yf, nxl, nyl, (16 + kHalfAtoms * g) / 2, hw1, lw1);
+                build_quarter(xf, yf, lane, 2 * q, kBuildGroups + g, hw1, lw1);
                 // every read of this stage's factor blocks is done: hand the buffer back
                 __syncwarp();
                 if (lane == 0) trj_mbar_arrive(&empty_xy[slot]);
-                tmem_wait_st();  // half-stage 0's stores
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) trj_mbar_arrive(&full_a[hb0]);
-                if (!__all_sync(0xffffffffu, ok1)) {
-                    if (lane == 0) trj_raise(p.status, TRJ_DEV_TIMEOUT);
-                    abort_flag = 1;
-                    stop = true;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t ta1 = tmem + lanes + p.a_col + (uint32_t)(32 * hb1 + kHalfAtoms * g);
-                tmem_st_cols<kHalfAtoms>(ta1, hw1);
-                tmem_st_cols<kHalfAtoms>(ta1 + 16, lw1);
+                tmem_st_quarter(ta + kStageSlots / 2, hw1);
+                tmem_st_quarter(ta + kStageSlots / 2 + kStageSlots, lw1);
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) trj_mbar_arrive(&full_a[hb1]);
+                if (lane == 0) trj_mbar_arrive(&full_a[ab]);
+                if (++ab == NA) {
+                    ab = 0;
+                    aphase ^= 1;
+                }
                 if (++slot == kXyStages) {
                     slot = 0;
                     phase ^= 1;
@@ -1453,7 +1483,7 @@ int trj_sq_tc_prepare(trj_sq_plan* plan) {
     st->table_rows = 2 * (nz_max - nz_min + 1);
     // A ring from the first multiple of 32 columns after the accumulator
     st->a_col = (st->bmax + 31) / 32 * 32;
-    st->nabuf = std::min(k1MaxABufs, (int)(kTmemCols - st->a_col) / 32);  // 9 for every bmax <= 224
+    st->nabuf = std::min(k1MaxABufs, (int)(kTmemCols - st->a_col) / (2 * kStageSlots));  // at least 4
     const int ntiles = (int)plan->tiles.size();
     std::vector<TcTile> tt(ntiles);
     int64_t acc = 0;
