@@ -16,7 +16,7 @@ parameters.  The loop:
   host, stamps the latency and frees the slot for the next request;
 * packs small requests (at most ``fuse_max_atoms`` atoms, reference bins within the batch's shared
   histogram) into one fused launch per turn instead of slots: one frame of each packed request goes
-  through a single table copy and five kernels (layout, all-pairs histogram, direct sum, shell
+  through a single table copy and eight kernels (layout, cell sort, pair histogram, direct sum, shell
   reduction) over all of them (``engine.Batch``), replayed from a CUDA graph captured once per staging
   buffer; their S(Q) is the direct sum, bit-identical to the per-request plain method;
 * ``cancel(rid)`` (from any thread) drops a request that is still waiting, or stops a running one
