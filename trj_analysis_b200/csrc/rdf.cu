@@ -557,6 +557,7 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const fl
                                 near = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
                             }
                             m = __ballot_sync(0xffffffffu, near);
+                            __syncwarp();  // the readers of the last 32 groups' starts (a ballot orders no memory)
                             if (near) {
                                 ws->gs[lane] = fstart[out.y + s];
                                 ws->gn[lane] = fcount[out.y + s];
