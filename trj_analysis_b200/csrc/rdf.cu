@@ -216,7 +216,8 @@ constexpr size_t kWarpBytes = 16 * kRing + (sizeof(WarpState) + 15) / 16 * 16;  
 // (sqrt.approx 2^-23, 1/deltar 2^-24, the reference's own root and quotient 2^-24 each), and less than
 // 0.47 q 2^-20 after a change of rr2 by one ulp (2^-24) or to its FMA-contracted value (1.25*2^-23); so a
 // pair whose q is farther than edge_thr allows from any bin edge has the reference's bin, and no edge
-// statistic.  rr2 < side2 is exact.  FLOOR: floor(q) + 1 = the integer nearest to q + 1/2.
+// statistic.  rr2 < side2 is exact.  FLOOR: floor(q) + 1 = the integer nearest to q + 1/2, whose sum is rounded
+// once more (2^-24: 0.38 and 0.53 in all).
 // Every pair in range is counted at once in its approximate bin; a block in which some test lies in the
 // window of an edge (or, with EDGE, within 2^-20 of the cutoff, where one-ulp changes decide) is looked at
 // again and the few wrong counts are moved.  QMODE instead leaves those out of the first count, since a
@@ -1338,10 +1339,12 @@ static void fill_geom(PairGeom& g, const float box[3], float side2, float deltar
     g.deltar = deltar;
     g.inv_deltar = 1.0f / deltar;
     // Window around a bin edge outside which the approximate q has the reference's bin (test_run): 0.34 (with
-    // edge statistics 0.5) x 2^-20 of the largest q of a pair in range, plus 2^-22.  Cutoffs whose squares leave the normal range (and bins
-    // beyond the integer trick) take the exact path throughout.
+    // edge statistics 0.5) x 2^-20 of the largest q of a pair in range, plus 2^-22; floor bins round q + 1/2 once
+    // more: 0.41 (0.57).  Cutoffs whose squares leave the normal range (and bins beyond the integer trick) take the
+    // exact path throughout.
     const double qmax = sqrt((double)g.side2_hi) / (double)deltar + 1.0;
-    const double thr = 0.5 - (qmax * (want_edge ? 0.5 : 0.34) / 1048576.0 + 1.0 / 4194304.0);
+    const double window = floor_bins ? (want_edge ? 0.57 : 0.41) : (want_edge ? 0.5 : 0.34);
+    const double thr = 0.5 - (qmax * window / 1048576.0 + 1.0 / 4194304.0);
     g.edge_thr = (side2 > 1e-30f && thr > 0.0) ? (float)thr : -1.0f;
     g.lsmax = lsmax;
     g.nsp = nsp;
