@@ -1298,6 +1298,9 @@ static float nint_threshold(float L, float q) {
     return x;
 }
 
+// Most work items a fused frame's neighbour lists are cut into (frames of more groups have one per group).
+constexpr int64_t kBatchItemsMost = (int64_t)1 << 20;
+
 static int nint_host(float x) {  // Fortran NINT: half away from zero
     double v = (double)x;
     return (int)(v >= 0 ? floor(v + 0.5) : -floor(-v + 0.5));
@@ -1461,7 +1464,7 @@ static void set_segments(RdfParams& P, int nseg, int nkey) {
     P.per_seg = (P.list + nseg - 1) / nseg;
     P.nseg = (P.list + P.per_seg - 1) / P.per_seg;
     P.div_nseg = make_fast_div(P.nseg);
-    P.nitems = (unsigned)nkey * (unsigned)P.nseg;  // below 2^31: nseg > 1 only for few keys
+    P.nitems = (unsigned)nkey * (unsigned)P.nseg;  // below 2^31: the callers bound nseg by the number of keys
 }
 
 struct PairShape {
@@ -1852,8 +1855,10 @@ int trj_batch_fill_rdf(trj_rdf_plan* plan, int64_t n, const float box[3], int hi
     cells_for(box, plan->side2, P.nc);
     fill_grid(P, n, box, plan->side2, plan->rcrdf_eff, 3, batch_keys_most(n));
     *nkey = (int64_t)P.nc[0] * P.nc[1] * P.nc[2] * P.nsub;
-    // about ten neighbour groups per item; one-atom frames have no pairs
-    if (n >= 2) set_segments(P, std::max(1, P.list / 10), (int)*nkey);
+    // About ten neighbour groups per item, but no more items than keep every warp of the GPU busy some 300 times
+    // over: the list grows with the frame, and items are numbered in 31 bits.  One-atom frames have no pairs.
+    const int64_t most = std::max<int64_t>(1, kBatchItemsMost / std::max<int64_t>(1, *nkey));
+    if (n >= 2) set_segments(P, (int)std::max<int64_t>(1, std::min<int64_t>(P.list / 10, most)), (int)*nkey);
     // a row per ordered species pair where those fit (floor bins: the general layout only)
     it->square = !plan->floor_bins &&
                  (int64_t)plan->nsp * plan->nsp * P.g.row_words <= (int64_t)batch_hist_smem_words(hist_words);
