@@ -1777,11 +1777,11 @@ extern "C" int trj_rdf_s2n(trj_rdf_plan* plan, int nrandom, uint64_t* gi_dev, ui
         return trj_fail(ctx, TRJ_ERR_INVALID, "rdf s2n: no frame accumulated (call trj_rdf_accumulate first)");
     if (nrandom == 0) return TRJ_OK;
     trj_device_guard g(ctx->device);
-    const size_t smem = sizeof(unsigned) * (size_t)(plan->lsmax + 1);
-    if (2 * smem > (size_t)ctx->smem_optin - 64)
-        return trj_fail(ctx, TRJ_ERR_UNSUPPORTED, "rdf s2n: lsmax=%d too large", plan->lsmax);
-    if (smem > 48 * 1024)
-        TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(s2n_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = sizeof(unsigned) * (size_t)(plan->lsmax + 1), most = ((size_t)ctx->smem_optin - 64) / 2;
+    if (smem > most) return trj_fail(ctx, TRJ_ERR_UNSUPPORTED, "rdf s2n: lsmax=%d too large", plan->lsmax);
+    // Always, and always the same: without it the kernel's static shared memory counts against 48 KB as well, and a
+    // value of this call's own could be lowered by another thread's before the launch.
+    TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(s2n_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     PairGeom geom;
     fill_geom(geom, plan->box_last, plan->side2, plan->deltar, plan->lsmax, plan->nsp, 0, false);
     s2n_kernel<<<(unsigned)nrandom, kS2nThreads, smem, (cudaStream_t)stream>>>(
