@@ -62,9 +62,9 @@ extern "C" int trj_batch_create(trj_ctx* ctx, int max_items, int64_t max_atoms, 
     if (!ctx || !out) return TRJ_ERR_INVALID;
     *out = nullptr;
     if (max_items < 1 || max_items > 4096 || max_atoms < 1 || max_atoms > ((int64_t)1 << 31) || hist_words < 1 ||
-        hist_words > 24576)
+        hist_words > kBatchMaxHistWords)
         return trj_fail(ctx, TRJ_ERR_INVALID, "batch: max_items=%d (1..4096), max_atoms=%lld (1..2^31), "
-                        "hist_words=%d (1..24576)", max_items, (long long)max_atoms, hist_words);
+                        "hist_words=%d (1..%d)", max_items, (long long)max_atoms, hist_words, kBatchMaxHistWords);
     trj_device_guard g(ctx->device);
     trj_batch* b = new trj_batch();
     b->ctx = ctx;
@@ -119,7 +119,7 @@ extern "C" int trj_batch_create(trj_ctx* ctx, int max_items, int64_t max_atoms, 
         b->device_bytes += (int64_t)dev;
         memset(B.table_host, 0, b->table_bytes);
     }
-    if (trj_batch_pairs_prepare(hist_words) != 0) {
+    if (trj_batch_pairs_prepare() != 0) {
         batch_free(b);
         delete b;
         return trj_fail(ctx, TRJ_ERR_UNSUPPORTED, "batch: %zu bytes of shared memory for the pair kernel",

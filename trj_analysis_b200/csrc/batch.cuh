@@ -14,6 +14,7 @@
 constexpr int kBatchChunk = 1024;        // atoms per layout unit
 constexpr int kBatchThreads = 256;
 constexpr int kBatchMaxSpecies = 16;
+constexpr int kBatchMaxHistWords = 24576;  // largest pair histogram of a batch
 constexpr int kBatchCounters = 4;        // dynamic work counters: pairs, direct sum, reduction, spare
 
 struct __align__(16) BatchItem {
@@ -89,7 +90,7 @@ void trj_batch_launch_layout(const BatchHeader* hdr, const BatchItem* items, con
 int trj_batch_launch_pairs(BatchHeader* hdr, const BatchItem* items, const float4* packed, const BatchSort& st,
                            size_t zero_bytes, int hist_words, int grid_layout, int grid, cudaStream_t s);  // rdf.cu
 size_t trj_batch_pairs_smem(int hist_words);                                                  // rdf.cu
-int trj_batch_pairs_prepare(int hist_words);                                                  // rdf.cu
+int trj_batch_pairs_prepare();                                                                // rdf.cu
 int trj_batch_pairs_occupancy(int hist_words, int* per_sm);                                   // rdf.cu
 void trj_batch_launch_sq(BatchHeader* hdr, const BatchItem* items, const uint4* phase, const float2* turn, int grid_sq,
                          int grid_red, cudaStream_t s);                                       // sq.cu

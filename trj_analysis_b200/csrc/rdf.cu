@@ -1814,9 +1814,10 @@ size_t trj_batch_pairs_smem(int hist_words) {
     return (size_t)(kBatchThreads / 32) * kWarpBytes + 4 * (size_t)batch_hist_smem_words(hist_words);
 }
 
-int trj_batch_pairs_prepare(int hist_words) {
+int trj_batch_pairs_prepare() {
+    // for the largest batch: a limit of this batch's own would refuse the launches of a larger one made before
     return cudaFuncSetAttribute(batch_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)trj_batch_pairs_smem(hist_words)) == cudaSuccess ? 0 : -1;
+                                (int)trj_batch_pairs_smem(kBatchMaxHistWords)) == cudaSuccess ? 0 : -1;
 }
 
 int trj_batch_launch_pairs(BatchHeader* hdr, const BatchItem* items, const float4* packed, const BatchSort& st,
