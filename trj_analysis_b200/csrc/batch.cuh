@@ -68,13 +68,17 @@ __device__ __forceinline__ int batch_item_of(const BatchItem* __restrict__ items
 }
 
 // Device arrays of the turn's cell sort.  Zeroed together at the start of a turn's pair work: state (per item:
-// pair work counter, atoms placed, frame flags, spare), fcount and cflag.
+// pair work counter, frame flags, atoms placed, rounds of homes), fcount and cflag.
 struct BatchSort {
     unsigned* state;
     int32_t *fcount, *cflag, *fstart;    // per group (cflag: per cell), an item's at its key_begin
+    int2* rounds;                        // per round of homes, an item's at batch_rounds_begin
     int32_t *akey, *aslot;               // per atom
     float4* sorted;                      // per atom: an item's atoms by group
 };
+
+// First round of homes of an item: its groups' ceil(atoms / 32) add up to at most its groups + n / 32.
+__host__ __device__ inline int64_t batch_rounds_begin(const BatchItem& it) { return it.key_begin + it.atom_off / 32; }
 
 // Most groups of an item of n atoms (choose_groups keeps to it), and the shared-memory words of the pair kernel's
 // bin rows: triangular rows always fit (hist_words plus two words for each of up to 136 rows), square rows are

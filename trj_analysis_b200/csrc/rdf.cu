@@ -39,6 +39,10 @@ constexpr int kMaxWarps = 32;         // per SM: 64 registers a thread (24 warps
 
 typedef unsigned long long u64;
 
+// A frame's words of work state (in a fused turn: an item's): work counter, frame flags, then one 64-bit sum of the
+// atoms placed (low half) and the rounds of homes (high half).
+enum { kWorkNext = 0, kWorkFlags = 1, kWorkAtoms = 2, kWorkRounds = 3, kWorkWords = 4 };
+
 // Frame flags raised by cell_assign_kernel: how far coordinates reach outside [0, L).  They decide
 // whether |d| < 3L/2 holds for every pair of the frame (see frame_within).
 enum : unsigned { kFrameLow = 1u, kFrameVeryLow = 2u, kFrameHigh = 4u };
@@ -393,10 +397,12 @@ __device__ __forceinline__ bool frame_within(unsigned f) {
     return !(f & kFrameLow) || !(f & (kFrameVeryLow | kFrameHigh));
 }
 
-// One work item of a frame: home group key = item / nseg against segment item % nseg of its neighbour list.
-// hist: shared-memory address of the bin rows (SQUARE), rowtab: of the row table (otherwise).
+// One work item of a frame: round item / nseg (up to 32 atoms of one group, see emit_rounds) against segment
+// item % nseg of its group's neighbour list.  hist: shared-memory address of the bin rows (SQUARE), rowtab: of the
+// row table (otherwise).
 template <bool FLOOR, bool QMODE, bool SQUARE, bool EDGE, int UNROLL>
-__device__ __forceinline__ void pair_item(const RdfParams& p, int item, const float4* __restrict__ sorted,
+__device__ __forceinline__ void pair_item(const RdfParams& p, int item, const int2* __restrict__ rounds,
+                                          const float4* __restrict__ sorted,
                                           const int32_t* __restrict__ fstart, const int32_t* __restrict__ fcount,
                                           const int32_t* __restrict__ cflag, bool frame_ok,
                                           const float* __restrict__ sorted_q, float* ring, double* ring_q,
@@ -405,9 +411,9 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const fl
     const PairGeom& g = p.g;
     const int lane = (int)(threadIdx.x & 31u);
     const unsigned lt = (1u << lane) - 1u;
-    const int key = fast_div((int)item, p.div_nseg), seg = (int)item - key * p.nseg;
+    const int round = fast_div(item, p.div_nseg), seg = item - round * p.nseg;
+    const int key = rounds[round].x, h0 = rounds[round].y;
     const int hbeg = fstart[key], hend = hbeg + fcount[key];
-    if (hbeg >= hend) return;
     const int c = fast_div(key, p.div_nsub), own = key - c * p.nsub;
     const int cxy = fast_div(c, p.div_nc2), cz = c - cxy * p.nc[2];
     const int cx = fast_div(cxy, p.div_nc1), cy = cxy - cx * p.nc[1];
@@ -438,183 +444,181 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const fl
             ws->half = w;
         }
     }
-    for (int h0 = hbeg; h0 < hend; h0 += kGroup) {
+    {
+        const int nh = min(kGroup, hend - h0);
+        const bool has = lane < nh;
+        float4 a = has ? sorted[h0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const unsigned wa = __float_as_uint(a.w);  // species * row bytes (64 with the row table)
+        a.x = -a.x;
+        a.y = -a.y;
+        a.z = -a.z;
+        a.w = __uint_as_float(SQUARE ? hist_base + wa * (unsigned)g.nsp - 4u * kBinBias : rowtab + (wa >> 4));
+        ws->home[lane] = a;
+        if (QMODE) ws->home_q[lane] = has ? sorted_q[h0 + lane] : 0.f;
+        if (lane == 0) ws->nh = nh;
+    }
+    for (int t = t0; t < t1;) {
+        // entries [e_lo, e_hi) of offset o: group e, or (own cell) the e-th after the homes' own
+        const int o = t < p.nself ? 0 : 1 + fast_div(t - p.nself, p.div_nsub);
+        const int first = o == 0 ? 0 : p.nself + (o - 1) * p.nsub;
+        const int e_lo = t - first, e_hi = min(o == 0 ? p.nself : p.nsub, t1 - first);
+        const int ex = cx + p.off[o][0], ey = cy + p.off[o][1], ez = cz + p.off[o][2];
+        const int c2 = (wrapc(ex, p.nc[0]) * p.nc[1] + wrapc(ey, p.nc[1])) * p.nc[2] + wrapc(ez, p.nc[2]);
+        const int f2 = fl | cflag[c2];
+        const bool far = f2 & 2;
+        const bool plain = p.split_all && !(f2 & 1);  // image known from the cells
+        int mode;
         {
-            const int nh = min(kGroup, hend - h0);
-            const bool has = lane < nh;
-            float4 a = has ? sorted[h0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-            const unsigned wa = __float_as_uint(a.w);  // species * row bytes (64 with the row table)
-            a.x = -a.x;
-            a.y = -a.y;
-            a.z = -a.z;
-            a.w = __uint_as_float(SQUARE ? hist_base + wa * (unsigned)g.nsp - 4u * kBinBias : rowtab + (wa >> 4));
-            ws->home[lane] = a;
-            if (QMODE) ws->home_q[lane] = has ? sorted_q[h0 + lane] : 0.f;
-            if (lane == 0) ws->nh = nh;
-        }
-        for (int t = t0; t < t1;) {
-            // entries [e_lo, e_hi) of offset o: group e, or (own cell) the e-th after the homes' own
-            const int o = t < p.nself ? 0 : 1 + fast_div(t - p.nself, p.div_nsub);
-            const int first = o == 0 ? 0 : p.nself + (o - 1) * p.nsub;
-            const int e_lo = t - first, e_hi = min(o == 0 ? p.nself : p.nsub, t1 - first);
-            const int ex = cx + p.off[o][0], ey = cy + p.off[o][1], ez = cz + p.off[o][2];
-            const int c2 = (wrapc(ex, p.nc[0]) * p.nc[1] + wrapc(ey, p.nc[1])) * p.nc[2] + wrapc(ez, p.nc[2]);
-            const int f2 = fl | cflag[c2];
-            const bool far = f2 & 2;
-            const bool plain = p.split_all && !(f2 & 1);  // image known from the cells
-            int mode;
-            {
-                const float4 img = make_float4(ex < 0 ? -g.L[0] : (ex >= p.nc[0] ? g.L[0] : 0.f),
-                                               ey < 0 ? -g.L[1] : (ey >= p.nc[1] ? g.L[1] : 0.f),
-                                               ez < 0 ? -g.L[2] : (ez >= p.nc[2] ? g.L[2] : 0.f), 0.f);
-                mode = plain ? ((img.x != 0.f || img.y != 0.f || img.z != 0.f) ? kImgShift : kImgNone)
-                             : far ? kImgAny : p.split_all ? kImgRound : frame_ok ? kImgFold : kImgAny;
-                __syncwarp();  // the group's box, homes and the last offset's readers
-                if (lane == 0) {
-                    const float4 c = ws->box;
-                    ws->img = img;
-                    ws->cut = plain ? make_float4(c.x - img.x, c.y - img.y, c.z - img.z, 0.f) : c;
-                    ws->outer = make_int4(first + e_hi, c2 * p.nsub, own, h0);
-                }
-                __syncwarp();
+            const float4 img = make_float4(ex < 0 ? -g.L[0] : (ex >= p.nc[0] ? g.L[0] : 0.f),
+                                           ey < 0 ? -g.L[1] : (ey >= p.nc[1] ? g.L[1] : 0.f),
+                                           ez < 0 ? -g.L[2] : (ez >= p.nc[2] ? g.L[2] : 0.f), 0.f);
+            mode = plain ? ((img.x != 0.f || img.y != 0.f || img.z != 0.f) ? kImgShift : kImgNone)
+                         : far ? kImgAny : p.split_all ? kImgRound : frame_ok ? kImgFold : kImgAny;
+            __syncwarp();  // the group's box, homes and the last offset's readers
+            if (lane == 0) {
+                const float4 c = ws->box;
+                ws->img = img;
+                ws->cut = plain ? make_float4(c.x - img.x, c.y - img.y, c.z - img.z, 0.f) : c;
+                ws->outer = make_int4(first + e_hi, c2 * p.nsub, own, h0);
             }
-            int head = 0, tail = 0;
-            auto append = [&](float x, float y, float z, float w, float qb, bool keep) {
-                const unsigned m = __ballot_sync(0xffffffffu, keep);
-                if (keep) {
-                    const int e = (tail + __popc(m & lt)) & (kRing - 1);
-                    ring[e] = x;
-                    ring[kRing + e] = y;
-                    ring[2 * kRing + e] = z;
-                    ring[3 * kRing + e] = w;
-                    if (QMODE) ring_q[e] = (double)qb;
-                }
-                tail += __popc(m);
-            };
-            // Fills the buffer up to a multiple of four with NaN entries (in no range, near no edge).
-            auto pad = [&]() {
-                const int n = tail - head, up = (n + 3) & ~3;
-                if (lane < up - n) {
-                    const int e = (tail + lane) & (kRing - 1);
-                    ring[e] = ring[kRing + e] = ring[2 * kRing + e] = NAN;
-                    ring[3 * kRing + e] = 0.f;
-                    if (QMODE) ring_q[e] = 0.0;
-                }
-                return up >> 2;
-            };
-#define TRJ_RUN(M, S, N4) test_run<M, S, FLOOR, QMODE, SQUARE, EDGE, UNROLL>(ring, ring_q, head, N4, ws, g, pc, qhist)
-            if (o == 0 && e_lo == 0) {
-                // pairs j > i of the round's own atoms, through the buffer in lane order
-                const int nh = ws->nh;
-                const float4 a = lane < nh ? sorted[h0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-                append(a.x, a.y, a.z, a.w, QMODE ? ws->home_q[lane] : 0.f, lane < nh);
-                const int n4 = pad();
-                __syncwarp();
-                if (plain) TRJ_RUN(kImgNone, true, n4);
-                else if (mode == kImgRound) TRJ_RUN(kImgRound, true, n4);
-                else if (mode == kImgFold) TRJ_RUN(kImgFold, true, n4);
-                else TRJ_RUN(kImgAny, true, n4);
-                __syncwarp();
-                if (EDGE && lane < nh) n_tested += (unsigned)(nh - 1 - lane);
-                tail = 0;
-            }
-            int e0 = e_lo - 32, j = 0, je = 0;
-            unsigned m = 0;
-            bool more = true;
-            do {
-                // survivors into the buffer until a run is full or the segment's groups are used up
-                while (tail - head < kRingRun) {
-                    if (j >= je) {
-                        if (!m) {
-                            e0 += 32;
-                            if (e0 >= e_hi) {
-                                more = false;
-                                break;
-                            }
-                            // lanes over the neighbour groups: which can hold an atom in range of the homes' box
-                            const int4 out = ws->outer;
-                            const int e = e0 + lane;
-                            int s = o == 0 ? out.z + e : e;
-                            if (s >= p.nsub) s -= p.nsub;
-                            // half-way round an even number of groups each pair is met twice: the lower has it
-                            bool near = e < e_hi && (o > 0 || 2 * e != p.nsub || 2 * out.z < p.nsub);
-                            if (near && !far) {
-                                const float4 b = ws->box, w = ws->half, img = ws->img;
-                                const int q = (int)(((float)s + 0.5f) * p.inv_sub[2]), sz = s - q * p.sub[2];
-                                const int sx = (int)(((float)q + 0.5f) * p.inv_sub[1]), sy = q - sx * p.sub[1];
-                                const float gx = ((float)ex + ((float)sx + 0.5f) * p.inv_sub[0]) * p.edge[0];
-                                const float gy = ((float)ey + ((float)sy + 0.5f) * p.inv_sub[1]) * p.edge[1];
-                                const float gz = ((float)ez + ((float)sz + 0.5f) * p.inv_sub[2]) * p.edge[2];
-                                float dx, dy, dz;
-                                if (p.split_all) {
-                                    dx = axis_gap<false>(gx, b.x, w.x + p.half[0], 0.f);
-                                    dy = axis_gap<false>(gy, b.y, w.y + p.half[1], 0.f);
-                                    dz = axis_gap<false>(gz, b.z, w.z + p.half[2], 0.f);
-                                } else {
-                                    dx = axis_gap<true>(gx - img.x, b.x, w.x + p.half[0], g.L[0]);
-                                    dy = axis_gap<true>(gy - img.y, b.y, w.y + p.half[1], g.L[1]);
-                                    dz = axis_gap<true>(gz - img.z, b.z, w.z + p.half[2], g.L[2]);
-                                }
-                                near = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
-                            }
-                            m = __ballot_sync(0xffffffffu, near);
-                            __syncwarp();  // the readers of the last 32 groups' starts (a ballot orders no memory)
-                            if (near) {
-                                ws->gs[lane] = fstart[out.y + s];
-                                ws->gn[lane] = fcount[out.y + s];
-                            }
-                            __syncwarp();
-                            continue;
-                        }
-                        const int k = __ffs(m) - 1;
-                        m &= m - 1u;
-                        j = ws->gs[k];
-                        je = j + ws->gn[k];
-                        if (o == 0 && e0 + k == 0) j = ws->outer.w + ws->nh;  // the round's own atoms are done
-                        continue;
-                    }
-                    bool keep = j + lane < je;
-                    const float4 b = keep ? sorted[j + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    const float qb = (QMODE && keep) ? sorted_q[j + lane] : 0.f;
-                    j += 32;
-                    if (keep && !far) {
-                        const float4 c = ws->cut, w = ws->half;
-                        float dx, dy, dz;
-                        if (plain) {
-                            dx = axis_gap<false>(b.x, c.x, w.x, 0.f);
-                            dy = axis_gap<false>(b.y, c.y, w.y, 0.f);
-                            dz = axis_gap<false>(b.z, c.z, w.z, 0.f);
-                        } else {
-                            dx = axis_gap<true>(wrap_cull(b.x, g.L[0]), c.x, w.x, g.L[0]);
-                            dy = axis_gap<true>(wrap_cull(b.y, g.L[1]), c.y, w.y, g.L[1]);
-                            dz = axis_gap<true>(wrap_cull(b.z, g.L[2]), c.z, w.z, g.L[2]);
-                        }
-                        keep = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
-                    }
-                    const int before = tail;
-                    append(b.x, b.y, b.z, b.w, qb, keep);
-                    if (EDGE && lane < ws->nh) n_tested += (unsigned)(tail - before);
-                }
-                const int n4 = tail - head >= kRingRun ? kRingRun / 4 : pad();
-                if (lane == 0) ws->walk = make_int4(j, je, (int)m, e0);
-                __syncwarp();  // the other lanes' entries
-                if (mode == kImgNone) TRJ_RUN(kImgNone, false, n4);
-                else if (mode == kImgShift) TRJ_RUN(kImgShift, false, n4);
-                else if (mode == kImgRound) TRJ_RUN(kImgRound, false, n4);
-                else if (mode == kImgFold) TRJ_RUN(kImgFold, false, n4);
-                else TRJ_RUN(kImgAny, false, n4);
-                const int4 walk = ws->walk;
-                __syncwarp();  // before the buffer and the state are written again
-                j = walk.x;
-                je = walk.y;
-                m = (unsigned)walk.z;
-                e0 = walk.w;
-                head += 4 * n4;
-            } while (more);
-#undef TRJ_RUN
-            t = ws->outer.x;
             __syncwarp();
         }
+        int head = 0, tail = 0;
+        auto append = [&](float x, float y, float z, float w, float qb, bool keep) {
+            const unsigned m = __ballot_sync(0xffffffffu, keep);
+            if (keep) {
+                const int e = (tail + __popc(m & lt)) & (kRing - 1);
+                ring[e] = x;
+                ring[kRing + e] = y;
+                ring[2 * kRing + e] = z;
+                ring[3 * kRing + e] = w;
+                if (QMODE) ring_q[e] = (double)qb;
+            }
+            tail += __popc(m);
+        };
+        // Fills the buffer up to a multiple of four with NaN entries (in no range, near no edge).
+        auto pad = [&]() {
+            const int n = tail - head, up = (n + 3) & ~3;
+            if (lane < up - n) {
+                const int e = (tail + lane) & (kRing - 1);
+                ring[e] = ring[kRing + e] = ring[2 * kRing + e] = NAN;
+                ring[3 * kRing + e] = 0.f;
+                if (QMODE) ring_q[e] = 0.0;
+            }
+            return up >> 2;
+        };
+#define TRJ_RUN(M, S, N4) test_run<M, S, FLOOR, QMODE, SQUARE, EDGE, UNROLL>(ring, ring_q, head, N4, ws, g, pc, qhist)
+        if (o == 0 && e_lo == 0) {
+            // pairs j > i of the round's own atoms, through the buffer in lane order
+            const int nh = ws->nh;
+            const float4 a = lane < nh ? sorted[h0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+            append(a.x, a.y, a.z, a.w, QMODE ? ws->home_q[lane] : 0.f, lane < nh);
+            const int n4 = pad();
+            __syncwarp();
+            if (plain) TRJ_RUN(kImgNone, true, n4);
+            else if (mode == kImgRound) TRJ_RUN(kImgRound, true, n4);
+            else if (mode == kImgFold) TRJ_RUN(kImgFold, true, n4);
+            else TRJ_RUN(kImgAny, true, n4);
+            __syncwarp();
+            if (EDGE && lane < nh) n_tested += (unsigned)(nh - 1 - lane);
+            tail = 0;
+        }
+        int e0 = e_lo - 32, j = 0, je = 0;
+        unsigned m = 0;
+        bool more = true;
+        do {
+            // survivors into the buffer until a run is full or the segment's groups are used up
+            while (tail - head < kRingRun) {
+                if (j >= je) {
+                    if (!m) {
+                        e0 += 32;
+                        if (e0 >= e_hi) {
+                            more = false;
+                            break;
+                        }
+                        // lanes over the neighbour groups: which can hold an atom in range of the homes' box
+                        const int4 out = ws->outer;
+                        const int e = e0 + lane;
+                        int s = o == 0 ? out.z + e : e;
+                        if (s >= p.nsub) s -= p.nsub;
+                        // half-way round an even number of groups each pair is met twice: the lower has it
+                        bool near = e < e_hi && (o > 0 || 2 * e != p.nsub || 2 * out.z < p.nsub);
+                        if (near && !far) {
+                            const float4 b = ws->box, w = ws->half, img = ws->img;
+                            const int q = (int)(((float)s + 0.5f) * p.inv_sub[2]), sz = s - q * p.sub[2];
+                            const int sx = (int)(((float)q + 0.5f) * p.inv_sub[1]), sy = q - sx * p.sub[1];
+                            const float gx = ((float)ex + ((float)sx + 0.5f) * p.inv_sub[0]) * p.edge[0];
+                            const float gy = ((float)ey + ((float)sy + 0.5f) * p.inv_sub[1]) * p.edge[1];
+                            const float gz = ((float)ez + ((float)sz + 0.5f) * p.inv_sub[2]) * p.edge[2];
+                            float dx, dy, dz;
+                            if (p.split_all) {
+                                dx = axis_gap<false>(gx, b.x, w.x + p.half[0], 0.f);
+                                dy = axis_gap<false>(gy, b.y, w.y + p.half[1], 0.f);
+                                dz = axis_gap<false>(gz, b.z, w.z + p.half[2], 0.f);
+                            } else {
+                                dx = axis_gap<true>(gx - img.x, b.x, w.x + p.half[0], g.L[0]);
+                                dy = axis_gap<true>(gy - img.y, b.y, w.y + p.half[1], g.L[1]);
+                                dz = axis_gap<true>(gz - img.z, b.z, w.z + p.half[2], g.L[2]);
+                            }
+                            near = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
+                        }
+                        m = __ballot_sync(0xffffffffu, near);
+                        __syncwarp();  // the readers of the last 32 groups' starts (a ballot orders no memory)
+                        if (near) {
+                            ws->gs[lane] = fstart[out.y + s];
+                            ws->gn[lane] = fcount[out.y + s];
+                        }
+                        __syncwarp();
+                        continue;
+                    }
+                    const int k = __ffs(m) - 1;
+                    m &= m - 1u;
+                    j = ws->gs[k];
+                    je = j + ws->gn[k];
+                    if (o == 0 && e0 + k == 0) j = ws->outer.w + ws->nh;  // the round's own atoms are done
+                    continue;
+                }
+                bool keep = j + lane < je;
+                const float4 b = keep ? sorted[j + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float qb = (QMODE && keep) ? sorted_q[j + lane] : 0.f;
+                j += 32;
+                if (keep && !far) {
+                    const float4 c = ws->cut, w = ws->half;
+                    float dx, dy, dz;
+                    if (plain) {
+                        dx = axis_gap<false>(b.x, c.x, w.x, 0.f);
+                        dy = axis_gap<false>(b.y, c.y, w.y, 0.f);
+                        dz = axis_gap<false>(b.z, c.z, w.z, 0.f);
+                    } else {
+                        dx = axis_gap<true>(wrap_cull(b.x, g.L[0]), c.x, w.x, g.L[0]);
+                        dy = axis_gap<true>(wrap_cull(b.y, g.L[1]), c.y, w.y, g.L[1]);
+                        dz = axis_gap<true>(wrap_cull(b.z, g.L[2]), c.z, w.z, g.L[2]);
+                    }
+                    keep = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
+                }
+                const int before = tail;
+                append(b.x, b.y, b.z, b.w, qb, keep);
+                if (EDGE && lane < ws->nh) n_tested += (unsigned)(tail - before);
+            }
+            const int n4 = tail - head >= kRingRun ? kRingRun / 4 : pad();
+            if (lane == 0) ws->walk = make_int4(j, je, (int)m, e0);
+            __syncwarp();  // the other lanes' entries
+            if (mode == kImgNone) TRJ_RUN(kImgNone, false, n4);
+            else if (mode == kImgShift) TRJ_RUN(kImgShift, false, n4);
+            else if (mode == kImgRound) TRJ_RUN(kImgRound, false, n4);
+            else if (mode == kImgFold) TRJ_RUN(kImgFold, false, n4);
+            else TRJ_RUN(kImgAny, false, n4);
+            const int4 walk = ws->walk;
+            __syncwarp();  // before the buffer and the state are written again
+            j = walk.x;
+            je = walk.y;
+            m = (unsigned)walk.z;
+            e0 = walk.w;
+            head += 4 * n4;
+        } while (more);
+#undef TRJ_RUN
+        t = ws->outer.x;
+        __syncwarp();
     }
 }
 
@@ -658,8 +662,8 @@ __device__ __forceinline__ void add_edges(u64* __restrict__ edge_g, const PairCo
     }
 }
 
-// Work item = (home group, segment of its neighbour list), taken from a global counter by one warp at a
-// time; no warp waits for another.  Shared memory: bin rows (count), charge rows (QMODE, FP64 [row_words]),
+// Work item = (round of homes, segment of their group's neighbour list), taken from a global counter by one warp at
+// a time; no warp waits for another.  Shared memory: bin rows (count), charge rows (QMODE, FP64 [row_words]),
 // the warps' buffers.  SQUARE: a bin row per ordered species pair, so that a pair's row address is a sum of
 // two registers; otherwise the rows of ind_ij through a 16 x 16 table of addresses.
 //
@@ -676,7 +680,7 @@ template <bool FLOOR, bool QMODE, bool SQUARE, bool EDGE>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     rdf_pairs_kernel(const __grid_constant__ RdfParams p, const float4* __restrict__ sorted,
                      const int32_t* __restrict__ fstart, const int32_t* __restrict__ fcount,
-                     const int32_t* __restrict__ cflag, const unsigned* __restrict__ fflag, unsigned* __restrict__ work,
+                     const int32_t* __restrict__ cflag, const int2* __restrict__ rounds, unsigned* __restrict__ work,
                      u64* __restrict__ hist_g, u64* __restrict__ edge_g, unsigned* __restrict__ status,
                      const float* __restrict__ sorted_q, double* __restrict__ gqq_frame) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -714,16 +718,17 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     __syncthreads();
     if (stalled) return;
 
-    const bool frame_ok = frame_within(*fflag);
+    const bool frame_ok = frame_within(work[kWorkFlags]);
+    const unsigned nitems = work[kWorkRounds] * (unsigned)p.nseg;
     PairCounters pc;
     u64 n_tested = 0;
     for (;;) {
         unsigned item = 0;
         if (lane == 0) item = atomicAdd(work, 1u);
         item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= p.nitems) break;
-        pair_item<FLOOR, QMODE, SQUARE, EDGE, QMODE ? 1 : 2>(p, (int)item, sorted, fstart, fcount, cflag, frame_ok,
-                                                             sorted_q, ring, ring_q, ws, hist_base,
+        if (item >= nitems) break;
+        pair_item<FLOOR, QMODE, SQUARE, EDGE, QMODE ? 1 : 2>(p, (int)item, rounds, sorted, fstart, fcount, cflag,
+                                                             frame_ok, sorted_q, ring, ring_q, ws, hist_base,
                                                              trj_smem_addr(rowtab), qhist, pc, n_tested);
     }
     __syncthreads();
@@ -799,33 +804,54 @@ __global__ void cell_assign_kernel(const float4* __restrict__ packed, int64_t n,
     if ((threadIdx.x & 31) == 0 && (ff & ~*(volatile unsigned*)fflag)) atomicOr(fflag, ff);
 }
 
-// Start of every group in the sorted array.  Groups need only be contiguous, not in key order, so a block
-// takes the room of its 256 groups from a counter instead of waiting for the sums before it: one short
-// kernel in place of a scan over all keys.
-__global__ void __launch_bounds__(256) group_offsets_kernel(const int32_t* __restrict__ fcount, int nkey,
-                                                            int32_t* __restrict__ total, int32_t* __restrict__ fstart) {
-    __shared__ int wsum[8], base;
-    const int k = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int v = k < nkey ? fcount[k] : 0;
-    int x = v;
+// Atoms (low half) and rounds of homes (high half) of a group of v atoms: sums of both in one scan.
+__device__ __forceinline__ u64 group_sums(int v) { return (u64)((v + kGroup - 1) / kGroup) << 32 | (unsigned)v; }
+
+__device__ __forceinline__ u64 warp_scan(u64 x, int lane) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        const u64 y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
+    return x;
+}
+
+// A group's rounds of homes: (key, first atom) of every 32 atoms.  The pair kernel's work goes by rounds, not by
+// groups, because the groups of a frame of uneven density hold anything from no atom to all of them.  A ball of
+// 62,500 atoms in a box 7.5 times as wide has groups of up to 3,900; with a warp for all homes of a group, and items
+// for the empty ones too, 312 ms, with rounds 1.62; 20,000 atoms in one clump 343 and 1.33 ms.  Even frames gain as
+// well, from items of one round instead of one or two: 62,500 atoms 0.36 -> 0.33 ms, 1e6 2.59 -> 2.43.
+__device__ __forceinline__ void emit_rounds(int2* __restrict__ rounds, unsigned first, int key, int start, int v) {
+    for (int i = 0; i * kGroup < v; ++i) rounds[first + i] = make_int2(key, start + i * kGroup);
+}
+
+// Start of every group in the sorted array, and its rounds.  Groups need only be contiguous, not in key order, so a
+// block takes the room of its 256 groups from a counter instead of waiting for the sums before it: one short
+// kernel in place of a scan over all keys.
+__global__ void __launch_bounds__(256) group_offsets_kernel(const int32_t* __restrict__ fcount, int nkey,
+                                                            u64* __restrict__ total, int32_t* __restrict__ fstart,
+                                                            int2* __restrict__ rounds) {
+    __shared__ u64 wsum[8], base;
+    const int k = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int v = k < nkey ? fcount[k] : 0;
+    const u64 x = warp_scan(group_sums(v), lane);
     if (lane == 31) wsum[warp] = x;
     __syncthreads();
     if (threadIdx.x == 0) {
-        int sum = 0;
+        u64 sum = 0;
         for (int w = 0; w < 8; ++w) {
-            const int y = wsum[w];
+            const u64 y = wsum[w];
             wsum[w] = sum;
             sum += y;
         }
         base = atomicAdd(total, sum);
     }
     __syncthreads();
-    if (k < nkey) fstart[k] = base + wsum[warp] + x - v;
+    if (k < nkey) {
+        const u64 at = base + wsum[warp] + x - group_sums(v);
+        fstart[k] = (int)(unsigned)at;
+        emit_rounds(rounds, (unsigned)(at >> 32), k, (int)(unsigned)at, v);
+    }
 }
 
 // Sum over a block of v (FP64, fixed order): warp shuffles, then warps in order; thread 0 has it.
@@ -868,11 +894,12 @@ constexpr int kSmallAtoms = kSmallThreads * kSmallRounds;
 constexpr int kSmallKeys = 4096;  // most groups, and most cells, of a frame sorted this way
 __global__ void __launch_bounds__(kSmallThreads) cell_sort_small_kernel(
     const float4* __restrict__ packed, int n, const __grid_constant__ RdfParams p, int ncell, int nkey, unsigned wscale,
-    unsigned* __restrict__ work, unsigned* __restrict__ fflag, int32_t* __restrict__ cflag, int32_t* __restrict__ fcount,
-    int32_t* __restrict__ fstart, float4* __restrict__ sorted, const float* __restrict__ q,
+    unsigned* __restrict__ work, int32_t* __restrict__ cflag, int32_t* __restrict__ fcount,
+    int32_t* __restrict__ fstart, int2* __restrict__ rounds, float4* __restrict__ sorted, const float* __restrict__ q,
     float* __restrict__ sorted_q, double* __restrict__ q2) {
     __shared__ double red[32];
-    __shared__ int cnt[kSmallKeys], flag[kSmallKeys], wsum[32];
+    __shared__ int cnt[kSmallKeys], flag[kSmallKeys];
+    __shared__ u64 wsum[32];
     __shared__ unsigned frame;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int k = tid; k < nkey; k += kSmallThreads) cnt[k] = 0;
@@ -900,43 +927,37 @@ __global__ void __launch_bounds__(kSmallThreads) cell_sort_small_kernel(
     __syncthreads();
     // starts: every thread scans kSmallKeys / kSmallThreads consecutive keys
     constexpr int kPer = kSmallKeys / kSmallThreads;
-    int v[kPer], sum = 0;
+    int v[kPer];
+    u64 sum = 0;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
         const int g = tid * kPer + k;
         v[k] = g < nkey ? cnt[g] : 0;
-        sum += v[k];
+        sum += group_sums(v[k]);
     }
-    int x = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
+    const u64 x = warp_scan(sum, lane);
     if (lane == 31) wsum[warp] = x;
     __syncthreads();
-    int w = wsum[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-    }
-    const int before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
-    int run = (warp > 0 ? before : 0) + x - sum;
+    const u64 w = warp_scan(wsum[lane], lane);
+    const u64 before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+    u64 run = (warp > 0 ? before : 0) + x - sum;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
         const int g = tid * kPer + k;
         if (g < nkey) {
-            fstart[g] = run;
+            const int at = (int)(unsigned)run;
+            fstart[g] = at;
             fcount[g] = v[k];
-            cnt[g] = run;
+            cnt[g] = at;
+            emit_rounds(rounds, (unsigned)(run >> 32), g, at, v[k]);
         }
-        run += v[k];
+        run += group_sums(v[k]);
     }
     for (int k = tid; k < ncell; k += kSmallThreads) cflag[k] = flag[k];
+    if (tid == kSmallThreads - 1) work[kWorkRounds] = (unsigned)(run >> 32);
     if (tid == 0) {
-        *work = 0u;
-        *fflag = frame;
+        work[kWorkNext] = 0u;
+        work[kWorkFlags] = frame;
     }
     __syncthreads();
     double s2 = 0.0;
@@ -1134,7 +1155,7 @@ __global__ void __launch_bounds__(kBatchThreads) batch_keys_kernel(const BatchHe
                 if (a.flag) atomicOr(&st.cflag[it.key_begin + a.cell], a.flag);
             }
             ff = __reduce_or_sync(0xffffffffu, ff);
-            if ((threadIdx.x & 31) == 0 && ff) atomicOr(&st.state[4 * r + 2], ff);
+            if ((threadIdx.x & 31) == 0 && ff) atomicOr(&st.state[kWorkWords * r + kWorkFlags], ff);
         }
     }
 }
@@ -1146,16 +1167,13 @@ __global__ void __launch_bounds__(kBatchThreads) batch_offsets_kernel(const Batc
          k0 += (int64_t)gridDim.x * kBatchThreads) {
         const int r = batch_item_of<&BatchItem::key_begin>(items, hdr->nitems, k0);
         const int v = st.fcount[k0 + lane];
-        int x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        int base = 0;
-        if (lane == 31) base = (int)atomicAdd(&st.state[4 * r + 1], (unsigned)x);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        st.fstart[k0 + lane] = base + x - v;
+        const u64 x = warp_scan(group_sums(v), lane);
+        u64 base = 0;
+        if (lane == 31) base = atomicAdd(reinterpret_cast<u64*>(&st.state[kWorkWords * r + kWorkAtoms]), x);
+        const u64 at = __shfl_sync(0xffffffffu, base, 31) + x - group_sums(v);
+        st.fstart[k0 + lane] = (int)(unsigned)at;
+        emit_rounds(st.rounds + batch_rounds_begin(items[r]), (unsigned)(at >> 32), (int)(k0 + lane - items[r].key_begin),
+                    (int)(unsigned)at, v);
     }
 }
 
@@ -1205,7 +1223,8 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
         __syncthreads();
         for (int k = tid; k < nitems; k += kBatchThreads) {
             const int q = r + k < nitems ? r + k : r + k - nitems;
-            if (*(volatile unsigned*)&st.state[4 * q] < items[q].pair.nitems && items[q].hist) {
+            const volatile unsigned* work = &st.state[kWorkWords * q];
+            if (items[q].hist && work[kWorkNext] < work[kWorkRounds] * (unsigned)items[q].pair.nseg) {
                 atomicMin(&next, k);
                 break;
             }
@@ -1227,18 +1246,20 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
         __syncthreads();
         PairCounters pc;
         u64 n_tested = 0;
-        const bool frame_ok = frame_within(st.state[4 * r + 2]);
+        const bool frame_ok = frame_within(st.state[kWorkWords * r + kWorkFlags]);
+        const unsigned nwork = st.state[kWorkWords * r + kWorkRounds] * (unsigned)p.nseg;
+        const int2* rounds = st.rounds + batch_rounds_begin(it);
         const float4* sorted = st.sorted + it.atom_off;
         const int32_t *fstart = st.fstart + it.key_begin, *fcount = st.fcount + it.key_begin,
                       *cflag = st.cflag + it.key_begin;
         for (;;) {
             unsigned item = 0;
-            if (lane == 0) item = atomicAdd(&st.state[4 * r], 1u);
+            if (lane == 0) item = atomicAdd(&st.state[kWorkWords * r + kWorkNext], 1u);
             item = __shfl_sync(0xffffffffu, item, 0);
-            if (item >= p.nitems) break;
+            if (item >= nwork) break;
 #define TRJ_ITEM(F, S, E)                                                                                       \
-    pair_item<F, false, S, E, 1>(p, (int)item, sorted, fstart, fcount, cflag, frame_ok, nullptr, ring, nullptr, ws, \
-                                 hist_base, rowtab_base, nullptr, pc, n_tested)
+    pair_item<F, false, S, E, 1>(p, (int)item, rounds, sorted, fstart, fcount, cflag, frame_ok, nullptr, ring, nullptr, \
+                                 ws, hist_base, rowtab_base, nullptr, pc, n_tested)
             if (p.g.floor_bins) TRJ_ITEM(true, false, true);
             else if (!square) TRJ_ITEM(false, false, true);
             else if (p.g.want_edge) TRJ_ITEM(false, true, true);
@@ -1271,9 +1292,10 @@ struct trj_rdf_plan {
     int nc[3] = {1, 1, 1};      // cells per axis of the cutoff
     int64_t key_cap = 0;        // capacity of the per-group arrays
     int32_t* fstart = nullptr;  // key_cap: first atom of every (cell, group) in `sorted`
-    // Zeroed per frame by one memset: work counter (8 bytes), atoms placed, frame flags, cell flags
-    // (ncell: bit 0 a coordinate outside [0, L), bit 1 outside [-L, L)), atoms per group (nkey).
-    int32_t* zeroed = nullptr;  // 4 + ncell_cap + key_cap
+    // Zeroed per frame by one memset: work state (kWorkWords), cell flags (ncell: bit 0 a coordinate outside
+    // [0, L), bit 1 outside [-L, L)), atoms per group (nkey).
+    int32_t* zeroed = nullptr;  // kWorkWords + ncell_cap + key_cap
+    int2* rounds = nullptr;     // key_cap + n_max / 32: key and first atom of every round of homes
     int32_t* akey = nullptr;    // n_max: (cell, group) key per atom
     int32_t* aslot = nullptr;   // n_max
     int grid_nc[3] = {1, 1, 1}, nsub = 1;  // cells and groups per cell of the last accumulated frame
@@ -1298,7 +1320,7 @@ static float nint_threshold(float L, float q) {
     return x;
 }
 
-// Most work items a fused frame's neighbour lists are cut into (frames of more groups have one per group).
+// Most work items a fused frame's neighbour lists are cut into (frames of more rounds have one segment each).
 constexpr int64_t kBatchItemsMost = (int64_t)1 << 20;
 
 static int nint_host(float x) {  // Fortran NINT: half away from zero
@@ -1459,12 +1481,15 @@ static void fill_grid(RdfParams& P, int64_t n, const float box[3], float side2, 
     P.div_nc2 = make_fast_div(P.nc[2]);
 }
 
-// Work items of nkey home groups with neighbour lists cut into about nseg segments.
-static void set_segments(RdfParams& P, int nseg, int nkey) {
-    P.per_seg = (P.list + nseg - 1) / nseg;
+// Neighbour lists cut into about nseg segments, at most so many that the work items of n atoms in nkey groups
+// (the groups' rounds: ceil(atoms / 32) each) are below 2^31.
+static void set_segments(RdfParams& P, int64_t nseg, int64_t nkey, int64_t n) {
+    const int64_t rounds = nkey + n / kGroup;
+    nseg = std::max<int64_t>(1, std::min(nseg, ((int64_t)1 << 30) / rounds));
+    P.per_seg = (int)((P.list + nseg - 1) / nseg);
     P.nseg = (P.list + P.per_seg - 1) / P.per_seg;
     P.div_nseg = make_fast_div(P.nseg);
-    P.nitems = (unsigned)nkey * (unsigned)P.nseg;  // below 2^31: the callers bound nseg by the number of keys
+    P.nitems = (unsigned)(rounds * P.nseg);
 }
 
 struct PairShape {
@@ -1496,7 +1521,7 @@ static bool pair_shape(const trj_ctx* ctx, int nsp, int nit, int row_words, bool
     return false;
 }
 
-typedef void (*PairKernel)(RdfParams, const float4*, const int32_t*, const int32_t*, const int32_t*, const unsigned*, unsigned*,
+typedef void (*PairKernel)(RdfParams, const float4*, const int32_t*, const int32_t*, const int32_t*, const int2*, unsigned*,
                            u64*, u64*, unsigned*, const float*, double*);
 template <bool FLOOR, bool SQUARE>
 static PairKernel pair_kernel_of(bool charged, bool edge) {
@@ -1550,18 +1575,19 @@ static int rdf_plan_create_impl(trj_ctx* ctx, int nsp, float deltar, float rcrdf
     // Groups: one per cell, or at least 16 atoms per group on average (choose_groups).
     p->key_cap = (int64_t)p->ncell_cap + n_max / 16 + 64;
     const size_t na = (size_t)std::max<int64_t>(n_max, 1);
-    size_t bytes = 64 + sizeof(int32_t) * (size_t)(4 + p->ncell_cap + 2 * p->key_cap) +
-                   (sizeof(int32_t) * 2 + sizeof(float4)) * na;
+    size_t bytes = 64 + sizeof(int32_t) * (size_t)(kWorkWords + p->ncell_cap + 2 * p->key_cap) +
+                   (sizeof(int32_t) * 2 + sizeof(float4)) * na + sizeof(int2) * ((size_t)p->key_cap + na / kGroup + 1);
     char* base = nullptr;
     if (trj_dev_alloc(ctx, (void**)&base, bytes + 256) != cudaSuccess) {
         delete p;
         return trj_fail(ctx, TRJ_ERR_NOMEM, "rdf plan: %zu bytes of scratch", bytes);
     }
     p->sorted = reinterpret_cast<float4*>(base);
-    p->akey = reinterpret_cast<int32_t*>(p->sorted + na);
+    p->rounds = reinterpret_cast<int2*>(p->sorted + na);
+    p->akey = reinterpret_cast<int32_t*>(p->rounds + (size_t)p->key_cap + na / kGroup + 1);
     p->aslot = p->akey + na;
     p->zeroed = reinterpret_cast<int32_t*>((reinterpret_cast<uintptr_t>(p->aslot + na) + 15) & ~(uintptr_t)15);
-    p->fstart = p->zeroed + 4 + p->ncell_cap + p->key_cap;
+    p->fstart = p->zeroed + kWorkWords + p->ncell_cap + p->key_cap;
     p->scratch_bytes = (int64_t)bytes;
     *out = p;
     return TRJ_OK;
@@ -1700,16 +1726,15 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
     // Segments: about twelve items per resident warp, so that the last ones end together (six: 62,500 atoms
     // 485 us instead of 455; twenty-four: 459), but at least two neighbour groups per item.
     const int64_t warps = (int64_t)ctx->sm_count * shape.ctas * shape.warps;
-    set_segments(P, (int)std::max<int64_t>(1, std::min<int64_t>((12 * warps + nkey - 1) / nkey, P.list / 2)), nkey);
+    set_segments(P, std::min<int64_t>((12 * warps + nkey - 1) / nkey, P.list / 2), nkey, n);
 
     const PairKernel kern = pair_kernel(plan->floor_bins, charged, shape.square, edge_dev != nullptr);
     TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem));
 
     // Cell binning: count, group offsets, scatter.
     unsigned* work = reinterpret_cast<unsigned*>(plan->zeroed);
-    int32_t* total = plan->zeroed + 2;
-    unsigned* fflag = reinterpret_cast<unsigned*>(plan->zeroed + 3);
-    int32_t* cflag = plan->zeroed + 4;
+    unsigned* fflag = work + kWorkFlags;
+    int32_t* cflag = plan->zeroed + kWorkWords;
     int32_t* fcount = cflag + ncell;
     plan->fcount_last = fcount;
     plan->nsub = P.nsub;
@@ -1719,16 +1744,17 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
     int q2_parts = 0;  // sums of squared charges, one per sorting block
     if (n <= kSmallAtoms && nkey <= kSmallKeys) {
         cell_sort_small_kernel<<<1, kSmallThreads, 0, s>>>((const float4*)packed_dev, (int)n, P, ncell, nkey, wscale, work,
-                                                           fflag, cflag, fcount, plan->fstart, plan->sorted, q_dev,
-                                                           plan->sorted_q, plan->q2_part);
+                                                           cflag, fcount, plan->fstart, plan->rounds, plan->sorted,
+                                                           q_dev, plan->sorted_q, plan->q2_part);
         q2_parts = 1;
         ctx->launches += 1;
     } else {
-        TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->zeroed, 0, sizeof(int32_t) * (size_t)(4 + ncell + nkey), s));
+        TRJ_CUDA_TRY(ctx, cudaMemsetAsync(plan->zeroed, 0, sizeof(int32_t) * (size_t)(kWorkWords + ncell + nkey), s));
         const unsigned nb = (unsigned)((n + 255) / 256);
         cell_assign_kernel<<<nb, 256, 0, s>>>((const float4*)packed_dev, n, P, fcount, cflag, fflag, plan->akey,
                                               plan->aslot);
-        group_offsets_kernel<<<(unsigned)((nkey + 255) / 256), 256, 0, s>>>(fcount, nkey, total, plan->fstart);
+        group_offsets_kernel<<<(unsigned)((nkey + 255) / 256), 256, 0, s>>>(
+            fcount, nkey, reinterpret_cast<u64*>(work + kWorkAtoms), plan->fstart, plan->rounds);
         cell_scatter_kernel<<<nb, 256, 0, s>>>((const float4*)packed_dev, n, plan->akey, plan->aslot, plan->fstart,
                                                wscale, plan->sorted, q_dev, plan->sorted_q, plan->q2_part);
         q2_parts = (int)nb;
@@ -1738,8 +1764,8 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
     const int64_t grid = std::min<int64_t>((int64_t)ctx->sm_count * shape.ctas,
                                            ((int64_t)P.nitems + shape.warps - 1) / shape.warps);
     plan->timer.begin(ctx, s);
-    kern<<<(unsigned)grid, shape.warps * 32, shape.smem, s>>>(P, plan->sorted, plan->fstart, fcount, cflag, fflag, work,
-                                                              (u64*)hist_dev, (u64*)edge_dev, ctx->status_dev,
+    kern<<<(unsigned)grid, shape.warps * 32, shape.smem, s>>>(P, plan->sorted, plan->fstart, fcount, cflag,
+                                                              plan->rounds, work, (u64*)hist_dev, (u64*)edge_dev, ctx->status_dev,
                                                               charged ? plan->sorted_q : nullptr,
                                                               charged ? plan->gqq_frame : nullptr);
     plan->timer.end(ctx, s);
@@ -1858,8 +1884,8 @@ int trj_batch_fill_rdf(trj_rdf_plan* plan, int64_t n, const float box[3], int hi
     *nkey = (int64_t)P.nc[0] * P.nc[1] * P.nc[2] * P.nsub;
     // About ten neighbour groups per item, but no more items than keep every warp of the GPU busy some 300 times
     // over: the list grows with the frame, and items are numbered in 31 bits.  One-atom frames have no pairs.
-    const int64_t most = std::max<int64_t>(1, kBatchItemsMost / std::max<int64_t>(1, *nkey));
-    if (n >= 2) set_segments(P, (int)std::max<int64_t>(1, std::min<int64_t>(P.list / 10, most)), (int)*nkey);
+    const int64_t most = kBatchItemsMost / (*nkey + n / kGroup);
+    if (n >= 2) set_segments(P, std::min<int64_t>(P.list / 10, most), *nkey, n);
     // a row per ordered species pair where those fit (floor bins: the general layout only)
     it->square = !plan->floor_bins &&
                  (int64_t)plan->nsp * plan->nsp * P.g.row_words <= (int64_t)batch_hist_smem_words(hist_words);
