@@ -1007,24 +1007,27 @@ __global__ void one_charge_kernel(const float* __restrict__ q, double* __restric
 // atoms within each radius r_k = k*deltar (cumulative over nint(r/deltar) bins, the reference's
 // gi_s(ind:lsmax) += 1) from the cells around it, and adds N_k and N_k^2 to the int64 sums.
 //
-// What bounds it: latency of the groups' starts and atoms.  A warp takes eight groups of the 27 cells at a
-// time, their starts in one load and an atom of four groups per lane in flight; the cumulative counts are a
-// block scan.  4,096 points at 1e6 atoms: 0.268 ms, as with threads over whole cells of atoms sorted otherwise
-// (0.269); a warp per group with its start loaded each time, a division per axis and one thread summing the
-// counts 0.364; without the division-free minimum image 0.347.
-constexpr int kS2nThreads = 256, kS2nGroups = 8, kS2nFlight = 4;
+// What bounds it: latency of the groups' starts and atoms.  A lane looks at a group of the point's cells (a warp
+// at every eighth, so that the warps have equal shares) and drops it where its box is out of reach; the warp then
+// has an atom of four groups per lane in flight, and groups of more than 128 atoms (frames of uneven density) go
+// to the whole block.  The cumulative counts are a block scan.
+constexpr int kS2nThreads = 256, kS2nFlight = 4, kS2nLarge = 128, kS2nList = 64;
 __global__ void __launch_bounds__(kS2nThreads, 5)
     s2n_kernel(const float4* __restrict__ sorted, const int32_t* __restrict__ fstart,
-               const int32_t* __restrict__ fcount, int nsub, PairGeom g, int ncx, int ncy, int ncz,
+               const int32_t* __restrict__ fcount, const int32_t* __restrict__ cflag, const __grid_constant__ RdfParams p,
                unsigned long long* __restrict__ gi, unsigned long long* __restrict__ g2i, float* __restrict__ points,
                int dim) {
+    const PairGeom& g = p.g;
     extern __shared__ unsigned s2n_cnt[];  // lsmax + 1
     unsigned* cnt = s2n_cnt;
     __shared__ float pt[3];
     __shared__ unsigned wsum[kS2nThreads / 32];
+    __shared__ int2 large[kS2nList];  // groups left to the whole block: start and atoms
+    __shared__ int nlarge;
     const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5), lsmax = g.lsmax;
     for (int k = threadIdx.x; k <= lsmax; k += kS2nThreads) cnt[k] = 0u;
     if (threadIdx.x == 0) {
+        nlarge = 0;
         curandStateXORWOW_t h;
         curand_init((unsigned long long)blockIdx.x + 1ull + 12345ull, 0ull, 0ull, &h);
         pt[0] = g.L[0] * curand_uniform(&h);
@@ -1037,13 +1040,13 @@ __global__ void __launch_bounds__(kS2nThreads, 5)
         }
     }
     __syncthreads();
-    const int nc[3] = {ncx, ncy, ncz};
     int pc[3];
+    float pw[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {  // the point's cell, as cell_assign_kernel bins an atom
-        const float w = pt[d] - g.L[d] * floorf(pt[d] / g.L[d]);
-        int c = (int)(w * ((float)nc[d] / g.L[d]));
-        pc[d] = c < 0 ? 0 : (c >= nc[d] ? nc[d] - 1 : c);
+        pw[d] = pt[d] - g.L[d] * floorf(pt[d] / g.L[d]);
+        int c = (int)(pw[d] * ((float)p.nc[d] / g.L[d]));
+        pc[d] = c < 0 ? 0 : (c >= p.nc[d] ? p.nc[d] - 1 : c);
     }
     const float px = pt[0], py = pt[1], pz = pt[2];
     auto count = [&](const float4& a) {
@@ -1058,27 +1061,54 @@ __global__ void __launch_bounds__(kS2nThreads, 5)
         }
     };
     // an axis that is not split has one cell, a split one three or more
-    const int sx = ncx > 1 ? 3 : 1, sy = ncy > 1 ? 3 : 1, sz = ncz > 1 ? 3 : 1;
-    const int total = sx * sy * sz * nsub;
-    for (int base = kS2nGroups * warp; base < total; base += kS2nGroups * (kS2nThreads / 32)) {
+    const int sx = p.nc[0] > 1 ? 3 : 1, sy = p.nc[1] > 1 ? 3 : 1, sz = p.nc[2] > 1 ? 3 : 1;
+    const int total = sx * sy * sz * p.nsub;
+    for (int base = 0; base < total; base += kS2nThreads) {
+        const int t = base + lane * (kS2nThreads / 32) + warp;
         int j0 = 0, na = 0;
-        if (lane < kS2nGroups && base + lane < total) {
-            const int e = (base + lane) / nsub, sg = base + lane - e * nsub;
-            const int cx = (pc[0] + e / (sy * sz) - (sx >> 1) + ncx) % ncx;
-            const int cy = (pc[1] + e / sz % sy - (sy >> 1) + ncy) % ncy;
-            const int cz = (pc[2] + e % sz - (sz >> 1) + ncz) % ncz;
-            const int key = ((cx * ncy + cy) * ncz + cz) * nsub + sg;
-            j0 = fstart[key];
-            na = fcount[key];
+        if (t < total) {
+            const int e = fast_div(t, p.div_nsub), s = t - e * p.nsub;
+            const int cx = wrapc(pc[0] + e / (sy * sz) - (sx >> 1), p.nc[0]);
+            const int cy = wrapc(pc[1] + e / sz % sy - (sy >> 1), p.nc[1]);
+            const int cz = wrapc(pc[2] + e % sz - (sz >> 1), p.nc[2]);
+            const int cell = (cx * p.nc[1] + cy) * p.nc[2] + cz;
+            bool near = cflag[cell] & 2;  // coordinates outside [-L, L): anywhere
+            if (!near) {
+                // nearest image of the group's box, as pair_item culls a neighbour group
+                const int q = (int)(((float)s + 0.5f) * p.inv_sub[2]), bz = s - q * p.sub[2];
+                const int bx = (int)(((float)q + 0.5f) * p.inv_sub[1]), by = q - bx * p.sub[1];
+                const float dx = axis_gap<true>(((float)cx + ((float)bx + 0.5f) * p.inv_sub[0]) * p.edge[0], pw[0],
+                                                p.half[0], g.L[0]);
+                const float dy = axis_gap<true>(((float)cy + ((float)by + 0.5f) * p.inv_sub[1]) * p.edge[1], pw[1],
+                                                p.half[1], g.L[1]);
+                const float dz = axis_gap<true>(((float)cz + ((float)bz + 0.5f) * p.inv_sub[2]) * p.edge[2], pw[2],
+                                                p.half[2], g.L[2]);
+                near = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= p.cull2;
+            }
+            if (near) {
+                const int key = cell * p.nsub + s;
+                j0 = fstart[key];
+                na = fcount[key];
+                if (na > kS2nLarge) {
+                    const int k = atomicAdd(&nlarge, 1);
+                    if (k < kS2nList) {
+                        large[k] = make_int2(j0, na);
+                        na = 0;
+                    }
+                }
+            }
         }
-#pragma unroll
-        for (int k0 = 0; k0 < kS2nGroups; k0 += kS2nFlight) {
+        unsigned m = __ballot_sync(0xffffffffu, na > 0);
+        while (m) {
             float4 a[kS2nFlight];
             int n[kS2nFlight], j[kS2nFlight];
 #pragma unroll
             for (int k = 0; k < kS2nFlight; ++k) {
-                j[k] = __shfl_sync(0xffffffffu, j0, k0 + k);
-                n[k] = __shfl_sync(0xffffffffu, na, k0 + k);
+                const int from = m ? __ffs(m) - 1 : 0;
+                j[k] = __shfl_sync(0xffffffffu, j0, from);
+                n[k] = __shfl_sync(0xffffffffu, na, from);
+                if (!m) n[k] = 0;
+                m &= m - 1u;
                 if (lane < n[k]) a[k] = sorted[j[k] + lane];
             }
 #pragma unroll
@@ -1088,6 +1118,9 @@ __global__ void __launch_bounds__(kS2nThreads, 5)
             }
         }
     }
+    __syncthreads();
+    for (int k = 0; k < min(nlarge, kS2nList); ++k)
+        for (int q = (int)threadIdx.x; q < large[k].y; q += kS2nThreads) count(sorted[large[k].x + q]);
     __syncthreads();
     // cumulative counts N_k = sum_{j <= k} cnt[j] (at most the frame's atoms): a thread's run, then the runs before it
     const int run = (lsmax + kS2nThreads) / kS2nThreads, k0 = (int)threadIdx.x * run, k1 = min(k0 + run, lsmax + 1);
@@ -1298,12 +1331,11 @@ struct trj_rdf_plan {
     int2* rounds = nullptr;     // key_cap + n_max / 32: key and first atom of every round of homes
     int32_t* akey = nullptr;    // n_max: (cell, group) key per atom
     int32_t* aslot = nullptr;   // n_max
-    int grid_nc[3] = {1, 1, 1}, nsub = 1;  // cells and groups per cell of the last accumulated frame
+    RdfParams frame_last;       // geometry, cells and groups of the last accumulated frame
     float4* sorted = nullptr;   // n_max
     float* sorted_q = nullptr;  // n_max charges in cell order (first charged call)
-    int32_t* fcount_last = nullptr;  // atoms per group of the last accumulated frame (in `zeroed`)
+    int32_t *cflag_last = nullptr, *fcount_last = nullptr;  // its cell flags and atoms per group (in `zeroed`)
     int cells_valid = 0;        // sorted, fstart and the counts hold the last accumulated frame
-    float box_last[3] = {0.f, 0.f, 0.f};
     double* gqq_frame = nullptr;  // lsmax: this frame's charge-product sums
     double* q2_part = nullptr;    // one per sorting block: sums of squared charges
     int64_t scratch_bytes = 0;
@@ -1708,10 +1740,7 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
     P.stall_test = plan->stall_test;
     P.nit = plan->nit;
     cells_for(box, plan->side2, P.nc, plan->dim);
-    for (int d = 0; d < 3; ++d) {
-        plan->nc[d] = P.nc[d];
-        plan->box_last[d] = box[d];
-    }
+    for (int d = 0; d < 3; ++d) plan->nc[d] = P.nc[d];
     if (P.nc[0] * P.nc[1] * P.nc[2] > plan->ncell_cap)
         return trj_fail(ctx, TRJ_ERR_CAPACITY, "rdf accumulate: %d cells exceed plan capacity %d",
                         P.nc[0] * P.nc[1] * P.nc[2], plan->ncell_cap);
@@ -1737,8 +1766,8 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
     int32_t* cflag = plan->zeroed + kWorkWords;
     int32_t* fcount = cflag + ncell;
     plan->fcount_last = fcount;
-    plan->nsub = P.nsub;
-    for (int d = 0; d < 3; ++d) plan->grid_nc[d] = P.nc[d];
+    plan->cflag_last = cflag;
+    plan->frame_last = P;
     const unsigned wscale = shape.square ? 4u * (unsigned)P.g.row_words : 64u;
     const float* q_dev = charged ? charge_dev : nullptr;
     int q2_parts = 0;  // sums of squared charges, one per sorting block
@@ -1808,11 +1837,9 @@ extern "C" int trj_rdf_s2n(trj_rdf_plan* plan, int nrandom, uint64_t* gi_dev, ui
     // Always, and always the same: without it the kernel's static shared memory counts against 48 KB as well, and a
     // value of this call's own could be lowered by another thread's before the launch.
     TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(s2n_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
-    PairGeom geom;
-    fill_geom(geom, plan->box_last, plan->side2, plan->deltar, plan->lsmax, plan->nsp, 0, false);
     s2n_kernel<<<(unsigned)nrandom, kS2nThreads, smem, (cudaStream_t)stream>>>(
-        plan->sorted, plan->fstart, plan->fcount_last, plan->nsub, geom, plan->grid_nc[0], plan->grid_nc[1],
-        plan->grid_nc[2], (unsigned long long*)gi_dev, (unsigned long long*)g2i_dev, points_dev, plan->dim);
+        plan->sorted, plan->fstart, plan->fcount_last, plan->cflag_last, plan->frame_last, (unsigned long long*)gi_dev,
+        (unsigned long long*)g2i_dev, points_dev, plan->dim);
     ctx->launches += 1;
     TRJ_CUDA_TRY(ctx, cudaGetLastError());
     return TRJ_OK;
