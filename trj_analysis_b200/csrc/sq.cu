@@ -100,9 +100,10 @@ __device__ __forceinline__ void terms2(unsigned pa, unsigned pb, const char* tab
 
 // Shape of a direct sum.  A slice (of nsplit) is the unit of the FP32 partial sums: runs of 64 atoms are
 // counted from its start within each species; parts cut a slice's runs further, between blocks.  A block
-// takes tv threads x VPT vectors and walks tg runs at a time (tv * tg <= 256 threads).
+// takes tv threads x VPT vectors and walks tg runs at a time (tv * tg <= 256 threads); the species are shared out
+// between `cuts` blocks.
 struct PlainShape {
-    int vpt, tv, tg, nvblk, nsplit, parts;
+    int vpt, tv, tg, nvblk, nsplit, parts, cuts;
 };
 
 // Shared memory of a direct-sum block: replicated turn table, staged atoms, FP64 sums of the tg > 1 threads.
@@ -121,7 +122,7 @@ __device__ __forceinline__ void fill_turn_table(PlainSmem& sm, const float2* __r
     }
 }
 
-// Sums of one block of vectors (bx) over one part (by = slice * parts + part) of every species.  Species qsp
+// Sums of one block of vectors (bx) over one part (by = slice * parts + part) of species [sp0, sp1).  Species qsp
 // (if any) is the charge species: each term is weighted by the charge in the entry's w.  Partials by position
 // in the subset: part[by][species][nsub].  The turn table must be filled; the first barrier orders it.
 //
@@ -133,7 +134,7 @@ __device__ __forceinline__ void fill_turn_table(PlainSmem& sm, const float2* __r
 // one slice: 235 -> 12 us.
 template <int VPT>
 __device__ __forceinline__ void plain_block(const uint4* __restrict__ phase, const int64_t* __restrict__ sp_off,
-                                            int nsp, int qsp, const int4* __restrict__ vecs,
+                                            int nsp, int sp0, int sp1, int qsp, const int4* __restrict__ vecs,
                                             const int32_t* __restrict__ subset, int nsub, const PlainShape& shape,
                                             double2* __restrict__ part, int64_t bx, int64_t by, PlainSmem& sm) {
     const int tid = threadIdx.x, tv = shape.tv, tg = shape.tg;
@@ -152,7 +153,7 @@ __device__ __forceinline__ void plain_block(const uint4* __restrict__ phase, con
         nz[q] = (unsigned)n.z;
     }
     const int64_t slice = by / shape.parts, cut = by - slice * shape.parts;
-    for (int a = 0; a < nsp; ++a) {
+    for (int a = sp0; a < sp1; ++a) {
         const int64_t a0 = sp_off[a], len = sp_off[a + 1] - a0;
         const int64_t s0 = a0 + len * slice / shape.nsplit, s1 = a0 + len * (slice + 1) / shape.nsplit;
         const int64_t runs = (s1 - s0 + kPlainSub - 1) / kPlainSub;
@@ -224,7 +225,9 @@ __global__ void __launch_bounds__(kPlainThreads, kPlainCtas) sq_plain_kernel(
     const float2* __restrict__ turn, double2* __restrict__ part) {
     __shared__ __align__(16) PlainSmem sm;
     fill_turn_table(sm, turn);
-    plain_block<VPT>(phase, sp_off, nsp, qsp, vecs, subset, nsub, shape, part, blockIdx.x, blockIdx.y, sm);
+    const int cut = (int)blockIdx.z;
+    plain_block<VPT>(phase, sp_off, nsp, nsp * cut / shape.cuts, nsp * (cut + 1) / shape.cuts, qsp, vecs, subset, nsub,
+                     shape, part, blockIdx.x, blockIdx.y, sm);
 }
 
 // Sums over `n` partials `stride` apart for 32 vectors at a time (consecutive vectors in a warp's lanes:
@@ -376,14 +379,14 @@ __global__ void __launch_bounds__(kPlainThreads, 2) batch_sq_kernel(BatchHeader*
         __syncthreads();
         if (u >= total) break;
         const BatchItem& it = items[batch_item_of<&BatchItem::sq_begin>(items, nitems, u)];
-        const PlainShape shape = {it.vpt, it.tv, it.tg, it.nvblk, it.nsplit, it.parts};
+        const PlainShape shape = {it.vpt, it.tv, it.tg, it.nvblk, it.nsplit, it.parts, 1};
         const int64_t t = u - it.sq_begin, bx = t % it.nvblk, by = t / it.nvblk;
         if (it.vpt == 2)
-            plain_block<2>(phase + it.atom_off, it.sp_off_dev, it.nsp, -1, it.vecs, it.subset, it.nvec, shape,
-                           it.part, bx, by, sm);
+            plain_block<2>(phase + it.atom_off, it.sp_off_dev, it.nsp, 0, it.nsp, -1, it.vecs, it.subset, it.nvec,
+                           shape, it.part, bx, by, sm);
         else
-            plain_block<4>(phase + it.atom_off, it.sp_off_dev, it.nsp, -1, it.vecs, it.subset, it.nvec, shape,
-                           it.part, bx, by, sm);
+            plain_block<4>(phase + it.atom_off, it.sp_off_dev, it.nsp, 0, it.nsp, -1, it.vecs, it.subset, it.nvec,
+                           shape, it.part, bx, by, sm);
     }
 }
 
@@ -454,7 +457,8 @@ int plain_nsplit(const trj_ctx* ctx, int64_t nsub, int64_t n_total) {
 // Launch shape: four vectors per thread where that still makes enough warps, two otherwise (one packed
 // instruction serves two); tv threads cover a block's vectors with the fewest idle lanes, the other threads
 // take further runs.  Slices are cut into parts, at least a run per run lane, while the partials stay below
-// 256 MB.
+// 256 MB; where that makes fewer than three waves of blocks (a few atoms in each of many groups), the species are
+// shared out as well: 64 groups of 256 atoms x 773 vectors 280 -> 64 us, 64 of 469 x 7,904 460 -> 310 us.
 PlainShape plain_shape(const trj_ctx* ctx, int64_t nsub, int64_t n_total, int nsp) {
     PlainShape s;
     s.nsplit = plain_nsplit(ctx, nsub, n_total);
@@ -485,6 +489,7 @@ PlainShape plain_shape(const trj_ctx* ctx, int64_t nsub, int64_t n_total, int ns
             s.parts = (int)k;
         }
     }
+    s.cuts = (int)std::min<int64_t>(nsp, std::max<int64_t>(1, (int64_t)ceil(3.0 * slots / (double)(blocks * s.parts))));
     return s;
 }
 
@@ -729,7 +734,7 @@ extern "C" int trj_sq_plan_info(const trj_sq_plan* p, int64_t* n_dense, int64_t*
 
 static void launch_plain(const trj_ctx* ctx, const PlainShape& sh, const uint4* phase, const int64_t* sp_off, int nsp,
                          int qsp, const int4* vecs, const int32_t* subset, int64_t nsub, double2* part, cudaStream_t s) {
-    const dim3 grid((unsigned)sh.nvblk, (unsigned)(sh.nsplit * sh.parts));
+    const dim3 grid((unsigned)sh.nvblk, (unsigned)(sh.nsplit * sh.parts), (unsigned)sh.cuts);
     auto kern = sh.vpt == 2 ? sq_plain_kernel<2> : sq_plain_kernel<4>;
     kern<<<grid, sh.tv * sh.tg, 0, s>>>(phase, sp_off, nsp, qsp, vecs, subset, (int)nsub, sh, ctx->turn_dev, part);
 }
