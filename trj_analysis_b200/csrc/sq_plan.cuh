@@ -43,7 +43,8 @@ struct trj_sq_plan {
     int64_t tile_slots = 0;                // sum over tiles of 128 * ncols/2
     int64_t tc_out_doubles = 0;
     int64_t* dense_src_dev = nullptr;      // per plan vector: offset into TC output (re at +0, im at +128) or -1
-    // scratch
+    // scratch: parts of one allocation
+    char* scratch = nullptr;
     uint4* phase_dev = nullptr;            // n_total x (ux, uy, uz, species)
     double2* part_dev = nullptr;           // direct-sum partials [slice, part][nsp][nvec]
     double* tc_out_dev = nullptr;          // tensor-core rho blocks (FP64)

@@ -183,6 +183,7 @@ struct TcState {
     TcChunk* chunks_dev = nullptr;
     int64_t* pad_off_dev = nullptr;  // nsp+1 offsets, then nsp slot -> atom multipliers
     int32_t* chunk_begin_dev = nullptr;
+    char* scratch = nullptr;  // tables and partial sums, parts of one allocation
     __nv_bfloat16* tab_hi = nullptr;
     __nv_bfloat16* tab_lo = nullptr;
     uint2* uxy = nullptr;
@@ -1336,8 +1337,7 @@ void trj_sq_tc_release(trj_sq_plan* plan) {
     TcState* st = reinterpret_cast<TcState*>(plan->tc_state);
     if (!st) return;
     void* ptrs[] = {st->sched_dev, st->tiles_dev, st->chunks_dev, st->pad_off_dev, st->chunk_begin_dev,
-                    st->tab_hi,    st->tab_lo,    st->uxy,        st->part,           st->pairs_dev,
-                    st->sched2_dev, st->xtab,     st->ytab};
+                    st->scratch,   st->pairs_dev, st->sched2_dev};
     for (void* q : ptrs) trj_dev_free(plan->ctx, q);
     delete st;
     plan->tc_state = nullptr;
@@ -1573,26 +1573,29 @@ int trj_sq_tc_prepare(trj_sq_plan* plan) {
     }
 
     const int64_t kdim = 2 * st->total_slots;
-    size_t tab_bytes = (size_t)st->table_rows * (size_t)kdim * sizeof(__nv_bfloat16);
-    size_t uxy_bytes = sizeof(uint2) * (size_t)st->total_slots;
+    auto a256 = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t tab_bytes = a256((size_t)st->table_rows * (size_t)kdim * sizeof(__nv_bfloat16));
+    const size_t uxy_bytes = a256(sizeof(uint2) * (size_t)st->total_slots);
     const int64_t nstage_tot = st->total_slots / kStageSlots;
     const size_t xtab_bytes = (size_t)nstage_tot * st->nxb * kXBlockBytes;
     const size_t ytab_bytes = (size_t)nstage_tot * st->nyb * kYBlockBytes;
-    size_t part_bytes = sizeof(float) * (size_t)st->acc_stride * st->chunks.size();
+    const size_t part_bytes = sizeof(float) * (size_t)st->acc_stride * st->chunks.size();
+    const size_t bytes = 2 * tab_bytes + uxy_bytes + xtab_bytes + ytab_bytes + part_bytes;
     std::vector<int32_t> cb(st->chunk_of_species_begin.begin(), st->chunk_of_species_begin.end());
-    if (trj_dev_alloc(ctx, (void**)&st->tab_hi, tab_bytes) != cudaSuccess ||
-        trj_dev_alloc(ctx, (void**)&st->tab_lo, tab_bytes) != cudaSuccess ||
-        trj_dev_alloc(ctx, (void**)&st->uxy, uxy_bytes) != cudaSuccess ||
-        trj_dev_alloc(ctx, (void**)&st->xtab, xtab_bytes) != cudaSuccess ||
-        trj_dev_alloc(ctx, (void**)&st->ytab, ytab_bytes) != cudaSuccess ||
-        trj_dev_alloc(ctx, (void**)&st->part, part_bytes) != cudaSuccess ||
+    if (trj_dev_alloc(ctx, (void**)&st->scratch, bytes) != cudaSuccess ||
         trj_dev_alloc(ctx, (void**)&st->tiles_dev, sizeof(TcTile) * tt.size()) != cudaSuccess ||
         trj_dev_alloc(ctx, (void**)&st->chunks_dev, sizeof(TcChunk) * st->chunks.size()) != cudaSuccess ||
         trj_dev_alloc(ctx, (void**)&st->pad_off_dev, sizeof(int64_t) * (2 * nsp + 1)) != cudaSuccess ||
         trj_dev_alloc(ctx, (void**)&st->chunk_begin_dev, sizeof(int32_t) * (nsp + 1)) != cudaSuccess ||
         trj_dev_alloc(ctx, (void**)&st->sched_dev, sizeof(int32_t) * sched.size()) != cudaSuccess)
-        return trj_fail(ctx, TRJ_ERR_NOMEM, "tensor path: %zu bytes of tables",
-                        2 * tab_bytes + uxy_bytes + xtab_bytes + ytab_bytes + part_bytes);
+        return trj_fail(ctx, TRJ_ERR_NOMEM, "tensor path: %zu bytes of tables", bytes);
+    char* at = st->scratch;
+    st->xtab = reinterpret_cast<float4*>(at);  // X/Y blocks are whole multiples of 2 KB
+    st->ytab = reinterpret_cast<float4*>(at += xtab_bytes);
+    st->tab_hi = reinterpret_cast<__nv_bfloat16*>(at += ytab_bytes);
+    st->tab_lo = reinterpret_cast<__nv_bfloat16*>(at += tab_bytes);
+    st->uxy = reinterpret_cast<uint2*>(at += tab_bytes);
+    st->part = reinterpret_cast<float*>(at += uxy_bytes);
     cudaMemcpy(st->tiles_dev, tt.data(), sizeof(TcTile) * tt.size(), cudaMemcpyHostToDevice);
     cudaMemcpy(st->chunks_dev, st->chunks.data(), sizeof(TcChunk) * st->chunks.size(), cudaMemcpyHostToDevice);
     // pad offsets, then the per-species slot -> atom multipliers
@@ -1614,7 +1617,7 @@ int trj_sq_tc_prepare(trj_sq_plan* plan) {
     cudaMemcpy(st->pad_off_dev, pad_mul.data(), sizeof(int64_t) * (2 * nsp + 1), cudaMemcpyHostToDevice);
     cudaMemcpy(st->chunk_begin_dev, cb.data(), sizeof(int32_t) * (nsp + 1), cudaMemcpyHostToDevice);
     cudaMemcpy(st->sched_dev, sched.data(), sizeof(int32_t) * sched.size(), cudaMemcpyHostToDevice);
-    plan->scratch_bytes += (int64_t)(2 * tab_bytes + uxy_bytes + xtab_bytes + ytab_bytes + part_bytes);
+    plan->scratch_bytes += (int64_t)bytes;
     // Blocked table: [total_slots / 32][table_rows][64 bf16] as a 2-D map of 128-byte rows.
     const int64_t brows = (st->total_slots / kStageSlots) * (int64_t)st->table_rows;
     int rc = encode_map(ctx, &st->map_hi, st->tab_hi, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, 64, brows, 64, 16,
