@@ -203,7 +203,7 @@ extern "C" int trj_batch_add(trj_batch* b, int buf, trj_rdf_plan* rdf, trj_sq_pl
     }
     if (rdf) {
         int p_nsp = 0;
-        int rc = trj_batch_fill_rdf(rdf, n, box, b->hist_words, edge_dev != nullptr, &it, &p_nsp, &nkey);
+        int rc = trj_batch_fill_rdf(rdf, n, box, b->hist_words, b->max_items, edge_dev != nullptr, &it, &p_nsp, &nkey);
         if (rc != TRJ_OK) return rc;
         if (sq && p_nsp != nsp)
             return trj_fail(ctx, TRJ_ERR_INVALID, "batch: pair plan has %d species, S(Q) plan %d", p_nsp, nsp);

