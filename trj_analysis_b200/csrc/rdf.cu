@@ -207,6 +207,7 @@ struct WarpState {
     int4 walk;                  // j, je, m, e0 of the neighbour walk
     int4 outer;                 // position in the neighbour list, cell of the homes and its flags, first home
     int nh;
+    int blocks;                 // blocks tested since the warp last merged the CTA's rows
 };
 
 constexpr size_t kWarpBytes = 16 * kRing + (sizeof(WarpState) + 15) / 16 * 16;  // buffer and state of a warp
@@ -395,6 +396,53 @@ __device__ __forceinline__ void axis_box(unsigned lo, unsigned hi, float pad, fl
 // reaches 0.749 L (frames centred on the origin).  (Coordinates outside [-L, L) are flagged per cell.)
 __device__ __forceinline__ bool frame_within(unsigned f) {
     return !(f & kFrameLow) || !(f & (kFrameVeryLow | kFrameHigh));
+}
+
+// The CTA's rows into the frame's uint64 histogram, elements first, first + step, ...; returns their total, the
+// counted pairs.  EARLY: taken out while other warps count on.  A count is then a signed number: a pair that another
+// warp has just counted in its approximate bin and is about to move may be taken out of that bin before it moves.
+template <bool SQUARE, bool EARLY>
+__device__ __forceinline__ u64 merge_rows(int nsp, int nit, int lsmax, unsigned* hist, u64* __restrict__ hist_g, int first,
+                                          int step) {
+    const int rw = lsmax + 2, hsz = nit * lsmax;
+    auto take = [&](unsigned* c) { return (long long)(int)(EARLY ? atomicExch(c, 0u) : *c); };
+    u64 total = 0;
+    int row = 0, sa = 0, sb = 0;  // species of the row of element k
+#pragma unroll 1
+    for (int k = first; k < hsz; k += step) {
+        while (row < k / lsmax) {
+            ++row;
+            if (++sb == nsp) sb = ++sa;
+        }
+        const int bin = k - row * lsmax + 1;
+        long long s;
+        if (SQUARE) {
+            s = take(&hist[(sa * nsp + sb) * rw + bin]);
+            if (sa != sb) s += take(&hist[(sb * nsp + sa) * rw + bin]);
+        } else {
+            s = take(&hist[row * rw + bin]);
+        }
+        if (s) atomicAdd(&hist_g[k], (u64)s);
+        total += (u64)s;
+    }
+    return total;
+}
+
+// Rows hold 32 bits per bin.  A warp that has tested 2^22 pairs since it last did so moves the CTA's rows to the
+// frame's histogram after its item.  A bin then holds less than 2^31 as long as no item meets 8e6 atoms at one distance
+// (eight warps per CTA; 2e6 with the 32 of CTAs that share a histogram of many bins).  Without it a CTA of a frame of
+// 1e7 atoms puts 4e9 pairs into a coarse bin at half the box.
+constexpr int kMergeBlocks = (1 << 22) / (4 * kGroup);
+template <bool SQUARE>
+__device__ __forceinline__ void merge_early(WarpState* ws, int nsp, int nit, int lsmax, unsigned* hist, u64* hist_g,
+                                            u64* edge_g) {
+    if (ws->blocks < kMergeBlocks) return;
+    const int lane = (int)(threadIdx.x & 31u);
+    const u64 counted = merge_rows<SQUARE, true>(nsp, nit, lsmax, hist, hist_g, lane, 32);
+    if (edge_g) atomicAdd(&edge_g[TRJ_EDGE_COUNTED], counted);
+    __syncwarp();
+    if (lane == 0) ws->blocks = 0;
+    __syncwarp();
 }
 
 // One work item of a frame: round item / nseg (up to 32 atoms of one group, see emit_rounds) against segment
@@ -601,7 +649,10 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const in
                 if (EDGE && lane < ws->nh) n_tested += (unsigned)(tail - before);
             }
             const int n4 = tail - head >= kRingRun ? kRingRun / 4 : pad();
-            if (lane == 0) ws->walk = make_int4(j, je, (int)m, e0);
+            if (lane == 0) {
+                ws->walk = make_int4(j, je, (int)m, e0);
+                ws->blocks += n4;
+            }
             __syncwarp();  // the other lanes' entries
             if (mode == kImgNone) TRJ_RUN(kImgNone, false, n4);
             else if (mode == kImgShift) TRJ_RUN(kImgShift, false, n4);
@@ -619,30 +670,6 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const in
 #undef TRJ_RUN
         t = ws->outer.x;
         __syncwarp();
-    }
-}
-
-// The CTA's rows into the frame's uint64 histogram (their total is the counted pairs).
-template <bool SQUARE>
-__device__ __forceinline__ void merge_rows(const RdfParams& p, const unsigned* hist, u64* __restrict__ hist_g,
-                                           PairCounters& pc) {
-    const int nsp = p.g.nsp, rw = p.g.row_words, lsmax = p.g.lsmax, hsz = p.nit * lsmax;
-    int row = 0, sa = 0, sb = 0;  // species of the row of element k
-    for (int k = threadIdx.x; k < hsz; k += blockDim.x) {
-        while (row < k / lsmax) {
-            ++row;
-            if (++sb == nsp) sb = ++sa;
-        }
-        const int bin = k - row * lsmax + 1;
-        u64 s;
-        if (SQUARE) {
-            s = hist[(sa * nsp + sb) * rw + bin];
-            if (sa != sb) s += hist[(sb * nsp + sa) * rw + bin];
-        } else {
-            s = hist[row * rw + bin];
-        }
-        if (s) atomicAdd(&hist_g[k], s);
-        pc.counted += s;
     }
 }
 
@@ -705,6 +732,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
         for (int k = tid; k < nsp * nsp; k += blockDim.x)
             rowtab[(k / nsp) * 16 + k % nsp] =
                 hist_base + (unsigned)(trj_pair_row(k / nsp, k % nsp, nsp) * rw * 4) - 4u * kBinBias;
+    if (lane == 0) ws->blocks = 0;
     if (tid == 0) {
         trj_mbar_init(&never, 1);
         trj_fence_mbar_init();
@@ -730,9 +758,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
         pair_item<FLOOR, QMODE, SQUARE, EDGE, QMODE ? 1 : 2>(p, (int)item, rounds, sorted, fstart, fcount, cflag,
                                                              frame_ok, sorted_q, ring, ring_q, ws, hist_base,
                                                              trj_smem_addr(rowtab), qhist, pc, n_tested);
+        merge_early<SQUARE>(ws, nsp, p.nit, g.lsmax, hist, hist_g, EDGE ? edge_g : nullptr);
     }
     __syncthreads();
-    merge_rows<SQUARE>(p, hist, hist_g, pc);
+    pc.counted += merge_rows<SQUARE, false>(nsp, p.nit, g.lsmax, hist, hist_g, tid, (int)blockDim.x);
     if (QMODE) {
         for (int k = tid; k < g.lsmax; k += blockDim.x) {
             const double s = qhist[k + 1];
@@ -1248,6 +1277,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
     unsigned* hist = reinterpret_cast<unsigned*>(smem + (size_t)(kBatchThreads / 32) * kWarpBytes);
     const unsigned hist_base = trj_smem_addr(hist), rowtab_base = trj_smem_addr(rowtab);
     for (int k = tid; k < batch_hist_smem_words(hist_words); k += kBatchThreads) hist[k] = 0u;
+    if (lane == 0) ws->blocks = 0;
     const int nitems = hdr->nitems;
     if (nitems == 0) return;
     // CTAs start spread over the turn's work; each then moves on cyclically to frames with items left
@@ -1299,10 +1329,12 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
             else if (p.g.want_edge) TRJ_ITEM(false, true, true);
             else TRJ_ITEM(false, true, false);
 #undef TRJ_ITEM
+            if (square) merge_early<true>(ws, p.g.nsp, p.nit, p.g.lsmax, hist, it.hist, it.edge);
+            else merge_early<false>(ws, p.g.nsp, p.nit, p.g.lsmax, hist, it.hist, it.edge);
         }
         __syncthreads();
-        if (square) merge_rows<true>(p, hist, it.hist, pc);
-        else merge_rows<false>(p, hist, it.hist, pc);
+        pc.counted += square ? merge_rows<true, false>(p.g.nsp, p.nit, p.g.lsmax, hist, it.hist, tid, kBatchThreads)
+                             : merge_rows<false, false>(p.g.nsp, p.nit, p.g.lsmax, hist, it.hist, tid, kBatchThreads);
         if (it.edge) add_edges(it.edge, pc, n_tested);
         __syncthreads();
         const int rows = square ? p.g.nsp * p.g.nsp : p.nit;
