@@ -63,10 +63,19 @@ extern "C" int trj_ctx_create(int device, trj_ctx** out) {
         delete ctx;
         return TRJ_ERR_NOMEM;
     }
-    cudaMemset(ctx->status_dev, 0, 8 * sizeof(unsigned));
     ctx->turn_dev = reinterpret_cast<float2*>(ctx->status_dev + 8);
-    turn_table_kernel<<<1, 256>>>(ctx->turn_dev);
-    cudaDeviceSynchronize();
+    cudaError_t e = cudaMemset(ctx->status_dev, 0, 8 * sizeof(unsigned));
+    if (e == cudaSuccess) {
+        turn_table_kernel<<<1, 256>>>(ctx->turn_dev);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) {  // every direct sum reads the table
+        cudaFree(ctx->status_dev);
+        cudaFreeHost(ctx->status_host);
+        delete ctx;
+        return TRJ_ERR_CUDA;
+    }
     *out = ctx;
     return TRJ_OK;
 }
