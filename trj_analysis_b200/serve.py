@@ -4,7 +4,7 @@ A request is a short trajectory (1..F frames of one system) with its own g(r) an
 parameters.  The loop:
 
 * admits queued requests when a slot (CUDA stream + pinned staging) is free and the
-  request's device footprint fits the HBM budget still unused by running requests;
+  request's plans fit the HBM budget still unused by running requests;
 * creates the request's plans with the library's device memory drawn from PyTorch's
   caching allocator (``trj_ctx_set_allocator``), so plan set-up and tear-down never
   synchronise the device while other requests run;
@@ -208,6 +208,11 @@ class _Job:
         self.cancelled = False
         self.fused = False
 
+    def held_bytes(self) -> int:
+        """Device memory of the job's plans and outputs."""
+        return (self.rdf.scratch_bytes + self.sq.scratch_bytes + self.hist.numel() * self.hist.element_size()
+                + self.out.numel() * self.out.element_size())
+
 
 class Server:
     def __init__(self, device: int = 0, slots: int = 8, hbm_budget: Optional[int] = None, n_max: int = 1 << 18,
@@ -227,6 +232,7 @@ class Server:
         self.in_use = 0
         self.peak_in_use = 0
         self.admission_waits = 0
+        self._sizes: Dict[tuple, int] = {}  # of requests sent back to the queue
         self.cancelled: List[int] = []
         self._cancel: set = set()
         self._cancel_lock = threading.Lock()
@@ -283,13 +289,46 @@ class Server:
             job.slot.req = None
 
     # ---- footprint / admission ---------------------------------------------------------
+    # A request is admitted on a first guess of its size or, once its plans have been too large for the budget, on
+    # what they hold; what counts against the budget is always what the plans hold.
     def footprint(self, req: Request, ks: refsem.KSet, method: str) -> int:
+        """First guess, without the launch shape of the direct sum and the tensor path's tables."""
         n, nsp, nv = req.n, req.nsp, ks.nvec
         rdf = 64 * n + 3 * 4 * 4096
         sq = 16 * n + 16 * nsp * nv * 9 + 16 * nsp * nv + 24 * nv
         if method == "split":
             sq += 2 * (2 * 64) * 2 * (n + 32 * nsp) + 2 * 8 * 128 * (n + 32 * nsp) + 8 * nsp * nv * 4
         return int(rdf + sq)
+
+    @staticmethod
+    def _size_key(req: Request, counts: np.ndarray, cols: int, fused: bool) -> tuple:
+        return (tuple(int(c) for c in counts), tuple(float(v) for v in req.frames[0].box), req.deltar, req.rcrdf,
+                req.kset, req.qmax, req.qmin, cols, fused)
+
+    def _fits(self, nbytes: int) -> bool:
+        if self.in_use + nbytes > self.hbm_budget and self.in_use > 0:
+            self.admission_waits += 1
+            return False
+        return True
+
+    def _account(self, job: _Job) -> None:
+        """Counts what the job's plans and outputs hold against the budget."""
+        self.in_use -= job.footprint
+        job.footprint = job.held_bytes()
+        self.in_use += job.footprint
+        self.peak_in_use = max(self.peak_in_use, self.in_use)
+
+    def _keep(self, job: _Job, key: tuple) -> bool:
+        """Whether the job's plans fit beside the others'; if not they are given back and their size remembered
+        until the request is admitted."""
+        if not self._fits(job.held_bytes()):
+            self._sizes[key] = job.held_bytes()
+            job.rdf.close()
+            job.sq.close()
+            return False
+        self._sizes.pop(key, None)
+        self._account(job)
+        return True
 
     # ---- fused launches -------------------------------------------------------------------
     def _fusable(self, req: Request) -> bool:
@@ -314,9 +353,8 @@ class Server:
         bsc = list(req.bsc) if req.bsc is not None else [1.0] * req.nsp
         ks = refsem.make_kset(req.kset, fr0.box, req.qmax, req.qmin)
         counts = np.bincount(sp[sp >= 0], minlength=req.nsp)
-        fp = self.footprint(req, ks, "plain") - 64 * req.n  # no cell arrays
-        if self.in_use + fp > self.hbm_budget and self.in_use > 0:
-            self.admission_waits += 1
+        key = self._size_key(req, counts, 0, True)
+        if not self._fits(self._sizes.get(key, self.footprint(req, ks, "plain") - 64 * req.n)):  # no cell arrays
             return None
         job = _Job(req, None)
         job.fused = True
@@ -333,9 +371,8 @@ class Server:
         job.method = "plain"
         job.cols = 0
         job.tune = False
-        job.footprint = fp
-        self.in_use += fp
-        self.peak_in_use = max(self.peak_in_use, self.in_use)
+        if not self._keep(job, key):
+            return None
         self.fused_requests += 1
         return job
 
@@ -390,9 +427,8 @@ class Server:
         tuned = self.tuner.lookup(req.n, req.nsp, req.kset)
         method = req.method or self.method or (tuned[0] if tuned else "split")
         cols = tuned[1] if (tuned and req.method is None and self.method is None) else 0
-        fp = self.footprint(req, ks, method)
-        if self.in_use + fp > self.hbm_budget and self.in_use > 0:
-            self.admission_waits += 1
+        key = self._size_key(req, counts, cols, False)
+        if not self._fits(self._sizes.get(key, self.footprint(req, ks, method))):
             return None
         job = _Job(req, slot)
         job.species = sp
@@ -411,9 +447,8 @@ class Server:
         job.method = method
         job.cols = cols
         job.tune = req.method is None and self.method is None and tuned is None
-        job.footprint = fp
-        self.in_use += fp
-        self.peak_in_use = max(self.peak_in_use, self.in_use)
+        if not self._keep(job, key):
+            return None
         slot.req = req
         return job
 
@@ -454,6 +489,7 @@ class Server:
                     finally:
                         self.ctx.set_sq_tile_cols(0)
                     job.cols = cols
+                    self._account(job)
             graphed = self.use_graphs and len(req.frames) >= 4
             if graphed and k >= 1 and job.graphs[buf] is None:
                 # capture this frame's launch sequence (no device synchronisation: other requests keep
@@ -565,6 +601,7 @@ class Server:
                     time.sleep(max(0.0, min(0.002, pending[0].arrival - (time.perf_counter() - t0))))
         self.ctx.check()
         self._fuse_cache.clear()
+        self._sizes.clear()
         return results
 
 
