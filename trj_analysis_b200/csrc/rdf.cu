@@ -1557,6 +1557,8 @@ static void set_segments(RdfParams& P, int64_t nseg, int64_t nkey, int64_t n) {
     P.nitems = (unsigned)(rounds * P.nseg);
 }
 
+constexpr size_t kPairStatic = 1200;  // more than the pair kernel's static shared memory
+
 struct PairShape {
     int ctas, warps;  // per SM, per CTA
     bool square;      // a bin row per ordered species pair
@@ -1576,7 +1578,7 @@ static bool pair_shape(const trj_ctx* ctx, int nsp, int nit, int row_words, bool
             const size_t smem = (size_t)kWarps[i] * (kWarpBytes + (charged ? 8 * kRing : 0)) +
                                 (size_t)row_words * (4 * rows + (charged ? 8 : 0)) + 16;
             // the driver's reserve and the static shared memory of a CTA
-            if (smem + 1200 > optin || (smem + 1024 + 1200) * kCtas[i] > per_sm) continue;
+            if (smem + kPairStatic > optin || (smem + 1024 + kPairStatic) * kCtas[i] > per_sm) continue;
             out->ctas = kCtas[i];
             out->warps = kWarps[i];
             out->square = square;
@@ -1791,7 +1793,10 @@ static int rdf_accumulate_impl(trj_rdf_plan* plan, const float* packed_dev, cons
     set_segments(P, std::min<int64_t>((12 * warps + nkey - 1) / nkey, P.list / 2), nkey, n);
 
     const PairKernel kern = pair_kernel(plan->floor_bins, charged, shape.square, edge_dev != nullptr);
-    TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shape.smem));
+    // the most pair_shape gives any plan: a limit of this call's own could be lowered by another thread's before the
+    // launch
+    TRJ_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(ctx->smem_optin - kPairStatic)));
 
     // Cell binning: count, group offsets, scatter.
     unsigned* work = reinterpret_cast<unsigned*>(plan->zeroed);
