@@ -739,7 +739,6 @@ def run_fused(args):
     ctx.check()
     n = np.array([e["r"].n for e in st], np.float64)
     nvec = np.array([e["ks"].nvec for e in st], np.float64)
-    pairs = float((n * (n - 1) / 2).sum())
     terms = float((n * nvec).sum())
     f_ms, u_ms = statistics.median(fus), statistics.median(unf)
     return {"metric": "fused turn: frame 0 of 64 small requests (g(r) + plain S(Q))", "value": 64.0 / (f_ms * 1e-3),
@@ -747,8 +746,7 @@ def run_fused(args):
             "higher_is_better": True, "dtype": "f32 terms, f64 sums", "data": "synthetic",
             "config": {"workload": "64 serving requests, N log-uniform [1e3, 16384]", "atoms": int(n.sum()),
                        "kvec": int(nvec.sum()), "l2": "256 MB buffer written between steps"},
-            "fused": {"ms": f_ms, "launches": 8, "copies": 1, "pair_tests_per_s": pairs / (f_ms * 1e-3),
-                      "sq_terms_per_s": terms / (f_ms * 1e-3)},
+            "fused": {"ms": f_ms, "launches": 8, "copies": 1, "sq_terms_per_s": terms / (f_ms * 1e-3)},
             "per_request": {"ms": u_ms, "launches": unfused_launches, "frames_per_s": 64.0 / (u_ms * 1e-3)},
             "fused_vs_per_request": u_ms / f_ms, "launches_before_timing": int(launches0)}
 

@@ -352,7 +352,7 @@ TRJ_API int trj_dyn_plan_destroy(trj_dyn_plan* plan);
  * executes.  Counts are those of trj_rdf_accumulate and S(Q) sums those of
  * trj_sq_accumulate(TRJ_SQ_PLAIN_FP32) for the same plans, bit for bit.
  * max_atoms: staged atoms per turn; hist_words: the largest nit*lsmax of a
- * pair plan the batch takes (shared memory: 8 bytes per word + 20 KB). */
+ * pair plan the batch takes (shared memory: 8 bytes per word + 26 KB). */
 TRJ_API int trj_batch_create(trj_ctx* ctx, int max_items, int64_t max_atoms, int hist_words, trj_batch** out);
 /* Host staging of buffer buf: xyz[3 * max_atoms] float and species[max_atoms]
  * int32 (0-based species ids), pinned and mapped into the device's address

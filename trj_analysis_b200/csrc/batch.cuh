@@ -15,7 +15,7 @@ constexpr int kBatchChunk = 1024;        // atoms per layout unit
 constexpr int kBatchThreads = 256;
 constexpr int kBatchMaxSpecies = 16;
 constexpr int kBatchMaxHistWords = 24576;  // largest pair histogram of a batch
-constexpr int kBatchCounters = 4;        // dynamic work counters: pairs, direct sum, reduction, spare
+constexpr int kBatchCounters = 2;        // dynamic work counters: direct sum, reduction
 
 struct __align__(16) BatchItem {
     // frame: atoms [atom_off, atom_off + n) of the staging and device arrays

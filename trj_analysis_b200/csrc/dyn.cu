@@ -37,33 +37,6 @@ constexpr int kDynSub = 64;       // FP32 run length before the FP64 add
 constexpr int kDynCtas = 4;       // blocks of 256 threads per SM the launch shapes count on
 constexpr float kTwoPiOver2_32 = 1.4629180792671596e-09f;
 
-typedef unsigned long long u64;
-
-// Packed FP32: two independent IEEE operations per instruction, each rounded to nearest once.
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-    u64 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
-    u64 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ u64 pack2(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
 // Vectors in launch order: a thread's kDynVPT vectors are consecutive slots.  Slots hold the components with
 // axis `axis` first; shared: the vectors of a thread have that component in common, so its product is formed
 // once per atom.

@@ -23,7 +23,6 @@
 #include <math.h>
 
 #include <algorithm>
-#include <vector>
 
 #include "batch.cuh"
 #include "pairs.cuh"
@@ -37,8 +36,6 @@ constexpr int kRing = 128;            // surviving neighbours buffered per warp 
 constexpr int kRingRun = 64;          // survivors tested per run
 constexpr int kMaxWarps = 32;         // per SM: 64 registers a thread (24 warps of 80 registers: 4 % slower at 1e6 atoms)
 
-typedef unsigned long long u64;
-
 // A frame's words of work state (in a fused turn: an item's): work counter, frame flags, then one 64-bit sum of the
 // atoms placed (low half) and the rounds of homes (high half).
 enum { kWorkNext = 0, kWorkFlags = 1, kWorkAtoms = 2, kWorkRounds = 3, kWorkWords = 4 };
@@ -51,30 +48,6 @@ __device__ __forceinline__ int fast_div(int n, const FastDiv& f) {
     return f.d == 1u ? n : (int)(__umulhi((unsigned)n, f.mul) >> f.shift);
 }
 
-// ---- packed FP32 (two independent IEEE operations per instruction, each rounded to nearest once) ----
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-    u64 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
-    u64 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ u64 pack2(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
 __device__ __forceinline__ float fast_sqrt(float x) {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -1039,7 +1012,9 @@ __global__ void one_charge_kernel(const float* __restrict__ q, double* __restric
 // What bounds it: latency of the groups' starts and atoms.  A lane looks at a group of the point's cells (a warp
 // at every eighth, so that the warps have equal shares) and drops it where its box is out of reach; the warp then
 // has an atom of four groups per lane in flight, and groups of more than 128 atoms (frames of uneven density) go
-// to the whole block.  The cumulative counts are a block scan.
+// to the whole block.  The cumulative counts are a block scan.  4,096 points, every group of the cells read and eight
+// consecutive ones to a warp against this: 1e6 atoms (cutoff 8) 0.268 and 0.122 ms, 62,500 atoms 0.334 and 0.131, a
+// ball of them in a box of 400 0.432 and 0.077.
 constexpr int kS2nThreads = 256, kS2nFlight = 4, kS2nLarge = 128, kS2nList = 64;
 __global__ void __launch_bounds__(kS2nThreads, 5)
     s2n_kernel(const float4* __restrict__ sorted, const int32_t* __restrict__ fstart,
@@ -1349,7 +1324,7 @@ struct trj_rdf_plan {
     trj_ctx* ctx = nullptr;
     int nsp = 0, nit = 0, lsmax = 0;
     int floor_bins = 0;
-    long long wait_clocks = TRJ_WAIT_CLOCKS;  // limit of the pair kernel's waits for staged chunks
+    long long wait_clocks = TRJ_WAIT_CLOCKS;  // limit of the stall test's wait
     int stall_test = 0;
     int dim = 3;                // 2: frames in the xy plane (z = 0); z is neither clipped nor split
     float deltar = 0.f, rcrdf_eff = 0.f, side2 = 0.f;

@@ -31,33 +31,6 @@ constexpr int kPlainStage = 512;       // atoms staged per pass, at most
 constexpr int kPlainCtas = 4;          // direct-sum blocks of 256 threads per SM
 constexpr int kTurnCopies = 16;        // copies of the turn table in shared memory, one per lane of a half-warp
 
-typedef unsigned long long u64;
-
-// Packed FP32: two independent IEEE operations per instruction, each rounded to nearest once.
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-    u64 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
-    u64 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ u64 pack2(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(u64 v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
 // Fixed-point phase coordinates of every atom.  With charges (q non-null) every atom is written a
 // second time at n + i as a member of the charge species qsp, its charge (FP32 bits) in place of the
 // species index: rho_q(k) = sum_j q_j exp(i k.r_j) (sq.cuf:569-573) is then the sum of that species.
@@ -373,7 +346,7 @@ __global__ void __launch_bounds__(kPlainThreads, 2) batch_sq_kernel(BatchHeader*
     const int nitems = hdr->nitems;
     const int64_t total = hdr->total_sq;
     while (true) {
-        if (threadIdx.x == 0) unit_s = (long long)atomicAdd(&hdr->counter[1], 1ull);
+        if (threadIdx.x == 0) unit_s = (long long)atomicAdd(&hdr->counter[0], 1ull);
         __syncthreads();
         const int64_t u = unit_s;
         __syncthreads();
@@ -398,7 +371,7 @@ __global__ void __launch_bounds__(256, 4) batch_reduce_kernel(BatchHeader* __res
     const int nitems = hdr->nitems;
     const int64_t total = hdr->total_red;
     while (true) {
-        if (threadIdx.x == 0) unit_s = (long long)atomicAdd(&hdr->counter[2], 1ull);
+        if (threadIdx.x == 0) unit_s = (long long)atomicAdd(&hdr->counter[1], 1ull);
         __syncthreads();
         const int64_t u = unit_s;
         __syncthreads();
