@@ -180,7 +180,7 @@ struct WarpState {
     int4 walk;                  // j, je, m, e0 of the neighbour walk
     int4 outer;                 // position in the neighbour list, cell of the homes and its flags, first home
     int nh;
-    int blocks;                 // blocks tested since the warp last merged the CTA's rows
+    unsigned since;             // clock when the CTA's rows were last merged
 };
 
 constexpr size_t kWarpBytes = 16 * kRing + (sizeof(WarpState) + 15) / 16 * 16;  // buffer and state of a warp
@@ -369,53 +369,6 @@ __device__ __forceinline__ void axis_box(unsigned lo, unsigned hi, float pad, fl
 // reaches 0.749 L (frames centred on the origin).  (Coordinates outside [-L, L) are flagged per cell.)
 __device__ __forceinline__ bool frame_within(unsigned f) {
     return !(f & kFrameLow) || !(f & (kFrameVeryLow | kFrameHigh));
-}
-
-// The CTA's rows into the frame's uint64 histogram, elements first, first + step, ...; returns their total, the
-// counted pairs.  EARLY: taken out while other warps count on.  A count is then a signed number: a pair that another
-// warp has just counted in its approximate bin and is about to move may be taken out of that bin before it moves.
-template <bool SQUARE, bool EARLY>
-__device__ __forceinline__ u64 merge_rows(int nsp, int nit, int lsmax, unsigned* hist, u64* __restrict__ hist_g, int first,
-                                          int step) {
-    const int rw = lsmax + 2, hsz = nit * lsmax;
-    auto take = [&](unsigned* c) { return (long long)(int)(EARLY ? atomicExch(c, 0u) : *c); };
-    u64 total = 0;
-    int row = 0, sa = 0, sb = 0;  // species of the row of element k
-#pragma unroll 1
-    for (int k = first; k < hsz; k += step) {
-        while (row < k / lsmax) {
-            ++row;
-            if (++sb == nsp) sb = ++sa;
-        }
-        const int bin = k - row * lsmax + 1;
-        long long s;
-        if (SQUARE) {
-            s = take(&hist[(sa * nsp + sb) * rw + bin]);
-            if (sa != sb) s += take(&hist[(sb * nsp + sa) * rw + bin]);
-        } else {
-            s = take(&hist[row * rw + bin]);
-        }
-        if (s) atomicAdd(&hist_g[k], (u64)s);
-        total += (u64)s;
-    }
-    return total;
-}
-
-// Rows hold 32 bits per bin.  A warp that has tested 2^22 pairs since it last did so moves the CTA's rows to the
-// frame's histogram after its item.  A bin then holds less than 2^31 as long as no item meets 8e6 atoms at one distance
-// (eight warps per CTA; 2e6 with the 32 of CTAs that share a histogram of many bins).  Without it a CTA of a frame of
-// 1e7 atoms puts 4e9 pairs into a coarse bin at half the box.
-constexpr int kMergeBlocks = (1 << 22) / (4 * kGroup);
-template <bool SQUARE>
-__device__ __forceinline__ void merge_early(WarpState* ws, int nsp, int nit, int lsmax, unsigned* hist, u64* hist_g,
-                                            u64* edge_g) {
-    if (ws->blocks < kMergeBlocks) return;
-    const int lane = (int)(threadIdx.x & 31u);
-    const u64 counted = merge_rows<SQUARE, true>(nsp, nit, lsmax, hist, hist_g, lane, 32);
-    if (edge_g) atomicAdd(&edge_g[TRJ_EDGE_COUNTED], counted);
-    __syncwarp();
-    if (lane == 0) ws->blocks = 0;
-    __syncwarp();
 }
 
 // One work item of a frame: round item / nseg (up to 32 atoms of one group, see emit_rounds) against segment
@@ -622,10 +575,7 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const in
                 if (EDGE && lane < ws->nh) n_tested += (unsigned)(tail - before);
             }
             const int n4 = tail - head >= kRingRun ? kRingRun / 4 : pad();
-            if (lane == 0) {
-                ws->walk = make_int4(j, je, (int)m, e0);
-                ws->blocks += n4;
-            }
+            if (lane == 0) ws->walk = make_int4(j, je, (int)m, e0);
             __syncwarp();  // the other lanes' entries
             if (mode == kImgNone) TRJ_RUN(kImgNone, false, n4);
             else if (mode == kImgShift) TRJ_RUN(kImgShift, false, n4);
@@ -646,6 +596,36 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const in
     }
 }
 
+// The CTA's rows into the frame's uint64 histogram (their total is the counted pairs); they are cleared.
+template <bool SQUARE>
+__device__ __forceinline__ void merge_rows(const RdfParams& p, unsigned* hist, u64* __restrict__ hist_g,
+                                           PairCounters& pc) {
+    const int nsp = p.g.nsp, rw = p.g.row_words, lsmax = p.g.lsmax, hsz = p.nit * lsmax;
+    auto take = [&](int row, int bin) {
+        const u64 c = hist[row * rw + bin];
+        hist[row * rw + bin] = 0u;
+        return c;
+    };
+    int row = 0, sa = 0, sb = 0;  // species of the row of element k
+#pragma unroll 1
+    for (int k = threadIdx.x; k < hsz; k += blockDim.x) {
+        while (row < k / lsmax) {
+            ++row;
+            if (++sb == nsp) sb = ++sa;
+        }
+        const int bin = k - row * lsmax + 1;
+        u64 s;
+        if (SQUARE) {
+            s = take(sa * nsp + sb, bin);
+            if (sa != sb) s += take(sb * nsp + sa, bin);
+        } else {
+            s = take(row, bin);
+        }
+        if (s) atomicAdd(&hist_g[k], s);
+        pc.counted += s;
+    }
+}
+
 __device__ __forceinline__ void add_edges(u64* __restrict__ edge_g, const PairCounters& pc, u64 n_tested) {
     u64 n_ulp = pc.ulp, n_fma = pc.fma, n_counted = pc.counted;
     for (int off = 16; off > 0; off >>= 1) {
@@ -660,6 +640,22 @@ __device__ __forceinline__ void add_edges(u64* __restrict__ edge_g, const PairCo
         if (n_counted) atomicAdd(&edge_g[TRJ_EDGE_COUNTED], n_counted);
         if (n_tested) atomicAdd(&edge_g[TRJ_EDGE_TESTED], n_tested);
     }
+}
+
+// Rows hold 32 bits per bin.  2^26 clocks (35 ms) after its CTA last merged its rows a warp takes no further item, and
+// once the CTA's other warps have come to that point (or to the end) the rows are merged and cleared.  An SM tests
+// about eight pairs per clock, so that a bin stays below 2^32 as long as no item meets 1e7 atoms at one distance (eight
+// warps per CTA; 3e6 with the 32 of CTAs that share a histogram of many bins).  Without it a CTA of a frame of 1e7
+// atoms puts 4e9 pairs into a coarse bin at half the box.  It costs 1 % without and nothing with edge statistics (2.45
+// -> 2.475 and 2.88 -> 2.875 ms at 1e6 atoms); the test loop's registers are tight: counting the tests instead, or
+// merging by single warps, 2.55 and 3.04 to 3.19.
+constexpr unsigned kMergeClocks = 1u << 26;
+
+// The next work item, for a whole warp; past every item also when the rows are due to be merged.
+__device__ __forceinline__ unsigned next_item(unsigned* next, const WarpState* ws) {
+    unsigned item = 0xffffffffu;
+    if ((threadIdx.x & 31u) == 0u && (unsigned)clock() - ws->since < kMergeClocks) item = atomicAdd(next, 1u);
+    return __shfl_sync(0xffffffffu, item, 0);
 }
 
 // Work item = (round of homes, segment of their group's neighbour list), taken from a global counter by one warp at
@@ -705,7 +701,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
         for (int k = tid; k < nsp * nsp; k += blockDim.x)
             rowtab[(k / nsp) * 16 + k % nsp] =
                 hist_base + (unsigned)(trj_pair_row(k / nsp, k % nsp, nsp) * rw * 4) - 4u * kBinBias;
-    if (lane == 0) ws->blocks = 0;
+    if (lane == 0) ws->since = (unsigned)clock();
     if (tid == 0) {
         trj_mbar_init(&never, 1);
         trj_fence_mbar_init();
@@ -721,27 +717,32 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 
     const bool frame_ok = frame_within(work[kWorkFlags]);
     const unsigned nitems = work[kWorkRounds] * (unsigned)p.nseg;
-    PairCounters pc;
-    u64 n_tested = 0;
-    for (;;) {
-        unsigned item = 0;
-        if (lane == 0) item = atomicAdd(work, 1u);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= nitems) break;
-        pair_item<FLOOR, QMODE, SQUARE, EDGE, QMODE ? 1 : 2>(p, (int)item, rounds, sorted, fstart, fcount, cflag,
-                                                             frame_ok, sorted_q, ring, ring_q, ws, hist_base,
-                                                             trj_smem_addr(rowtab), qhist, pc, n_tested);
-        merge_early<SQUARE>(ws, nsp, p.nit, g.lsmax, hist, hist_g, EDGE ? edge_g : nullptr);
+#pragma unroll 1
+    for (bool more = true; more;) {
+        PairCounters pc;
+        u64 n_tested = 0;
+        for (;;) {
+            const unsigned item = next_item(work, ws);
+            if (item >= nitems) {
+                more = item == 0xffffffffu;
+                break;
+            }
+            pair_item<FLOOR, QMODE, SQUARE, EDGE, QMODE ? 1 : 2>(p, (int)item, rounds, sorted, fstart, fcount, cflag,
+                                                                 frame_ok, sorted_q, ring, ring_q, ws, hist_base,
+                                                                 trj_smem_addr(rowtab), qhist, pc, n_tested);
+        }
+        more = __syncthreads_or(more);
+        merge_rows<SQUARE>(p, hist, hist_g, pc);
+        if (edge_g) add_edges(edge_g, pc, n_tested);
+        if (lane == 0) ws->since = (unsigned)clock();
+        __syncthreads();
     }
-    __syncthreads();
-    pc.counted += merge_rows<SQUARE, false>(nsp, p.nit, g.lsmax, hist, hist_g, tid, (int)blockDim.x);
     if (QMODE) {
         for (int k = tid; k < g.lsmax; k += blockDim.x) {
             const double s = qhist[k + 1];
             if (s != 0.0) atomicAdd(&gqq_frame[k], s);
         }
     }
-    if (edge_g) add_edges(edge_g, pc, n_tested);
 }
 
 // Group of a folded coordinate along one axis: cell, then box within the cell (NaN: the first ones).
@@ -1252,7 +1253,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
     unsigned* hist = reinterpret_cast<unsigned*>(smem + (size_t)(kBatchThreads / 32) * kWarpBytes);
     const unsigned hist_base = trj_smem_addr(hist), rowtab_base = trj_smem_addr(rowtab);
     for (int k = tid; k < batch_hist_smem_words(hist_words); k += kBatchThreads) hist[k] = 0u;
-    if (lane == 0) ws->blocks = 0;
+    if (lane == 0) ws->since = (unsigned)clock();
     const int nitems = hdr->nitems;
     if (nitems == 0) return;
     // CTAs start spread over the turn's work; each then moves on cyclically to frames with items left
@@ -1292,9 +1293,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
         const int32_t *fstart = st.fstart + it.key_begin, *fcount = st.fcount + it.key_begin,
                       *cflag = st.cflag + it.key_begin;
         for (;;) {
-            unsigned item = 0;
-            if (lane == 0) item = atomicAdd(&st.state[kWorkWords * r + kWorkNext], 1u);
-            item = __shfl_sync(0xffffffffu, item, 0);
+            const unsigned item = next_item(&st.state[kWorkWords * r + kWorkNext], ws);
             if (item >= nwork) break;
 #define TRJ_ITEM(F, S, E)                                                                                       \
     pair_item<F, false, S, E, 1>(p, (int)item, rounds, sorted, fstart, fcount, cflag, frame_ok, nullptr, ring, nullptr, \
@@ -1304,16 +1303,16 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
             else if (p.g.want_edge) TRJ_ITEM(false, true, true);
             else TRJ_ITEM(false, true, false);
 #undef TRJ_ITEM
-            if (square) merge_early<true>(ws, p.g.nsp, p.nit, p.g.lsmax, hist, it.hist, it.edge);
-            else merge_early<false>(ws, p.g.nsp, p.nit, p.g.lsmax, hist, it.hist, it.edge);
         }
         __syncthreads();
-        pc.counted += square ? merge_rows<true, false>(p.g.nsp, p.nit, p.g.lsmax, hist, it.hist, tid, kBatchThreads)
-                             : merge_rows<false, false>(p.g.nsp, p.nit, p.g.lsmax, hist, it.hist, tid, kBatchThreads);
+        if (square) merge_rows<true>(p, hist, it.hist, pc);
+        else merge_rows<false>(p, hist, it.hist, pc);
         if (it.edge) add_edges(it.edge, pc, n_tested);
         __syncthreads();
+        // the words before and after a row's bins as well: the next frame's rows lie elsewhere
         const int rows = square ? p.g.nsp * p.g.nsp : p.nit;
         for (int q = tid; q < rows * p.g.row_words; q += kBatchThreads) hist[q] = 0u;
+        if (lane == 0) ws->since = (unsigned)clock();
         r = r + 1 < nitems ? r + 1 : 0;
     }
 }
