@@ -80,7 +80,7 @@ extern "C" int trj_batch_create(trj_ctx* ctx, int max_items, int64_t max_atoms, 
         const size_t dev = a256(b->table_bytes) + 3 * a256(sizeof(float4) * (size_t)max_atoms) +
                            a256(sizeof(int32_t) * kBatchMaxSpecies * (size_t)B.chunk_cap) + a256(B.zero_bytes) +
                            a256(sizeof(int32_t) * (size_t)B.key_cap) + 2 * a256(sizeof(int32_t) * (size_t)max_atoms) +
-                           a256(sizeof(int2) * (size_t)(B.key_cap + max_atoms / 32 + 1));
+                           a256(sizeof(int4) * (size_t)(B.key_cap + max_atoms / 32 + 1));
         if (cudaHostAlloc((void**)&B.table_host, b->table_bytes, cudaHostAllocDefault) != cudaSuccess ||
             cudaHostAlloc((void**)&B.xyz_host, sizeof(float) * 3 * (size_t)max_atoms,
                           cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
@@ -117,7 +117,7 @@ extern "C" int trj_batch_create(trj_ctx* ctx, int max_items, int64_t max_atoms, 
         p += a256(sizeof(int32_t) * (size_t)max_atoms);
         B.sort.aslot = reinterpret_cast<int32_t*>(p);
         p += a256(sizeof(int32_t) * (size_t)max_atoms);
-        B.sort.rounds = reinterpret_cast<int2*>(p);
+        B.sort.rounds = reinterpret_cast<int4*>(p);
         B.sort.sorted = B.raw;  // the staged atoms are read for the last time by the layout
         b->device_bytes += (int64_t)dev;
         memset(B.table_host, 0, b->table_bytes);

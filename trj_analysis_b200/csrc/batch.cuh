@@ -77,7 +77,7 @@ __device__ __forceinline__ int batch_item_of(const BatchItem* __restrict__ items
 struct BatchSort {
     unsigned* state;
     int32_t *fcount, *cflag, *fstart;    // per group (cflag: per cell), an item's at its key_begin
-    int2* rounds;                        // per round of homes, an item's at batch_rounds_begin
+    int4* rounds;                        // per round of homes, an item's at batch_rounds_begin
     int32_t *akey, *aslot;               // per atom
     float4* sorted;                      // per atom: an item's atoms by group
 };

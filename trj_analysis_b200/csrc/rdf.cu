@@ -375,7 +375,7 @@ __device__ __forceinline__ bool frame_within(unsigned f) {
 // item % nseg of its group's neighbour list.  hist: shared-memory address of the bin rows (SQUARE), rowtab: of the
 // row table (otherwise).
 template <bool FLOOR, bool QMODE, bool SQUARE, bool EDGE, int UNROLL>
-__device__ __forceinline__ void pair_item(const RdfParams& p, int item, const int2* __restrict__ rounds,
+__device__ __forceinline__ void pair_item(const RdfParams& p, int item, const int4* __restrict__ rounds,
                                           const float4* __restrict__ sorted,
                                           const int32_t* __restrict__ fstart, const int32_t* __restrict__ fcount,
                                           const int32_t* __restrict__ cflag, bool frame_ok,
@@ -386,8 +386,17 @@ __device__ __forceinline__ void pair_item(const RdfParams& p, int item, const in
     const int lane = (int)(threadIdx.x & 31u);
     const unsigned lt = (1u << lane) - 1u;
     const int round = fast_div(item, p.div_nseg), seg = item - round * p.nseg;
-    const int key = rounds[round].x, h0 = rounds[round].y;
-    const int hbeg = fstart[key], hend = hbeg + fcount[key];
+    // one 16-byte load wants four neighbouring registers, which the uncharged loops do not have (2.54 ms at 1e6 atoms
+    // against 2.47); the charged ones gain from it (255,000 ions, cutoff 3.5: 394 -> 390 us)
+    int4 rd;
+    if constexpr (QMODE) {
+        rd = rounds[round];
+    } else {
+        const int2* r2 = reinterpret_cast<const int2*>(rounds + round);
+        const int2 lo = r2[0], hi = r2[1];
+        rd = make_int4(lo.x, lo.y, hi.x, hi.y);
+    }
+    const int key = rd.x, h0 = rd.y, hbeg = rd.z, hend = rd.w;
     const int c = fast_div(key, p.div_nsub), own = key - c * p.nsub;
     const int cxy = fast_div(c, p.div_nc2), cz = c - cxy * p.nc[2];
     const int cx = fast_div(cxy, p.div_nc1), cy = cxy - cx * p.nc[1];
@@ -676,7 +685,7 @@ template <bool FLOOR, bool QMODE, bool SQUARE, bool EDGE>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     rdf_pairs_kernel(const __grid_constant__ RdfParams p, const float4* __restrict__ sorted,
                      const int32_t* __restrict__ fstart, const int32_t* __restrict__ fcount,
-                     const int32_t* __restrict__ cflag, const int2* __restrict__ rounds, unsigned* __restrict__ work,
+                     const int32_t* __restrict__ cflag, const int4* __restrict__ rounds, unsigned* __restrict__ work,
                      u64* __restrict__ hist_g, u64* __restrict__ edge_g, unsigned* __restrict__ status,
                      const float* __restrict__ sorted_q, double* __restrict__ gqq_frame) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -819,13 +828,13 @@ __device__ __forceinline__ u64 warp_scan(u64 x, int lane) {
     return x;
 }
 
-// A group's rounds of homes: (key, first atom) of every 32 atoms.  The pair kernel's work goes by rounds, not by
+// A group's rounds of homes: key and first atom of every 32 atoms, begin and end of the group.  The pair kernel's work goes by rounds, not by
 // groups, because the groups of a frame of uneven density hold anything from no atom to all of them.  A ball of
 // 62,500 atoms in a box 7.5 times as wide has groups of up to 3,900; with a warp for all homes of a group, and items
 // for the empty ones too, 312 ms, with rounds 1.62; 20,000 atoms in one clump 343 and 1.33 ms.  Even frames gain as
 // well, from items of one round instead of one or two: 62,500 atoms 0.36 -> 0.33 ms, 1e6 2.59 -> 2.43.
-__device__ __forceinline__ void emit_rounds(int2* __restrict__ rounds, unsigned first, int key, int start, int v) {
-    for (int i = 0; i * kGroup < v; ++i) rounds[first + i] = make_int2(key, start + i * kGroup);
+__device__ __forceinline__ void emit_rounds(int4* __restrict__ rounds, unsigned first, int key, int start, int v) {
+    for (int i = 0; i * kGroup < v; ++i) rounds[first + i] = make_int4(key, start + i * kGroup, start, start + v);
 }
 
 // Start of every group in the sorted array, and its rounds.  Groups need only be contiguous, not in key order, so a
@@ -833,7 +842,7 @@ __device__ __forceinline__ void emit_rounds(int2* __restrict__ rounds, unsigned 
 // kernel in place of a scan over all keys.
 __global__ void __launch_bounds__(256) group_offsets_kernel(const int32_t* __restrict__ fcount, int nkey,
                                                             u64* __restrict__ total, int32_t* __restrict__ fstart,
-                                                            int2* __restrict__ rounds) {
+                                                            int4* __restrict__ rounds) {
     __shared__ u64 wsum[8], base;
     const int k = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int v = k < nkey ? fcount[k] : 0;
@@ -898,7 +907,7 @@ constexpr int kSmallKeys = 4096;  // most groups, and most cells, of a frame sor
 __global__ void __launch_bounds__(kSmallThreads) cell_sort_small_kernel(
     const float4* __restrict__ packed, int n, const __grid_constant__ RdfParams p, int ncell, int nkey, unsigned wscale,
     unsigned* __restrict__ work, int32_t* __restrict__ cflag, int32_t* __restrict__ fcount,
-    int32_t* __restrict__ fstart, int2* __restrict__ rounds, float4* __restrict__ sorted, const float* __restrict__ q,
+    int32_t* __restrict__ fstart, int4* __restrict__ rounds, float4* __restrict__ sorted, const float* __restrict__ q,
     float* __restrict__ sorted_q, double* __restrict__ q2) {
     __shared__ double red[32];
     __shared__ int cnt[kSmallKeys], flag[kSmallKeys];
@@ -1288,7 +1297,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
         u64 n_tested = 0;
         const bool frame_ok = frame_within(st.state[kWorkWords * r + kWorkFlags]);
         const unsigned nwork = st.state[kWorkWords * r + kWorkRounds] * (unsigned)p.nseg;
-        const int2* rounds = st.rounds + batch_rounds_begin(it);
+        const int4* rounds = st.rounds + batch_rounds_begin(it);
         const float4* sorted = st.sorted + it.atom_off;
         const int32_t *fstart = st.fstart + it.key_begin, *fcount = st.fcount + it.key_begin,
                       *cflag = st.cflag + it.key_begin;
@@ -1335,7 +1344,7 @@ struct trj_rdf_plan {
     // Zeroed per frame by one memset: work state (kWorkWords), cell flags (ncell: bit 0 a coordinate outside
     // [0, L), bit 1 outside [-L, L)), atoms per group (nkey).
     int32_t* zeroed = nullptr;  // kWorkWords + ncell_cap + key_cap
-    int2* rounds = nullptr;     // key_cap + n_max / 32: key and first atom of every round of homes
+    int4* rounds = nullptr;     // key_cap + n_max / 32: every round of homes (emit_rounds)
     int32_t* akey = nullptr;    // n_max: (cell, group) key per atom
     int32_t* aslot = nullptr;   // n_max
     RdfParams frame_last;       // geometry, cells and groups of the last accumulated frame
@@ -1562,7 +1571,7 @@ static bool pair_shape(const trj_ctx* ctx, int nsp, int nit, int row_words, bool
     return false;
 }
 
-typedef void (*PairKernel)(RdfParams, const float4*, const int32_t*, const int32_t*, const int32_t*, const int2*, unsigned*,
+typedef void (*PairKernel)(RdfParams, const float4*, const int32_t*, const int32_t*, const int32_t*, const int4*, unsigned*,
                            u64*, u64*, unsigned*, const float*, double*);
 template <bool FLOOR, bool SQUARE>
 static PairKernel pair_kernel_of(bool charged, bool edge) {
@@ -1617,14 +1626,14 @@ static int rdf_plan_create_impl(trj_ctx* ctx, int nsp, float deltar, float rcrdf
     p->key_cap = (int64_t)p->ncell_cap + n_max / 16 + 64;
     const size_t na = (size_t)std::max<int64_t>(n_max, 1);
     size_t bytes = 64 + sizeof(int32_t) * (size_t)(kWorkWords + p->ncell_cap + 2 * p->key_cap) +
-                   (sizeof(int32_t) * 2 + sizeof(float4)) * na + sizeof(int2) * ((size_t)p->key_cap + na / kGroup + 1);
+                   (sizeof(int32_t) * 2 + sizeof(float4)) * na + sizeof(int4) * ((size_t)p->key_cap + na / kGroup + 1);
     char* base = nullptr;
     if (trj_dev_alloc(ctx, (void**)&base, bytes + 256) != cudaSuccess) {
         delete p;
         return trj_fail(ctx, TRJ_ERR_NOMEM, "rdf plan: %zu bytes of scratch", bytes);
     }
     p->sorted = reinterpret_cast<float4*>(base);
-    p->rounds = reinterpret_cast<int2*>(p->sorted + na);
+    p->rounds = reinterpret_cast<int4*>(p->sorted + na);
     p->akey = reinterpret_cast<int32_t*>(p->rounds + (size_t)p->key_cap + na / kGroup + 1);
     p->aslot = p->akey + na;
     p->zeroed = reinterpret_cast<int32_t*>((reinterpret_cast<uintptr_t>(p->aslot + na) + 15) & ~(uintptr_t)15);
