@@ -668,7 +668,7 @@ __device__ __forceinline__ unsigned next_item(unsigned* next, const WarpState* w
 }
 
 // Work item = (round of homes, segment of their group's neighbour list), taken from a global counter by one warp at
-// a time; no warp waits for another.  Shared memory: bin rows (count), charge rows (QMODE, FP64 [row_words]),
+// a time; no warp waits for another until the rows are merged.  Shared memory: bin rows (count), charge rows (QMODE, FP64 [row_words]),
 // the warps' buffers.  SQUARE: a bin row per ordered species pair, so that a pair's row address is a sum of
 // two registers; otherwise the rows of ind_ij through a 16 x 16 table of addresses.
 //
@@ -678,9 +678,10 @@ __device__ __forceinline__ unsigned next_item(unsigned* next, const WarpState* w
 // together a quarter of the time.  With the culling's variables in registers across the tests 64 registers do
 // not hold both (100 bytes spilled in the inner loop, 97 instructions a block): 2.95 ms at 1e6 atoms, 0.437 ms
 // at 62,500 (cutoff 10, four cells per axis), 6.08 ms for the 4e6-atom slab, 1.83 ms for 256,000 ions; with
-// them in WarpState and two blocks per turn of the loop 2.64, 0.394, 5.50 and 1.63 ms.  (The ions' loop keeps
-// one block per turn: two take 1.97 ms.)  64-atom homes, two per lane, that a CTA walks over staged neighbour
-// cells with a branch per pair: 7.37, 1.69, 19.5 and 3.75 ms.
+// them in WarpState and two blocks per turn of the loop 2.64, 0.394, 5.50 and 1.63 ms, with rounds for items
+// 2.54, 0.370, 5.45 and 1.53 (layout and sort included).  (The ions' loop keeps one block per turn: two take
+// 1.97 ms.)  64-atom homes, two per lane, that a CTA walks over staged neighbour cells with a branch per pair:
+// 7.37, 1.69, 19.5 and 3.75 ms.
 template <bool FLOOR, bool QMODE, bool SQUARE, bool EDGE>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
     rdf_pairs_kernel(const __grid_constant__ RdfParams p, const float4* __restrict__ sorted,

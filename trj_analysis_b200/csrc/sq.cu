@@ -103,7 +103,7 @@ __device__ __forceinline__ void fill_turn_table(PlainSmem& sm, const float2* __r
 // scheduler in a loop of nothing else: 1.46e12 terms/s; all-scalar FP32 27 clocks, without the integer
 // multiply-adds of the phase 22.7).  One copy of the table had a lane's load conflict with three to six
 // others'.  62,500 atoms x 14,116 vectors: 846 -> 700 us; 1e6 atoms x 363 vectors: 538 -> 360 us;
-// 16,379 atoms with the reference's vectors, where eight slices left most SMs idle: 144 -> 43 us; 4,000 atoms,
+// 16,379 atoms with the reference's vectors, where eight slices left most SMs idle: 144 -> 39 us; 4,000 atoms,
 // one slice: 235 -> 12 us.
 template <int VPT>
 __device__ __forceinline__ void plain_block(const uint4* __restrict__ phase, const int64_t* __restrict__ sp_off,
