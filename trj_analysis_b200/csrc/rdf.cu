@@ -1263,7 +1263,6 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
     unsigned* hist = reinterpret_cast<unsigned*>(smem + (size_t)(kBatchThreads / 32) * kWarpBytes);
     const unsigned hist_base = trj_smem_addr(hist), rowtab_base = trj_smem_addr(rowtab);
     for (int k = tid; k < batch_hist_smem_words(hist_words); k += kBatchThreads) hist[k] = 0u;
-    if (lane == 0) ws->since = (unsigned)clock();
     const int nitems = hdr->nitems;
     if (nitems == 0) return;
     // CTAs start spread over the turn's work; each then moves on cyclically to frames with items left
@@ -1302,6 +1301,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
         const float4* sorted = st.sorted + it.atom_off;
         const int32_t *fstart = st.fstart + it.key_begin, *fcount = st.fcount + it.key_begin,
                       *cflag = st.cflag + it.key_begin;
+        if (lane == 0) ws->since = (unsigned)clock();  // here, so that the first item is always taken
         for (;;) {
             const unsigned item = next_item(&st.state[kWorkWords * r + kWorkNext], ws);
             if (item >= nwork) break;
@@ -1322,7 +1322,6 @@ __global__ void __launch_bounds__(kBatchThreads, 3) batch_pairs_kernel(const Bat
         // the words before and after a row's bins as well: the next frame's rows lie elsewhere
         const int rows = square ? p.g.nsp * p.g.nsp : p.nit;
         for (int q = tid; q < rows * p.g.row_words; q += kBatchThreads) hist[q] = 0u;
-        if (lane == 0) ws->since = (unsigned)clock();
         r = r + 1 < nitems ? r + 1 : 0;
     }
 }
