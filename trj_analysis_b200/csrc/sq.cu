@@ -95,7 +95,7 @@ __device__ __forceinline__ void fill_turn_table(PlainSmem& sm, const float2* __r
     }
 }
 
-// Sums of one block of vectors (bx) over one part (by = slice * parts + part) of species [sp0, sp1).  Species qsp
+// Sums of one block of vectors (bx) over one part (by = slice * parts + part) of every gridDim.z-th species.  Species qsp
 // (if any) is the charge species: each term is weighted by the charge in the entry's w.  Partials by position
 // in the subset: part[by][species][nsub].  The turn table must be filled; the first barrier orders it.
 //
@@ -107,7 +107,7 @@ __device__ __forceinline__ void fill_turn_table(PlainSmem& sm, const float2* __r
 // one slice: 235 -> 12 us.
 template <int VPT>
 __device__ __forceinline__ void plain_block(const uint4* __restrict__ phase, const int64_t* __restrict__ sp_off,
-                                            int nsp, int sp0, int sp1, int qsp, const int4* __restrict__ vecs,
+                                            int nsp, int qsp, const int4* __restrict__ vecs,
                                             const int32_t* __restrict__ subset, int nsub, const PlainShape& shape,
                                             double2* __restrict__ part, int64_t bx, int64_t by, PlainSmem& sm) {
     const int tid = threadIdx.x, tv = shape.tv, tg = shape.tg;
@@ -126,7 +126,7 @@ __device__ __forceinline__ void plain_block(const uint4* __restrict__ phase, con
         nz[q] = (unsigned)n.z;
     }
     const int64_t slice = by / shape.parts, cut = by - slice * shape.parts;
-    for (int a = sp0; a < sp1; ++a) {
+    for (int a = (int)blockIdx.z; a < nsp; a += (int)gridDim.z) {
         const int64_t a0 = sp_off[a], len = sp_off[a + 1] - a0;
         const int64_t s0 = a0 + len * slice / shape.nsplit, s1 = a0 + len * (slice + 1) / shape.nsplit;
         const int64_t runs = (s1 - s0 + kPlainSub - 1) / kPlainSub;
@@ -198,9 +198,7 @@ __global__ void __launch_bounds__(kPlainThreads, kPlainCtas) sq_plain_kernel(
     const float2* __restrict__ turn, double2* __restrict__ part) {
     __shared__ __align__(16) PlainSmem sm;
     fill_turn_table(sm, turn);
-    const int cut = (int)blockIdx.z;
-    plain_block<VPT>(phase, sp_off, nsp, nsp * cut / shape.cuts, nsp * (cut + 1) / shape.cuts, qsp, vecs, subset, nsub,
-                     shape, part, blockIdx.x, blockIdx.y, sm);
+    plain_block<VPT>(phase, sp_off, nsp, qsp, vecs, subset, nsub, shape, part, blockIdx.x, blockIdx.y, sm);
 }
 
 // Sums over `n` partials `stride` apart for 32 vectors at a time (consecutive vectors in a warp's lanes:
@@ -355,10 +353,10 @@ __global__ void __launch_bounds__(kPlainThreads, 2) batch_sq_kernel(BatchHeader*
         const PlainShape shape = {it.vpt, it.tv, it.tg, it.nvblk, it.nsplit, it.parts, 1};
         const int64_t t = u - it.sq_begin, bx = t % it.nvblk, by = t / it.nvblk;
         if (it.vpt == 2)
-            plain_block<2>(phase + it.atom_off, it.sp_off_dev, it.nsp, 0, it.nsp, -1, it.vecs, it.subset, it.nvec,
+            plain_block<2>(phase + it.atom_off, it.sp_off_dev, it.nsp, -1, it.vecs, it.subset, it.nvec,
                            shape, it.part, bx, by, sm);
         else
-            plain_block<4>(phase + it.atom_off, it.sp_off_dev, it.nsp, 0, it.nsp, -1, it.vecs, it.subset, it.nvec,
+            plain_block<4>(phase + it.atom_off, it.sp_off_dev, it.nsp, -1, it.vecs, it.subset, it.nvec,
                            shape, it.part, bx, by, sm);
     }
 }
